@@ -608,24 +608,25 @@ int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint3
 
 // ---- stand-alone hand-over kernel ----------------------------------------------------------------------------
 namespace {
-__global__ void __launch_bounds__(256) publish_vector_kernel(const __grid_constant__ Publish p, int* status) {
-    __shared__ double red[8];
+constexpr int PUB_WARPS = 16;      // with two blocks of 256 a warp, vectors of up to 8192 are read once
+__global__ void __launch_bounds__(PUB_WARPS * 32) publish_vector_kernel(const __grid_constant__ Publish p, int* status) {
+    __shared__ double red[PUB_WARPS];
     __shared__ int ok;
     pdl_launch_dependents();
     pdl_wait();
-    if (p.npeers) {
+    if (p.npeers) {    // batches are single-GPU: one CTA
         if (threadIdx.x == 0) ok = publish_peer_gate(p, status) ? 1 : 0;
         __syncthreads();
         if (!ok) return;
     }
-    if (p.dst.qs != nullptr || p.dst.xn != nullptr) publish_vector<8, 1>(p, red, true);
+    if (p.dst.qs != nullptr || p.dst.xn != nullptr) publish_vector<PUB_WARPS, 1>(p, red, blockIdx.x);
 }
 }  // namespace
 
 cudaError_t launch_publish_vector(const Publish& p, int* status, cudaStream_t stream, bool pdl) {
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(1);
-    lc.blockDim = dim3(256);
+    lc.gridDim = dim3(p.npeers ? 1 : p.batch);
+    lc.blockDim = dim3(PUB_WARPS * 32);
     lc.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

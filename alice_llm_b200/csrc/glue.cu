@@ -16,15 +16,14 @@ __global__ void __launch_bounds__(256) embed_q8_0_kernel(const __grid_constant__
     __shared__ double red[8];
     pdl_launch_dependents();   // the next kernel may become resident (and prefetch its weights) while this one waits
     pdl_wait();
-    const uint32_t pos0 = (uint32_t)*a.pos;
-    for (uint32_t i = threadIdx.x; i < 64 * a.batch; i += blockDim.x) rope_table_entry(a.rope_tab + (size_t)(i >> 6) * 128, i & 63, pos0 + (i >> 6), a.rope_freq);
+    const uint32_t k = blockIdx.x;   // a CTA per token of the batch
+    if (threadIdx.x < 64) rope_table_entry(a.rope_tab + (size_t)k * 128, threadIdx.x, (uint32_t)*a.pos + k, a.rope_freq);
     // one thread per 34-byte block (f16 scale + 32 int8): 17 independent 16-bit loads, so the row costs one memory
     // round trip instead of one per element
     const uint32_t nblk = a.cols / 32;
-    for (uint32_t i = threadIdx.x; i < nblk * a.batch; i += blockDim.x) {
-        const uint32_t k = i / nblk, b = i % nblk;
-        uint32_t t = (uint32_t)a.tokens[k];
-        if (t >= a.vocab) t = 0;
+    uint32_t t = (uint32_t)a.tokens[k];
+    if (t >= a.vocab) t = 0;
+    for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x) {
         const unsigned short* src = reinterpret_cast<const unsigned short*>(a.table + (size_t)t * nblk * 34 + (size_t)b * 34);
         unsigned short h[17];
 #pragma unroll
@@ -40,7 +39,7 @@ __global__ void __launch_bounds__(256) embed_q8_0_kernel(const __grid_constant__
     if (a.pub.mode == PUB_VECTOR && (a.pub.dst.qs != nullptr || a.pub.dst.xn != nullptr)) {
         __threadfence();
         __syncthreads();
-        publish_vector<8, 0>(a.pub, red, true);
+        publish_vector<8, 0>(a.pub, red, k);
     }
 }
 
@@ -65,7 +64,7 @@ static void launch_cfg(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, dim3 gri
 
 cudaError_t launch_embed_q8_0(const EmbedArgs& a, cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t lc; cudaLaunchAttribute at[1];
-    launch_cfg(lc, at, dim3(1), dim3(256), st, pdl);
+    launch_cfg(lc, at, dim3(a.batch), dim3(256), st, pdl);
     return cudaLaunchKernelEx(&lc, embed_q8_0_kernel, a);
 }
 

@@ -60,7 +60,9 @@ struct LlamaModel final : alice_model {
         for (uint32_t p = 0; p < npeers; p++) cudaIpcCloseMemHandle(peer_base[p]);
     }
     uint32_t max_tokens() const override { return MAX_BATCH; }
-    int enqueue_step(uint32_t batch, bool greedy_feed) override;
+    int enqueue_step(uint32_t batch, bool greedy_feed) override { return step(batch, greedy_feed, nullptr, 0); }
+    // Logits of rows[0 .. nrows) of the batch only, each at its own place in `logits`; rows == nullptr: of all of them.
+    int step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows);
     int enqueue_rows(uint32_t n, const uint32_t* rows, uint32_t nrows, float* host_logits) override;
     int clear_state() override;
 };
@@ -123,7 +125,7 @@ void fill_dst(PublishDst& d, const Need& nd, uint8_t* q8_base, float* xn, uint32
 // rows into every peer's copy, with one flag per vector that a one-CTA kernel behind it raises on the peers and waits for
 // here before it prepares the vector for the next op. Attention runs on the rank's own KV heads (its q, k, v rows), so
 // only its output needs exchanging (it is the input of the output projection).
-int LlamaModel::enqueue_step(uint32_t batch, bool greedy_feed) {
+int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows) {
     LlamaModel* const m = this;
     const alice_model_config& c = m->cfg;
     cudaStream_t st = m->e->stream;
@@ -318,11 +320,21 @@ int LlamaModel::enqueue_step(uint32_t batch, bool greedy_feed) {
             if ((rc = gather_then_publish(m->hidden, m->lH, p))) return rc;
         }
     }
-    {   // output head on the prepared (normalised) hidden (src/llama3.rs:14590-14604)
-        GemvOp op; Q8KView view; Publish p;
+    // output head on the prepared (normalised) hidden (src/llama3.rs:14590-14604), a launch per run of consecutive rows: a prompt
+    // wants its last row only
+    const uint32_t runs_of = rows ? nrows : 1;
+    for (uint32_t i = 0; i < runs_of;) {
+        const uint32_t lo = rows ? rows[i] : 0;
+        uint32_t len = rows ? 1 : batch;
+        while (rows && i + len < nrows && rows[i + len] == lo + len) len++;
+        GemvOp op; Publish p;
         op.w[0] = &m->out;
-        if ((rc = hidden_input(op, m->out, m->out_norm, false, true))) return rc;
-        op.y = m->logits; op.y_off[0] = r * m->lV; op.y_stride = V;
+        if ((rc = hidden_input(op, m->out, m->out_norm, false, i == 0))) return rc;
+        Q8KView at;
+        op.batch = len;
+        if (op.q8) { at = *op.q8; at.qs += (size_t)lo * H; at.d += (size_t)lo * at.nb; at.bsums += (size_t)lo * at.nb * 16; op.q8 = &at; }
+        if (op.x) op.x += (size_t)lo * H;
+        op.y = m->logits + (size_t)lo * V; op.y_off[0] = r * m->lV; op.y_stride = V;
         if (batch == 1) op.argmax_key = m->argmax_key;   // greedy sampling: the head kernel leaves the packed maximum of its rows
         if (peer) {
             Need none;
@@ -337,6 +349,7 @@ int LlamaModel::enqueue_step(uint32_t batch, bool greedy_feed) {
             if ((rc = tp_all_gather(m->e, m->logits, (size_t)m->lV * sizeof(float)))) return rc;
             if ((rc = tp_all_gather(m->e, m->argmax_keys, sizeof(unsigned long long)))) return rc;
         }
+        i += rows ? len : 1;
     }
     MCU(launch_finish_step(m->argmax_keys, m->tp_n, m->d_token, m->d_pos, m->d_trace, greedy_feed ? 1 : 0, batch,
                            peer ? m->epoch : nullptr,   // the epoch counts steps whose rows were pushed (it is what the per-vector flags are compared with)
@@ -344,9 +357,9 @@ int LlamaModel::enqueue_step(uint32_t batch, bool greedy_feed) {
     return ALICE_OK;
 }
 
-// Every row of the batch has its logits (the head runs over the whole batch): the wanted ones are copied out.
+// A single token always has its logits (and its argmax) left on the device.
 int LlamaModel::enqueue_rows(uint32_t n, const uint32_t* rows, uint32_t nrows, float* host_logits) {
-    const int rc = enqueue_step(n, false);
+    const int rc = n == 1 ? step(1, false, nullptr, 0) : step(n, false, rows ? rows : &n, nrows);
     if (rc) return rc;
     for (uint32_t i = 0; i < nrows; i++)
         MCU(cudaMemcpyAsync(host_logits + (size_t)i * cfg.vocab_size, logits + (size_t)rows[i] * cfg.vocab_size, (size_t)cfg.vocab_size * 4,

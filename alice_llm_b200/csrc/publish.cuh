@@ -91,16 +91,15 @@ __device__ __forceinline__ Q8KLaneInput pub_scale(const Q8KLaneInput& v, float s
 }
 
 // One prepared 256-element block leaves the warp: Q8_K fields and / or f32.
-__device__ __forceinline__ void pub_emit_block(const PublishDst& dst, const Q8KLaneInput& v, uint32_t lane, uint32_t vec, uint32_t blk, uint32_t n,
-                                               bool store = true) {
+__device__ __forceinline__ void pub_emit_block(const PublishDst& dst, const Q8KLaneInput& v, uint32_t lane, uint32_t vec, uint32_t blk, uint32_t n) {
     const uint32_t nb = n / QK_K;
     const size_t bi = (size_t)vec * nb + blk;
-    if (dst.qs != nullptr) q8k_quantize_block_warp(v, lane, dst.qs + bi * QK_K, dst.d + bi, dst.bsums + bi * 16, nullptr, store);
+    if (dst.qs != nullptr) q8k_quantize_block_warp(v, lane, dst.qs + bi * QK_K, dst.d + bi, dst.bsums + bi * 16);
     if (dst.xn != nullptr) {
         float* out = dst.xn + (size_t)vec * n + (size_t)blk * QK_K;
         if (dst.roundtrip) {
-            q8k_quantize_block_warp<true>(v, lane, nullptr, nullptr, nullptr, out, store);
-        } else if (store) {
+            q8k_quantize_block_warp<true>(v, lane, nullptr, nullptr, nullptr, out);
+        } else {
             const uint32_t i0 = blk * QK_K + lane * 8;
             if (i0 + 8 <= n) {
                 reinterpret_cast<float4*>(out + lane * 8)[0] = v.a;
@@ -118,63 +117,57 @@ __device__ __forceinline__ void pub_emit_block(const PublishDst& dst, const Q8KL
 // blocks per warp stay in registers between the sum of squares and the second pass (one trip to L2 for vectors of up to
 // NW * PUB_REG_BLOCKS * 256 elements), longer vectors are read twice. `red` = NW doubles of shared memory.
 //
-// Only ONE CTA of a launch runs this, once: its instructions are then in nobody's instruction cache, and a cold walk
-// through a few hundred instructions costs on the order of 10 us (measured 14 us) - far more than the arithmetic.
-// So every CTA of the launch first calls it with store == false while it waits for the previous kernel anyway: same
-// instructions, results discarded, and the real call finds them in the SM's cache.
+// One CTA prepares vector k: a batch is a grid of as many CTAs. (One CTA walking through all of them took 24.4 us for eight
+// vectors of 4096, one CTA each 6 us.)
 constexpr int PUB_REG_BLOCKS = 2;
 template <int NW, int BAR>
-static __device__ __noinline__ void publish_vector(const Publish& p, double* red, bool store) {
+static __device__ __noinline__ void publish_vector(const Publish& p, double* red, uint32_t k) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = p.n, nblk = (n + QK_K - 1) / QK_K;
     const bool in_regs = nblk <= (uint32_t)(NW * PUB_REG_BLOCKS);
-    const uint32_t nvec = store ? p.batch : 1u;
-    for (uint32_t k = 0; k < nvec; k++) {
-        const float* x = p.src + (size_t)k * n;
-        Q8KLaneInput xv[PUB_REG_BLOCKS], wv[PUB_REG_BLOCKS];
-        float scale = 1.0f;
-        if (in_regs) {
+    const float* x = p.src + (size_t)k * n;
+    Q8KLaneInput xv[PUB_REG_BLOCKS], wv[PUB_REG_BLOCKS];
+    float scale = 1.0f;
+    if (in_regs) {
 #pragma unroll
-            for (int i = 0; i < PUB_REG_BLOCKS; i++) {
-                const uint32_t b = warp + (uint32_t)i * NW;
-                if (b < nblk) {
-                    xv[i] = pub_load8(x, b * QK_K + lane * 8, n);
-                    if (p.norm_w != nullptr) wv[i] = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
-                }
+        for (int i = 0; i < PUB_REG_BLOCKS; i++) {
+            const uint32_t b = warp + (uint32_t)i * NW;
+            if (b < nblk) {
+                xv[i] = pub_load8(x, b * QK_K + lane * 8, n);
+                if (p.norm_w != nullptr) wv[i] = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
             }
         }
-        if (p.norm_w != nullptr) {
-            double ss = 0.0;
-            if (in_regs) {
-#pragma unroll
-                for (int i = 0; i < PUB_REG_BLOCKS; i++)
-                    if (warp + (uint32_t)i * NW < nblk) ss += pub_sumsq(xv[i]);
-            } else {
-                for (uint32_t b = warp; b < nblk; b += NW) ss += pub_sumsq(pub_load8(x, b * QK_K + lane * 8, n));
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");   // `red` free (previous vector read it)
-            if (lane == 0) red[warp] = ss;
-            asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");
-            double tot = 0.0;
-#pragma unroll
-            for (int w = 0; w < NW; w++) tot += red[w];
-            const float mean = (float)(tot / (double)n);
-            scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
-        }
+    }
+    if (p.norm_w != nullptr) {
+        double ss = 0.0;
         if (in_regs) {
 #pragma unroll
-            for (int i = 0; i < PUB_REG_BLOCKS; i++) {
-                const uint32_t b = warp + (uint32_t)i * NW;
-                if (b < nblk) pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv[i], scale, wv[i]) : xv[i], lane, k, b, n, store);
-            }
+            for (int i = 0; i < PUB_REG_BLOCKS; i++)
+                if (warp + (uint32_t)i * NW < nblk) ss += pub_sumsq(xv[i]);
         } else {
-            for (uint32_t b = warp; b < nblk; b += NW) {
-                const Q8KLaneInput v = pub_load8(x, b * QK_K + lane * 8, n);
-                if (p.norm_w != nullptr) pub_emit_block(p.dst, pub_scale(v, scale, pub_load8_w(p.norm_w, b * QK_K + lane * 8, n)), lane, k, b, n, store);
-                else pub_emit_block(p.dst, v, lane, k, b, n, store);
-            }
+            for (uint32_t b = warp; b < nblk; b += NW) ss += pub_sumsq(pub_load8(x, b * QK_K + lane * 8, n));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) red[warp] = ss;
+        asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");
+        double tot = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) tot += red[w];
+        const float mean = (float)(tot / (double)n);
+        scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
+    }
+    if (in_regs) {
+#pragma unroll
+        for (int i = 0; i < PUB_REG_BLOCKS; i++) {
+            const uint32_t b = warp + (uint32_t)i * NW;
+            if (b < nblk) pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv[i], scale, wv[i]) : xv[i], lane, k, b, n);
+        }
+    } else {
+        for (uint32_t b = warp; b < nblk; b += NW) {
+            const Q8KLaneInput v = pub_load8(x, b * QK_K + lane * 8, n);
+            if (p.norm_w != nullptr) pub_emit_block(p.dst, pub_scale(v, scale, pub_load8_w(p.norm_w, b * QK_K + lane * 8, n)), lane, k, b, n);
+            else pub_emit_block(p.dst, v, lane, k, b, n);
         }
     }
 }
