@@ -10,6 +10,7 @@
 #include "gemv_kq_mma.cuh"
 #include "gemv_launch.cuh"
 #include "gemv_plan.cuh"
+#include "gemv_planes.cuh"
 
 namespace alice {
 
@@ -559,31 +560,53 @@ static int launch_dense_rows(const GemvOp& op, const LaunchCfg& cfg) {
     return ALICE_OK;
 }
 
+// Vectors [k, k + n) of a batch.
+static GemvOp sub_batch(const GemvOp& op, uint32_t k, uint32_t n, Q8KView& v) {
+    GemvOp o = op;
+    o.batch = n;
+    uint32_t total_rows = 0;
+    for (uint32_t i = 0; i < op.nw && i < 3; i++) if (op.w[i]) total_rows += op.w[i]->rows;
+    const uint32_t cols = op.w[0]->cols, nb = cols / QK_K;
+    const size_t ys = op.y_stride ? op.y_stride : total_rows;
+    o.y_stride = (uint32_t)ys;
+    if (op.q8) { v = *op.q8; v.qs += (size_t)k * cols; v.d += (size_t)k * nb; v.bsums += (size_t)k * nb * 16; o.q8 = &v; }
+    if (op.x) o.x = op.x + (size_t)k * cols;
+    o.y = op.y + k * ys;
+    if (op.resid) o.resid = op.resid + k * ys;
+    for (uint32_t p = 0; p < op.npeers && p < MAX_PEERS; p++) o.peer_y[p] = op.peer_y[p] + k * ys;
+    return o;
+}
+
+static int launch_planes_split(const GemvOp& op, const LaunchCfg& cfg) {
+    if (!op.w[0] || (op.w[0]->fmt != WF_TERNARY && op.w[0]->fmt != WF_SPARSE_TERNARY)) return ALICE_E_SHAPE;
+    for (uint32_t n = op.batch; n; n /= 2) {
+        Q8KView v;
+        int rc = launch_planes(sub_batch(op, 0, n, v), cfg, false);
+        if (rc == ALICE_E_SHAPE) continue;
+        for (uint32_t k = n; k < op.batch && !rc; k += n) rc = launch_planes(sub_batch(op, k, std::min(n, op.batch - k), v), cfg, false);
+        return rc;
+    }
+    return ALICE_E_SHAPE;
+}
+
 int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
     if (op.batch == 0 || op.batch > (uint32_t)MAX_BATCH) return ALICE_E_SHAPE;
     if (op.w[0] && op.w[0]->fmt == WF_BF16) return launch_dense_rows(op, cfg);
+    if (op.batch > 1 && op.argmax_key) return ALICE_E_INVALID;
+    {   // ternary planes and codes: the whole batch in one pass; halves of it where the digits of all vectors fit no cluster
+        const int prc = launch_planes_split(op, cfg);
+        if (prc != ALICE_E_SHAPE) return prc;
+    }
     if (op.batch == 1) return launch_single(op, cfg);
-    if (op.argmax_key) return ALICE_E_INVALID;
     {   // K-quants with prepared Q8_K input: the int8 tensor-core kernel serves the whole batch in one pass over the weights
         const int brc = launch_kq_batch(op, cfg, false, nullptr);
         if (brc != ALICE_E_SHAPE) return brc;
     }
     // Formats without a batch kernel: one launch per input vector (the weights stream once per vector).
     if (!op.w[0]) return ALICE_E_INVALID;
-    uint32_t total_rows = 0;
-    for (uint32_t i = 0; i < op.nw && i < 3; i++) if (op.w[i]) total_rows += op.w[i]->rows;
-    const uint32_t ys = op.y_stride ? op.y_stride : total_rows;
-    const uint32_t cols = op.w[0]->cols, nb = cols / QK_K;
     for (uint32_t k = 0; k < op.batch; k++) {
-        GemvOp o = op;
-        o.batch = 1;
         Q8KView v;
-        if (op.q8) { v = *op.q8; v.qs += (size_t)k * cols; v.d += (size_t)k * nb; v.bsums += (size_t)k * nb * 16; o.q8 = &v; }
-        if (op.x) o.x = op.x + (size_t)k * cols;
-        o.y = op.y + (size_t)k * ys;
-        if (op.resid) o.resid = op.resid + (size_t)k * ys;
-        for (uint32_t p = 0; p < op.npeers && p < MAX_PEERS; p++) o.peer_y[p] = op.peer_y[p] + (size_t)k * ys;
-        const int rc = launch_single(o, cfg);
+        const int rc = launch_single(sub_batch(op, k, 1, v), cfg);
         if (rc) return rc;
     }
     return ALICE_OK;
@@ -598,6 +621,7 @@ size_t mma_prep_bytes(uint32_t cols) {
 int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint32_t* weight_passes) {
     uint32_t n = 0;
     if (op.batch > 1 && launch_kq_batch(op, cfg, true, &n) == ALICE_OK) { *launches = n; *weight_passes = 1; return ALICE_OK; }
+    if (launch_planes(op, cfg, true) == ALICE_OK) { *launches = *weight_passes = 1; return ALICE_OK; }
     GemvOp one = op; one.batch = 1;
     StreamPlan pl;
     const int rc = plan_stream_gemv(one, cfg, pl);

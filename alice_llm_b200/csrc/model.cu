@@ -10,6 +10,7 @@
 
 #include "abi_internal.cuh"
 #include "attn_body.cuh"
+#include "gemv_planes.cuh"
 #include "glue.cuh"
 #include "model_base.cuh"
 #include "tp.cuh"
@@ -466,7 +467,8 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     if (!rc) rc = dev_alloc(m, &m->ffn_q8, Q8KLayout::make((c.intermediate_dim + 255) / 256, B).total);
     if (!rc) rc = dev_alloc(m, &m->hid_xn, (size_t)B * c.hidden_dim);
     if (!rc) {
-        m->prep_bytes = mma_prep_bytes(std::max({c.hidden_dim, c.intermediate_dim, q_dim}));
+        const uint32_t widest = std::max({c.hidden_dim, c.intermediate_dim, q_dim});
+        m->prep_bytes = std::max(mma_prep_bytes(widest), plane_prep_bytes(widest, B));
         rc = dev_alloc(m, &m->prep, m->prep_bytes);
     }
     if (!rc) rc = dev_alloc(m, &m->d_pos, 1);
