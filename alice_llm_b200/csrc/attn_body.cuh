@@ -1,7 +1,5 @@
-// Device body of the fused decode attention: RoPE + KV append + split-KV GQA attention + split combine, for one
-// token or a batch of consecutive tokens (causal). Arithmetic: ALICE-LLM src/llama3.rs apply_rope :5323-5333,
-// :5367-5378, KvCache::append :4773, gqa_attention :5431-5690, evaluated as an online softmax over KV splits; the
-// batch form is the causal rule of src/shaders/attention.wgsl:45 (token k at position base + k attends base + k + 1 rows).
+// Device body of the fused decode attention: RoPE + KV append + split-KV GQA attention + split combine, for one token. Arithmetic: ALICE-LLM src/llama3.rs apply_rope :5323-5333,
+// :5367-5378, KvCache::append :4773, gqa_attention :5431-5690, evaluated as an online softmax over KV splits.
 #pragma once
 #include "common.cuh"
 #include "glue.cuh"
@@ -60,13 +58,11 @@ __device__ __forceinline__ float4 rope4(float4 v, uint32_t lane, const RopeCoef&
 }
 
 // GQA decode attention with RoPE, KV append and the split combine fused in.
-// One CTA = one KV head x one slice of positions x one token of the batch; its GROUP = num_heads/num_kv_heads query
+// One CTA = one KV head x one slice of positions; its GROUP = num_heads/num_kv_heads query
 // heads share every K and V row it reads. Each warp walks positions t, t+NW, ...; a lane owns 4 of the 128 dims.
-// qkv[k] = [q | k | v] of batch token k, un-rotated: q and k are rotated here. Rows of the tokens of this very batch
-// (positions >= pos0) are taken from qkv, not from the cache - their cache rows are being written by this launch -
-// and token k's own row is written to the cache at pos0 + k by the CTA whose slice contains it.
-// Per (token, split, head) the CTA leaves (max, sum, accumulator); the last CTA of a (token, KV head) to finish
-// (ticket counter) folds the splits into attn_out for its heads.
+// qkv = [q | k | v], un-rotated: q and k are rotated here. The token's own row (position pos) is taken from qkv and
+// written to the cache by the CTA whose slice contains it.
+// Per (split, head) the CTA leaves (max, sum, accumulator); the last CTA of a KV head to finish (ticket counter) folds the splits into attn_out for its heads.
 template <int GROUP>
 struct AttnSmem {
     float m[8][GROUP], l[8][GROUP];
@@ -77,19 +73,17 @@ struct AttnSmem {
 };
 
 template <int GROUP>
-__device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0, uint32_t kvh, uint32_t split, uint32_t bk,
+__device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos, uint32_t kvh, uint32_t split,
                                                 AttnSmem<GROUP>* sh) {
     constexpr int NW = 8;
     const AttnShape s = a.shape;
-    const uint32_t pos = pos0 + bk;            // position of this CTA's token
     const uint32_t seq = pos + 1;
     const uint32_t nsplit = a.nsplit;
     const uint32_t per = (seq + nsplit - 1) / nsplit;
     const uint32_t t0 = split * per, t1 = min(seq, t0 + per);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t q_dim = s.num_heads * s.head_dim, kv_dim = s.num_kv_heads * s.head_dim;
-    const uint32_t qkv_stride = q_dim + 2 * kv_dim;
-    const float* __restrict__ qkv = a.qkv + (size_t)bk * qkv_stride;
+    const float* __restrict__ qkv = a.qkv;
     float* __restrict__ kcache = a.kcache;
     float* __restrict__ vcache = a.vcache;
     const float inv_sqrt_d = __fdiv_rn(1.0f, sqrtf((float)s.head_dim));
@@ -105,7 +99,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
         for (int j = 0; j < KB; j++) {
             const uint32_t t = tb + j * NW;
             k[j] = v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t < t1 && t < pos0) {
+            if (t < t1 && t < pos) {
                 k[j] = __ldcg(reinterpret_cast<const float4*>(kcache + (size_t)t * kv_dim + kvh * s.head_dim) + lane);
                 v[j] = __ldcg(reinterpret_cast<const float4*>(vcache + (size_t)t * kv_dim + kvh * s.head_dim) + lane);
             }
@@ -115,7 +109,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
 #pragma unroll
     for (int g = 0; g < GROUP; g++) q[g] = __ldcg(reinterpret_cast<const float4*>(qkv + (size_t)(kvh * GROUP + g) * s.head_dim) + lane);
     if (t0 + warp < t1) load_round(t0 + warp);
-    const RopeCoef rc = rope_coef(a.rope_tab + (size_t)bk * 128, lane, neox);
+    const RopeCoef rc = rope_coef(a.rope_tab, lane, neox);
 #pragma unroll
     for (int g = 0; g < GROUP; g++) q[g] = rope4(q[g], lane, rc, neox);
     float m[GROUP], l[GROUP];
@@ -129,16 +123,11 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
         for (int j = 0; j < KB; j++) {
             const uint32_t t = tb + j * NW;
             if (t < t1) {
-                if (t >= pos0) {   // a token of this batch: rotate its K here; the token's own CTA appends K and V (KvCache::append, src/llama3.rs:4773)
-                    const uint32_t bj = t - pos0;
-                    const float* __restrict__ src = a.qkv + (size_t)bj * qkv_stride;
-                    const RopeCoef rj = bj == bk ? rc : rope_coef(a.rope_tab + (size_t)bj * 128, lane, neox);
-                    k[j] = rope4(__ldcg(reinterpret_cast<const float4*>(src + q_dim + (size_t)kvh * s.head_dim) + lane), lane, rj, neox);
-                    v[j] = __ldcg(reinterpret_cast<const float4*>(src + q_dim + kv_dim + (size_t)kvh * s.head_dim) + lane);
-                    if (bj == bk) {
-                        reinterpret_cast<float4*>(kcache + (size_t)t * kv_dim + kvh * s.head_dim)[lane] = k[j];
-                        reinterpret_cast<float4*>(vcache + (size_t)t * kv_dim + kvh * s.head_dim)[lane] = v[j];
-                    }
+                if (t == pos) {   // the token itself: rotate its K, append K and V (KvCache::append, src/llama3.rs:4773)
+                    k[j] = rope4(__ldcg(reinterpret_cast<const float4*>(qkv + q_dim + (size_t)kvh * s.head_dim) + lane), lane, rc, neox);
+                    v[j] = __ldcg(reinterpret_cast<const float4*>(qkv + q_dim + kv_dim + (size_t)kvh * s.head_dim) + lane);
+                    reinterpret_cast<float4*>(kcache + (size_t)t * kv_dim + kvh * s.head_dim)[lane] = k[j];
+                    reinterpret_cast<float4*>(vcache + (size_t)t * kv_dim + kvh * s.head_dim)[lane] = v[j];
                 }
                 float sc[GROUP];
 #pragma unroll
@@ -168,7 +157,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
     }
     __syncthreads();
     const uint32_t stride = s.head_dim + 4;   // (m, l, pad, pad, acc[128]): keeps acc 16-byte aligned
-    float* __restrict__ part = a.part + (size_t)bk * nsplit * s.num_heads * stride;
+    float* __restrict__ part = a.part;
     if (warp < GROUP) {
         const int g = warp;
         float M = -INFINITY;
@@ -189,10 +178,10 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
         if (lane == 0) { out[0] = M; out[1] = L; }
         reinterpret_cast<float4*>(out + 4)[lane] = A;
     }
-    // last CTA of this (token, KV head) folds the splits
+    // last CTA of this KV head folds the splits
     __threadfence();
     __syncthreads();
-    unsigned int* ticket_p = a.tickets + bk * s.num_kv_heads + kvh;
+    unsigned int* ticket_p = a.tickets + kvh;
     if (threadIdx.x == 0) {
         const unsigned int ticket = atomicAdd(ticket_p, 1u);
         sh->last = (ticket == nsplit - 1) ? 1u : 0u;
@@ -201,7 +190,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
     __syncthreads();
     if (!sh->last) return;
     __threadfence();
-    float* __restrict__ attn_out = a.attn_out + (size_t)bk * a.out_stride;
+    float* __restrict__ attn_out = a.attn_out;
     float4 o_keep = make_float4(0.f, 0.f, 0.f, 0.f);   // this warp's head, this lane's 4 dims
     if (warp < GROUP) {
         // one warp per head; lane <-> split for the (max, sum) pairs, so all loads are in flight at once
@@ -244,7 +233,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
         const float4 o = make_float4(A.x * inv, A.y * inv, A.z * inv, A.w * inv);
         reinterpret_cast<float4*>(attn_out + (size_t)head * s.head_dim)[lane] = o;
         for (uint32_t p = 0; p < a.npeers; p++)
-            reinterpret_cast<float4*>(a.peer_out[p] + (size_t)bk * a.out_stride + (size_t)head * s.head_dim)[lane] = o;
+            reinterpret_cast<float4*>(a.peer_out[p] + (size_t)head * s.head_dim)[lane] = o;
         o_keep = o;
     }
     if (a.q8.qs != nullptr && (GROUP % 2) == 0) {
@@ -254,8 +243,7 @@ __device__ __forceinline__ void attn_fused_body(const AttnArgs& a, uint32_t pos0
         if (warp < GROUP) sh->acc[0][warp][lane] = o_keep;
         __syncthreads();
         if (warp < GROUP / 2) {
-            const uint32_t nb = q_dim / QK_K;
-            const size_t blk = (size_t)bk * nb + (kvh * GROUP) / 2 + warp;
+            const size_t blk = (kvh * GROUP) / 2 + warp;
             const int hsel = 2 * (int)warp + (int)(lane >> 4);
             Q8KLaneInput in;
             in.a = sh->acc[0][hsel][(lane & 15) * 2];

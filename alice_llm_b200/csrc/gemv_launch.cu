@@ -8,6 +8,7 @@
 #include "formats.cuh"
 #include "gemv_mma.cuh"
 #include "gemv_kq_mma.cuh"
+#include "gemm_kq.cuh"
 #include "gemv_launch.cuh"
 #include "gemv_plan.cuh"
 #include "gemv_planes.cuh"
@@ -577,24 +578,37 @@ static GemvOp sub_batch(const GemvOp& op, uint32_t k, uint32_t n, Q8KView& v) {
     return o;
 }
 
-static int launch_planes_split(const GemvOp& op, const LaunchCfg& cfg) {
-    if (!op.w[0] || (op.w[0]->fmt != WF_TERNARY && op.w[0]->fmt != WF_SPARSE_TERNARY)) return ALICE_E_SHAPE;
+// A kernel that takes the whole batch in one pass, or halves of it where the digits of all vectors fit no cluster.
+static int launch_split(int (*launch)(const GemvOp&, const LaunchCfg&, bool), const GemvOp& op, const LaunchCfg& cfg) {
     for (uint32_t n = op.batch; n; n /= 2) {
         Q8KView v;
-        int rc = launch_planes(sub_batch(op, 0, n, v), cfg, false);
+        int rc = launch(sub_batch(op, 0, n, v), cfg, false);
         if (rc == ALICE_E_SHAPE) continue;
-        for (uint32_t k = n; k < op.batch && !rc; k += n) rc = launch_planes(sub_batch(op, k, std::min(n, op.batch - k), v), cfg, false);
+        for (uint32_t k = n; k < op.batch && !rc; k += n) rc = launch(sub_batch(op, k, std::min(n, op.batch - k), v), cfg, false);
         return rc;
     }
     return ALICE_E_SHAPE;
 }
 
 int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
-    if (op.batch == 0 || op.batch > (uint32_t)MAX_BATCH) return ALICE_E_SHAPE;
+    if (op.batch == 0) return ALICE_E_SHAPE;
     if (op.w[0] && op.w[0]->fmt == WF_BF16) return launch_dense_rows(op, cfg);
+    if (!op.w[0]) return ALICE_E_INVALID;
+    if (op.batch > (uint32_t)MAX_BATCH) {
+        // the tokens of a prompt: K-quants in tiles of tokens (for up to eight the streaming kernel below is faster: 74 against 90 us
+        // for the feed-forward block of an 8B model and four tokens), everything else eight at a time
+        const int grc = launch_kq_gemm(op, cfg, false);
+        if (grc != ALICE_E_SHAPE) return grc;
+        for (uint32_t k = 0; k < op.batch; k += MAX_BATCH) {
+            Q8KView v;
+            const int rc = launch_stream_gemv_op(sub_batch(op, k, std::min<uint32_t>(MAX_BATCH, op.batch - k), v), cfg);
+            if (rc) return rc;
+        }
+        return ALICE_OK;
+    }
     if (op.batch > 1 && op.argmax_key) return ALICE_E_INVALID;
-    {   // ternary planes and codes: the whole batch in one pass; halves of it where the digits of all vectors fit no cluster
-        const int prc = launch_planes_split(op, cfg);
+    if (op.w[0]->fmt == WF_TERNARY || op.w[0]->fmt == WF_SPARSE_TERNARY) {
+        const int prc = launch_split(launch_planes, op, cfg);
         if (prc != ALICE_E_SHAPE) return prc;
     }
     if (op.batch == 1) return launch_single(op, cfg);
@@ -603,7 +617,6 @@ int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
         if (brc != ALICE_E_SHAPE) return brc;
     }
     // Formats without a batch kernel: one launch per input vector (the weights stream once per vector).
-    if (!op.w[0]) return ALICE_E_INVALID;
     for (uint32_t k = 0; k < op.batch; k++) {
         Q8KView v;
         const int rc = launch_single(sub_batch(op, k, 1, v), cfg);

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(256, GROUP <= 5 ? 2 : 1) attn_fused_kernel(con
     __shared__ AttnSmem<GROUP> sh;
     pdl_launch_dependents();   // the next kernel may become resident (and prefetch its weights) while this one waits
     pdl_wait();
-    attn_fused_body<GROUP>(a, (uint32_t)*a.pos, blockIdx.x, blockIdx.y, blockIdx.z, &sh);
+    attn_fused_body<GROUP>(a, (uint32_t)*a.pos, blockIdx.x, blockIdx.y, &sh);
 }
 
 static void launch_cfg(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, dim3 grid, dim3 block, cudaStream_t st, bool pdl) {
@@ -68,12 +68,12 @@ cudaError_t launch_embed_q8_0(const EmbedArgs& a, cudaStream_t st, bool pdl) {
     return cudaLaunchKernelEx(&lc, embed_q8_0_kernel, a);
 }
 
-cudaError_t launch_attention(const AttnArgs& a, uint32_t batch, cudaStream_t st, bool pdl) {
+cudaError_t launch_attention(const AttnArgs& a, cudaStream_t st, bool pdl) {
     const AttnShape& s = a.shape;
     if (s.head_dim != 128 || s.num_heads % s.num_kv_heads) return cudaErrorInvalidValue;
     const uint32_t group = s.num_heads / s.num_kv_heads;
     cudaLaunchConfig_t lc; cudaLaunchAttribute at[1];
-    launch_cfg(lc, at, dim3(s.num_kv_heads, a.nsplit, batch), dim3(256), st, pdl);
+    launch_cfg(lc, at, dim3(s.num_kv_heads, a.nsplit), dim3(256), st, pdl);
     switch (group) {
         case 1: return cudaLaunchKernelEx(&lc, attn_fused_kernel<1>, a);
         case 2: return cudaLaunchKernelEx(&lc, attn_fused_kernel<2>, a);

@@ -53,7 +53,10 @@ struct EmbedArgs {
 // hidden[k] <- dequantized row tokens[k] of the Q8_0 table; rope_tab[k] <- (sin, cos) of (pos + k) * freq[j]; then the
 // prepared form of hidden for the first projection. One CTA.
 cudaError_t launch_embed_q8_0(const EmbedArgs& a, cudaStream_t st, bool pdl);
-cudaError_t launch_attention(const AttnArgs& a, uint32_t batch, cudaStream_t st, bool pdl);
+cudaError_t launch_attention(const AttnArgs& a, cudaStream_t st, bool pdl);      // one token
+// `batch` consecutive tokens from position pos0 (the host's copy of *a.pos, which only sizes the split): rotates the queries
+// inside qkv, appends to the cache, attends (csrc/attn_tokens.cu). a.part holds part_vectors * (head_dim + 4) floats. Single GPU.
+cudaError_t launch_attention_tokens(const AttnArgs& a, float* qkv, uint32_t batch, uint32_t pos0, uint32_t part_vectors, int num_sms, cudaStream_t st, bool pdl);
 // token <- index held in the largest of keys[0 .. nkeys) (packed maxima written by the output-head kernels, one per
 // tensor-parallel rank) when write_token; pos <- pos + advance; keys <- 0; *epoch += 1 (decode steps completed: the
 // tensor-parallel hand-over counters are compared against it)

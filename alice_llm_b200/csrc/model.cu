@@ -29,10 +29,14 @@ struct LlamaModel final : alice_model {
     std::vector<Layer> layers;
     WeightDesc emb{}, out{};
     float* out_norm = nullptr;
-    // activations, each for up to MAX_BATCH tokens: [k][dim]
+    // Tokens a piece of a prompt may have (tensor parallel: MAX_BATCH). The products of a K-quant piece are bound by arithmetic from
+    // 64 tokens on; a larger piece than 256 would only save launches.
+    uint32_t cap = MAX_BATCH;
+    // activations, each for up to `cap` tokens: [k][dim]; logits for MAX_BATCH
     float *hidden = nullptr, *qkv = nullptr, *attn_out = nullptr, *ffn_h = nullptr;   // and the base's logits
     float *kcache = nullptr, *vcache = nullptr;  // [layer][max_seq][kv_dim]
     float* attn_part = nullptr;
+    uint32_t part_vectors = 0;   // vectors of head_dim + 4 it holds
     float* rope_freq = nullptr;  // 1 / theta^(2j / head_dim), j < 64, computed on the host (libm powf, as the CPU path)
     float* rope_tab = nullptr;   // [k][(sin, cos) per rotation pair] at the current positions, rewritten every step
     // Prepared forms of the vectors the matvecs read (csrc/publish.cuh), written once by the kernel that produced the
@@ -61,9 +65,11 @@ struct LlamaModel final : alice_model {
         for (uint32_t p = 0; p < npeers; p++) cudaIpcCloseMemHandle(peer_base[p]);
     }
     uint32_t max_tokens() const override { return MAX_BATCH; }
-    int enqueue_step(uint32_t batch, bool greedy_feed) override { return step(batch, greedy_feed, nullptr, 0); }
-    // Logits of rows[0 .. nrows) of the batch only, each at its own place in `logits`; rows == nullptr: of all of them.
-    int step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows);
+    uint32_t piece_tokens() const override { return cap; }
+    int enqueue_step(uint32_t batch, bool greedy_feed) override { return step(batch, greedy_feed, nullptr, 0, nullptr); }
+    // rows == nullptr: logits of the whole batch (at most MAX_BATCH tokens) stay on the device. Else those of rows[0 .. nrows) are
+    // copied to host_logits; the last run of up to MAX_BATCH consecutive rows stays in `logits`.
+    int step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows, float* host_logits);
     int enqueue_rows(uint32_t n, const uint32_t* rows, uint32_t nrows, float* host_logits) override;
     int clear_state() override;
 };
@@ -88,8 +94,8 @@ int gemv(LlamaModel* m, GemvOp& op, const char* what) {
 // projections see the vector rounded to the Q8_K grid.
 bool preq_roundtrip(const WeightDesc& w) { return w.fmt == WF_Q1_0 || w.fmt == WF_Q2_0; }
 
-Q8KView q8_view(uint8_t* base, uint32_t n) {
-    const Q8KLayout l = Q8KLayout::make(n / 256, MAX_BATCH);
+Q8KView q8_view(uint8_t* base, uint32_t n, uint32_t cap) {
+    const Q8KLayout l = Q8KLayout::make(n / 256, cap);
     Q8KView v;
     v.qs = reinterpret_cast<const int8_t*>(base + l.qs_off);
     v.d = reinterpret_cast<const float*>(base + l.d_off);
@@ -111,10 +117,10 @@ void need_of(Need& nd, const WeightDesc& w, bool via_preq) {
     nd.xn = true;
     if (via_preq && preq_roundtrip(w)) nd.roundtrip = true;
 }
-void fill_dst(PublishDst& d, const Need& nd, uint8_t* q8_base, float* xn, uint32_t n) {
+void fill_dst(PublishDst& d, const Need& nd, uint8_t* q8_base, float* xn, uint32_t n, uint32_t cap) {
     d = PublishDst{};
     if (nd.q8) {
-        const Q8KView v = q8_view(q8_base, n);
+        const Q8KView v = q8_view(q8_base, n, cap);
         d.qs = const_cast<int8_t*>(v.qs); d.d = const_cast<float*>(v.d); d.bsums = const_cast<int16_t*>(v.bsums);
     }
     if (nd.xn) { d.xn = xn; d.roundtrip = nd.roundtrip ? 1u : 0u; }
@@ -126,7 +132,7 @@ void fill_dst(PublishDst& d, const Need& nd, uint8_t* q8_base, float* xn, uint32
 // rows into every peer's copy, with one flag per vector that a one-CTA kernel behind it raises on the peers and waits for
 // here before it prepares the vector for the next op. Attention runs on the rank's own KV heads (its q, k, v rows), so
 // only its output needs exchanging (it is the input of the output projection).
-int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows) {
+int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uint32_t nrows, float* host_logits) {
     LlamaModel* const m = this;
     const alice_model_config& c = m->cfg;
     cudaStream_t st = m->e->stream;
@@ -146,7 +152,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
                           uint32_t flag_idx) {
         p = Publish{};
         p.mode = PUB_VECTOR; p.n = len; p.batch = batch; p.src = src; p.norm_w = norm_w; p.eps = c.eps;
-        fill_dst(p.dst, nd, q8_base, xn, len);
+        fill_dst(p.dst, nd, q8_base, xn, len, m->cap);
         p.wait_limit = m->e->wait_limit;
         if (peer) {
             p.npeers = m->npeers; p.wait_flag = m->flags + flag_idx; p.epoch = m->epoch;
@@ -186,7 +192,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     // are resident and streaming weights meanwhile (measured on the 8B decode step: 2.23 ms per token this way, 2.28
     // with every CTA of the matvec normalising and quantizing the vector itself); else the raw vector plus the norm
     // weights, prepared per CTA. `fresh` = the hidden state has changed since the last such preparation.
-    Q8KView hid_view = q8_view(m->hid_q8, H);
+    Q8KView hid_view = q8_view(m->hid_q8, H, m->cap);
     auto hidden_input = [&](GemvOp& op, const WeightDesc& w, const float* norm_w, bool via_preq, bool fresh) -> int {
         op.batch = batch;
         if (wants_prepared(w)) { op.x = m->hid_xn; return ALICE_OK; }
@@ -195,7 +201,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
                 Publish p{};
                 p.mode = PUB_VECTOR; p.n = H; p.batch = batch; p.src = m->hidden; p.norm_w = norm_w; p.eps = c.eps;
                 Need nd; nd.q8 = true;
-                fill_dst(p.dst, nd, m->hid_q8, nullptr, H);
+                fill_dst(p.dst, nd, m->hid_q8, nullptr, H, m->cap);
                 MCU(launch_publish_vector(p, m->e->status, st, pdl));
             }
             op.q8 = &hid_view;
@@ -255,9 +261,9 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
         Publish attn_pub{};
         // a K-quant output projection takes the attention output as Q8_K: written by the attention kernel itself when a
         // KV head's outputs are whole blocks, else quantized in the projection's own prologue
-        const bool per_head_q8 = format_uses_q8k(L.o.fmt) && n == 1 && group % 2 == 0 && q_dim % 256 == 0;
-        if (per_head_q8) {
-            const Q8KView v = q8_view(m->attn_q8, q_dim);
+        const bool o_q8 = format_uses_q8k(L.o.fmt) && n == 1 && q_dim % 256 == 0 && (batch > 1 || group % 2 == 0);
+        if (o_q8 && batch == 1) {
+            const Q8KView v = q8_view(m->attn_q8, q_dim, m->cap);
             aa.q8.qs = const_cast<int8_t*>(v.qs); aa.q8.d = const_cast<float*>(v.d); aa.q8.bsums = const_cast<int16_t*>(v.bsums);
         }
         if (n > 1) {   // tensor parallel: the hand-over of the pushed rows
@@ -268,12 +274,17 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
             aa.npeers = m->npeers;
             for (uint32_t q = 0; q < m->npeers; q++) aa.peer_out[q] = reinterpret_cast<float*>(on_peer(q, m->attn_out)) + (size_t)r * lq;
         }
-        MCU(launch_attention(aa, batch, st, pdl));
+        if (batch == 1) {
+            MCU(launch_attention(aa, st, pdl));
+        } else {
+            MCU(launch_attention_tokens(aa, m->qkv, batch, m->pos, m->part_vectors, m->e->num_sms, st, pdl));
+            if (o_q8) { launch_quantize_q8k(m->attn_out, q_dim, batch, m->attn_q8, st, pdl, m->cap); MCU(cudaGetLastError()); }
+        }
         if ((rc = gather_then_publish(m->attn_out, lq, attn_pub))) return rc;
         {   // output projection + residual (src/llama3.rs:14423, 14468); leaves hidden prepared for gate / up
             GemvOp op; Q8KView view; Publish p;
             op.w[0] = &L.o;
-            if (per_head_q8) { view = q8_view(m->attn_q8, q_dim); op.q8 = &view; } else op.x = m->attn_out;
+            if (o_q8) { view = q8_view(m->attn_q8, q_dim, m->cap); op.q8 = &view; } else op.x = m->attn_out;
             op.batch = batch;
             op.resid = m->hidden; op.y = m->hidden; op.y_off[0] = r * m->lH; op.y_stride = H;
             Need nd; need_of(nd, L.gate, true);
@@ -296,13 +307,13 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
             }
             push_rows(op, m->ffn_h);
             if ((rc = gemv(m, op, "gate/up"))) return rc;
-            if (down_q8) { launch_quantize_q8k(m->ffn_h, F, batch, m->ffn_q8, st, pdl, MAX_BATCH); MCU(cudaGetLastError()); }
+            if (down_q8) { launch_quantize_q8k(m->ffn_h, F, batch, m->ffn_q8, st, pdl, m->cap); MCU(cudaGetLastError()); }
             if (n > 1 && (rc = gather_then_publish(m->ffn_h, m->lF, p))) return rc;
         }
         {   // down projection + residual (src/llama3.rs:14536-14555); leaves hidden prepared for the next layer / the head
             GemvOp op; Q8KView view; Publish p;
             op.w[0] = &L.down;
-            if (n == 1 && format_uses_q8k(L.down.fmt)) { view = q8_view(m->ffn_q8, F); op.q8 = &view; } else op.x = m->ffn_h;
+            if (n == 1 && format_uses_q8k(L.down.fmt)) { view = q8_view(m->ffn_q8, F, m->cap); op.q8 = &view; } else op.x = m->ffn_h;
             op.batch = batch;
             op.resid = m->hidden; op.y = m->hidden; op.y_off[0] = r * m->lH; op.y_stride = H;
             Need nd;
@@ -327,7 +338,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     for (uint32_t i = 0; i < runs_of;) {
         const uint32_t lo = rows ? rows[i] : 0;
         uint32_t len = rows ? 1 : batch;
-        while (rows && i + len < nrows && rows[i + len] == lo + len) len++;
+        while (rows && len < (uint32_t)MAX_BATCH && i + len < nrows && rows[i + len] == lo + len) len++;
         GemvOp op; Publish p;
         op.w[0] = &m->out;
         if ((rc = hidden_input(op, m->out, m->out_norm, false, i == 0))) return rc;
@@ -335,7 +346,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
         op.batch = len;
         if (op.q8) { at = *op.q8; at.qs += (size_t)lo * H; at.d += (size_t)lo * at.nb; at.bsums += (size_t)lo * at.nb * 16; op.q8 = &at; }
         if (op.x) op.x += (size_t)lo * H;
-        op.y = m->logits + (size_t)lo * V; op.y_off[0] = r * m->lV; op.y_stride = V;
+        op.y = m->logits; op.y_off[0] = r * m->lV; op.y_stride = V;
         if (batch == 1) op.argmax_key = m->argmax_key;   // greedy sampling: the head kernel leaves the packed maximum of its rows
         if (peer) {
             Need none;
@@ -350,6 +361,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
             if ((rc = tp_all_gather(m->e, m->logits, (size_t)m->lV * sizeof(float)))) return rc;
             if ((rc = tp_all_gather(m->e, m->argmax_keys, sizeof(unsigned long long)))) return rc;
         }
+        if (rows) MCU(cudaMemcpyAsync(host_logits + (size_t)i * V, m->logits, (size_t)len * V * 4, cudaMemcpyDeviceToHost, st));
         i += rows ? len : 1;
     }
     MCU(launch_finish_step(m->argmax_keys, m->tp_n, m->d_token, m->d_pos, m->d_trace, greedy_feed ? 1 : 0, batch,
@@ -360,12 +372,11 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
 
 // A single token always has its logits (and its argmax) left on the device.
 int LlamaModel::enqueue_rows(uint32_t n, const uint32_t* rows, uint32_t nrows, float* host_logits) {
-    const int rc = n == 1 ? step(1, false, nullptr, 0) : step(n, false, rows ? rows : &n, nrows);
-    if (rc) return rc;
-    for (uint32_t i = 0; i < nrows; i++)
-        MCU(cudaMemcpyAsync(host_logits + (size_t)i * cfg.vocab_size, logits + (size_t)rows[i] * cfg.vocab_size, (size_t)cfg.vocab_size * 4,
-                            cudaMemcpyDeviceToHost, e->stream));
-    return ALICE_OK;
+    static const uint32_t none = 0;
+    if (n > 1) return step(n, false, rows ? rows : &none, nrows, host_logits);
+    const int rc = step(1, false, nullptr, 0, nullptr);
+    if (!rc && nrows) MCU(cudaMemcpyAsync(host_logits, logits, (size_t)cfg.vocab_size * 4, cudaMemcpyDeviceToHost, e->stream));
+    return rc;
 }
 
 int LlamaModel::clear_state() {
@@ -434,11 +445,13 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     // (measured on the 8B and 27B decode steps: one wave of 2 CTAs per SM is the optimum; 18 or 64 splits cost 4-10 %)
     const size_t kv_elems = (size_t)c.num_layers * c.max_seq_len * lkv;
     if (!rc) rc = upload_norm(m, &m->out_norm, output_norm, c.hidden_dim);
-    constexpr uint32_t B = MAX_BATCH;
+    constexpr uint32_t PIECE = 256;
+    m->cap = n > 1 ? (uint32_t)MAX_BATCH : std::max<uint32_t>(MAX_BATCH, std::min(PIECE, c.max_seq_len));
+    const uint32_t B = m->cap;
     {   // the vectors other ranks need, the argmax keys and the hand-over counters share one allocation
         auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
         const size_t o_hidden = 0, o_attn = o_hidden + up((size_t)B * c.hidden_dim * 4), o_ffn = o_attn + up((size_t)B * q_dim * 4),
-                     o_logits = o_ffn + up((size_t)B * c.intermediate_dim * 4), o_keys = o_logits + up((size_t)B * c.vocab_size * 4),
+                     o_logits = o_ffn + up((size_t)B * c.intermediate_dim * 4), o_keys = o_logits + up((size_t)MAX_BATCH * c.vocab_size * 4),
                      o_flags = o_keys + up(8 * 8), o_epoch = o_flags + up(((size_t)4 * c.num_layers + 2) * 4);
         m->xchg_bytes = o_epoch + 256;
         if (!rc) rc = dev_alloc(m, &m->xchg, m->xchg_bytes);
@@ -458,8 +471,9 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     if (!rc) rc = dev_alloc(m, &m->qkv, (size_t)B * (lq + 2 * lkv));
     if (!rc) rc = dev_alloc(m, &m->kcache, kv_elems);
     if (!rc) rc = dev_alloc(m, &m->vcache, kv_elems);
-    if (!rc) rc = dev_alloc(m, &m->attn_part, (size_t)B * m->nsplit * (c.num_heads / n) * (c.head_dim + 4));
-    if (!rc) rc = dev_alloc(m, &m->attn_tickets, (size_t)B * (c.num_kv_heads / n));
+    m->part_vectors = MAX_BATCH * m->nsplit * (c.num_heads / n);
+    if (!rc) rc = dev_alloc(m, &m->attn_part, (size_t)m->part_vectors * (c.head_dim + 4));
+    if (!rc) rc = dev_alloc(m, &m->attn_tickets, c.num_kv_heads / n);
     if (!rc) rc = dev_alloc(m, &m->rope_tab, (size_t)B * 128);
     if (!rc) rc = dev_alloc(m, &m->rope_freq, 64);
     if (!rc) rc = dev_alloc(m, &m->hid_q8, Q8KLayout::make((c.hidden_dim + 255) / 256, B).total);
@@ -468,7 +482,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     if (!rc) rc = dev_alloc(m, &m->hid_xn, (size_t)B * c.hidden_dim);
     if (!rc) {
         const uint32_t widest = std::max({c.hidden_dim, c.intermediate_dim, q_dim});
-        m->prep_bytes = std::max(mma_prep_bytes(widest), plane_prep_bytes(widest, B));
+        m->prep_bytes = std::max(mma_prep_bytes(widest), plane_prep_bytes(widest, MAX_BATCH));
         rc = dev_alloc(m, &m->prep, m->prep_bytes);
     }
     if (!rc) rc = dev_alloc(m, &m->d_pos, 1);
@@ -482,7 +496,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
         if (err == cudaSuccess) err = cudaMemsetAsync(m->kcache, 0, kv_elems * 4, e->stream);
         if (err == cudaSuccess) err = cudaMemsetAsync(m->vcache, 0, kv_elems * 4, e->stream);
         if (err == cudaSuccess) err = cudaMemsetAsync(m->d_pos, 0, 4, e->stream);
-        if (err == cudaSuccess) err = cudaMemsetAsync(m->attn_tickets, 0, (size_t)B * (c.num_kv_heads / n) * 4, e->stream);
+        if (err == cudaSuccess) err = cudaMemsetAsync(m->attn_tickets, 0, (size_t)(c.num_kv_heads / n) * 4, e->stream);
         if (err == cudaSuccess) err = cudaMemsetAsync(m->d_token, 0, 4 * B, e->stream);
         if (err == cudaSuccess) err = cudaMemsetAsync(m->d_trace, 0, (size_t)c.max_seq_len * 4, e->stream);
         if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);

@@ -72,7 +72,7 @@ int32_t alice_model_forward_rows(alice_model* m, const uint32_t* tokens, uint32_
     uint32_t done = 0;
     std::vector<uint32_t> local;
     for (uint32_t lo = 0; lo < n && !rc;) {
-        const uint32_t k = std::min(m->max_tokens(), n - lo);
+        const uint32_t k = std::min(m->piece_tokens(), n - lo);
         local.clear();
         while (done + local.size() < nrows && rows[done + local.size()] < lo + k) local.push_back(rows[done + local.size()] - lo);
         rc = set_tokens(m, tokens + lo, k);

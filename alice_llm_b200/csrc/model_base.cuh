@@ -19,8 +19,9 @@ struct alice_model {
     std::vector<void*> owned;                    // device allocations freed with the model
 
     virtual ~alice_model() = default;
-    // Most consecutive tokens one enqueue_* call takes.
+    // Most consecutive tokens enqueue_step takes, and the pieces a prompt is cut into for enqueue_rows.
     virtual uint32_t max_tokens() const = 0;
+    virtual uint32_t piece_tokens() const { return max_tokens(); }
     // Queues n consecutive tokens (read from d_token) at the current position: leaves logits and advances *d_pos. With
     // greedy_feed (n == 1) the argmax becomes the next token and is recorded in d_trace.
     virtual int enqueue_step(uint32_t n, bool greedy_feed) = 0;
