@@ -13,6 +13,7 @@
 
 #include "abi_internal.cuh"
 #include "gemv_plan.cuh"
+#include "gemv_blocks.cuh"
 #include "gemv_planes.cuh"
 #include "tp.cuh"
 
@@ -246,9 +247,9 @@ static int run_gemv(alice_engine* e, const alice_weights* w0, const alice_weight
                     float* y, uint32_t batch, const char* who, bool may_alloc = true) {
     GemvOp op;
     const WeightFormat f = w0->d.fmt;
-    if (f == WF_Q1_0 || f == WF_Q2_0 || f == WF_TERNARY || f == WF_SPARSE_TERNARY) {
+    if (!format_uses_q8k(f) && f != WF_BF16) {
         // room for the activation digit table, prepared once ahead of the matvec (csrc/gemv_mma.cuh)
-        if (may_alloc) { const int rc = ensure_prep(e, std::max(mma_prep_bytes(w0->d.cols), plane_prep_bytes(w0->d.cols, batch))); if (rc) return rc; }
+        if (may_alloc) { const int rc = ensure_prep(e, std::max({mma_prep_bytes(w0->d.cols), plane_prep_bytes(w0->d.cols, batch), blocks_prep_bytes(w0->d.cols, batch)})); if (rc) return rc; }
         op.prep = e->prep; op.prep_bytes = e->prep_bytes;
     }
     op.w[0] = &w0->d; op.up = w1 ? &w1->d : nullptr;

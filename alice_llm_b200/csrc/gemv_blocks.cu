@@ -1,0 +1,498 @@
+// Kernels and launch of csrc/gemv_blocks.cuh.
+//
+// A block is an f16 scale and 32 int8 (Q8_0), 128 signs (Q1_0) or 128 two-bit slots (Q2_0); blocks are 2-byte aligned. The f32
+// activations become 31-bit fixed point (unit 2^-30 of a power of two above the largest) in four signed base-256 digits; the
+// digits of two vectors fill the eight B columns. A operand: the int8 weights themselves, or bytes & (1 << j). A block's sum is an exact integer (two digits joined in
+// 32 bits: at most 16 bytes x 255 x 128 x 257), the offset of the one- and two-bit codes is taken off in integers too (2 S - T, S - T with T summed over the same
+// digits), and one f32 multiply-add per block scales it.
+//
+// Every warp has a ring of its own in shared memory (16 rows x 8 blocks a stage, cp.async, no barrier between warps); the digit
+// table of a CTA's columns stays in shared memory for the whole launch. A cluster of S CTAs shares the columns where the table
+// fits no single CTA or a matrix has few rows; the (tile, stage) pairs of a CTA are dealt evenly to its warps and the parts of a
+// tile are added in a fixed order.
+//
+// What bounds it: Q8_0 HBM at any batch (one product per 544 bytes); Q1_0 and Q2_0 the instructions for one or two vectors
+// (about 95 per 576 bytes, an SM issues 100 while those stream), the products (8 per 16 rows and block, for each pair of vectors) for more.
+#include <algorithm>
+
+#include "../../include/alice_cuda.h"
+#include "gemv_blocks.cuh"
+#include "gemv_mma.cuh"
+
+namespace alice {
+namespace {
+
+constexpr int BLK_WARPS = 16;
+constexpr uint32_t BLK_ITEM = 8;                 // blocks of a row a stage holds
+constexpr uint32_t BLK_SMEM = 224 * 1024, BLK_HDR = 128;
+
+template <int FMT> struct BlkFmt;                // bytes and elements of a block, digit bytes per block and pair of vectors, row pitch of a stage
+// pitch: 32-bit reads of 8 rows x 16 bytes fill the banks once (48 modulo 128)
+template <> struct BlkFmt<0> { static constexpr uint32_t BB = 34, EL = 32, DIG = 256, PITCH = 304; static constexpr bool T = false; };
+template <> struct BlkFmt<1> { static constexpr uint32_t BB = 18, EL = 128, DIG = 1024, PITCH = 176; static constexpr bool T = true; };
+template <> struct BlkFmt<2> { static constexpr uint32_t BB = 34, EL = 128, DIG = 2048, PITCH = 304; static constexpr bool T = true; };
+
+struct BlkArgs {
+    const uint8_t* w[3];
+    uint32_t rows[3], y_off[3], tile0[4], nw;
+    const uint8_t* up;
+    uint32_t row_bytes, nb;                      // blocks of a row
+    const uint8_t* digits;                       // [nb][NT][DIG]
+    const int* tsum;                             // [nb][NT][4]
+    const float* kappa;
+    float* y;
+    const float* resid;
+    uint32_t y_stride, batch;
+    unsigned long long* argmax_key;
+    uint32_t tiles_max, stages, tsum_off, main_off, head_off;      // shared memory: header | rings | digits | tsum | main | head
+    int* status;
+    long long wait_limit;
+};
+
+constexpr int BLK_FIX_BITS = 30;
+// A vector that is not finite has a unit of NaN: so have all its results.
+__device__ __forceinline__ void block_fixed_scale(float amax, bool finite, float& to_fixed, float& kappa) {
+    const uint32_t ebits = (__float_as_uint(amax) >> 23) & 0xffu;
+    const int e = !finite || ebits == 0u ? 0 : max((int)ebits - 126, -96);      // 2^(30 - e) stays an f32
+    to_fixed = finite ? ldexpf(1.0f, BLK_FIX_BITS - e) : 0.0f;
+    kappa = finite ? ldexpf(1.0f, e - BLK_FIX_BITS) : __int_as_float(0x7fffffff);
+}
+// four signed base-256 digits of f, |f| <= 2^30, most significant first
+__device__ __forceinline__ void block_digits(int f, int (&d)[4]) {
+    d[3] = (int)(int8_t)(f & 255); f = (f - d[3]) >> 8;
+    d[2] = (int)(int8_t)(f & 255); f = (f - d[2]) >> 8;
+    d[1] = (int)(int8_t)(f & 255); f = (f - d[1]) >> 8;
+    d[0] = f;
+}
+
+// Digit table of vector blockIdx.y; see the indexing of the consumer below.
+template <int FMT>
+__global__ void __launch_bounds__(256) block_table_kernel(const float* x, uint32_t cols, uint32_t batch, uint32_t nb, uint32_t nt, uint8_t* digits, int* tsum, float* kappa_out) {
+    using F = BlkFmt<FMT>;
+    __shared__ float red[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t v = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+    const float* xv = x + (size_t)v * cols;
+    float amax = 0.0f, odd = 0.0f;         // odd: stays 0 for a finite vector (inf * 0 and NaN * 0 are NaN)
+    if (v < batch) {
+        for (uint32_t base = 0; base < cols / 4; base += 256 * 8) {
+            float4 q[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint32_t i = base + k * 256 + tid;
+                q[k] = i < cols / 4 ? __ldcg(reinterpret_cast<const float4*>(xv) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(q[k].x), fabsf(q[k].y))), fmaxf(fabsf(q[k].z), fabsf(q[k].w)));
+                odd = fmaf(q[k].x, 0.0f, fmaf(q[k].y, 0.0f, fmaf(q[k].z, 0.0f, fmaf(q[k].w, 0.0f, odd))));
+            }
+        }
+    }
+    const int finite = __syncthreads_and(odd == 0.0f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red[tid >> 5] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++) amax = fmaxf(amax, red[w]);
+    float to_fixed, kappa;
+    block_fixed_scale(amax, finite != 0, to_fixed, kappa);
+    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
+    constexpr uint32_t TPB = FMT == 0 ? 8 : FMT == 1 ? 8 : 16;     // threads of a block of weights
+    const uint32_t i = blockIdx.x * 256 + tid, blk = i / TPB, u = i % TPB;
+    const bool live = blk < nb;
+    uint32_t out[4][4] = {};
+    int ts[4] = {0, 0, 0, 0};
+    const uint32_t t = u & 3u, h = (u >> 2) & 1u, w = u >> 3;
+#pragma unroll
+    for (uint32_t b = 0; b < 4; b++) {
+        // FMT 0: byte 16 h + 4 t + b of the block; 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte 16 w + 4 t + b, bits 4 h .. 4 h + 3
+        const uint32_t e = FMT == 0 ? 16 * h + 4 * t + b : FMT == 1 ? 8 * (4 * t + b) + 4 * h : 4 * (16 * w + 4 * t + b) + 2 * h;
+        float xe[4] = {0.f, 0.f, 0.f, 0.f};
+        if (live && v < batch) {
+            const float* p = xv + (size_t)blk * F::EL + e;
+#pragma unroll
+            for (uint32_t k = 0; k < (FMT == 0 ? 1u : FMT == 1 ? 4u : 2u); k++) xe[k] = __ldcg(p + k);
+        }
+#pragma unroll
+        for (uint32_t jj = 0; jj < (FMT == 0 ? 1u : 4u); jj++) {
+            const int sh = FMT == 0 ? 0 : FMT == 1 ? (int)(4 * h + jj) : (int)(2 * (2 * h + (jj >> 1)));
+            const int f = (__float2int_rn(xe[FMT == 2 ? jj >> 1 : jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
+            int dg[4];
+            block_digits(f, dg);
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                out[d][jj] |= (uint32_t)(dg[d] & 255) << (8 * b);
+                if (FMT == 1 || (FMT == 2 && !(jj & 1u))) ts[d] += dg[d] * (1 << sh);
+            }
+        }
+    }
+    if (F::T) {
+#pragma unroll
+        for (int d = 0; d < 4; d++)
+#pragma unroll
+            for (uint32_t o = 1; o < TPB; o *= 2) ts[d] += __shfl_xor_sync(0xffffffffu, ts[d], o);
+        if (live && u < 2) tsum[((size_t)blk * nt + (v >> 1)) * 4 + (v & 1u) * 2 + u] = u ? ts[2] * 256 + ts[3] : ts[0] * 256 + ts[1];
+    }
+    if (!live) return;
+    uint8_t* rec = digits + ((size_t)blk * nt + (v >> 1)) * F::DIG;
+#pragma unroll
+    for (uint32_t d = 0; d < 4; d++) {
+        const uint32_t col = (v & 1u) * 4 + d;
+        if (FMT == 0) reinterpret_cast<uint32_t*>(rec)[(col * 4 + t) * 2 + h] = out[d][0];
+        else reinterpret_cast<uint4*>(rec)[(w * 2 + h) * 32 + col * 4 + t] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
+    }
+}
+
+__device__ __forceinline__ uint32_t w4(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+__device__ __forceinline__ void mma_s8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+
+// AL: rows are multiples of 16 bytes, so a stage starts on a 16-byte boundary.
+template <int FMT, int NT, bool SW, bool AL>
+__global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __grid_constant__ BlkArgs a, const uint32_t S) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    using F = BlkFmt<FMT>;
+    constexpr int MATS = SW ? 2 : 1;
+    constexpr uint32_t CH = F::BB * BLK_ITEM / 16 + (AL ? 0 : 1), STAGE = 16 * F::PITCH;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3u;
+    const uint32_t rank = S > 1 ? blockIdx.x % S : 0u, cl = blockIdx.x / S, ncl = gridDim.x / S;
+    const uint32_t tiles = a.tile0[a.nw];
+    const uint32_t t_lo = (uint32_t)((uint64_t)tiles * cl / ncl), nt_loc = (uint32_t)((uint64_t)tiles * (cl + 1) / ncl) - t_lo;
+    const uint32_t all = (a.nb + BLK_ITEM - 1) / BLK_ITEM, s_lo = all * rank / S, ns = all * (rank + 1) / S - s_lo;
+    const uint32_t b_lo = s_lo * BLK_ITEM, b_hi = min(a.nb, (s_lo + ns) * BLK_ITEM), nblk = b_hi - b_lo;
+    const uint32_t bar = smem_u32(smem), ring = bar + BLK_HDR + warp * a.stages * STAGE, tab = bar + BLK_HDR + BLK_WARPS * a.stages * STAGE;
+    const uint32_t tsm = bar + a.tsum_off;
+    float* mainp = reinterpret_cast<float*>(smem + a.main_off);     // [mat][tile][16 rows][2 NT]
+    float* head = reinterpret_cast<float*>(smem + a.head_off);      // [warp][16 rows][2 NT]
+    if (tid == 0) { mbar_init(bar, 1); mbar_fence_init(); }
+    __syncthreads();
+    pdl_launch_dependents();
+
+    const uint32_t items = MATS * nt_loc * ns;
+    const uint32_t i_lo = items * warp / BLK_WARPS, i_hi = items * (warp + 1) / BLK_WARPS;
+    auto matrix_of = [&](uint32_t tile, uint32_t& s, const uint8_t*& w, uint32_t& r0) {     // tile: gate tiles, then up tiles
+        const bool up = SW && tile >= nt_loc;
+        const uint32_t tl = t_lo + (up ? tile - nt_loc : tile);
+        s = 0;
+        if (!SW) while (s + 1 < a.nw && tl >= a.tile0[s + 1]) s++;
+        w = up ? a.up : a.w[s];
+        r0 = (tl - a.tile0[s]) * 16;
+    };
+    uint32_t l_item = i_lo, l_tile = i_lo / ns, l_seg = i_lo - l_tile * ns, l_slot = 0;
+    const uint8_t* lw = nullptr;
+    uint32_t ls = 0, lr0 = 0;
+    if (i_lo < i_hi) matrix_of(l_tile, ls, lw, lr0);
+    auto fetch = [&]() {
+        if (l_item < i_hi) {
+            const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
+            const uint32_t at = (s_lo + l_seg) * (BLK_ITEM * F::BB), dst = ring + l_slot * STAGE;
+#pragma unroll
+            for (uint32_t i = lane; i < 16 * CH; i += 32) {
+                const uint32_t r = i / CH, c = i - r * CH;
+                const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
+                const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * F::PITCH + c * 16), "l"(n ? lw + off : lw), "r"(n) : "memory");
+            }
+            l_item++;
+            if (++l_seg == ns) { l_seg = 0; l_tile++; if (l_item < i_hi) matrix_of(l_tile, ls, lw, lr0); }
+            if (++l_slot == a.stages) l_slot = 0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (uint32_t k = 0; k + 1 < a.stages; k++) fetch();
+
+    pdl_wait();
+    if (tid == 0) {
+        const uint32_t db = nblk * NT * F::DIG, tb = F::T ? nblk * NT * 16u : 0u;
+        mbar_arrive_expect_tx(bar, db + tb);
+        bulk_g2s(tab, a.digits + (size_t)b_lo * NT * F::DIG, db, bar);
+        if (F::T) bulk_g2s(tsm, a.tsum + (size_t)b_lo * NT * 4, tb, bar);
+    }
+    const bool ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
+    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
+
+    float acc[NT][2] = {};
+    uint32_t tile = i_lo / ns, seg = i_lo - tile * ns, slot = 0, padA = 0, padB = 0;
+    bool mid = seg != 0;                     // this warp took the tile up in its middle
+    auto pads = [&]() {
+        if (AL) return;
+        uint32_t s, r0;
+        const uint8_t* w;
+        matrix_of(tile, s, w, r0);
+        padA = (min(r0 + g, a.rows[s] - 1) * a.row_bytes) & 15u;
+        padB = (min(r0 + g + 8, a.rows[s] - 1) * a.row_bytes) & 15u;
+    };
+    if (i_lo < i_hi) pads();
+    auto flush = [&]() {
+        float* dst = mid ? head + warp * (16 * 2 * NT) : mainp + (size_t)((tile >= nt_loc ? a.tiles_max + (tile - nt_loc) : tile) * 16) * (2 * NT);
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float f = (t & 1u) ? acc[n][h] : acc[n][h] * 65536.0f;
+                const float y = f + __shfl_xor_sync(0xffffffffu, f, 1);
+                if (!(t & 1u)) dst[(g + 8 * h) * (2 * NT) + 2 * n + (t >> 1)] = y;
+                acc[n][h] = 0.0f;
+            }
+        mid = false;
+    };
+    for (uint32_t it = i_lo; ok && it < i_hi; it++) {
+        if (a.stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        else if (a.stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncwarp();                        // the stage is in for every lane, and every lane is done with the one before
+        fetch();
+        const uint32_t rowA = ring + slot * STAGE + g * F::PITCH + padA, rowB = ring + slot * STAGE + (g + 8) * F::PITCH + padB;
+        if (++slot == a.stages) slot = 0;
+        const uint32_t b0 = seg * BLK_ITEM, nbi = min(BLK_ITEM, nblk - b0);
+        const uint32_t rec = tab + b0 * (NT * F::DIG), trec = tsm + b0 * (NT * 16u) + t * 4;
+        auto block = [&](uint32_t b) {
+            const uint32_t pA = rowA + b * F::BB, pB = rowB + b * F::BB;
+            const float dA = f16_bits_to_f32(lds16(pA)), dB = f16_bits_to_f32(lds16(pB));
+            if constexpr (FMT == 0) {
+                const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t), a2 = lds32_u2(pA + 18 + 4 * t), a3 = lds32_u2(pB + 18 + 4 * t);
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                    const uint2 x = lds64(rec + (b * NT + n) * F::DIG + lane * 8);
+                    int c[4];
+                    mma_s8s8_k32(c, a0, a1, a2, a3, x.x, x.y);
+                    acc[n][0] = fmaf(dA, (float)(c[0] * 256 + c[1]), acc[n][0]);
+                    acc[n][1] = fmaf(dB, (float)(c[2] * 256 + c[3]), acc[n][1]);
+                }
+            } else {
+                int c[NT][2][4] = {};        // even and odd bits: two chains
+                if constexpr (FMT == 1) {
+                    const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint4 x[NT];
+#pragma unroll
+                        for (int n = 0; n < NT; n++) x[n] = lds128(rec + (b * NT + n) * F::DIG + h * 512 + lane * 16);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const uint32_t m = 0x01010101u << (4 * h + j), m0 = a0 & m, m1 = a1 & m;
+#pragma unroll
+                            for (int n = 0; n < NT; n++) mma_u8s8_k16(c[n][j & 1], m0, m1, w4(x[n], j));
+                        }
+                    }
+                } else {
+                    const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t), a2 = lds32_u2(pA + 18 + 4 * t), a3 = lds32_u2(pB + 18 + 4 * t);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint4 x[NT], z[NT];
+#pragma unroll
+                        for (int n = 0; n < NT; n++) {
+                            x[n] = lds128(rec + (b * NT + n) * F::DIG + h * 512 + lane * 16);
+                            z[n] = lds128(rec + (b * NT + n) * F::DIG + 1024 + h * 512 + lane * 16);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const uint32_t m = 0x01010101u << (4 * h + j), m0 = a0 & m, m1 = a1 & m, m2 = a2 & m, m3 = a3 & m;
+#pragma unroll
+                            for (int n = 0; n < NT; n++) mma_u8s8_k32(c[n][j & 1], m0, m1, m2, m3, w4(x[n], j), w4(z[n], j));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                    const int T = (int)lds32(trec + (b * NT + n) * 16);
+                    int vA = (c[n][0][0] + c[n][1][0]) * 256 + (c[n][0][1] + c[n][1][1]), vB = (c[n][0][2] + c[n][1][2]) * 256 + (c[n][0][3] + c[n][1][3]);
+                    vA = (FMT == 1 ? 2 * vA : vA) - T;
+                    vB = (FMT == 1 ? 2 * vB : vB) - T;
+                    acc[n][0] = fmaf(dA, (float)vA, acc[n][0]);
+                    acc[n][1] = fmaf(dB, (float)vB, acc[n][1]);
+                }
+            }
+        };
+        if (nbi == BLK_ITEM) {
+#pragma unroll(FMT == 0 ? 4 : 2)
+            for (uint32_t b = 0; b < BLK_ITEM; b++) block(b);
+        } else {
+#pragma unroll 1
+            for (uint32_t b = 0; b < nbi; b++) block(b);
+        }
+        if (++seg == ns) { flush(); seg = 0; tile++; if (it + 1 < i_hi) pads(); }
+    }
+    if (ok && seg != 0 && i_lo < i_hi) flush();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // parts of tiles that another warp began, in the order of the warps
+    if (tid < 16 * 2 * NT) {
+        for (uint32_t w = 1; w < (uint32_t)BLK_WARPS; w++) {
+            const uint32_t lo = items * w / BLK_WARPS, hi = items * (w + 1) / BLK_WARPS, tl = lo / ns;
+            if (lo < hi && lo != tl * ns) mainp[(size_t)((tl >= nt_loc ? a.tiles_max + (tl - nt_loc) : tl) * 16) * (2 * NT) + tid] += head[w * (16 * 2 * NT) + tid];
+        }
+    }
+    if (S > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+    const uint32_t R = nt_loc * 16, outs = R * a.batch;
+    const uint32_t main_s = bar + a.main_off;
+    unsigned long long key = 0ull;
+    for (uint32_t i = rank * (BLK_WARPS * 32) + tid; ok && i < outs; i += S * (BLK_WARPS * 32)) {
+        const uint32_t v = i / R, lr = i - v * R, tl = t_lo + lr / 16;
+        uint32_t s = 0;
+        if (!SW) while (s + 1 < a.nw && tl >= a.tile0[s + 1]) s++;
+        const uint32_t row = (tl - a.tile0[s]) * 16 + lr % 16;
+        if (row >= a.rows[s]) continue;
+        float f[MATS];
+#pragma unroll
+        for (int q = 0; q < MATS; q++) {
+            const uint32_t at = main_s + ((q * a.tiles_max * 16 + lr) * (2 * NT) + v) * 4;
+            float y = ldsf(at);
+            if (S > 1) {
+                for (uint32_t r = 0; r < S; r++) {
+                    uint32_t remote;
+                    float p;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(r));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p) : "r"(remote) : "memory");
+                    y = r ? y + p : p;
+                }
+            }
+            f[q] = __ldg(a.kappa + v) * y;
+        }
+        float r = SW ? silu_ref(f[0]) * f[MATS - 1] : f[0];
+        const uint32_t yi = a.y_off[s] + row;
+        const size_t at = (size_t)v * a.y_stride + yi;
+        if (a.resid != nullptr) r = __fadd_rn(__ldcg(a.resid + at), r);
+        a.y[at] = r;
+        const uint32_t b = __float_as_uint(r), ordered = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+        const unsigned long long k = r == r ? ((unsigned long long)ordered << 32) | (0xFFFFFFFFu - yi) : 0ull;
+        key = k > key ? k : key;
+    }
+    if (a.argmax_key != nullptr) stream_argmax(a.argmax_key, key, lane);
+    if (S > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+template <int FMT, int NT, bool SW, bool AL>
+int plan_and_launch(BlkArgs a, const LaunchCfg& cfg, bool dry) {
+    using F = BlkFmt<FMT>;
+    static bool attr_done[64] = {};
+    static int clusters[64][4] = {};
+    auto kern = block_rows_kernel<FMT, NT, SW, AL>;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ALICE_E_CUDA;
+    if (!attr_done[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLK_SMEM) != cudaSuccess) return ALICE_E_CUDA;
+        attr_done[dev] = true;
+    }
+    const uint32_t sms = (uint32_t)std::max(cfg.num_sms, 1), tiles = a.tile0[a.nw], all = (a.nb + BLK_ITEM - 1) / BLK_ITEM;
+    cudaLaunchConfig_t lc = {};
+    lc.blockDim = dim3(BLK_WARPS * 32); lc.stream = cfg.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    for (uint32_t S = 1, l2 = 0; S <= 8 && S <= all; S *= 2, l2++) {
+        uint32_t ncl = sms;
+        if (S > 1) {      // a cluster's CTAs sit in one GPC: what the chip holds at once is asked for, once per kernel and device
+            int& known = clusters[dev][l2];
+            if (!known) {
+                at[0].val.clusterDim.x = S;
+                lc.attrs = at; lc.numAttrs = 1; lc.gridDim = dim3(sms / S * S); lc.dynamicSmemBytes = BLK_SMEM;
+                int n = 0;
+                if (sms < S || cudaOccupancyMaxActiveClusters(&n, kern, &lc) != cudaSuccess || n < 1) { cudaGetLastError(); break; }
+                known = n;
+            }
+            ncl = std::min<uint32_t>((uint32_t)known, sms / S);
+        }
+        ncl = std::min(ncl, tiles);
+        const uint32_t per = (tiles + ncl - 1) / ncl, slice = (all + S - 1) / S * BLK_ITEM;
+        const size_t dig = (size_t)slice * NT * F::DIG, ts = F::T ? (size_t)slice * NT * 16 : 0, mn = (size_t)(SW ? 2 : 1) * per * 16 * 2 * NT * 4,
+                     hd = (size_t)BLK_WARPS * 16 * 2 * NT * 4, stage = (size_t)BLK_WARPS * 16 * F::PITCH, fixed = BLK_HDR + dig + ts + mn + hd;
+        if (fixed + 2 * stage > BLK_SMEM) continue;
+        // fewer tiles than half the SMs: let more CTAs share a tile's columns
+        if (S < 8 && tiles * S * 2 <= sms && all >= 2 * S) continue;
+        if (dry) return ALICE_OK;
+        a.stages = (uint32_t)std::min<size_t>(4, (BLK_SMEM - fixed) / stage);
+        a.tiles_max = per;
+        a.tsum_off = (uint32_t)(BLK_HDR + a.stages * stage + dig);
+        a.main_off = (uint32_t)(a.tsum_off + ts); a.head_off = (uint32_t)(a.main_off + mn);
+        at[0].val.clusterDim.x = S;
+        lc.gridDim = dim3(ncl * S); lc.dynamicSmemBytes = fixed + a.stages * stage;
+        lc.attrs = S > 1 ? at : at + 1;
+        lc.numAttrs = (S > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
+        return cudaLaunchKernelEx(&lc, kern, a, S) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
+    }
+    return ALICE_E_SHAPE;
+}
+
+template <int FMT, int NT>
+int launch_nt(const BlkArgs& a, const LaunchCfg& cfg, bool dry) {
+    const bool al = a.row_bytes % 16 == 0;
+    if (a.up) return al ? plan_and_launch<FMT, NT, true, true>(a, cfg, dry) : plan_and_launch<FMT, NT, true, false>(a, cfg, dry);
+    return al ? plan_and_launch<FMT, NT, false, true>(a, cfg, dry) : plan_and_launch<FMT, NT, false, false>(a, cfg, dry);
+}
+uint32_t pairs_of(uint32_t batch) { return batch <= 2 ? 1u : batch <= 4 ? 2u : 4u; }
+
+template <int FMT>
+int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+    using F = BlkFmt<FMT>;
+    const uint32_t nt = pairs_of(op.batch), cols = op.w[0]->cols;
+    a.nb = cols / F::EL;
+    const size_t dig = (size_t)a.nb * nt * F::DIG, ts = F::T ? (size_t)a.nb * nt * 16 : 0;
+    if (!dry) {
+        if (!op.prep || ((uintptr_t)op.prep & 15) || dig + ts + 64 > op.prep_bytes) return ALICE_E_SHAPE;
+        uint8_t* base = static_cast<uint8_t*>(op.prep);
+        a.digits = base; a.tsum = reinterpret_cast<const int*>(base + dig); a.kappa = reinterpret_cast<const float*>(base + dig + ts);
+    }
+    auto rows = [&](bool plan) { return nt == 1 ? launch_nt<FMT, 1>(a, cfg, plan) : nt == 2 ? launch_nt<FMT, 2>(a, cfg, plan) : launch_nt<FMT, 4>(a, cfg, plan); };
+    const int rc = rows(true);
+    if (rc || dry) return rc;
+    cudaLaunchConfig_t lc = {};
+    const uint32_t per_vec = a.nb * (FMT == 2 ? 16u : 8u);
+    lc.gridDim = dim3((per_vec + 255) / 256, 2 * nt); lc.blockDim = dim3(256); lc.stream = cfg.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at; lc.numAttrs = cfg.pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&lc, block_table_kernel<FMT>, op.x, cols, op.batch, a.nb, nt, const_cast<uint8_t*>(a.digits), const_cast<int*>(a.tsum), const_cast<float*>(a.kappa)) != cudaSuccess)
+        return ALICE_E_CUDA;
+    return rows(false);
+}
+
+}  // namespace
+
+size_t blocks_prep_bytes(uint32_t cols, uint32_t batch) {
+    // Q2_0 has the largest: 2048 + 16 bytes per 128 columns and pair
+    return (size_t)((cols + 127) / 128) * pairs_of(batch) * (2048 + 16) + 256;
+}
+
+int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+    const WeightDesc& w0 = *op.w[0];
+    if ((w0.fmt != WF_Q8_0 && w0.fmt != WF_Q1_0 && w0.fmt != WF_Q2_0) || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || (op.argmax_key && op.batch > 1)) return ALICE_E_SHAPE;
+    if (op.nw < 1 || op.nw > 3 || (op.up && op.nw != 1) || !op.y || !op.x || ((uintptr_t)op.x & 15)) return ALICE_E_SHAPE;
+    BlkArgs a = {};
+    uint32_t total = 0;
+    for (uint32_t i = 0; i < op.nw; i++) {
+        const WeightDesc* w = op.w[i];
+        if (!w || !w->data || !w->rows || ((uintptr_t)w->data & 15) || w->fmt != w0.fmt || w->cols != w0.cols || w->row_bytes != w0.row_bytes) return ALICE_E_SHAPE;
+        a.w[i] = w->data; a.rows[i] = w->rows; a.y_off[i] = op.y_off[i];
+        a.tile0[i + 1] = a.tile0[i] + (w->rows + 15) / 16;
+        total += w->rows;
+    }
+    if (op.up) {
+        const WeightDesc& u = *op.up;
+        if (u.fmt != w0.fmt || u.rows != w0.rows || u.cols != w0.cols || u.row_bytes != w0.row_bytes || !u.data || ((uintptr_t)u.data & 15)) return ALICE_E_SHAPE;
+        a.up = u.data;
+    }
+    a.nw = op.nw; a.row_bytes = w0.row_bytes;
+    a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch;
+    a.argmax_key = op.argmax_key; a.status = cfg.status; a.wait_limit = op.wait_limit;
+    return w0.fmt == WF_Q8_0 ? launch_blk<0>(a, op, cfg, dry) : w0.fmt == WF_Q1_0 ? launch_blk<1>(a, op, cfg, dry) : launch_blk<2>(a, op, cfg, dry);
+}
+
+}  // namespace alice

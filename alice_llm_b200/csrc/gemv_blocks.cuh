@@ -1,0 +1,12 @@
+// Matvec over Q8_0, Q1_0 and Q2_0 blocks for 1..8 input vectors in ONE pass over the weights, on the int8 tensor path.
+#pragma once
+#include "gemv_launch.cuh"
+
+namespace alice {
+
+// Scratch for the digit table of `batch` vectors, for any of the three formats.
+size_t blocks_prep_bytes(uint32_t cols, uint32_t batch);
+// ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only.
+int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry);
+
+}  // namespace alice

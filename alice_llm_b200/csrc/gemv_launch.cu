@@ -11,6 +11,7 @@
 #include "gemm_kq.cuh"
 #include "gemv_launch.cuh"
 #include "gemv_plan.cuh"
+#include "gemv_blocks.cuh"
 #include "gemv_planes.cuh"
 
 namespace alice {
@@ -607,8 +608,10 @@ int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
         return ALICE_OK;
     }
     if (op.batch > 1 && op.argmax_key) return ALICE_E_INVALID;
-    if (op.w[0]->fmt == WF_TERNARY || op.w[0]->fmt == WF_SPARSE_TERNARY) {
-        const int prc = launch_split(launch_planes, op, cfg);
+    const WeightFormat f = op.w[0]->fmt;
+    const bool planes = f == WF_TERNARY || f == WF_SPARSE_TERNARY;
+    if (planes || f == WF_Q8_0 || f == WF_Q1_0 || f == WF_Q2_0) {
+        const int prc = launch_split(planes ? launch_planes : launch_blocks, op, cfg);
         if (prc != ALICE_E_SHAPE) return prc;
     }
     if (op.batch == 1) return launch_single(op, cfg);
@@ -634,7 +637,7 @@ size_t mma_prep_bytes(uint32_t cols) {
 int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint32_t* weight_passes) {
     uint32_t n = 0;
     if (op.batch > 1 && launch_kq_batch(op, cfg, true, &n) == ALICE_OK) { *launches = n; *weight_passes = 1; return ALICE_OK; }
-    if (launch_planes(op, cfg, true) == ALICE_OK) { *launches = *weight_passes = 1; return ALICE_OK; }
+    if (launch_planes(op, cfg, true) == ALICE_OK || launch_blocks(op, cfg, true) == ALICE_OK) { *launches = *weight_passes = 1; return ALICE_OK; }
     GemvOp one = op; one.batch = 1;
     StreamPlan pl;
     const int rc = plan_stream_gemv(one, cfg, pl);

@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32
     const uint32_t v = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     const float* xv = x + (size_t)v * cols;
     const bool vec4 = cols % 4 == 0 && ((uintptr_t)xv & 15) == 0;
-    float amax = 0.0f;
+    float amax = 0.0f, odd = 0.0f;         // odd: stays 0 for a finite vector (inf * 0 and NaN * 0 are NaN)
     if (v < batch) {
         if (vec4) {
             for (uint32_t base = 0; base < cols / 4; base += 256 * 8) {
@@ -33,12 +33,20 @@ __global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32
                     q[k] = i < cols / 4 ? __ldcg(reinterpret_cast<const float4*>(xv) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
-                for (int k = 0; k < 8; k++) amax = fmaxf(fmaxf(amax, fmaxf(fabsf(q[k].x), fabsf(q[k].y))), fmaxf(fabsf(q[k].z), fabsf(q[k].w)));
+                for (int k = 0; k < 8; k++) {
+                    amax = fmaxf(fmaxf(amax, fmaxf(fabsf(q[k].x), fabsf(q[k].y))), fmaxf(fabsf(q[k].z), fabsf(q[k].w)));
+                    odd = fmaf(q[k].x, 0.0f, fmaf(q[k].y, 0.0f, fmaf(q[k].z, 0.0f, fmaf(q[k].w, 0.0f, odd))));
+                }
             }
         } else {
-            for (uint32_t i = tid; i < cols; i += 256) amax = fmaxf(amax, fabsf(__ldcg(xv + i)));
+            for (uint32_t i = tid; i < cols; i += 256) {
+                const float q = __ldcg(xv + i);
+                amax = fmaxf(amax, fabsf(q));
+                odd = fmaf(q, 0.0f, odd);
+            }
         }
     }
+    const bool finite = __syncthreads_and(odd == 0.0f);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if (lane == 0) red[tid >> 5] = amax;
@@ -47,7 +55,7 @@ __global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32
     for (int w = 0; w < 8; w++) amax = fmaxf(amax, red[w]);
     float to_fixed, kappa;
     mma_fixed_scale(amax, to_fixed, kappa);
-    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
+    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = finite ? kappa : __int_as_float(0x7fffffff);      // all results of a vector that is not finite are NaN
     const uint32_t seg = blockIdx.x * 8 + (tid >> 5), t = lane & 3u, wh = lane >> 2, h = wh & 1u;   // wh = 2 w + h
     if (seg >= segs) return;
     uint32_t out[4][4] = {};          // [digit][bit 4 h + jj]

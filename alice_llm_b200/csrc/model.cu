@@ -10,6 +10,7 @@
 
 #include "abi_internal.cuh"
 #include "attn_body.cuh"
+#include "gemv_blocks.cuh"
 #include "gemv_planes.cuh"
 #include "glue.cuh"
 #include "model_base.cuh"
@@ -104,11 +105,11 @@ Q8KView q8_view(uint8_t* base, uint32_t n, uint32_t cap) {
     return v;
 }
 
-// The bit-plane tensor-core kernels (Q1_0, Q2_0, ternary formats) take their input as a finished f32 vector in global
-// memory, left there by the kernel that produced the vector; the K-quant kernels take Q8_K blocks that a one-CTA kernel
-// prepares between producer and consumer; the rest (Q8_0) prepare the raw vector per CTA in their own prologue.
+// The int8 kernels of Q8_0, Q1_0, Q2_0 and the ternary formats take their input as a finished f32 vector in global memory, left
+// there by the kernel that produced the vector; the K-quant kernels take Q8_K blocks that a small kernel prepares between producer
+// and consumer. A Q8_0 matrix beside one that wants the vector on the Q8_K grid prepares the raw vector in its own prologue.
 bool wants_prepared(const WeightDesc& w) {
-    return (w.fmt == WF_Q1_0 || w.fmt == WF_Q2_0 || w.fmt == WF_TERNARY || w.fmt == WF_SPARSE_TERNARY) && w.cols % 4 == 0;
+    return (w.fmt == WF_Q8_0 || w.fmt == WF_Q1_0 || w.fmt == WF_Q2_0 || w.fmt == WF_TERNARY || w.fmt == WF_SPARSE_TERNARY) && w.cols % 4 == 0;
 }
 // Which prepared forms of a vector its consumers need from the kernel that produces it.
 struct Need { bool q8 = false, xn = false, roundtrip = false; };
@@ -193,9 +194,9 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     // with every CTA of the matvec normalising and quantizing the vector itself); else the raw vector plus the norm
     // weights, prepared per CTA. `fresh` = the hidden state has changed since the last such preparation.
     Q8KView hid_view = q8_view(m->hid_q8, H, m->cap);
-    auto hidden_input = [&](GemvOp& op, const WeightDesc& w, const float* norm_w, bool via_preq, bool fresh) -> int {
+    auto hidden_input = [&](GemvOp& op, const WeightDesc& w, const float* norm_w, bool via_preq, bool fresh, bool beside_grid = false) -> int {
         op.batch = batch;
-        if (wants_prepared(w)) { op.x = m->hid_xn; return ALICE_OK; }
+        if (wants_prepared(w) && !(w.fmt == WF_Q8_0 && beside_grid)) { op.x = m->hid_xn; return ALICE_OK; }
         if (format_uses_q8k(w.fmt)) {
             if (fresh) {
                 Publish p{};
@@ -247,7 +248,8 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
             for (int i = 0; i < 3; i++) {
                 GemvOp op; Q8KView view;
                 op.w[0] = ws[i];
-                if ((rc = hidden_input(op, *ws[i], L.attn_norm, true, i == 0))) return rc;
+                const bool beside_grid = preq_roundtrip(L.q) || preq_roundtrip(L.k) || preq_roundtrip(L.v);
+                if ((rc = hidden_input(op, *ws[i], L.attn_norm, true, i == 0, beside_grid))) return rc;
                 op.y = m->qkv + offs[i]; op.y_stride = qkv_stride;
                 if ((rc = gemv(m, op, "q/k/v"))) return rc;
             }
@@ -482,7 +484,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     if (!rc) rc = dev_alloc(m, &m->hid_xn, (size_t)B * c.hidden_dim);
     if (!rc) {
         const uint32_t widest = std::max({c.hidden_dim, c.intermediate_dim, q_dim});
-        m->prep_bytes = std::max(mma_prep_bytes(widest), plane_prep_bytes(widest, MAX_BATCH));
+        m->prep_bytes = std::max({mma_prep_bytes(widest), plane_prep_bytes(widest, MAX_BATCH), blocks_prep_bytes(widest, MAX_BATCH)});
         rc = dev_alloc(m, &m->prep, m->prep_bytes);
     }
     if (!rc) rc = dev_alloc(m, &m->d_pos, 1);
