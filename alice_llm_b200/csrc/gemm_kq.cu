@@ -3,9 +3,9 @@
 // 6- or 8-bit scale in int32, one f32 step per block of 256. That is why the products are mma.sync u8 x s8: scale times
 // quant needs more than 8 bits, and up to 13 bits for Q6_K, more than an f16 holds.
 //
-// A CTA (4 warps, 2 x 2) owns 64 rows x 16 NTW tokens and walks the 256-column blocks: raw weight blocks and Q8_K blocks come in
-// with cp.async one to two blocks ahead, a warp unpacks 32 rows of a sub-block into A fragments and uses them for its NTW x 8
-// tokens. The min / bias term is a pair of products of the scales with base-64 digits of the activation sums, once per block.
+// A CTA (WM x WN warps) owns 32 WM rows x 8 NTW WN tokens and walks the 256-column blocks: raw weight blocks and Q8_K blocks come
+// in with cp.async one to two blocks ahead, a warp unpacks 32 rows of a sub-block into A fragments and uses them for its NTW x 8
+// tokens (32: sums in int32 and f32 then leave room for two CTAs of eight warps an SM). The min / bias term is a pair of products of the scales with base-64 digits of the activation sums, once per block.
 // What bounds it: from 64 tokens on the int8 products (8 clk each and SM quarter) together with the four multiply-adds that
 // scale each of them; below, HBM. Where tiles are fewer than two per SM, a cluster shares the columns of a tile and adds its
 // parts through distributed shared memory in a fixed order.
@@ -18,8 +18,6 @@
 
 namespace alice {
 namespace {
-
-constexpr uint32_t G_ROWS = 64, G_THREADS = 128;
 
 struct KqGemmArgs {
     const uint8_t* w[3];
@@ -40,9 +38,9 @@ template <> struct KqBlock<4> { static constexpr uint32_t BB = 144, CH = 9, PITC
 template <> struct KqBlock<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 224, XP = 288, DG = 16; };
 template <> struct KqBlock<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, XP = 272, DG = 32; };
 
-template <int FMT, int NTW>
+template <int FMT, int WM, int WN, int NTW>
 struct KqStage {      // byte offsets inside a stage
-    static constexpr uint32_t N = 16 * NTW, A = 0, X = G_ROWS * KqBlock<FMT>::PITCH, D = X + N * KqBlock<FMT>::XP, DIG = D + N * 4,
+    static constexpr uint32_t ROWS = 32 * WM, N = 8 * NTW * WN, THREADS = 32 * WM * WN, X = ROWS * KqBlock<FMT>::PITCH, D = X + N * KqBlock<FMT>::XP, DIG = D + N * 4,
                               BYTES = (DIG + N * KqBlock<FMT>::DG + 127) & ~127u;
 };
 
@@ -53,49 +51,37 @@ __device__ __forceinline__ void cp4z(uint32_t dst, const void* src, uint32_t n) 
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void mma0_u8s8_k32(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 __device__ __forceinline__ void mma0_u8s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+    asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                  : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
-__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
-
-// Signed base-64 digits (v = 64 hi + lo) of a token's activation sums: K4 the 8 sums of 32 (lo 0..7 | hi 8..15), Q6_K the 16 sums of 16.
-template <int FMT>
-__device__ __forceinline__ void store_digits(uint32_t at, const uint4& s0, const uint4& s1) {
-    const uint32_t w[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-    constexpr int NV = FMT == 6 ? 16 : 8;
-    uint32_t lo[NV / 4] = {}, hi[NV / 4] = {};
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        int v;
-        if (FMT == 6) v = (int)(int16_t)(i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu);
-        else v = (int)(int16_t)(w[i] & 0xffffu) + (int)(int16_t)(w[i] >> 16);
-        const int l = ((v + 32) & 63) - 32, h = (v - l) >> 6;
-        lo[i >> 2] |= (uint32_t)(l & 0xff) << (8 * (i & 3));
-        hi[i >> 2] |= (uint32_t)(h & 0xff) << (8 * (i & 3));
-    }
-#pragma unroll
-    for (int i = 0; i < NV / 4; i++) { sts32(at + 4 * i, lo[i]); sts32(at + NV + 4 * i, hi[i]); }
+// Plain loads: the products are no volatile assembly here either, so the compiler may bring operands in ahead of earlier products.
+template <class V> __device__ __forceinline__ V ld(const uint8_t* p) { return *reinterpret_cast<const V*>(p); }
+__device__ __forceinline__ uint32_t ld_u2(const uint8_t* p) {      // a 32-bit word at a 2-byte boundary
+    const uint32_t a = smem_u32(p) & 2u;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - a);
+    return __funnelshift_r(q[0], q[1], a * 8u);
 }
 
-template <int FMT, int NTW, bool SW>
-__global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_constant__ KqGemmArgs a, const uint32_t KS) {
+template <int FMT, int WM, int WN, int NTW, bool SW>
+__global__ void __launch_bounds__(32 * WM * WN, 2) kq_gemm_kernel(const __grid_constant__ KqGemmArgs a, const uint32_t KS) {
     extern __shared__ __align__(128) uint8_t smem[];
     using B = KqBlock<FMT>;
-    using St = KqStage<FMT, NTW>;
-    constexpr uint32_t N = St::N;
+    using St = KqStage<FMT, WM, WN, NTW>;
+    constexpr uint32_t N = St::N, G_ROWS = St::ROWS, G_THREADS = St::THREADS;
+    static_assert(N <= G_THREADS, "a thread per token prepares the activation sums");
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
-    const uint32_t wm = warp & 1, wn = warp >> 1;
+    const uint32_t wm = warp % WM, wn = warp / WM;
     const uint32_t rank = KS > 1 ? blockIdx.x % KS : 0u, tile = blockIdx.x / KS, tok0 = blockIdx.y * N;
     const uint32_t ring = smem_u32(smem);
     uint32_t s = 0;
     if (!SW) while (s + 1 < a.nw && tile >= a.tile0[s + 1]) s++;
-    const uint32_t seg_rows = a.rows[s], r0 = (tile - a.tile0[s]) * (SW ? 32u : 64u);
+    const uint32_t seg_rows = a.rows[s], r0 = (tile - a.tile0[s]) * (SW ? G_ROWS / 2 : G_ROWS);
     const uint64_t total = (uint64_t)seg_rows * a.row_bytes;
     const uint32_t b_lo = a.nb * rank / KS, nblk = a.nb * (rank + 1) / KS - b_lo;
     pdl_launch_dependents();
@@ -139,7 +125,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
     float acc[2][NTW][4] = {};
     for (uint32_t k = 0; k < nblk; k++) {
         const uint32_t st = ring + (k % a.stages) * St::BYTES, blk = b_lo + k;
-        if (tid < N) store_digits<FMT>(st + St::DIG + tid * B::DG, s0, s1);
+        if (tid < N) kq_store_digits<FMT == 6>(st + St::DIG + tid * B::DG, s0, s1);
         sums(k + 1);
         if (a.stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
         else asm volatile("cp.async.wait_group 1;" ::: "memory");      // 3 stages: one younger group may be in flight
@@ -148,31 +134,29 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
         asm volatile("cp.async.commit_group;" ::: "memory");
 
         int tot[2][NTW][4] = {};
-        uint32_t p[2][2];      // rows g and g + 8 of both 16-row tiles
+        const uint8_t* const sp = smem + (k % a.stages) * St::BYTES;
+        const uint8_t* p[2][2];      // rows g and g + 8 of both 16-row tiles
 #pragma unroll
         for (int m = 0; m < 2; m++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const uint32_t r = wm * 32 + m * 16 + h * 8 + g;
-                p[m][h] = st + r * B::PITCH;
+                p[m][h] = sp + r * B::PITCH;
                 if (FMT == 6) p[m][h] += ((uint32_t)min(stage_row(r), seg_rows - 1) * a.row_bytes + blk * B::BB) & 15u;
             }
-        const uint32_t xa = st + St::X + (wn * NTW * 8 + g) * B::XP;
-        const uint32_t dg = st + St::DIG + (wn * NTW * 8 + g) * B::DG;
+        const uint8_t* const xa = sp + St::X + (wn * NTW * 8 + g) * B::XP;
+        const uint8_t* const dg = sp + St::DIG + (wn * NTW * 8 + g) * B::DG;
         if constexpr (FMT != 6) {
             constexpr uint32_t LO = 0x0f0f0f0fu, QS = FMT == 5 ? 48u : 16u;
-            uint32_t sc[2][2][2], mn[2][2][2], dm[2][2];     // [tile][row half][sub-blocks 0..3 / 4..7]
-            uint2 qh[2][2];
+            uint32_t sc[2][2][2];                            // [tile][row half]: scales of the sub-blocks to come, two a step
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const uint4 hd = lds128(p[m][h]);
-                    dm[m][h] = hd.x;
-                    k4_unpack(hd, sc[m][h][0], sc[m][h][1], mn[m][h][0], mn[m][h][1]);
-                    if (FMT == 5) qh[m][h] = lds64(p[m][h] + 16 + 8 * t);
+                    uint32_t mn_lo, mn_hi;
+                    k4_unpack(ld<uint4>(p[m][h]), sc[m][h][0], sc[m][h][1], mn_lo, mn_hi);
                 }
-#pragma unroll
+#pragma unroll 1                                                // unrolled it needs more than the 128 registers two CTAs leave
             for (int j = 0; j < 4; j++) {
                 uint32_t lo[2][4], hi[2][4];
                 int w0[2][2], w1[2][2];
@@ -180,20 +164,22 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
                 for (int m = 0; m < 2; m++)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const uint2 w = lds64(p[m][h] + QS + 32 * j + 8 * t);
+                        const uint2 w = ld<uint2>(p[m][h] + QS + 32 * j + 8 * t);
                         lo[m][h] = w.x & LO; lo[m][2 + h] = w.y & LO;
                         hi[m][h] = (w.x >> 4) & LO; hi[m][2 + h] = (w.y >> 4) & LO;
                         if (FMT == 5) {
-                            constexpr uint32_t B0 = 0x01010101u;
-                            lo[m][h] |= ((qh[m][h].x >> (2 * j)) & B0) << 4; lo[m][2 + h] |= ((qh[m][h].y >> (2 * j)) & B0) << 4;
-                            hi[m][h] |= ((qh[m][h].x >> (2 * j + 1)) & B0) << 4; hi[m][2 + h] |= ((qh[m][h].y >> (2 * j + 1)) & B0) << 4;
+                            constexpr uint32_t H4 = 0x10101010u;
+                            const uint2 qh = ld<uint2>(p[m][h] + 16 + 8 * t);
+                            const uint32_t x = __funnelshift_l(qh.x, qh.x, 4 - 2 * j), y = __funnelshift_l(qh.y, qh.y, 4 - 2 * j);   // bit 2 j of each byte to bit 4
+                            lo[m][h] |= x & H4; lo[m][2 + h] |= y & H4;
+                            hi[m][h] |= (x >> 1) & H4; hi[m][2 + h] |= (y >> 1) & H4;
                         }
-                        const uint32_t ws = sc[m][h][j >> 1] >> (16 * (j & 1));
-                        w0[m][h] = (int)(ws & 0xffu); w1[m][h] = (int)((ws >> 8) & 0xffu);
+                        w0[m][h] = (int)(sc[m][h][0] & 0xffu); w1[m][h] = (int)((sc[m][h][0] >> 8) & 0xffu);
+                        sc[m][h][0] = __funnelshift_r(sc[m][h][0], sc[m][h][1], 16); sc[m][h][1] >>= 16;
                     }
 #pragma unroll
                 for (int n = 0; n < NTW; n++) {
-                    const uint2 xl = lds64(xa + n * 8 * B::XP + 64 * j + 8 * t), xh = lds64(xa + n * 8 * B::XP + 64 * j + 32 + 8 * t);
+                    const uint2 xl = ld<uint2>(xa + n * 8 * B::XP + 64 * j + 8 * t), xh = ld<uint2>(xa + n * 8 * B::XP + 64 * j + 32 + 8 * t);
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         int c0[4], c1[4];
@@ -205,13 +191,18 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
                 }
             }
 #pragma unroll
-            for (int n = 0; n < NTW; n++) {
-                const uint32_t bl = t < 2 ? lds32(dg + n * 8 * B::DG + 4 * t) : 0u, bh = t < 2 ? lds32(dg + n * 8 * B::DG + 8 + 4 * t) : 0u;
-                const uint2 d8 = lds64(st + St::D + (wn * NTW * 8 + n * 8 + 2 * t) * 4);
-                const float e0 = __uint_as_float(d8.x), e1 = __uint_as_float(d8.y);
+            for (int m = 0; m < 2; m++) {
+                const uint4 hA = ld<uint4>(p[m][0]), hB = ld<uint4>(p[m][1]);
+                uint32_t u0, u1, mA[2], mB[2];
+                k4_unpack(hA, u0, u1, mA[0], mA[1]);
+                k4_unpack(hB, u0, u1, mB[0], mB[1]);
+                const uint32_t a0 = t == 0 ? mA[0] : t == 1 ? mA[1] : 0u, a1 = t == 0 ? mB[0] : t == 1 ? mB[1] : 0u;
+                const float2 fA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), fB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
 #pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    const uint32_t a0 = t == 0 ? mn[m][0][0] : t == 1 ? mn[m][0][1] : 0u, a1 = t == 0 ? mn[m][1][0] : t == 1 ? mn[m][1][1] : 0u;
+                for (int n = 0; n < NTW; n++) {
+                    const uint32_t bl = t < 2 ? ld<uint32_t>(dg + n * 8 * B::DG + 4 * t) : 0u, bh = t < 2 ? ld<uint32_t>(dg + n * 8 * B::DG + 8 + 4 * t) : 0u;
+                    const float2 d8 = ld<float2>(sp + St::D + (wn * NTW * 8 + n * 8 + 2 * t) * 4);
+                    const float e0 = d8.x, e1 = d8.y;
                     int sm[4];
                     mma0_u8s8_k16(sm, a0, a1, bh);
 #pragma unroll
@@ -219,7 +210,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
                     mma_u8s8_k16(sm, a0, a1, bl);
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&dm[m][i >> 1]));
+                        const float2 f = i >> 1 ? fB : fA;
                         const float e = i & 1 ? e1 : e0;
                         acc[m][n][i] += (f.x * e) * (float)tot[m][n][i] - (f.y * e) * (float)sm[i];
                     }
@@ -227,9 +218,9 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
             }
         } else {
             constexpr uint32_t LO = 0x0f0f0f0fu, H2 = 0x30303030u;
-#pragma unroll
+#pragma unroll 1
             for (int n2 = 0; n2 < 2; n2++)
-#pragma unroll
+#pragma unroll 1
                 for (int i2 = 0; i2 < 2; i2++) {
                     uint32_t q[2][2][4], sc[2][2][2];     // [tile][row half][quadrant]; scales of quadrants 0, 1 / 2, 3 in bytes 0 and 2
                     const uint32_t o = 16 * i2 + 4 * t;
@@ -237,18 +228,18 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
                     for (int m = 0; m < 2; m++)
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
-                            const uint32_t b = p[m][h];
-                            const uint32_t l0 = lds32_u2(b + 64 * n2 + o), l1 = lds32_u2(b + 64 * n2 + 32 + o), hb = lds32_u2(b + 128 + 32 * n2 + o);
+                            const uint8_t* const b = p[m][h];
+                            const uint32_t l0 = ld_u2(b + 64 * n2 + o), l1 = ld_u2(b + 64 * n2 + 32 + o), hb = ld_u2(b + 128 + 32 * n2 + o);
                             q[m][h][0] = (l0 & LO) | ((hb << 4) & H2); q[m][h][1] = (l1 & LO) | ((hb << 2) & H2);
                             q[m][h][2] = ((l0 >> 4) & LO) | (hb & H2); q[m][h][3] = ((l1 >> 4) & LO) | ((hb >> 2) & H2);
-                            sc[m][h][0] = lds32_u2(b + 192 + 8 * n2) >> (8 * i2);
-                            sc[m][h][1] = lds32_u2(b + 196 + 8 * n2) >> (8 * i2);
+                            sc[m][h][0] = ld_u2(b + 192 + 8 * n2) >> (8 * i2);
+                            sc[m][h][1] = ld_u2(b + 196 + 8 * n2) >> (8 * i2);
                         }
 #pragma unroll
                     for (int z = 0; z < 4; z++)
 #pragma unroll
                         for (int n = 0; n < NTW; n++) {
-                            const uint32_t bx = lds32(xa + n * 8 * B::XP + 128 * n2 + 32 * z + 16 * i2 + 4 * t);
+                            const uint32_t bx = ld<uint32_t>(xa + n * 8 * B::XP + 128 * n2 + 32 * z + 16 * i2 + 4 * t);
 #pragma unroll
                             for (int m = 0; m < 2; m++) {
                                 int c[4];
@@ -263,12 +254,12 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
-                for (int h = 0; h < 2; h++) { as[m][h] = lds32_u2(p[m][h] + 192 + 4 * t); d[m][h] = f16_bits_to_f32(lds16(p[m][h] + 208)); }
+                for (int h = 0; h < 2; h++) { as[m][h] = ld_u2(p[m][h] + 192 + 4 * t); d[m][h] = f16_bits_to_f32(ld<uint16_t>(p[m][h] + 208)); }
 #pragma unroll
             for (int n = 0; n < NTW; n++) {
-                const uint32_t bl = lds32(dg + n * 8 * B::DG + 4 * t), bh = lds32(dg + n * 8 * B::DG + 16 + 4 * t);
-                const uint2 d8 = lds64(st + St::D + (wn * NTW * 8 + n * 8 + 2 * t) * 4);
-                const float e0 = __uint_as_float(d8.x), e1 = __uint_as_float(d8.y);
+                const uint32_t bl = ld<uint32_t>(dg + n * 8 * B::DG + 4 * t), bh = ld<uint32_t>(dg + n * 8 * B::DG + 16 + 4 * t);
+                const float2 d8 = ld<float2>(sp + St::D + (wn * NTW * 8 + n * 8 + 2 * t) * 4);
+                const float e0 = d8.x, e1 = d8.y;
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     int bias[4] = {0, 0, 0, 0};
@@ -304,7 +295,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
             }
         return;
     }
-    // every CTA leaves its part [token][64 rows] in shared memory; the outputs are dealt to the CTAs, parts added in rank order
+    // every CTA leaves its part [token][rows] in shared memory; the outputs are dealt to the CTAs, parts added in rank order
     __syncthreads();
     float* part = reinterpret_cast<float*>(smem);
     constexpr uint32_t PP = G_ROWS + 1;
@@ -328,7 +319,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
         }
         return f;
     };
-    constexpr uint32_t OUT = SW ? 32u : 64u;      // output rows of the tile
+    constexpr uint32_t OUT = SW ? G_ROWS / 2 : G_ROWS;      // output rows of the tile
     for (uint32_t i = rank * G_THREADS + tid; i < N * OUT; i += KS * G_THREADS) {
         const uint32_t v = i / OUT, r = i % OUT;
         if (SW) {
@@ -342,26 +333,29 @@ __global__ void __launch_bounds__(G_THREADS, 2) kq_gemm_kernel(const __grid_cons
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int FMT, int NTW, bool SW>
+template <int FMT, int WM, int WN, int NTW, bool SW>
 int launch_one(KqGemmArgs a, const LaunchCfg& cfg) {
     static bool done[64] = {};
-    using St = KqStage<FMT, NTW>;
-    auto kern = kq_gemm_kernel<FMT, NTW, SW>;
-    a.stages = NTW <= 4 ? 3 : 2;
+    using St = KqStage<FMT, WM, WN, NTW>;
+    auto kern = kq_gemm_kernel<FMT, WM, WN, NTW, SW>;
+    a.stages = 3 * St::BYTES <= 112 * 1024 ? 3 : 2;
     const size_t smem = (size_t)a.stages * St::BYTES;
-    static_assert(2 * St::BYTES >= St::N * (G_ROWS + 1) * 4, "the parts of a split reuse the stages");
+    static_assert(2 * St::BYTES <= 112 * 1024, "two CTAs an SM");
+    static_assert(2 * St::BYTES >= St::N * (St::ROWS + 1) * 4, "the parts of a split reuse the stages");
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return ALICE_E_CUDA;
     if (dev >= 64 || !done[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return ALICE_E_CUDA;
         if (dev < 64) done[dev] = true;
     }
+    constexpr uint32_t per = SW ? St::ROWS / 2 : St::ROWS;
+    for (uint32_t i = 0; i < a.nw; i++) a.tile0[i + 1] = a.tile0[i] + (a.rows[i] + per - 1) / per;
     const uint32_t tiles = a.tile0[a.nw], toks = (a.batch + St::N - 1) / St::N, slots = 2 * (uint32_t)std::max(cfg.num_sms, 1);
     // columns shared by a cluster while that fills the two CTAs an SM holds and leaves each at least four blocks
     uint32_t KS = 1;
     while (KS < 8 && tiles * toks * KS * 2 <= slots && a.nb >= 8 * KS) KS *= 2;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(tiles * KS, toks); lc.blockDim = dim3(G_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
+    lc.gridDim = dim3(tiles * KS, toks); lc.blockDim = dim3(St::THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = KS; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -373,10 +367,10 @@ int launch_one(KqGemmArgs a, const LaunchCfg& cfg) {
 }
 template <int FMT, bool SW>
 int launch_n(const KqGemmArgs& a, const LaunchCfg& cfg) {
-    if (a.batch <= 16) return launch_one<FMT, 1, SW>(a, cfg);
-    if (a.batch <= 32) return launch_one<FMT, 2, SW>(a, cfg);
-    if (a.batch <= 64) return launch_one<FMT, 4, SW>(a, cfg);
-    return launch_one<FMT, 8, SW>(a, cfg);
+    if (a.batch <= 16) return launch_one<FMT, 4, 1, 2, SW>(a, cfg);
+    if (a.batch <= 32) return launch_one<FMT, 4, 1, 4, SW>(a, cfg);
+    if (a.batch <= 64) return launch_one<FMT, 2, 2, 4, SW>(a, cfg);
+    return launch_one<FMT, 2, 4, 4, SW>(a, cfg);
 }
 template <int FMT>
 int launch_fmt(const KqGemmArgs& a, const LaunchCfg& cfg) { return a.up ? launch_n<FMT, true>(a, cfg) : launch_n<FMT, false>(a, cfg); }
@@ -395,8 +389,6 @@ int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
         const WeightDesc* w = op.w[i];
         if (!w || !w->rows || !w->data || ((uintptr_t)w->data & 15) || w->fmt != w0.fmt || w->cols != w0.cols || w->row_bytes != w0.row_bytes) return ALICE_E_SHAPE;
         a.w[i] = w->data; a.rows[i] = w->rows; a.y_off[i] = op.y_off[i];
-        const uint32_t per = op.up ? 32 : 64;
-        a.tile0[i + 1] = a.tile0[i] + (w->rows + per - 1) / per;
         total += w->rows;
     }
     if (op.up) {

@@ -79,6 +79,26 @@ static __device__ __noinline__ void kq_stage_acts(const StreamArgs& a, uint8_t* 
     asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
 }
 
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+// Signed base-64 digits (v = 64 hi + lo) of a token's activation sums: K4 the 8 sums of 32 (lo 0..7 | hi 8..15), Q6_K the 16 sums of 16.
+template <bool Q6>
+__device__ __forceinline__ void kq_store_digits(uint32_t at, const uint4& s0, const uint4& s1) {
+    const uint32_t w[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    constexpr int NV = Q6 ? 16 : 8;
+    uint32_t lo[NV / 4] = {}, hi[NV / 4] = {};
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        int v;
+        if (Q6) v = (int)(int16_t)(i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu);
+        else v = (int)(int16_t)(w[i] & 0xffffu) + (int)(int16_t)(w[i] >> 16);
+        const int l = ((v + 32) & 63) - 32, h = (v - l) >> 6;
+        lo[i >> 2] |= (uint32_t)(l & 0xff) << (8 * (i & 3));
+        hi[i >> 2] |= (uint32_t)(h & 0xff) << (8 * (i & 3));
+    }
+#pragma unroll
+    for (int i = 0; i < NV / 4; i++) { sts32(at + 4 * i, lo[i]); sts32(at + NV + 4 * i, hi[i]); }
+}
+
 // 6-bit scales (sc) and mins (m) of a K4 header as four words of four bytes each: sub-blocks 0..3 and 4..7
 // (get_scale_min_k4, src/gguf.rs:794-802).
 __device__ __forceinline__ void k4_unpack(const uint4& h, uint32_t& sc_lo, uint32_t& sc_hi, uint32_t& m_lo, uint32_t& m_hi) {
