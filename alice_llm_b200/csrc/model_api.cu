@@ -1,5 +1,6 @@
 // The alice_model_* entry points that are the same for every model family (include/alice_cuda.h): stepping, greedy decoding
 // from a captured graph, logits, position. GpuModel of ALICE-LLM src/gpu.rs:5010-6094.
+#include <cstring>
 #include <vector>
 
 #include "model_base.cuh"
@@ -12,16 +13,30 @@ int check_room(const alice_model* m, uint32_t steps, const char* who) {
     return ALICE_OK;
 }
 
+// A few words of the caller's, taken over before the call returns: a copy from pageable memory (which `own` is, whatever the caller's
+// memory is) has left it by then, so the stream need not be waited for (about 10 us a token).
+int to_device(alice_model* m, int* dst, const uint32_t* src, uint32_t n) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    MCU(cudaStreamIsCapturing(m->e->stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return alice_cuda_fail(cudaErrorStreamCaptureUnsupported, "alice_model: tokens and positions of a captured stream");
+    const std::vector<uint32_t> own(src, src + n);
+    MCU(cudaMemcpyAsync(dst, own.data(), (size_t)4 * n, cudaMemcpyHostToDevice, m->e->stream));
+    return ALICE_OK;
+}
+
 int set_tokens(alice_model* m, const uint32_t* tokens, uint32_t n) {
     for (uint32_t k = 0; k < n; k++)
         if (tokens[k] >= m->vocab) return alice_fail(ALICE_E_INVALID, "alice_model: token %u >= vocab %u", tokens[k], m->vocab);
     static_assert(sizeof(uint32_t) == sizeof(int), "tokens are copied as 32-bit words");
-    MCU(cudaMemcpyAsync(m->d_token, tokens, (size_t)4 * n, cudaMemcpyHostToDevice, m->e->stream));
-    MCU(cudaStreamSynchronize(m->e->stream));  // the caller's array is only borrowed
-    return ALICE_OK;
+    return to_device(m, m->d_token, tokens, n);
 }
 
 }  // namespace
+
+int alice_model::make_stage() {
+    MCU(cudaMallocHost(&stage, (size_t)STAGE_ROWS * vocab * 4));
+    return ALICE_OK;
+}
 
 extern "C" {
 
@@ -33,6 +48,7 @@ int32_t alice_model_destroy(alice_model* m) {
     if (m->graph_greedy) cudaGraphExecDestroy(m->graph_greedy);
     std::vector<void*> owned;
     owned.swap(m->owned);
+    if (m->stage) cudaFreeHost(m->stage);
     delete m;
     for (void* p : owned) cudaFree(p);
     alice_engine_release(e);
@@ -70,19 +86,22 @@ int32_t alice_model_forward_rows(alice_model* m, const uint32_t* tokens, uint32_
     MCU(cudaSetDevice(m->e->device));
     int rc = check_room(m, n, who);
     uint32_t done = 0;
+    float* const to = nrows <= alice_model::STAGE_ROWS ? m->stage : logits;
     std::vector<uint32_t> local;
     for (uint32_t lo = 0; lo < n && !rc;) {
         const uint32_t k = std::min(m->piece_tokens(), n - lo);
         local.clear();
         while (done + local.size() < nrows && rows[done + local.size()] < lo + k) local.push_back(rows[done + local.size()] - lo);
         rc = set_tokens(m, tokens + lo, k);
-        if (!rc) rc = m->enqueue_rows(k, local.data(), (uint32_t)local.size(), logits + (size_t)done * m->vocab);
+        if (!rc) rc = m->enqueue_rows(k, local.data(), (uint32_t)local.size(), to + (size_t)done * m->vocab);
         if (!rc) m->pos += k;
         done += (uint32_t)local.size();
         lo += k;
     }
     if (rc) return rc;
-    return alice_sync(m->e);
+    rc = alice_sync(m->e);
+    if (to != logits && nrows) memcpy(logits, to, (size_t)nrows * m->vocab * 4);
+    return rc;
 }
 
 int32_t alice_model_forward_batch_read(alice_model* m, const uint32_t* tokens, uint32_t n, float* logits) {
@@ -96,9 +115,10 @@ int32_t alice_model_forward_batch_read(alice_model* m, const uint32_t* tokens, u
 
 int32_t alice_model_read_logits(alice_model* m, float* logits) {
     if (!m || !logits) return alice_fail(ALICE_E_INVALID, "alice_model_read_logits: null argument");
-    MCU(cudaMemcpyAsync(logits, m->logits, (size_t)m->vocab * 4, cudaMemcpyDeviceToHost, m->e->stream));
-    MCU(cudaStreamSynchronize(m->e->stream));
-    return alice_sync(m->e);
+    MCU(cudaMemcpyAsync(m->stage, m->logits, (size_t)m->vocab * 4, cudaMemcpyDeviceToHost, m->e->stream));
+    const int rc = alice_sync(m->e);
+    memcpy(logits, m->stage, (size_t)m->vocab * 4);
+    return rc;
 }
 
 int32_t alice_model_forward_read(alice_model* m, uint32_t token, float* logits) {
@@ -166,10 +186,9 @@ int32_t alice_model_set_position(alice_model* m, uint32_t pos) {
     if (pos > m->max_seq) return alice_fail(ALICE_E_SHAPE, "alice_model_set_position: %u > max_seq_len %u", pos, m->max_seq);
     if (!m->can_return_to(pos))
         return alice_fail(ALICE_E_UNSUPPORTED, "alice_model_set_position: the recurrent state of position %u is not kept (only reset and the present position %u can be had)", pos, m->pos);
-    const int p = (int)pos;
     MCU(cudaSetDevice(m->e->device));
-    MCU(cudaMemcpyAsync(m->d_pos, &p, 4, cudaMemcpyHostToDevice, m->e->stream));
-    MCU(cudaStreamSynchronize(m->e->stream));
+    const int rc = to_device(m, m->d_pos, &pos, 1);
+    if (rc) return rc;
     m->pos = pos;
     return ALICE_OK;
 }
