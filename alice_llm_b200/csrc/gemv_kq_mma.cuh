@@ -1,4 +1,5 @@
-// Batched (2..8 input vectors) fused dequantize + matvec for the K-quant formats on the int8 tensor cores.
+// 16-row tiles of K-quant weights times up to eight Q8_K vectors on the int8 tensor cores (csrc/gemv_kq_rows.cu, and the digits of
+// the activation sums for csrc/gemm_kq.cu).
 //
 // The speculative-verify step feeds 4..8 tokens through every projection. The weights are streamed and unpacked ONCE:
 // a warp owns a tile of 16 rows (mma M), the unpacked 4/5/6-bit quants of a 32-element sub-block are the A operand
@@ -8,13 +9,8 @@
 // min term sum_is m[is] * bsum[is] is one more pair of small MMAs (A = the 6-bit mins, B = the sub-block sums of the
 // activations split into two signed base-64 digits). The reference does the same on the GPU with
 // dequant_matvec_q4k_batch4.wgsl / swiglu_fused_q4k_batch4.wgsl (weights decoded once for 4 inputs, in f32).
-//
-// Same producer / ring / partial-sum machinery as the batch-1 kernels, with row-wise staging: the shared-memory row
-// stride is padded to 32 mod 128 bytes so the 64-bit A loads of a half warp (4 rows x 4 column slices) hit 16 different
-// bank pairs. The activations of all vectors sit in shared memory too (row stride cols + 32 for the same reason).
 #pragma once
 #include "gemv_mma.cuh"
-#include "gemv_stream.cuh"
 
 namespace alice {
 
@@ -26,57 +22,10 @@ struct KqActs {
     uint32_t bs16;    // shared address of s8 [8][nb][32]: base-64 digits of the 16 sub-block (16-element) sums, low 0..15, high 16..31 (Q6_K)
     uint32_t nb;
 };
-__host__ __device__ constexpr uint32_t kq_acts_bytes(uint32_t cols) {
-    return ((8u * (cols + 32u) + 127u) & ~127u) + ((8u * (cols / 256u) * 4u + 127u) & ~127u) + ((8u * (cols / 256u) * 16u + 127u) & ~127u) +
-           ((8u * (cols / 256u) * 32u + 127u) & ~127u);
-}
-
 __device__ __forceinline__ void mma_s8s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(a1), "r"(b0));
-}
-
-// Brings the Q8_K blocks of the `batch` input vectors (global memory, prepared by an earlier kernel) into shared memory
-// in the layout above; columns past `batch` are zero. Run by the NCW consumer warps.
-static __device__ __noinline__ void kq_stage_acts(const StreamArgs& a, uint8_t* area, KqActs& x) {
-    const uint32_t tid = threadIdx.x, nb = a.cols / QK_K, cols = a.cols, B = a.batch;
-    const uint32_t vs = a.x_stride, vnb = a.x_stride / QK_K;   // strides between input vectors in global memory
-    const uint32_t xs = cols + 32u;
-    uint8_t* qs = area;
-    float* d = reinterpret_cast<float*>(area + ((8u * xs + 127u) & ~127u));
-    int8_t* bsd = reinterpret_cast<int8_t*>(reinterpret_cast<uint8_t*>(d) + ((8u * nb * 4u + 127u) & ~127u));
-    int8_t* bs16 = bsd + ((8u * nb * 16u + 127u) & ~127u);
-    for (uint32_t i = tid; i < 8u * (cols / 16u); i += NCW * 32) {
-        const uint32_t c = i / (cols / 16u), j = i % (cols / 16u);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (c < B) v = *reinterpret_cast<const uint4*>(a.q8.qs + (size_t)c * vs + (size_t)j * 16);
-        *reinterpret_cast<uint4*>(qs + (size_t)c * xs + (size_t)j * 16) = v;
-    }
-    for (uint32_t i = tid; i < 8u * nb; i += NCW * 32) {
-        const uint32_t c = i / nb, b = i % nb;
-        d[i] = c < B ? a.q8.d[(size_t)c * vnb + b] : 0.0f;
-    }
-    for (uint32_t i = tid; i < 8u * nb * 16u; i += NCW * 32) {
-        const uint32_t c = i / (nb * 16u), r = i % (nb * 16u), b = r / 16u, is = r % 16u;
-        int v16 = 0, v32 = 0;
-        if (c < B) {
-            const int16_t* bs = a.q8.bsums + ((size_t)c * vnb + b) * 16;
-            v16 = bs[is];
-            if (is < 8) v32 = (int)bs[2 * is] + (int)bs[2 * is + 1];
-        }
-        // signed base-64 digits: v = 64 * hi + lo, lo in [-32, 31]
-        const int lo16 = ((v16 + 32) & 63) - 32, hi16 = (v16 - lo16) >> 6;
-        bs16[((size_t)c * nb + b) * 32 + is] = (int8_t)lo16;
-        bs16[((size_t)c * nb + b) * 32 + 16 + is] = (int8_t)hi16;
-        if (is < 8) {
-            const int lo = ((v32 + 32) & 63) - 32, hi = (v32 - lo) >> 6;
-            bsd[((size_t)c * nb + b) * 16 + is] = (int8_t)lo;
-            bsd[((size_t)c * nb + b) * 16 + 8 + is] = (int8_t)hi;
-        }
-    }
-    x.qs = smem_u32(qs); x.xs = xs; x.d = smem_u32(d); x.bsd = smem_u32(bsd); x.bs16 = smem_u32(bs16); x.nb = nb;
-    asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
 }
 
 __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
@@ -229,116 +178,5 @@ struct KqQ6K {
         }
     }
 };
-
-// Shared-memory area for the partial sums of the P warps of a tile: [stage][warp][16 rows][8 vectors][gate | up]
-struct KqPartials { float v[2][NCW][16][8][2]; };
-
-// Consumer side (the NCW consumer warps). A stage holds slots * 16 rows; warp `part` of a tile covers blocks
-// [nb * part / P, nb * (part + 1) / P) of every row of its tile. Returns false after an abort.
-template <class T, bool SWIGLU>
-__device__ __forceinline__ bool stream_consume_kq(const StreamArgs& a, StreamCtx& cx, KqPartials* pp, uint8_t* act_area) {
-    StreamSmem* sm = cx.sm;
-    volatile int* abort_flag = &sm->abort_flag;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t P = a.P, slots = a.slots, rps = a.rps;   // rps == 16
-    const uint32_t rows_per_group = slots * rps;
-    const uint32_t slot = warp / P, part = warp % P;
-    KqActs x;
-    kq_stage_acts(a, act_area, x);
-    const uint32_t nb = a.cols / QK_K;                          // blocks of the (sub-)row this launch covers
-    const uint32_t b_lo = nb * part / P, b_hi = nb * (part + 1) / P;
-    const uint32_t t = lane & 3u, gid = lane >> 2;
-
-    const uint32_t g0 = (uint32_t)(((uint64_t)a.groups * blockIdx.x) / gridDim.x);
-    const uint32_t g1 = (uint32_t)(((uint64_t)a.groups * (blockIdx.x + 1)) / gridDim.x);
-    for (uint32_t g = g0; g < g1; g++) {
-        const uint32_t s = cx.cc % cx.nstages, ph = (cx.cc / cx.nstages) & 1;
-        cx.cc++;
-        uint32_t sg = 0;
-        while (sg + 1 < a.nseg && g >= a.seg_g0[sg + 1]) sg++;
-        const uint32_t seg_rows = a.seg_rows[sg];
-        const uint32_t r0 = (g - a.seg_g0[sg]) * rows_per_group;
-        const uint32_t set0 = slot * rps;
-        const uint32_t nrow = r0 + set0 < seg_rows ? min(rps, seg_rows - r0 - set0) : 0;
-        if (!wait_or_abort(smem_u32(&sm->full[s]), ph, abort_flag, a.status, KERR_WAIT_FULL, cx.limit)) return false;
-        const uint32_t sb = cx.ring + s * cx.stage_stride + set0 * a.row_stride;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
-        if (nrow > 0) {
-            // rows past nrow of a short last tile read whatever the stage holds; their results are never stored
-            const uint32_t rowA = sb + gid * a.row_stride + a.row_pad, rowB = sb + (gid + 8) * a.row_stride + a.row_pad;
-            T::tile(rowA, rowB, b_lo, b_hi, x, lane, acc);
-            if (SWIGLU) T::tile(rowA + a.cap, rowB + a.cap, b_lo, b_hi, x, lane, up);
-            if (P > 1) {
-                float (*pv)[8][2] = pp->v[s & 1][warp];
-                pv[gid][2 * t][0] = acc[0]; pv[gid][2 * t + 1][0] = acc[1]; pv[gid + 8][2 * t][0] = acc[2]; pv[gid + 8][2 * t + 1][0] = acc[3];
-                if (SWIGLU) { pv[gid][2 * t][1] = up[0]; pv[gid][2 * t + 1][1] = up[1]; pv[gid + 8][2 * t][1] = up[2]; pv[gid + 8][2 * t + 1][1] = up[3]; }
-            }
-        }
-        __syncwarp();
-        {
-            const uint32_t own0 = warp * rps;
-            const bool used = P > 1 && warp < slots && r0 + own0 < seg_rows;
-            if (!used && lane == 0) mbar_arrive_n(smem_u32(&sm->red[s][warp]), RED_COUNT);
-        }
-        if (nrow > 0) {
-            if (part != 0) {
-                if (lane == 0) mbar_arrive_n(smem_u32(&sm->red[s][slot]), RED_COUNT / (P - 1));
-            } else {
-                if (P > 1 && !wait_or_abort(smem_u32(&sm->red[s][slot]), ph, abort_flag, a.status, KERR_WAIT_PARTIALS, cx.limit)) return false;
-                if (P > 1) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) { acc[i] = 0.f; up[i] = 0.f; }
-                    for (uint32_t p = 0; p < P; p++) {
-                        float (*pv)[8][2] = pp->v[s & 1][warp + p];
-                        acc[0] += pv[gid][2 * t][0]; acc[1] += pv[gid][2 * t + 1][0]; acc[2] += pv[gid + 8][2 * t][0]; acc[3] += pv[gid + 8][2 * t + 1][0];
-                        if (SWIGLU) { up[0] += pv[gid][2 * t][1]; up[1] += pv[gid][2 * t + 1][1]; up[2] += pv[gid + 8][2 * t][1]; up[3] += pv[gid + 8][2 * t + 1][1]; }
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->empty[s]));
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const uint32_t rr = gid + 8 * (i >> 1), k = 2 * t + (i & 1);
-                    if (rr < nrow && k < a.batch) {
-                        float r = acc[i];
-                        if (SWIGLU) r = silu_ref(r) * up[i];
-                        const size_t yi = (size_t)k * a.y_stride + a.seg_y[sg] + r0 + set0 + rr;
-                        if (a.resid != nullptr) r = __fadd_rn(__ldcg(a.resid + yi), r);
-                        a.y[yi] = r;
-                    }
-                }
-                continue;   // this warp has already released the stage
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->empty[s]));
-    }
-    return true;
-}
-
-// The partial-sum area is double buffered by stage parity: a finalizer has read stage s before the producer may refill
-// it (it arrives on `empty` after reading), and the helpers write their partials of the next use of the same parity only
-// after that stage has landed again.
-template <class T, bool SWIGLU, int CTAS>
-__global__ void __launch_bounds__(STREAM_THREADS, CTAS) stream_gemv_kq_kernel(const __grid_constant__ StreamArgs a) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    StreamSmem* sm = reinterpret_cast<StreamSmem*>(smem_raw);
-    constexpr uint32_t HDR = (sizeof(StreamSmem) + 127) & ~127u;
-    constexpr uint32_t PART = (sizeof(KqPartials) + 127) & ~127u;
-    StreamCtx cx;
-    cx.sm = sm; cx.smem_raw = smem_raw; cx.ring = smem_u32(smem_raw) + HDR + PART;
-    cx.stage_stride = a.cap * (SWIGLU ? 2u : 1u); cx.nstages = a.nstages; cx.cc = 0;
-    cx.limit = a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT;
-    stream_init_ring(sm, a.nstages);
-    __syncthreads();
-    pdl_launch_dependents();
-    if ((threadIdx.x >> 5) == NCW) {
-        stream_produce_rows(a, cx);
-        if ((threadIdx.x & 31) == 0 && sm->abort_flag) stream_drain(cx);
-        return;
-    }
-    pdl_wait();
-    stream_consume_kq<T, SWIGLU>(a, cx, reinterpret_cast<KqPartials*>(smem_raw + HDR), smem_raw + a.tab_off);
-}
 
 }  // namespace alice
