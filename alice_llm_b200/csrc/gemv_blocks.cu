@@ -2,7 +2,7 @@
 //
 // A block is an f16 scale and 32 int8 (Q8_0), 128 signs (Q1_0) or 128 two-bit slots (Q2_0); blocks are 2-byte aligned. The f32
 // activations become 31-bit fixed point (unit 2^-30 of a power of two above the largest) in four signed base-256 digits; the
-// digits of two vectors fill the eight B columns. A operand: the int8 weights themselves, or bytes & (1 << j). A block's sum is an exact integer (two digits joined in
+// digits of two vectors fill the eight B columns. A operand: the int8 weights themselves, or bytes & (1 << j), or the two bits of a slot at once (0 .. 3 times 4^q). A block's sum is an exact integer (two digits joined in
 // 32 bits: at most 16 bytes x 255 x 128 x 257), the offset of the one- and two-bit codes is taken off in integers too (2 S - T, S - T with T summed over the same
 // digits), and one f32 multiply-add per block scales it.
 //
@@ -12,10 +12,11 @@
 // tile are added in a fixed order.
 //
 // What bounds it: Q8_0 HBM at any batch (one product per 544 bytes); Q1_0 and Q2_0 the instructions for one or two vectors
-// (about 95 per 576 bytes, an SM issues 100 while those stream), the products (8 per 16 rows and block, for each pair of vectors) for more.
+// (Q1_0 about 95 per 576 bytes, an SM issues 100 while those stream), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
+#include "digits_dev.cuh"
 #include "gemv_blocks.cuh"
 #include "gemv_mma.cuh"
 
@@ -30,13 +31,14 @@ template <int FMT> struct BlkFmt;                // bytes and elements of a bloc
 // pitch: 32-bit reads of 8 rows x 16 bytes fill the banks once (48 modulo 128)
 template <> struct BlkFmt<0> { static constexpr uint32_t BB = 34, EL = 32, DIG = 256, PITCH = 304; static constexpr bool T = false; };
 template <> struct BlkFmt<1> { static constexpr uint32_t BB = 18, EL = 128, DIG = 1024, PITCH = 176; static constexpr bool T = true; };
-template <> struct BlkFmt<2> { static constexpr uint32_t BB = 34, EL = 128, DIG = 2048, PITCH = 304; static constexpr bool T = true; };
+template <> struct BlkFmt<2> { static constexpr uint32_t BB = 34, EL = 128, DIG = 1024, PITCH = 304; static constexpr bool T = true; };
 
 struct BlkArgs {
     const uint8_t* w[3];
     uint32_t rows[3], y_off[3], tile0[4], nw;
     const uint8_t* up;
     uint32_t row_bytes, nb;                      // blocks of a row
+    const float* x;                              // one or two vectors: the kernel makes the digits itself; more: the table
     const uint8_t* digits;                       // [nb][NT][DIG]
     const int* tsum;                             // [nb][NT][4]
     const float* kappa;
@@ -65,90 +67,91 @@ __device__ __forceinline__ void block_digits(int f, int (&d)[4]) {
     d[0] = f;
 }
 
-// Digit table of vector blockIdx.y; see the indexing of the consumer below.
+// Digits of one block by eight consecutive lanes (t = u & 3, h = u >> 2) into the block's record, columns 4 col .. + 3, and its two joined
+// digit sums into tsum[0 .. 1]; `live` lanes store. FMT 0: byte 16 h + 4 t + b of the block; 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte
+// 16 h + 4 t + b, its four slots.
 template <int FMT>
-__global__ void __launch_bounds__(256) block_table_kernel(const float* x, uint32_t cols, uint32_t batch, uint32_t nb, uint32_t nt, uint8_t* digits, int* tsum, float* kappa_out) {
-    using F = BlkFmt<FMT>;
-    __shared__ float red[8];
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t v = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
-    const float* xv = x + (size_t)v * cols;
-    float amax = 0.0f, odd = 0.0f;         // odd: stays 0 for a finite vector (inf * 0 and NaN * 0 are NaN)
-    if (v < batch) {
-        for (uint32_t base = 0; base < cols / 4; base += 256 * 8) {
-            float4 q[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t i = base + k * 256 + tid;
-                q[k] = i < cols / 4 ? __ldcg(reinterpret_cast<const float4*>(xv) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                amax = fmaxf(fmaxf(amax, fmaxf(fabsf(q[k].x), fabsf(q[k].y))), fmaxf(fabsf(q[k].z), fabsf(q[k].w)));
-                odd = fmaf(q[k].x, 0.0f, fmaf(q[k].y, 0.0f, fmaf(q[k].z, 0.0f, fmaf(q[k].w, 0.0f, odd))));
-            }
-        }
-    }
-    const int finite = __syncthreads_and(odd == 0.0f);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) red[tid >> 5] = amax;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < 8; w++) amax = fmaxf(amax, red[w]);
-    float to_fixed, kappa;
-    block_fixed_scale(amax, finite != 0, to_fixed, kappa);
-    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
-    constexpr uint32_t TPB = FMT == 0 ? 8 : FMT == 1 ? 8 : 16;     // threads of a block of weights
-    const uint32_t i = blockIdx.x * 256 + tid, blk = i / TPB, u = i % TPB;
-    const bool live = blk < nb;
+__device__ __forceinline__ void block_record(const float* x, bool live, uint32_t u, uint32_t col, float to_fixed, uint8_t* rec, int* tsum) {
     uint32_t out[4][4] = {};
     int ts[4] = {0, 0, 0, 0};
-    const uint32_t t = u & 3u, h = (u >> 2) & 1u, w = u >> 3;
+    const uint32_t t = u & 3u, h = u >> 2;
 #pragma unroll
     for (uint32_t b = 0; b < 4; b++) {
-        // FMT 0: byte 16 h + 4 t + b of the block; 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte 16 w + 4 t + b, bits 4 h .. 4 h + 3
-        const uint32_t e = FMT == 0 ? 16 * h + 4 * t + b : FMT == 1 ? 8 * (4 * t + b) + 4 * h : 4 * (16 * w + 4 * t + b) + 2 * h;
+        const uint32_t e = FMT == 0 ? 16 * h + 4 * t + b : FMT == 1 ? 8 * (4 * t + b) + 4 * h : 4 * (16 * h + 4 * t + b);
         float xe[4] = {0.f, 0.f, 0.f, 0.f};
-        if (live && v < batch) {
-            const float* p = xv + (size_t)blk * F::EL + e;
-#pragma unroll
-            for (uint32_t k = 0; k < (FMT == 0 ? 1u : FMT == 1 ? 4u : 2u); k++) xe[k] = __ldcg(p + k);
+        if (live) {
+            if (FMT == 0) {
+                xe[0] = __ldcg(x + e);
+            } else {
+                const float4 q = __ldcg(reinterpret_cast<const float4*>(x + e));
+                xe[0] = q.x; xe[1] = q.y; xe[2] = q.z; xe[3] = q.w;
+            }
         }
 #pragma unroll
         for (uint32_t jj = 0; jj < (FMT == 0 ? 1u : 4u); jj++) {
-            const int sh = FMT == 0 ? 0 : FMT == 1 ? (int)(4 * h + jj) : (int)(2 * (2 * h + (jj >> 1)));
-            const int f = (__float2int_rn(xe[FMT == 2 ? jj >> 1 : jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
+            const int sh = FMT == 0 ? 0 : FMT == 1 ? (int)(4 * h + jj) : (int)(2 * jj);
+            const int f = (__float2int_rn(xe[jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
             int dg[4];
             block_digits(f, dg);
 #pragma unroll
             for (int d = 0; d < 4; d++) {
                 out[d][jj] |= (uint32_t)(dg[d] & 255) << (8 * b);
-                if (FMT == 1 || (FMT == 2 && !(jj & 1u))) ts[d] += dg[d] * (1 << sh);
+                if (FMT != 0) ts[d] += dg[d] * (1 << sh);
             }
         }
     }
-    if (F::T) {
+    if (FMT != 0) {
 #pragma unroll
         for (int d = 0; d < 4; d++)
 #pragma unroll
-            for (uint32_t o = 1; o < TPB; o *= 2) ts[d] += __shfl_xor_sync(0xffffffffu, ts[d], o);
-        if (live && u < 2) tsum[((size_t)blk * nt + (v >> 1)) * 4 + (v & 1u) * 2 + u] = u ? ts[2] * 256 + ts[3] : ts[0] * 256 + ts[1];
+            for (uint32_t o = 1; o < 8; o *= 2) ts[d] += __shfl_xor_sync(0xffffffffu, ts[d], o);
+        if (live && u < 2) tsum[u] = u ? ts[2] * 256 + ts[3] : ts[0] * 256 + ts[1];
     }
     if (!live) return;
-    uint8_t* rec = digits + ((size_t)blk * nt + (v >> 1)) * F::DIG;
 #pragma unroll
     for (uint32_t d = 0; d < 4; d++) {
-        const uint32_t col = (v & 1u) * 4 + d;
-        if (FMT == 0) reinterpret_cast<uint32_t*>(rec)[(col * 4 + t) * 2 + h] = out[d][0];
-        else reinterpret_cast<uint4*>(rec)[(w * 2 + h) * 32 + col * 4 + t] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
+        if (FMT == 0) reinterpret_cast<uint32_t*>(rec)[((col * 4 + d) * 4 + t) * 2 + h] = out[d][0];
+        else reinterpret_cast<uint4*>(rec)[h * 32 + (col * 4 + d) * 4 + t] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
     }
 }
 
+// Digit table of vector blockIdx.y; columns of vectors past the batch stay as they are (a column only reaches its own results).
+template <int FMT>
+__global__ void __launch_bounds__(256) block_table_kernel(const float* x, uint32_t cols, uint32_t nb, uint32_t nt, uint8_t* digits, int* tsum, float* kappa_out) {
+    using F = BlkFmt<FMT>;
+    __shared__ float red[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t v = blockIdx.y, tid = threadIdx.x;
+    const float* xv = x + (size_t)v * cols;
+    bool finite;
+    float to_fixed, kappa;
+    const float amax = vec_amax<256>(xv, cols, true, red, finite);
+    block_fixed_scale(amax, finite, to_fixed, kappa);
+    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
+    const uint32_t i = blockIdx.x * 256 + tid, blk = i / 8;
+    const size_t at = (size_t)blk * nt + (v >> 1);
+    block_record<FMT>(xv + (size_t)blk * F::EL, blk < nb, i % 8, v & 1u, to_fixed, digits + at * F::DIG, tsum + at * 4 + (v & 1u) * 2);
+}
+
 __device__ __forceinline__ uint32_t w4(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+// Plain loads and products that are no volatile assembly: the compiler may bring operands in ahead of earlier products.
+template <class V> __device__ __forceinline__ V ld(const uint8_t* p) { return *reinterpret_cast<const V*>(p); }
+__device__ __forceinline__ uint32_t ld_u2(const uint8_t* p) {      // a 32-bit word at a 2-byte boundary
+    const uint32_t a = smem_u32(p) & 2u;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - a);
+    return __funnelshift_r(q[0], q[1], a * 8u);
+}
+__device__ __forceinline__ void mma_u8s8_k16p(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+__device__ __forceinline__ void mma_u8s8_k32p(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 __device__ __forceinline__ void mma_s8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
@@ -158,6 +161,7 @@ template <int FMT, int NT, bool SW, bool AL>
 __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __grid_constant__ BlkArgs a, const uint32_t S) {
     extern __shared__ __align__(128) uint8_t smem[];
     using F = BlkFmt<FMT>;
+    __shared__ float s_red[BLK_WARPS], s_kappa[2];
     constexpr int MATS = SW ? 2 : 1;
     constexpr uint32_t CH = F::BB * BLK_ITEM / 16 + (AL ? 0 : 1), STAGE = 16 * F::PITCH;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3u;
@@ -166,8 +170,9 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
     const uint32_t t_lo = (uint32_t)((uint64_t)tiles * cl / ncl), nt_loc = (uint32_t)((uint64_t)tiles * (cl + 1) / ncl) - t_lo;
     const uint32_t all = (a.nb + BLK_ITEM - 1) / BLK_ITEM, s_lo = all * rank / S, ns = all * (rank + 1) / S - s_lo;
     const uint32_t b_lo = s_lo * BLK_ITEM, b_hi = min(a.nb, (s_lo + ns) * BLK_ITEM), nblk = b_hi - b_lo;
-    const uint32_t bar = smem_u32(smem), ring = bar + BLK_HDR + warp * a.stages * STAGE, tab = bar + BLK_HDR + BLK_WARPS * a.stages * STAGE;
-    const uint32_t tsm = bar + a.tsum_off;
+    const uint32_t bar = smem_u32(smem), ring = bar + BLK_HDR + warp * a.stages * STAGE;
+    const uint8_t* const tab = smem + BLK_HDR + BLK_WARPS * a.stages * STAGE;
+    const uint8_t* const tsm = smem + a.tsum_off;
     float* mainp = reinterpret_cast<float*>(smem + a.main_off);     // [mat][tile][16 rows][2 NT]
     float* head = reinterpret_cast<float*>(smem + a.head_off);      // [warp][16 rows][2 NT]
     if (tid == 0) { mbar_init(bar, 1); mbar_fence_init(); }
@@ -208,14 +213,32 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
     for (uint32_t k = 0; k + 1 < a.stages; k++) fetch();
 
     pdl_wait();
-    if (tid == 0) {
-        const uint32_t db = nblk * NT * F::DIG, tb = F::T ? nblk * NT * 16u : 0u;
-        mbar_arrive_expect_tx(bar, db + tb);
-        bulk_g2s(tab, a.digits + (size_t)b_lo * NT * F::DIG, db, bar);
-        if (F::T) bulk_g2s(tsm, a.tsum + (size_t)b_lo * NT * 4, tb, bar);
+    bool ok = true;
+    if constexpr (NT == 1) {
+        // one or two vectors: every CTA makes the digits of its columns itself, which saves the launch of the table kernel in between
+        uint8_t* const dtab = smem + BLK_HDR + BLK_WARPS * a.stages * STAGE;
+        int* const dsum = reinterpret_cast<int*>(smem + a.tsum_off);
+        for (uint32_t v = 0; v < a.batch; v++) {
+            const float* xv = a.x + (size_t)v * a.nb * F::EL;
+            bool finite;
+            float to_fixed, kappa;
+            const float amax = vec_amax<BLK_WARPS * 32>(xv, a.nb * F::EL, true, s_red, finite);
+            block_fixed_scale(amax, finite, to_fixed, kappa);
+            if (tid == 0) s_kappa[v] = kappa;
+            for (uint32_t i = tid; i < ((nblk * 8 + 31) & ~31u); i += BLK_WARPS * 32)
+                block_record<FMT>(xv + (size_t)(b_lo + i / 8) * F::EL, i / 8 < nblk, i % 8, v, to_fixed, dtab + (i / 8) * F::DIG, dsum + (i / 8) * 4 + v * 2);
+        }
+        __syncthreads();
+    } else {
+        if (tid == 0) {
+            const uint32_t db = nblk * NT * F::DIG, tb = F::T ? nblk * NT * 16u : 0u;
+            mbar_arrive_expect_tx(bar, db + tb);
+            bulk_g2s(smem_u32(tab), a.digits + (size_t)b_lo * NT * F::DIG, db, bar);
+            if (F::T) bulk_g2s(smem_u32(tsm), a.tsum + (size_t)b_lo * NT * 4, tb, bar);
+        }
+        ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
+        if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
     }
-    const bool ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
-    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
 
     float acc[NT][2] = {};
     uint32_t tile = i_lo / ns, seg = i_lo - tile * ns, slot = 0, padA = 0, padB = 0;
@@ -248,18 +271,19 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
         else asm volatile("cp.async.wait_group 2;" ::: "memory");
         __syncwarp();                        // the stage is in for every lane, and every lane is done with the one before
         fetch();
-        const uint32_t rowA = ring + slot * STAGE + g * F::PITCH + padA, rowB = ring + slot * STAGE + (g + 8) * F::PITCH + padB;
+        const uint8_t* const rowA = smem + BLK_HDR + (warp * a.stages + slot) * STAGE + g * F::PITCH + padA;
+        const uint8_t* const rowB = smem + BLK_HDR + (warp * a.stages + slot) * STAGE + (g + 8) * F::PITCH + padB;
         if (++slot == a.stages) slot = 0;
         const uint32_t b0 = seg * BLK_ITEM, nbi = min(BLK_ITEM, nblk - b0);
-        const uint32_t rec = tab + b0 * (NT * F::DIG), trec = tsm + b0 * (NT * 16u) + t * 4;
+        const uint8_t *const rec = tab + b0 * (NT * F::DIG), *const trec = tsm + b0 * (NT * 16u) + t * 4;
         auto block = [&](uint32_t b) {
-            const uint32_t pA = rowA + b * F::BB, pB = rowB + b * F::BB;
-            const float dA = f16_bits_to_f32(lds16(pA)), dB = f16_bits_to_f32(lds16(pB));
+            const uint8_t *const pA = rowA + b * F::BB, *const pB = rowB + b * F::BB;
+            const float dA = f16_bits_to_f32(ld<uint16_t>(pA)), dB = f16_bits_to_f32(ld<uint16_t>(pB));
             if constexpr (FMT == 0) {
-                const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t), a2 = lds32_u2(pA + 18 + 4 * t), a3 = lds32_u2(pB + 18 + 4 * t);
+                const uint32_t a0 = ld_u2(pA + 2 + 4 * t), a1 = ld_u2(pB + 2 + 4 * t), a2 = ld_u2(pA + 18 + 4 * t), a3 = ld_u2(pB + 18 + 4 * t);
 #pragma unroll
                 for (int n = 0; n < NT; n++) {
-                    const uint2 x = lds64(rec + (b * NT + n) * F::DIG + lane * 8);
+                    const uint2 x = ld<uint2>(rec + (b * NT + n) * F::DIG + lane * 8);
                     int c[4];
                     mma_s8s8_k32(c, a0, a1, a2, a3, x.x, x.y);
                     acc[n][0] = fmaf(dA, (float)(c[0] * 256 + c[1]), acc[n][0]);
@@ -268,40 +292,37 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
             } else {
                 int c[NT][2][4] = {};        // even and odd bits: two chains
                 if constexpr (FMT == 1) {
-                    const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t);
+                    const uint32_t a0 = ld_u2(pA + 2 + 4 * t), a1 = ld_u2(pB + 2 + 4 * t);
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         uint4 x[NT];
 #pragma unroll
-                        for (int n = 0; n < NT; n++) x[n] = lds128(rec + (b * NT + n) * F::DIG + h * 512 + lane * 16);
+                        for (int n = 0; n < NT; n++) x[n] = ld<uint4>(rec + (b * NT + n) * F::DIG + h * 512 + lane * 16);
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             const uint32_t m = 0x01010101u << (4 * h + j), m0 = a0 & m, m1 = a1 & m;
 #pragma unroll
-                            for (int n = 0; n < NT; n++) mma_u8s8_k16(c[n][j & 1], m0, m1, w4(x[n], j));
+                            for (int n = 0; n < NT; n++) mma_u8s8_k16p(c[n][j & 1], m0, m1, w4(x[n], j));
                         }
                     }
                 } else {
-                    const uint32_t a0 = lds32_u2(pA + 2 + 4 * t), a1 = lds32_u2(pB + 2 + 4 * t), a2 = lds32_u2(pA + 18 + 4 * t), a3 = lds32_u2(pB + 18 + 4 * t);
+                    const uint32_t a0 = ld_u2(pA + 2 + 4 * t), a1 = ld_u2(pB + 2 + 4 * t), a2 = ld_u2(pA + 18 + 4 * t), a3 = ld_u2(pB + 18 + 4 * t);
+                    uint4 x[NT], z[NT];
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        uint4 x[NT], z[NT];
+                    for (int n = 0; n < NT; n++) {
+                        x[n] = ld<uint4>(rec + (b * NT + n) * F::DIG + lane * 16);
+                        z[n] = ld<uint4>(rec + (b * NT + n) * F::DIG + 512 + lane * 16);
+                    }
 #pragma unroll
-                        for (int n = 0; n < NT; n++) {
-                            x[n] = lds128(rec + (b * NT + n) * F::DIG + h * 512 + lane * 16);
-                            z[n] = lds128(rec + (b * NT + n) * F::DIG + 1024 + h * 512 + lane * 16);
-                        }
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t m = 0x03030303u << (2 * j), m0 = a0 & m, m1 = a1 & m, m2 = a2 & m, m3 = a3 & m;
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const uint32_t m = 0x01010101u << (4 * h + j), m0 = a0 & m, m1 = a1 & m, m2 = a2 & m, m3 = a3 & m;
-#pragma unroll
-                            for (int n = 0; n < NT; n++) mma_u8s8_k32(c[n][j & 1], m0, m1, m2, m3, w4(x[n], j), w4(z[n], j));
-                        }
+                        for (int n = 0; n < NT; n++) mma_u8s8_k32p(c[n][j & 1], m0, m1, m2, m3, w4(x[n], j), w4(z[n], j));
                     }
                 }
 #pragma unroll
                 for (int n = 0; n < NT; n++) {
-                    const int T = (int)lds32(trec + (b * NT + n) * 16);
+                    const int T = (int)ld<uint32_t>(trec + (b * NT + n) * 16);
                     int vA = (c[n][0][0] + c[n][1][0]) * 256 + (c[n][0][1] + c[n][1][1]), vB = (c[n][0][2] + c[n][1][2]) * 256 + (c[n][0][3] + c[n][1][3]);
                     vA = (FMT == 1 ? 2 * vA : vA) - T;
                     vB = (FMT == 1 ? 2 * vB : vB) - T;
@@ -358,7 +379,7 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
                     y = r ? y + p : p;
                 }
             }
-            f[q] = __ldg(a.kappa + v) * y;
+            f[q] = (NT == 1 ? s_kappa[v] : __ldg(a.kappa + v)) * y;
         }
         float r = SW ? silu_ref(f[0]) * f[MATS - 1] : f[0];
         const uint32_t yi = a.y_off[s] + row;
@@ -444,7 +465,8 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     const uint32_t nt = pairs_of(op.batch), cols = op.w[0]->cols;
     a.nb = cols / F::EL;
     const size_t dig = (size_t)a.nb * nt * F::DIG, ts = F::T ? (size_t)a.nb * nt * 16 : 0;
-    if (!dry) {
+    a.x = op.x;
+    if (!dry && nt > 1) {
         if (!op.prep || ((uintptr_t)op.prep & 15) || dig + ts + 64 > op.prep_bytes) return ALICE_E_SHAPE;
         uint8_t* base = static_cast<uint8_t*>(op.prep);
         a.digits = base; a.tsum = reinterpret_cast<const int*>(base + dig); a.kappa = reinterpret_cast<const float*>(base + dig + ts);
@@ -452,14 +474,15 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     auto rows = [&](bool plan) { return nt == 1 ? launch_nt<FMT, 1>(a, cfg, plan) : nt == 2 ? launch_nt<FMT, 2>(a, cfg, plan) : launch_nt<FMT, 4>(a, cfg, plan); };
     const int rc = rows(true);
     if (rc || dry) return rc;
+    if (nt == 1) return rows(false);
     cudaLaunchConfig_t lc = {};
-    const uint32_t per_vec = a.nb * (FMT == 2 ? 16u : 8u);
-    lc.gridDim = dim3((per_vec + 255) / 256, 2 * nt); lc.blockDim = dim3(256); lc.stream = cfg.stream;
+    const uint32_t per_vec = a.nb * 8u;
+    lc.gridDim = dim3((per_vec + 255) / 256, op.batch); lc.blockDim = dim3(256); lc.stream = cfg.stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = cfg.pdl ? 1 : 0;
-    if (cudaLaunchKernelEx(&lc, block_table_kernel<FMT>, op.x, cols, op.batch, a.nb, nt, const_cast<uint8_t*>(a.digits), const_cast<int*>(a.tsum), const_cast<float*>(a.kappa)) != cudaSuccess)
+    if (cudaLaunchKernelEx(&lc, block_table_kernel<FMT>, op.x, cols, a.nb, nt, const_cast<uint8_t*>(a.digits), const_cast<int*>(a.tsum), const_cast<float*>(a.kappa)) != cudaSuccess)
         return ALICE_E_CUDA;
     return rows(false);
 }
@@ -467,8 +490,7 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
 }  // namespace
 
 size_t blocks_prep_bytes(uint32_t cols, uint32_t batch) {
-    // Q2_0 has the largest: 2048 + 16 bytes per 128 columns and pair
-    return (size_t)((cols + 127) / 128) * pairs_of(batch) * (2048 + 16) + 256;
+    return (size_t)((cols + 127) / 128) * pairs_of(batch) * (1024 + 16) + 256;      // Q8_0: 256 per 32 columns, no sums
 }
 
 int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry) {

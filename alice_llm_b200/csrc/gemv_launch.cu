@@ -476,6 +476,26 @@ static int launch_split(int (*launch)(const GemvOp&, const LaunchCfg&, bool), co
     return ALICE_E_SHAPE;
 }
 
+// Whether one vector goes to the kernel for several (csrc/gemv_blocks.cu) rather than to the ring kernels.
+static bool one_vector_warp_ring(const GemvOp& op) {
+    const WeightDesc& w = *op.w[0];
+    switch (w.fmt) {
+        // Q2_0: 51200 x 5120 27.4 against 36.8 us, 4096 x 4096 8.2 against 9.1. Q1_0: 151936 x 1024 16.5 against 31.5, 5120 x 25600 19.8 against
+        // 21.0, 25600 x 5120 15.0 against 14.9, 7168 x 5120 10.7 against 9.8; a 27B model 13.03 against 13.48 ms for two tokens.
+        case WF_Q1_0: case WF_Q2_0: return true;
+        // Widths at which the ring kernel's lanes stand idle (it deals 16-column units to 32 P lanes, 1, 2 or 4 each): 151936 x 5120 148 against
+        // 262 us; 32768 x 4096 37.5 against 33.8, 4096 x 14336 27.7 against 22.3.
+        case WF_Q8_0: {
+            const uint32_t units = w.cols / 16;
+            uint32_t lanes = 32;
+            while (lanes < 256 && lanes < units) lanes *= 2;
+            const uint32_t each = (units + lanes - 1) / lanes;
+            return 10 * units < 7 * lanes * (each == 3 ? 4 : each);
+        }
+        default: return false;
+    }
+}
+
 int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
     if (op.batch == 0) return ALICE_E_SHAPE;
     if (op.w[0] && op.w[0]->fmt == WF_BF16) return launch_dense_rows(op, cfg);
@@ -495,13 +515,9 @@ int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
     if (op.batch > 1 && op.argmax_key) return ALICE_E_INVALID;
     const WeightFormat f = op.w[0]->fmt;
     const bool planes = f == WF_TERNARY || f == WF_SPARSE_TERNARY;
-    if (planes || f == WF_Q8_0 || f == WF_Q1_0 || f == WF_Q2_0) {
-        const int prc = launch_split(planes ? launch_planes : launch_blocks, op, cfg);
-        if (prc != ALICE_E_SHAPE) return prc;
-    }
-    if (op.batch > 1) {      // K-quants; for one vector the per-lane kernel is faster (feed-forward block of an 8B model 32.6 against 43.1 us)
-        const int krc = launch_split(launch_kq_rows, op, cfg);
-        if (krc != ALICE_E_SHAPE) return krc;
+    if (planes || op.batch > 1 || one_vector_warp_ring(op)) {
+        const int rc = launch_split(planes ? launch_planes : format_uses_q8k(f) ? launch_kq_rows : launch_blocks, op, cfg);
+        if (rc != ALICE_E_SHAPE) return rc;
     }
     if (op.batch == 1) return launch_single(op, cfg);
     // Formats without a batch kernel: one launch per input vector (the weights stream once per vector).
@@ -520,10 +536,10 @@ size_t mma_prep_bytes(uint32_t cols) {
 }
 
 int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint32_t* weight_passes) {
-    for (uint32_t n = op.batch; n; n /= 2) {
+    for (uint32_t n = op.batch > 1 ? op.batch : 0; n; n /= 2) {
         Q8KView v;
         const GemvOp part = sub_batch(op, 0, n, v);
-        if (launch_planes(part, cfg, true) == ALICE_OK || launch_blocks(part, cfg, true) == ALICE_OK || (op.batch > 1 && launch_kq_rows(part, cfg, true) == ALICE_OK)) {
+        if (launch_planes(part, cfg, true) == ALICE_OK || launch_blocks(part, cfg, true) == ALICE_OK || launch_kq_rows(part, cfg, true) == ALICE_OK) {
             *launches = *weight_passes = (op.batch + n - 1) / n;
             return ALICE_OK;
         }

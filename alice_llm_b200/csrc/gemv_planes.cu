@@ -2,6 +2,7 @@
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
+#include "digits_dev.cuh"
 #include "gemv_mma.cuh"
 #include "gemv_planes.cuh"
 
@@ -11,82 +12,59 @@ namespace {
 constexpr uint32_t PLANE_SMEM = 220 * 1024;
 constexpr uint32_t PLANE_HDR = 128;
 
-// Digit table of one vector per blockIdx.y (columns 4 (v & 1) .. + 3 of pair v >> 1); vectors past `batch` are zero columns.
-// Thread (segment, quad lane t, word w, half h) owns bits 4 h .. 4 h + 3 of the four bytes 64 seg + 16 t + 4 w + i and writes, for
-// each digit, the four B words of those bits: table[((seg * NT + pair) * 8 + 2 w + h) * 32 + 4 * column + t].
+// One thread's part of a digit table: word w of quad lane t in a 64-byte segment. Planes: bits 4 h .. 4 h + 3 of its four bytes; codes:
+// the four code places of its four bytes (h = 0). out[digit] = the B words of the four.
 template <bool CODES>
-__global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32_t cols, uint32_t batch, uint32_t segs, uint32_t nt, uint4* table, float* kappa_out) {
-    __shared__ float red[8];
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t v = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
-    const float* xv = x + (size_t)v * cols;
-    const bool vec4 = cols % 4 == 0 && ((uintptr_t)xv & 15) == 0;
-    float amax = 0.0f, odd = 0.0f;         // odd: stays 0 for a finite vector (inf * 0 and NaN * 0 are NaN)
-    if (v < batch) {
-        if (vec4) {
-            for (uint32_t base = 0; base < cols / 4; base += 256 * 8) {
-                float4 q[8];
+__device__ __forceinline__ void plane_digits(const float* x, uint32_t cols, bool vec4, float to_fixed, uint32_t seg, uint32_t t, uint32_t w, uint32_t h, uint32_t (&out)[4][4]) {
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const uint32_t i = base + k * 256 + tid;
-                    q[k] = i < cols / 4 ? __ldcg(reinterpret_cast<const float4*>(xv) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    amax = fmaxf(fmaxf(amax, fmaxf(fabsf(q[k].x), fabsf(q[k].y))), fmaxf(fabsf(q[k].z), fabsf(q[k].w)));
-                    odd = fmaf(q[k].x, 0.0f, fmaf(q[k].y, 0.0f, fmaf(q[k].z, 0.0f, fmaf(q[k].w, 0.0f, odd))));
-                }
-            }
-        } else {
-            for (uint32_t i = tid; i < cols; i += 256) {
-                const float q = __ldcg(xv + i);
-                amax = fmaxf(amax, fabsf(q));
-                odd = fmaf(q, 0.0f, odd);
-            }
-        }
-    }
-    const bool finite = __syncthreads_and(odd == 0.0f);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) red[tid >> 5] = amax;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < 8; w++) amax = fmaxf(amax, red[w]);
-    float to_fixed, kappa;
-    mma_fixed_scale(amax, to_fixed, kappa);
-    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = finite ? kappa : __int_as_float(0x7fffffff);      // all results of a vector that is not finite are NaN
-    const uint32_t seg = blockIdx.x * 8 + (tid >> 5), t = lane & 3u, wh = lane >> 2, h = wh & 1u;   // wh = 2 w + h
-    if (seg >= segs) return;
-    uint32_t out[4][4] = {};          // [digit][bit 4 h + jj]
+    for (int d = 0; d < 4; d++) out[d][0] = out[d][1] = out[d][2] = out[d][3] = 0u;
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) {
-        const uint32_t byte = seg * PLANE_SEG + t * 16 + (wh >> 1) * 4 + i;
-        const uint32_t e = CODES ? byte * 4 + 2 * h : byte * 8 + 4 * h;
+        const uint32_t byte = seg * PLANE_SEG + t * 16 + w * 4 + i;
+        const uint32_t e = CODES ? byte * 4 : byte * 8 + 4 * h;
         float xe[4] = {0.f, 0.f, 0.f, 0.f};
-        if (v < batch) {
-            if (!CODES && vec4 && e < cols) {
-                const float4 q = __ldcg(reinterpret_cast<const float4*>(xv + e));
-                xe[0] = q.x; xe[1] = q.y; xe[2] = q.z; xe[3] = q.w;
-            } else {
+        if (vec4 && e < cols) {
+            const float4 q = __ldcg(reinterpret_cast<const float4*>(x + e));
+            xe[0] = q.x; xe[1] = q.y; xe[2] = q.z; xe[3] = q.w;
+        } else {
 #pragma unroll
-                for (uint32_t k = 0; k < (CODES ? 2u : 4u); k++)
-                    if (e + k < cols) xe[k] = __ldcg(xv + e + k);
-            }
+            for (uint32_t k = 0; k < 4; k++)
+                if (e + k < cols) xe[k] = __ldcg(x + e + k);
         }
 #pragma unroll
         for (uint32_t jj = 0; jj < 4; jj++) {
-            // one bit per element: element 8 byte + j, fixed / 2^j; two bits per element: bits 2 q and 2 q + 1 are worth x and -2 x
-            const int sh = CODES ? (int)(2 * (2 * h + (jj >> 1))) : (int)(4 * h + jj);
-            int f = (__float2int_rn(xe[CODES ? jj >> 1 : jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
-            if (CODES && (jj & 1u)) f = -f;
+            // what the consumer's A bytes are worth: 2^j for bits 0 .. 6, 2^6 for bit 7; 2^(2 q) for code place q
+            const int sh = CODES ? (int)(2 * jj) : min((int)(4 * h + jj), 6);
+            const int f = (__float2int_rn(xe[jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
             uint8_t dg[193];          // digits land 64 apart
             mma_store_digits(dg, f);
 #pragma unroll
             for (int d = 0; d < 4; d++) out[d][jj] |= (uint32_t)dg[64 * d] << (8 * i);
         }
     }
-    uint4* rec = table + ((size_t)(seg * nt + (v >> 1)) * 8 + wh) * 32 + (v & 1u) * 16 + t;
+}
+__device__ __forceinline__ bool can_vec4(const float* x, uint32_t cols) { return cols % 4 == 0 && ((uintptr_t)x & 15) == 0; }
+
+// Digit table of one vector per blockIdx.y (columns 4 (v & 1) .. + 3 of pair v >> 1); vectors past `batch` are zero columns. With
+// RECS records of 512 bytes to a segment and pair: table[((seg * NT + pair) * RECS + record) * 32 + 4 * column + t].
+template <bool CODES>
+__global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32_t cols, uint32_t batch, uint32_t segs, uint32_t nt, uint4* table, float* kappa_out) {
+    __shared__ float red[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t v = blockIdx.y, tid = threadIdx.x;
+    const float* xv = x + (size_t)min(v, batch - 1) * cols;
+    const bool vec4 = can_vec4(xv, cols);
+    bool finite;
+    float to_fixed, kappa;
+    mma_fixed_scale(vec_amax<256>(xv, cols, vec4, red, finite), to_fixed, kappa);
+    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = finite ? kappa : __int_as_float(0x7fffffff);      // all results of a vector that is not finite are NaN
+    constexpr uint32_t RECS = CODES ? 4 : 8;
+    const uint32_t i = blockIdx.x * 256 + tid, seg = i / (RECS * 4), t = i & 3u, wh = (i >> 2) % RECS;
+    if (seg >= segs) return;
+    uint32_t out[4][4];
+    plane_digits<CODES>(xv, v < batch ? cols : 0u, vec4, to_fixed, seg, t, CODES ? wh : wh >> 1, CODES ? 0u : wh & 1u, out);
+    uint4* rec = table + ((size_t)(seg * nt + (v >> 1)) * RECS + wh) * 32 + (v & 1u) * 16 + t;
 #pragma unroll
     for (int d = 0; d < 4; d++) rec[d * 4] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
 }
@@ -121,11 +99,11 @@ __device__ __forceinline__ PlaneTile plane_tile(const PlaneArgs& a, uint32_t til
     return {w + (size_t)min(r0 + g, last) * a.row_bytes, w + (size_t)min(r0 + g + 8, last) * a.row_bytes};
 }
 
-__device__ __forceinline__ int ld_cluster_s32(uint32_t addr, uint32_t rank) {
+__device__ __forceinline__ long long ld_cluster_s64(uint32_t addr, uint32_t rank) {
     uint32_t remote;
-    int v;
+    long long v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+    asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(remote) : "memory");
     return v;
 }
 __device__ __forceinline__ void cluster_sync() {
@@ -133,10 +111,28 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// A signed A word of four weights: those whose bit is set in p are worth 2^j, those in n -2^j (bits j .. 7 of their bytes set). A
+// byte cannot be +2^7: bit 7 is moved to bit 6.
+__device__ __forceinline__ uint32_t signed_planes(uint32_t p, uint32_t n, int j) {
+    const int k = min(j, 6);
+    const uint32_t m = 0x01010101u << k, x = (j == 7 ? n >> 1 : n) & m;
+    return ((j == 7 ? p >> 1 : p) & m) | x * ((1u << (8 - k)) - 1u);
+}
+// Codes 00 = 0, 01 = +1, 11 = -1 at place q of four bytes, worth +-2^(2 q): the high bit is the sign.
+__device__ __forceinline__ uint32_t signed_codes(uint32_t w, int q) {
+    return (w & (0x01010101u << (2 * q))) | (w & (0x02020202u << (2 * q))) * ((1u << (7 - 2 * q)) - 1u);
+}
+__device__ __forceinline__ void mma_s8s8_acc(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // NT: pairs of vectors. PL: bit planes of a row (2: pos | neg, 1: packed codes). S CTAs to a cluster.
 template <int NT, int PL, bool SW, bool VEC16>
 __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const __grid_constant__ PlaneArgs a, const uint32_t S) {
     extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ float s_red[PLANE_WARPS], s_kappa[2];
     constexpr int MATS = SW ? 2 : 1;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3u;
     const uint32_t rank = S > 1 ? blockIdx.x % S : 0u, cl = blockIdx.x / S, ncl = gridDim.x / S;
@@ -144,10 +140,11 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
     const uint32_t t_lo = (uint32_t)((uint64_t)tiles * cl / ncl), nt_loc = (uint32_t)((uint64_t)tiles * (cl + 1) / ncl) - t_lo;
     const uint32_t s_lo = a.segs * rank / S, ns = a.segs * (rank + 1) / S - s_lo;
     const uint32_t bar = smem_u32(smem), tab = bar + PLANE_HDR;
-    int* acc = reinterpret_cast<int*>(smem + a.acc_off);
-    const uint32_t acc_n = MATS * a.tiles_max * 16 * NT * 4;
+    constexpr uint32_t SEGB = (PL == 2 ? 8u : 4u) * NT * 512u;        // table bytes of a segment
+    auto* acc = reinterpret_cast<unsigned long long*>(smem + a.acc_off);   // [mat][tile][16 rows][2 NT]: two's complement sums in fixed-point units
+    const uint32_t acc_n = MATS * a.tiles_max * 16 * NT * 2;
     if (tid == 0) { mbar_init(bar, 1); mbar_fence_init(); }
-    for (uint32_t i = tid; i < acc_n; i += PLANE_WARPS * 32) acc[i] = 0;
+    for (uint32_t i = tid; i < acc_n; i += PLANE_WARPS * 32) acc[i] = 0ull;
     __syncthreads();
     pdl_launch_dependents();
 
@@ -178,52 +175,78 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
     for (int k = 0; k < PF; k++) load(buf[k]);
 
     pdl_wait();
-    const uint32_t tab_bytes = ns * NT * 4096u;
-    if (tid == 0) {
-        mbar_arrive_expect_tx(bar, tab_bytes);
-        if (tab_bytes) bulk_g2s(tab, a.table + (size_t)s_lo * NT * 256, tab_bytes, bar);
-    }
-    const bool ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
-    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
-
-    int c[PL][NT][4] = {};
-    uint32_t tile = ns ? i_lo / ns : 0u, seg = i_lo - tile * ns;
-    auto flush = [&]() {
-        int* row = acc + ((tile >= nt_loc ? a.tiles_max + (tile - nt_loc) : tile) * 16 + g) * (NT * 4) + t;
+    bool ok = true;
+    if constexpr (NT == 1) {
+        // one or two vectors: every CTA makes the digits of its columns itself, which takes about as long as fetching them and saves
+        // the launch of the table kernel in between. Columns of a second vector that is not there only reach its own sums.
+        constexpr bool CODES = PL == 1;
+        constexpr uint32_t RECS = CODES ? 4 : 8;
+        for (uint32_t v = 0; v < a.batch; v++) {
+            const float* xv = a.x + (size_t)v * a.cols;
+            const bool vec4 = can_vec4(xv, a.cols);
+            bool finite;
+            float to_fixed, kappa;
+            mma_fixed_scale(vec_amax<PLANE_WARPS * 32>(xv, a.cols, vec4, s_red, finite), to_fixed, kappa);
+            if (tid == 0) s_kappa[v] = finite ? kappa : __int_as_float(0x7fffffff);
+            for (uint32_t i = tid; i < ns * RECS * 4; i += PLANE_WARPS * 32) {
+                const uint32_t sl = i / (RECS * 4), wh = (i >> 2) % RECS;
+                uint32_t out[4][4];
+                plane_digits<CODES>(xv, a.cols, vec4, to_fixed, s_lo + sl, t, CODES ? wh : wh >> 1, CODES ? 0u : wh & 1u, out);
+                uint4* rec = reinterpret_cast<uint4*>(smem + PLANE_HDR + sl * SEGB + wh * 512) + v * 16 + t;
 #pragma unroll
-        for (int n = 0; n < NT; n++) {
-            int lo = c[0][n][0] * 128 + c[0][n][1], hi = c[0][n][2] * 128 + c[0][n][3];
-            if (PL == 2) { lo -= c[PL - 1][n][0] * 128 + c[PL - 1][n][1]; hi -= c[PL - 1][n][2] * 128 + c[PL - 1][n][3]; }
-            atomicAdd(row + n * 4, lo);
-            atomicAdd(row + 8 * (NT * 4) + n * 4, hi);
-#pragma unroll
-            for (int p = 0; p < PL; p++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) c[p][n][q] = 0;
+                for (int d = 0; d < 4; d++) rec[d * 4] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
+            }
         }
+        __syncthreads();
+    } else {
+        const uint32_t tab_bytes = ns * SEGB;
+        if (tid == 0) {
+            mbar_arrive_expect_tx(bar, tab_bytes);
+            if (tab_bytes) bulk_g2s(tab, a.table + (size_t)s_lo * (SEGB / 16), tab_bytes, bar);
+        }
+        ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
+        if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
+    }
+
+    int c[NT][4] = {};
+    uint32_t tile = ns ? i_lo / ns : 0u, seg = i_lo - tile * ns;
+    // the digits of a sum meet in 64 bits (a row of equal signs over equal activations leaves 32): lanes 2 k and 2 k + 1 have two each
+    auto flush = [&]() {
+        unsigned long long* row = acc + ((tile >= nt_loc ? a.tiles_max + (tile - nt_loc) : tile) * 16 + g) * (NT * 2) + (t >> 1);
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                long long v = (long long)c[n][2 * r] * 128 + c[n][2 * r + 1];
+                const long long other = __shfl_xor_sync(0xffffffffu, v, 1);
+                v = v * 16384 + other;
+                if (!(t & 1u)) atomicAdd(row + r * 8 * (NT * 2) + n * 2, (unsigned long long)v);
+                c[n][2 * r] = c[n][2 * r + 1] = 0;
+            }
     };
     auto step = [&](const uint4 (&v)[PL][2]) {
-        const uint32_t rec = tab + seg * (NT * 4096u) + lane * 16;
+        const uint8_t* rec = smem + PLANE_HDR + seg * SEGB + lane * 16;
+        constexpr int H = PL == 2 ? 2 : 1;
 #pragma unroll
         for (int p = 0; p < 2; p++)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
+            for (int h = 0; h < H; h++) {
                 uint4 b0[NT], b1[NT];
 #pragma unroll
                 for (int n = 0; n < NT; n++) {
-                    b0[n] = lds128(rec + n * 4096 + (4 * p + h) * 512);
-                    b1[n] = lds128(rec + n * 4096 + (4 * p + 2 + h) * 512);
+                    b0[n] = *reinterpret_cast<const uint4*>(rec + (n * 4 * H + 2 * p * H + h) * 512);
+                    b1[n] = *reinterpret_cast<const uint4*>(rec + (n * 4 * H + (2 * p + 1) * H + h) * 512);
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const uint32_t m = 0x01010101u << (4 * h + j);
+                    uint32_t w[4];
 #pragma unroll
-                    for (int q = 0; q < PL; q++) {
-                        const uint32_t a0 = word_of(v[q][0], 2 * p) & m, a1 = word_of(v[q][1], 2 * p) & m;
-                        const uint32_t a2 = word_of(v[q][0], 2 * p + 1) & m, a3 = word_of(v[q][1], 2 * p + 1) & m;
-#pragma unroll
-                        for (int n = 0; n < NT; n++) mma_u8s8_k32(c[q][n], a0, a1, a2, a3, word_of(b0[n], j), word_of(b1[n], j));
+                    for (int q = 0; q < 4; q++) {
+                        const int r = q & 1, i = 2 * p + (q >> 1);
+                        w[q] = PL == 2 ? signed_planes(word_of(v[0][r], i), word_of(v[PL - 1][r], i), 4 * h + j) : signed_codes(word_of(v[0][r], i), j);
                     }
+#pragma unroll
+                    for (int n = 0; n < NT; n++) mma_s8s8_acc(c[n], w[0], w[1], w[2], w[3], word_of(b0[n], j), word_of(b1[n], j));
                 }
             }
         if (++seg == ns) { flush(); seg = 0; tile++; }
@@ -257,13 +280,10 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
         float f[MATS];
 #pragma unroll
         for (int q = 0; q < MATS; q++) {
-            const uint32_t at = acc_s + (((q * a.tiles_max * 16 + lr) * NT + (v >> 1)) * 4 + (v & 1u) * 2) * 4;
-            long long hi = 0, lo = 0;
-            for (uint32_t r = 0; r < S; r++) {
-                hi += S > 1 ? ld_cluster_s32(at, r) : (int)lds32(at);
-                lo += S > 1 ? ld_cluster_s32(at + 4, r) : (int)lds32(at + 4);
-            }
-            f[q] = __ldg(a.kappa + v) * (float)(hi * 16384 + lo) * __ldg((SW && q ? a.up_scale : a.scale[s]) + row);
+            const uint32_t at = acc_s + ((q * a.tiles_max * 16 + lr) * (NT * 2) + v) * 8;
+            long long sum = 0;
+            for (uint32_t r = 0; r < S; r++) sum += S > 1 ? ld_cluster_s64(at, r) : (long long)acc[(at - acc_s) / 8];
+            f[q] = (NT == 1 ? s_kappa[v] : __ldg(a.kappa + v)) * (float)sum * __ldg((SW && q ? a.up_scale : a.scale[s]) + row);
         }
         float r = SW ? silu_ref(f[0]) * f[MATS - 1] : f[0];
         const uint32_t yi = a.y_off[s] + row;
@@ -318,7 +338,7 @@ int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
         }
         ncl = std::min(ncl, tiles);
         const uint32_t per = (tiles + ncl - 1) / ncl, slice = (a.segs + S - 1) / S;
-        const size_t table = (size_t)slice * NT * 4096, acc = (size_t)(SW ? 2 : 1) * per * 16 * NT * 16;
+        const size_t table = (size_t)slice * NT * (PL == 2 ? 4096 : 2048), acc = (size_t)(SW ? 2 : 1) * per * 16 * NT * 16;
         const size_t smem = PLANE_HDR + table + acc;
         if (smem > PLANE_SMEM) continue;
         // fewer tiles than half the SMs: let more CTAs share a tile's columns
@@ -350,7 +370,7 @@ uint32_t plane_pairs(uint32_t batch) { return batch <= 2 ? 1u : batch <= 4 ? 2u 
 }  // namespace
 
 size_t plane_prep_bytes(uint32_t cols, uint32_t batch) {
-    return (size_t)((cols + 255) / 256) * plane_pairs(batch) * 4096 + 256;
+    return (size_t)((cols + 511) / 512) * plane_pairs(batch) * 4096 + 256 + 4096;   // codes: half the bytes for half the columns
 }
 
 int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
@@ -381,10 +401,11 @@ int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     vec16 = a.plane % 16 == 0;
     a.segs = (a.plane + PLANE_SEG - 1) / PLANE_SEG;
     const uint32_t nt = plane_pairs(op.batch);
-    const size_t table = (size_t)a.segs * nt * 4096;
+    const size_t table = (size_t)a.segs * nt * (codes ? 2048 : 4096);
     a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch;
     a.argmax_key = op.argmax_key; a.status = cfg.status; a.wait_limit = op.wait_limit;
-    if (!dry) {
+    a.x = op.x; a.cols = w0.cols;
+    if (!dry && nt > 1) {
         if (!op.prep || ((uintptr_t)op.prep & 15) || table + 64 > op.prep_bytes) return ALICE_E_SHAPE;
         a.table = static_cast<const uint4*>(op.prep);
         a.kappa = reinterpret_cast<const float*>(static_cast<const uint8_t*>(op.prep) + table);
@@ -392,8 +413,9 @@ int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     auto rows = [&](bool plan) { return nt == 1 ? launch_nt<1>(a, codes, vec16, cfg, plan) : nt == 2 ? launch_nt<2>(a, codes, vec16, cfg, plan) : launch_nt<4>(a, codes, vec16, cfg, plan); };
     int rc = rows(true);
     if (rc || dry) return rc;
+    if (nt == 1) return rows(false);
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((a.segs + 7) / 8, 2 * nt); lc.blockDim = dim3(256); lc.stream = cfg.stream;
+    lc.gridDim = dim3((a.segs + (codes ? 15 : 7)) / (codes ? 16 : 8), 2 * nt); lc.blockDim = dim3(256); lc.stream = cfg.stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;

@@ -1,19 +1,17 @@
 // Matvec over ternary bit planes and packed ternary codes for 1..8 input vectors in ONE pass over the weights.
 //
-// The weight bytes are the A operand of the int8 mma.sync, as in csrc/gemv_mma.cuh (A_j = bytes & (1 << j), B = the
-// fixed-point digits of the element bit j stands for, divided by 2^j), but they go from HBM straight into the fragment
-// registers: lane (g, t) of a warp loads 16 bytes of rows g and g + 8 at byte 16 t of a 64-byte segment, which is a whole
-// A fragment for any order of the columns that the B side shares. No ring, no barrier per stage, no shared-memory read
-// of a weight. The digits of two vectors fill the eight B columns, so a second vector costs nothing and every further pair
-// costs its products only: 8 clk per m16n8k32 and SM quarter, measured, against four mask operations for each A fragment.
-//
-// What bounds it: one or two vectors HBM (64 clk of products for the 2 KB a tile segment streams; 2 KB take 89 clk of an SM
-// at 6.5 TB/s), more vectors the int8 products.
+// The weights are the A operand of the int8 mma.sync and the fixed-point digits of the activations the B operand, as in
+// csrc/gemv_mma.cuh, but the bytes go from HBM straight into the fragment registers: lane (g, t) of a warp loads 16 bytes of rows
+// g and g + 8 at byte 16 t of a 64-byte segment, which is a whole A fragment for any order of the columns that the B side shares.
+// No ring, no barrier per stage, no shared-memory read of a weight. Three operations turn the two planes' bits j (or one code
+// place) of four weights into a signed byte each, +-2^j, so a weight takes part in one product, not two. The digits of two
+// vectors fill the eight B columns, so a second vector costs nothing and every further pair costs its products only: 8 clk
+// per m16n8k32 and SM quarter, measured.
 //
 // Split: a cluster of S CTAs owns a range of 16-row tiles, each of its CTAs 1 / S of the columns, whose digit table stays in
 // shared memory for the whole launch (S is the smallest that makes it fit, or larger where a matrix has fewer tiles than the
-// chip has SMs). Inside a CTA the (tile, segment) pairs are dealt evenly to 16 warps; sums are 32-bit integers, added in
-// shared memory with atomics (exact, so the order does not matter) and once per launch over the cluster.
+// chip has SMs). Inside a CTA the (tile, segment) pairs are dealt evenly to 16 warps; sums are integers, added in shared memory
+// with atomics (exact, so the order does not matter) and once per launch over the cluster.
 #pragma once
 #include "gemv_launch.cuh"
 
@@ -30,7 +28,9 @@ struct PlaneArgs {
     const uint8_t* up;                                  // fused SwiGLU: w[0] = gate
     const float* up_scale;
     uint32_t row_bytes, plane, segs;                    // bytes of a row and of a plane; 64-byte segments of a plane
-    const uint4* table;                                 // [segs][NT][8][32]: see plane_table_kernel
+    const float* x;                                     // one or two vectors: the kernel makes the digits itself
+    uint32_t cols;
+    const uint4* table;                                 // more: see plane_table_kernel
     const float* kappa;                                 // value of one fixed-point unit, per vector
     float* y;
     const float* resid;

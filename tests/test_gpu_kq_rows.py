@@ -1,0 +1,49 @@
+"""K-quants over 2..8 vectors (csrc/gemv_kq_rows.cu) against the kernel of a single vector, which other files hold against the oracle:
+edges of the 16-row tiles, of the one- or two-block stages, of the column split over a cluster, rows that begin anywhere.
+
+Both keep the integer block dots; a row adds the scale and the min term of every block in f32, in another order. Either term is up to
+a few times what is left of both (4), and a chain of them rounds a few times (8): 32 times 2^-23 of the sum of magnitudes."""
+import numpy as np
+import pytest
+
+from alice_llm_b200 import synth
+
+pytestmark = pytest.mark.gpu
+Q4_K, Q5_K, Q6_K = synth.Q4_K, synth.Q5_K, synth.Q6_K
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from alice_llm_b200.gpu import GpuEngine
+    e = GpuEngine(0)
+    yield e
+    e.close()
+
+
+def quant(qtype):
+    from alice_llm_b200.gpu import GpuQuantType as Q
+    return {Q4_K: Q.Q4K, Q5_K: Q.Q5K, Q6_K: Q.Q6K}[qtype]
+
+
+@pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("rows,blocks", [(1, 1), (15, 2), (16, 3), (17, 7), (300, 16), (2500, 1), (40, 56), (4099, 5)])
+def test_every_batch(eng, qtype, rows, blocks):
+    cols = 256 * blocks
+    rng = np.random.default_rng(rows + cols)
+    w = eng.upload_weights_typed(synth.make_weights(qtype, rng, rows, cols), rows, cols, quant(qtype))
+    mag = np.abs(eng.dequantize(w).reshape(rows, cols)).astype(np.float64)
+    x = synth.make_x(rng, cols, 8).reshape(8, cols)
+    y = eng.alloc_f32(8 * rows)
+    one = []
+    for k in range(8):
+        eng.matvec_dev(w, eng.upload_f32(x[k]), y, 1)
+        one.append(eng.read_f32(y)[:rows].copy())
+        eng.sync()
+    bound = 32 * 2.0 ** -23 * (1.1 * np.abs(x) @ mag.T) + 1e-30
+    xd = eng.upload_f32(x.reshape(-1))
+    for batch in (2, 3, 5, 8):
+        eng.matvec_dev(w, xd, y, batch)
+        got = eng.read_f32(y)[:batch * rows].reshape(batch, rows).astype(np.float64)
+        eng.sync()
+        err = np.abs(got - np.array(one[:batch], np.float64)) / bound[:batch]
+        assert err.max() <= 1.0, (batch, err.max())

@@ -58,6 +58,22 @@ def test_planes_every_batch(eng, oracle, rows, cols, sparse):
         assert np.array_equal(a, alone[-1][:len(a)])
 
 
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("value", [0.9, -0.9999])
+def test_equal_signs_over_equal_activations(eng, oracle, sparse, value):
+    """The largest sums there are: they need more than 32 bits in fixed-point units."""
+    rows, cols = 20, 28672
+    pos = np.full((rows, cols // 8), 255, np.uint8)
+    pos[1::2] = 0
+    m = (pos, 255 - pos, np.ones(rows, np.float32))
+    x = np.full((3, cols), value, np.float32)
+    w, y = upload(eng, oracle, m, rows, cols, sparse), eng.alloc_f32(3 * rows)
+    eng.matvec_dev(w, eng.upload_f32(x.reshape(-1)), y, 3)
+    got = eng.read_f32(y).reshape(3, rows)
+    eng.sync()
+    check(got, x, m, cols)
+
+
 @pytest.mark.parametrize("rows,cols,batch", [(17, 544, 1), (1000, 4096, 3), (150, 8192, 8), (40, 28672, 8)])
 def test_planes_swiglu(eng, oracle, rows, cols, batch):
     rng = np.random.default_rng(rows + cols)
