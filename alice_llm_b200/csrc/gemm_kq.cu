@@ -397,6 +397,10 @@ int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
         a.up = u.data;
     }
     if (dry) return ALICE_OK;
+    if (op.batch > 64) {
+        const int rc = launch_kq_gemm_tc(op, cfg);
+        if (rc != ALICE_E_SHAPE) return rc;
+    }
     a.nw = op.nw; a.row_bytes = w0.row_bytes; a.nb = w0.cols / 256;
     a.qs = op.q8->qs; a.d = op.q8->d; a.bsums = op.q8->bsums;
     a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch;

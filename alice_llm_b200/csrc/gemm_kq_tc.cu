@@ -1,0 +1,473 @@
+// K-quant products with more than 64 vectors on the fifth-generation tensor cores (tcgen05.mma kind::f16).
+//
+// A weight enters as the integer scale x quant, an activation as its Q8_K integer, both exact in f16: up to 63 * 31 for Q4_K / Q5_K;
+// for Q6_K (up to 128 * 32) as a multiple of 32 and a remainder, two products. The f32 accumulator of one 256-column block then holds
+// the integer dot of q4k_q8k_dot / q6k_q8k_dot (src/gguf.rs:3201-3251, :3282-3319; below 2^24 it is exact, and no sum of 256
+// such products of real weights comes near), a second one the min term (sums of 16 activations, at most 2048, times the
+// 6-bit mins), and both are scaled by the block's f16 and f32 factors and added up in f32 registers once per block.
+//
+// One CTA per SM, 128 rows x 128 vectors, 18 warps: 8 unpack raw blocks (cp.async, a block ahead) into the swizzled A tiles, half a row a
+// thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one thread
+// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM). Where
+// tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
+// What bounds it: shared memory, which the A tiles enter once and leave once beside the B tiles, and the unpacking, which is
+// as long as the products; the integer path of mma.sync (csrc/gemm_kq.cu) spends some 16 instructions per product on scaling.
+#include <algorithm>
+
+#include "../../include/alice_cuda.h"
+#include "common.cuh"
+#include "gemm_kq.cuh"
+#include "gemv_kq_mma.cuh"
+#include "tc_dev.cuh"
+
+namespace alice {
+namespace {
+
+constexpr uint32_t KT_M = 128, KT_N = 128, KT_PROD = 256, KT_EPI = 256, KT_THREADS = KT_PROD + KT_EPI + 64;
+constexpr int KERR_KT_WAIT = 7;      // as the bf16 product: operands or accumulators of a tensor-core product
+
+template <int FMT> struct KtFmt;     // bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles and ring depth
+template <> struct KtFmt<4> { static constexpr uint32_t BB = 144, CH = 9, PITCH = 144, TILES = 5, ASUB = 1, STAGES = 5; };
+template <> struct KtFmt<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 176, TILES = 5, ASUB = 1, STAGES = 4; };
+template <> struct KtFmt<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, TILES = 4, ASUB = 2, STAGES = 3; };
+
+template <int FMT>
+struct KtGeom {
+    using F = KtFmt<FMT>;
+    static constexpr uint32_t A = 16384 * F::ASUB, STAGE = A + 16384, RAW = KT_M * F::PITCH, RING = F::STAGES * STAGE, SMEM = 1024 + RING + 2 * RAW,
+                              KB = F::TILES * 64;      // columns of the prepared activations per block
+    static_assert(RING >= KT_N * (KT_M + 1) * 4, "the parts of the result reuse the ring");
+    static_assert(SMEM <= 226 * 1024, "shared memory of a CTA");
+};
+
+struct KtArgs {
+    const uint8_t* w[3];
+    uint32_t rows[3], y_off[3], tile0[4], nw;
+    const uint8_t* up;
+    uint32_t row_bytes, nb, dstride;
+    const float* dt;             // [nb][dstride]: Q8_K scales
+    float* y;
+    const float* resid;
+    uint32_t y_stride, batch;
+    int* status;
+    CUtensorMap tb;
+};
+
+// Activations as the B tiles want them: x[v][blk * KB + ...] in f16, the columns in the order the unpacked weights have (Q4_K / Q5_K: second
+// and third of every four exchanged), behind a Q4_K / Q5_K block its 16 sums and zeros; scales transposed, zero past the batch.
+template <int FMT>
+__global__ void __launch_bounds__(256) kt_prepare_kernel(const int8_t* qs, const float* d, const int16_t* bsums, uint32_t batch, uint32_t nb, uint32_t dstride, __half* x, float* dt) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr uint32_t KB = KtGeom<FMT>::KB;
+    const uint32_t lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);     // a warp per block
+    if (i >= batch * nb) return;
+    const uint32_t v = i / nb, b = i - v * nb;
+    __half* out = x + ((size_t)v * nb + b) * KB;
+    const uint2 q = __ldcg(reinterpret_cast<const uint2*>(qs + (size_t)i * 256) + lane);
+    uint32_t h[4];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const uint32_t w = k ? q.y : q.x;
+        __half e[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) e[j] = __int2half_rn((int)(int8_t)(w >> (8 * j)));
+        const __half2 p0 = FMT == 6 ? __halves2half2(e[0], e[1]) : __halves2half2(e[0], e[2]), p1 = FMT == 6 ? __halves2half2(e[2], e[3]) : __halves2half2(e[1], e[3]);
+        h[2 * k] = *reinterpret_cast<const uint32_t*>(&p0);
+        h[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&p1);
+    }
+    reinterpret_cast<uint4*>(out)[lane] = make_uint4(h[0], h[1], h[2], h[3]);
+    if (FMT != 6) {
+        const __half2 z = __half2half2(__ushort_as_half(0));
+        const __half2 s = lane < 8 ? __halves2half2(__int2half_rn(bsums[(size_t)i * 16 + 2 * lane]), __int2half_rn(bsums[(size_t)i * 16 + 2 * lane + 1])) : z;
+        reinterpret_cast<__half2*>(out + 256)[lane] = s;
+    }
+    if (lane == 0) dt[(size_t)b * dstride + v] = __ldcg(d + i);
+}
+
+__device__ __forceinline__ uint32_t h2u(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ __half2 u2h(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+template <class V> __device__ __forceinline__ V kld(const uint8_t* p) { return *reinterpret_cast<const V*>(p); }
+__device__ __forceinline__ uint32_t kld_u2(const uint8_t* p) {      // a 32-bit word at a 2-byte boundary
+    const uint32_t a = smem_u32(p) & 2u;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - a);
+    return __funnelshift_r(q[0], q[1], a * 8u);
+}
+
+// `scales`: those of the block half's sub-blocks, this thread's in bytes 0 and 2.
+// 32 weights (k-half `half` of k-tile c) of a raw block as f16 integers into logical 16-byte pieces 4 half .. of row r of the A tile at `at`.
+template <int FMT>
+__device__ __forceinline__ void kt_unpack(const uint8_t* raw, uint32_t scales, uint32_t c, uint32_t half, uint8_t* at, uint32_t r) {
+    if constexpr (FMT != 6) {
+        const uint32_t j = 2 * c + half, sc = (scales >> (16 * (c & 1))) & 0xffu;
+        // a high nibble stays where it is in its byte: 1024 + 16 quant, times scale / 16
+        const __half2 one = __half2half2(__ushort2half_rn((unsigned short)sc)), s2 = half ? __hmul2(one, __float2half2_rn(0.0625f)) : one;
+        const __half2 o2 = __hmul2(s2, __float2half2_rn(-1024.0f));
+        const uint32_t mask = half ? 0x00f000f0u : 0x000f000fu;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint4 q4 = kld<uint4>(raw + (FMT == 5 ? 48 : 16) + 32 * c + 16 * i);
+            const uint32_t w[4] = {q4.x, q4.y, q4.z, q4.w};
+            uint32_t hb[4] = {0u, 0u, 0u, 0u};
+            if (FMT == 5) {
+                const uint4 h4 = kld<uint4>(raw + 16 + 16 * i);
+                hb[0] = h4.x >> j; hb[1] = h4.y >> j; hb[2] = h4.z >> j; hb[3] = h4.w >> j;
+            }
+            uint32_t out[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                uint32_t e = (w[k] & mask) | 0x64006400u, o = ((w[k] >> 8) & mask) | 0x64006400u;
+                if (FMT == 5) {
+                    const uint32_t up = half ? 8 : 4;
+                    e |= (hb[k] & 0x00010001u) << up; o |= ((hb[k] >> 8) & 0x00010001u) << up;
+                }
+                out[2 * k] = h2u(__hfma2(u2h(e), s2, o2));
+                out[2 * k + 1] = h2u(__hfma2(u2h(o), s2, o2));
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const uint32_t piece = 4 * half + 2 * i + k;
+                *reinterpret_cast<uint4*>(at + r * 128 + ((piece ^ (r & 7u)) * 16)) = make_uint4(out[4 * k], out[4 * k + 1], out[4 * k + 2], out[4 * k + 3]);
+            }
+        }
+    } else {
+        const uint32_t n = c >> 1, z = 2 * (c & 1) + half;       // quadrant z of half n of the block
+        const uint8_t* ql = raw + 64 * n + 32 * (z & 1);
+        const uint8_t* qh = raw + 128 + 32 * n;
+        const __half2 m2 = __float2half2_rn(49152.0f);           // sums with it are multiples of 32
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int sc = (int)(int8_t)raw[192 + 8 * n + 2 * z + i];
+            const __half2 s2 = __half2half2(__int2half_rn(sc));
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t w = (k + (r >> 3)) & 3u;          // rows eight apart meet the same banks: let them take another word
+                const uint32_t l = kld_u2(ql + 16 * i + 4 * w) >> (z >> 1 ? 4 : 0), h = kld_u2(qh + 16 * i + 4 * w) >> (2 * z);
+                const uint32_t q = (l & 0x0f0f0f0fu) | ((h & 0x03030303u) << 4);
+                uint32_t hi[2], lo[2];
+#pragma unroll
+                for (int p = 0; p < 2; p++) {                    // bytes 2 p and 2 p + 1, in order
+                    const uint32_t b = __byte_perm(q, 0x64u, p ? 0x4342u : 0x4140u);
+                    const __half2 u = __hsub2(u2h(b), __float2half2_rn(1056.0f));          // quant - 32
+                    const __half2 a = __hsub2(__hfma2(u, s2, m2), m2);                     // the multiple of 32 next to scale * quant
+                    hi[p] = h2u(a);
+                    lo[p] = h2u(__hfma2(u, s2, __hneg2(a)));
+                }
+                const uint32_t to = r * 128 + (((4 * half + 2 * i + (w >> 1)) ^ (r & 7u)) * 16) + (w & 1u) * 8;
+                *reinterpret_cast<uint2*>(at + to) = make_uint2(hi[0], hi[1]);
+                *reinterpret_cast<uint2*>(at + 16384 + to) = make_uint2(lo[0], lo[1]);
+            }
+        }
+    }
+}
+// The mins of a Q4_K / Q5_K block, each for two sums of 16: pieces 0 and 1 of the row.
+__device__ __forceinline__ void kt_mins(uint32_t m, uint32_t half, uint8_t* at, uint32_t r) {
+    uint32_t out[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) out[k] = h2u(__half2half2(__ushort2half_rn((unsigned short)((m >> (8 * k)) & 0xffu))));
+    *reinterpret_cast<uint4*>(at + r * 128 + ((half ^ (r & 7u)) * 16)) = make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+__device__ __forceinline__ void tmem_get8(uint32_t (&r)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(addr)
+        : "memory");
+}
+// what tmem_get8 asked for is there
+__device__ __forceinline__ void tmem_got8(uint32_t (&r)[8], uint32_t (&q)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7])
+        :
+        : "memory");
+}
+
+template <int FMT, bool SW>
+__global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_constant__ KtArgs a, const uint32_t KS) {
+    using F = KtFmt<FMT>;
+    using G = KtGeom<FMT>;
+    extern __shared__ uint8_t raw_smem[];
+    __shared__ __align__(8) uint64_t full_[F::STAGES], empty_[F::STAGES], tfull_[2], tempty_[2], drain_;
+    __shared__ uint32_t tmem_base;
+    // Q8_K scales of the vectors, four blocks deep: when the copies of block k are asked for, block k - 3 has been drained
+    __shared__ __align__(16) float dts[4][KT_N];
+    uint8_t* const ring = raw_smem + (1024u - (smem_u32(raw_smem) & 1023u));
+    uint8_t* const raw = ring + G::RING;
+    const uint32_t ring_s = smem_u32(ring);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    auto bar = [](uint64_t* b, uint32_t i) { return smem_u32(b + i); };
+    const uint32_t rank = KS > 1 ? blockIdx.x % KS : 0u, tile = blockIdx.x / KS, tok0 = blockIdx.y * KT_N;
+    uint32_t s = 0;
+    if (!SW) while (s + 1 < a.nw && tile >= a.tile0[s + 1]) s++;
+    constexpr uint32_t OUT = SW ? KT_M / 2 : KT_M;
+    const uint32_t seg_rows = a.rows[s], r0 = (tile - a.tile0[s]) * OUT;
+    const uint32_t b_lo = a.nb * rank / KS, nblk = a.nb * (rank + 1) / KS - b_lo;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (uint32_t i = 0; i < F::STAGES; i++) { mbar_init(bar(full_, i), KT_PROD + 1); mbar_init(bar(empty_, i), 1); }
+        for (uint32_t i = 0; i < 2; i++) { mbar_init(bar(tfull_, i), 1); mbar_init(bar(tempty_, i), KT_EPI); }
+        mbar_init(smem_u32(&drain_), 1);
+        mbar_fence_init();
+        fence_proxy_async();
+    }
+    if (warp == 17) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "n"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    // row of the matrix behind row i of the tile: with SwiGLU 64 gate rows, then the same 64 of up
+    auto matrix = [&](uint32_t i) { return SW && i >= KT_M / 2 ? a.up : a.w[s]; };
+    auto matrix_row = [&](uint32_t i) { return min(r0 + (SW ? i & (KT_M / 2 - 1) : i), seg_rows - 1); };
+    float acc[64];
+    bool ok = true;
+
+    if (warp < 8) {                       // ---- unpack
+        const uint32_t r = tid >> 1, half = tid & 1u;
+        const uint64_t total = (uint64_t)seg_rows * a.row_bytes;
+        auto fetch = [&](uint32_t k) {
+            if (k < nblk) {
+                uint8_t* const dst = raw + (k & 1u) * G::RAW;
+#pragma unroll 2
+                for (uint32_t i = tid; i < KT_M * F::CH; i += KT_PROD) {
+                    const uint32_t row = i / F::CH, c = i - row * F::CH;
+                    const uint64_t off = (((uint64_t)matrix_row(row) * a.row_bytes + (uint64_t)(b_lo + k) * F::BB) & ~(uint64_t)15) + c * 16;
+                    const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
+                    const uint8_t* m = matrix(row);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + row * F::PITCH + c * 16)), "l"(n ? m + off : m), "r"(n) : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        fetch(0);                         // weights: nothing of the kernel ahead
+        uint32_t it = 0;
+        for (uint32_t k = 0; k < nblk; k++) {      // a warp whose wait ran out still meets the others at the barriers
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(KT_PROD) : "memory");          // block k is in, everyone is done with block k - 1
+            fetch(k + 1);
+            const uint8_t* src = raw + (k & 1u) * G::RAW + r * F::PITCH;
+            if (FMT == 6) src += (matrix_row(r) * a.row_bytes + (b_lo + k) * F::BB) & 15u;
+            uint32_t sl = 0, sh = 0, ml = 0, mh = 0;
+            if (FMT != 6) k4_unpack(kld<uint4>(src), sl, sh, ml, mh);
+#pragma unroll
+            for (uint32_t c = 0; c < F::TILES; c++, it++) {
+                const uint32_t st = it % F::STAGES;
+                ok = __all_sync(0xffffffffu, ok && mbar_wait(bar(empty_, st), ((it / F::STAGES) & 1) ^ 1));
+                if (!ok) break;
+                uint8_t* const at = ring + st * G::STAGE;
+                if (FMT != 6 && c == 4) kt_mins(half ? mh : ml, half, at, r); else kt_unpack<FMT>(src, half ? (c < 2 ? sl >> 8 : sh >> 8) : (c < 2 ? sl : sh), c, half, at, r);
+                fence_proxy_async();
+                mbar_arrive(bar(full_, st));
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else if (warp < 16) {               // ---- drain
+        const uint32_t quad = warp & 3u, ch = (warp - 8) >> 2, i = quad * 32 + lane;
+        const uint8_t* wrow = matrix(i) + (uint64_t)matrix_row(i) * a.row_bytes;
+#pragma unroll
+        for (int j = 0; j < 64; j++) acc[j] = 0.0f;
+        pdl_wait();
+        // scale (and min factor) of this row's block, a block ahead
+        auto head = [&](uint32_t k) -> uint32_t {
+            const uint8_t* blk = wrow + (uint64_t)(b_lo + min(k, nblk - 1)) * F::BB;
+            return FMT == 6 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(blk + 208)) : __ldg(reinterpret_cast<const uint32_t*>(blk));
+        };
+        uint32_t hd = head(0);
+        for (uint32_t k = 0; k < nblk; k++) {
+            const uint32_t b = k & 1u;
+            const float2 f = __half22float2(u2h(hd));
+            hd = head(k + 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(tfull_, b), (k >> 1) & 1));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t base = tmem + b * KT_N + ch * 64 + ((quad * 32) << 16);
+            const float* e = dts[k & 3u] + ch * 64;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                uint32_t p[8], m[8];
+                tmem_get8(p, base + c * 8);
+                tmem_get8(m, base + (FMT != 6 ? 256 + c * 8 : (c ^ 1) * 8));      // Q6_K has no second accumulator: two pieces at a time
+                tmem_got8(p, m);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float x = e[c * 8 + j];
+                    if (FMT != 6) {
+                        acc[c * 8 + j] = fmaf(x, fmaf(-f.y, __uint_as_float(m[j]), f.x * __uint_as_float(p[j])), acc[c * 8 + j]);
+                    } else {
+                        acc[c * 8 + j] = fmaf(f.x * x, __uint_as_float(p[j]), acc[c * 8 + j]);
+                        acc[c * 8 + 8 + j] = fmaf(f.x * e[c * 8 + 8 + j], __uint_as_float(m[j]), acc[c * 8 + 8 + j]);
+                    }
+                }
+                if (FMT == 6) c++;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(bar(tempty_, b));
+        }
+    } else if (warp == 16) {              // ---- B tiles
+        if (lane == 0) {
+            pdl_wait();
+            uint32_t it = 0;
+            for (uint32_t k = 0; k < nblk && ok; k++)
+                for (uint32_t c = 0; c < F::TILES; c++, it++) {
+                    const uint32_t st = it % F::STAGES;
+                    ok = mbar_wait(bar(empty_, st), ((it / F::STAGES) & 1) ^ 1);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(bar(full_, st), c == 0 ? 16384 + KT_N * 4 : 16384);
+                    if (c == 0) bulk_g2s(smem_u32(dts[k & 3u]), a.dt + (size_t)(b_lo + k) * a.dstride + tok0, KT_N * 4, bar(full_, st));
+                    tma_2d(ring_s + st * G::STAGE + G::A, &a.tb, (int)((b_lo + k) * G::KB + c * 64), (int)tok0, bar(full_, st));
+                }
+            // every copy has landed before the CTA may leave
+            const uint32_t last = it < F::STAGES ? it : F::STAGES;
+            for (uint32_t j = it - last; j < it; j++) mbar_wait(bar(full_, j % F::STAGES), (j / F::STAGES) & 1);
+        }
+        __syncwarp();
+    } else {                              // ---- products
+        if (lane == 0) {
+            constexpr uint32_t idesc = (1u << 4) | ((KT_N / 8) << 17) | ((KT_M / 16) << 24);      // f16 x f16 -> f32
+            uint32_t it = 0;
+            for (uint32_t k = 0; k < nblk && ok; k++) {
+                const uint32_t b = k & 1u, d = tmem + b * KT_N;
+                ok = mbar_wait(bar(tempty_, b), ((k >> 1) & 1) ^ 1);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (uint32_t c = 0; c < F::TILES; c++, it++) {
+                    const uint32_t st = it % F::STAGES;
+                    ok = mbar_wait(bar(full_, st), (it / F::STAGES) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t at = ring_s + st * G::STAGE;
+                    const uint64_t db = smem_desc(at + G::A);
+                    if (FMT != 6 && c == 4) {
+                        mma_f16(d + 256, smem_desc(at), db, idesc, false);
+                    } else {
+#pragma unroll
+                        for (uint32_t z = 0; z < F::ASUB; z++) {
+                            const uint64_t da = smem_desc(at + z * 16384);
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) mma_f16(d, da + 2 * kk, db + 2 * kk, idesc, c > 0 || z > 0 || kk > 0);
+                        }
+                    }
+                    mma_commit(bar(empty_, st));
+                }
+                if (ok) mma_commit(bar(tfull_, b));
+            }
+            mma_commit(smem_u32(&drain_));
+            ok = mbar_wait(smem_u32(&drain_), 0) && ok;
+        }
+        __syncwarp();
+    }
+    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_KT_WAIT);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();                      // the ring is free: all products and copies are done
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float* const part = reinterpret_cast<float*>(ring);            // [vector][128 rows]
+    constexpr uint32_t PP = KT_M + 1;
+    if (warp >= 8 && warp < 16) {
+        const uint32_t i = (warp & 3u) * 32 + lane, ch = (warp - 8) >> 2;
+#pragma unroll
+        for (int j = 0; j < 64; j++) part[(ch * 64 + j) * PP + i] = acc[j];
+    }
+    auto meet = [&]() {
+        if (KS > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    };
+    meet();
+    auto total_at = [&](uint32_t v, uint32_t i) {
+        if (KS == 1) return part[v * PP + i];
+        const uint32_t at = ring_s + (v * PP + i) * 4;
+        float f = 0.0f;
+        for (uint32_t q = 0; q < KS; q++) {
+            uint32_t remote;
+            float x;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(q));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
+            f = q ? f + x : x;
+        }
+        return f;
+    };
+    pdl_wait();                           // the residual may be what an earlier kernel wrote (threads that have not waited yet)
+    for (uint32_t i = rank * KT_THREADS + tid; i < KT_N * OUT; i += KS * KT_THREADS) {
+        const uint32_t v = i / OUT, r = i % OUT, tok = tok0 + v, row = r0 + r;
+        if (tok >= a.batch || row >= seg_rows) continue;
+        float f = total_at(v, r);
+        if (SW) f = silu_ref(f) * total_at(v, r + KT_M / 2);
+        const size_t at = (size_t)tok * a.y_stride + a.y_off[s] + row;
+        if (a.resid != nullptr) f = __fadd_rn(__ldcg(a.resid + at), f);
+        a.y[at] = f;
+    }
+    meet();
+    if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+}
+
+template <int FMT, bool SW>
+int launch_tc(KtArgs a, const GemvOp& op, const LaunchCfg& cfg) {
+    using G = KtGeom<FMT>;
+    static bool done[64] = {};
+    auto kern = kq_gemm_tc_kernel<FMT, SW>;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return ALICE_E_CUDA;
+    if (dev >= 64 || !done[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM) != cudaSuccess) return ALICE_E_CUDA;
+        if (dev < 64) done[dev] = true;
+    }
+    constexpr uint32_t per = SW ? KT_M / 2 : KT_M;
+    for (uint32_t i = 0; i < a.nw; i++) a.tile0[i + 1] = a.tile0[i] + (a.rows[i] + per - 1) / per;
+    const uint32_t toks = (a.batch + KT_N - 1) / KT_N;
+    a.dstride = toks * KT_N;
+    // scratch: prepared activations, then scales
+    const size_t xbytes = (size_t)a.batch * a.nb * G::KB * 2, need = xbytes + (size_t)a.nb * a.dstride * 4;
+    if (!op.prep || ((uintptr_t)op.prep & 15) || need > op.prep_bytes) return ALICE_E_SHAPE;
+    auto* x = static_cast<__half*>(op.prep);
+    auto* dt = reinterpret_cast<float*>(static_cast<uint8_t*>(op.prep) + xbytes);
+    a.dt = dt;
+    if (!encode_fn() || !tile_map(&a.tb, x, a.batch, a.nb * G::KB, a.nb * G::KB, KT_N)) return ALICE_E_SHAPE;
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    lc.stream = cfg.stream;
+    lc.gridDim = dim3((a.batch * a.nb + 7) / 8); lc.blockDim = dim3(256);
+    lc.attrs = at + 1; lc.numAttrs = cfg.pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&lc, kt_prepare_kernel<FMT>, op.q8->qs, op.q8->d, op.q8->bsums, a.batch, a.nb, a.dstride, x, dt) != cudaSuccess) return ALICE_E_CUDA;
+    const uint32_t tiles = a.tile0[a.nw], sms = (uint32_t)std::max(cfg.num_sms, 1);
+    uint32_t KS = 1;
+    while (KS < 8 && tiles * toks * KS * 2 <= sms && a.nb >= 8 * KS) KS *= 2;
+    at[0].val.clusterDim.x = KS;
+    lc.gridDim = dim3(tiles * KS, toks); lc.blockDim = dim3(KT_THREADS); lc.dynamicSmemBytes = G::SMEM;
+    lc.attrs = KS > 1 ? at : at + 1;
+    lc.numAttrs = (KS > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
+    return cudaLaunchKernelEx(&lc, kern, a, KS) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
+}
+
+}  // namespace
+
+size_t kq_tc_prep_bytes(uint32_t cols, uint32_t batch) {
+    const size_t nb = (cols + 255) / 256;
+    return (size_t)batch * nb * 640 + nb * ((batch + 127) / 128 * 128) * 4;
+}
+
+int launch_kq_gemm_tc(const GemvOp& op, const LaunchCfg& cfg) {
+    const WeightDesc& w0 = *op.w[0];
+    KtArgs a = {};
+    uint32_t total = 0;
+    for (uint32_t i = 0; i < op.nw; i++) {
+        a.w[i] = op.w[i]->data; a.rows[i] = op.w[i]->rows; a.y_off[i] = op.y_off[i];
+        total += op.w[i]->rows;
+    }
+    if (op.up) a.up = op.up->data;
+    a.nw = op.nw; a.row_bytes = w0.row_bytes; a.nb = w0.cols / 256;
+    a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch; a.status = cfg.status;
+    if (op.up) return w0.fmt == WF_Q4_K ? launch_tc<4, true>(a, op, cfg) : w0.fmt == WF_Q5_K ? launch_tc<5, true>(a, op, cfg) : launch_tc<6, true>(a, op, cfg);
+    return w0.fmt == WF_Q4_K ? launch_tc<4, false>(a, op, cfg) : w0.fmt == WF_Q5_K ? launch_tc<5, false>(a, op, cfg) : launch_tc<6, false>(a, op, cfg);
+}
+
+}  // namespace alice

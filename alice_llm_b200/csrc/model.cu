@@ -10,6 +10,7 @@
 
 #include "abi_internal.cuh"
 #include "attn_body.cuh"
+#include "gemm_kq.cuh"
 #include "gemv_blocks.cuh"
 #include "gemv_planes.cuh"
 #include "glue.cuh"
@@ -484,7 +485,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
     if (!rc) rc = dev_alloc(m, &m->hid_xn, (size_t)B * c.hidden_dim);
     if (!rc) {
         const uint32_t widest = std::max({c.hidden_dim, c.intermediate_dim, q_dim});
-        m->prep_bytes = std::max({mma_prep_bytes(widest), plane_prep_bytes(widest, MAX_BATCH), blocks_prep_bytes(widest, MAX_BATCH)});
+        m->prep_bytes = std::max({mma_prep_bytes(widest), plane_prep_bytes(widest, MAX_BATCH), blocks_prep_bytes(widest, MAX_BATCH), kq_tc_prep_bytes(widest, B)});
         rc = dev_alloc(m, &m->prep, m->prep_bytes);
     }
     if (!rc) rc = dev_alloc(m, &m->d_pos, 1);
