@@ -11,8 +11,9 @@
 // fits no single CTA or a matrix has few rows; the (tile, stage) pairs of a CTA are dealt evenly to its warps and the parts of a
 // tile are added in a fixed order.
 //
-// What bounds it: Q8_0 HBM at any batch (one product per 544 bytes); Q1_0 and Q2_0 the instructions for one or two vectors
-// (Q1_0 about 95 per 576 bytes, an SM issues 100 while those stream), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
+// What bounds it: Q8_0 HBM at any batch (one product per 544 bytes: 32768 x 4096 36.5 us for one vector, 56 for eight); Q1_0 and Q2_0
+// the instructions for one or two vectors (Q1_0 about 75 per 576 bytes for one, an SM issues 100 while those stream: 102400 x 5120 in
+// 32.5 us, 2.3 TB/s), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -156,8 +157,51 @@ __device__ __forceinline__ void mma_s8s8_k32(int (&c)[4], uint32_t a0, uint32_t 
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
-// AL: rows are multiples of 16 bytes, so a stage starts on a 16-byte boundary.
-template <int FMT, int NT, bool SW, bool AL>
+__device__ __forceinline__ void mma0_u8s8_k32p(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+// Two Q1_0 blocks of rows g and g + 8 for ONE vector in eight products of 32: the first block in k slots 0 .. 15 against columns 0 .. 3, the
+// second in slots 16 .. 31 against columns 4 .. 7 (their records are zero in the other four), so quad lanes 0 and 1 hold the digit sums of
+// the first, 2 and 3 those of the second, and each finishes one block. About 75 instructions per 576 bytes against 120 block by block.
+// With rows of whole 16 bytes the second block's signs are aligned words, the first one's lie between two.
+template <bool AL>
+__device__ __forceinline__ void q1_pair(const uint8_t* pA, const uint8_t* pB, const uint8_t* rec, const uint8_t* tsum, bool second, uint32_t lane, float (&acc)[2]) {
+    const uint32_t t = lane & 3u, which = t >> 1;
+    uint32_t a0, a1, a2, a3;
+    if (AL) {
+        const uint32_t *qA = reinterpret_cast<const uint32_t*>(pA) + t, *qB = reinterpret_cast<const uint32_t*>(pB) + t;
+        a0 = __byte_perm(qA[0], qA[1], 0x5432); a1 = __byte_perm(qB[0], qB[1], 0x5432);
+        a2 = qA[5]; a3 = qB[5];
+    } else {
+        a0 = ld_u2(pA + 2 + 4 * t); a1 = ld_u2(pB + 2 + 4 * t);
+        a2 = ld_u2(pA + 20 + 4 * t); a3 = ld_u2(pB + 20 + 4 * t);
+    }
+    float dA = f16_bits_to_f32(ld<uint16_t>(pA + 18 * which)), dB = f16_bits_to_f32(ld<uint16_t>(pB + 18 * which));
+    if (!second) {       // an odd number of blocks: what lies there is no block
+        a2 = a3 = 0u;
+        if (which) dA = dB = 0.0f;
+    }
+    int c0[4], c1[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint4 x = ld<uint4>(rec + h * 512 + lane * 16), z = ld<uint4>(rec + 1024 + h * 512 + lane * 16);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t m = 0x01010101u << (4 * h + j);
+            int (&c)[4] = j & 1 ? c1 : c0;
+            if (h == 0 && j < 2) mma0_u8s8_k32p(c, a0 & m, a1 & m, a2 & m, a3 & m, w4(x, j), w4(z, j));
+            else mma_u8s8_k32p(c, a0 & m, a1 & m, a2 & m, a3 & m, w4(x, j), w4(z, j));
+        }
+    }
+    const int T = (int)ld<uint32_t>(tsum + which * 16 + (t & 1u) * 4);
+    const int vA = 2 * ((c0[0] + c1[0]) * 256 + (c0[1] + c1[1])) - T, vB = 2 * ((c0[2] + c1[2]) * 256 + (c0[3] + c1[3])) - T;
+    acc[0] = fmaf(dA, (float)vA, acc[0]);
+    acc[1] = fmaf(dB, (float)vB, acc[1]);
+}
+
+// AL: rows are multiples of 16 bytes, so a stage starts on a 16-byte boundary. ONE: one vector, Q1_0 blocks in pairs.
+template <int FMT, int NT, bool SW, bool AL, bool ONE>
 __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __grid_constant__ BlkArgs a, const uint32_t S) {
     extern __shared__ __align__(128) uint8_t smem[];
     using F = BlkFmt<FMT>;
@@ -225,8 +269,18 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
             const float amax = vec_amax<BLK_WARPS * 32>(xv, a.nb * F::EL, true, s_red, finite);
             block_fixed_scale(amax, finite, to_fixed, kappa);
             if (tid == 0) s_kappa[v] = kappa;
-            for (uint32_t i = tid; i < ((nblk * 8 + 31) & ~31u); i += BLK_WARPS * 32)
+            for (uint32_t i = tid; i < ((nblk * 8 + 31) & ~31u); i += BLK_WARPS * 32) {
+                if (ONE) {       // odd blocks in columns 4 .. 7, zeros in the others
+                    const uint32_t b = i / 8, col = b & 1u;
+                    uint8_t* rec = dtab + b * F::DIG;
+                    if (b < nblk)
+#pragma unroll
+                        for (uint32_t d = 0; d < 4; d++) reinterpret_cast<uint4*>(rec)[((i >> 2) & 1u) * 32 + ((1 - col) * 4 + d) * 4 + (i & 3u)] = make_uint4(0u, 0u, 0u, 0u);
+                    block_record<FMT>(xv + (size_t)(b_lo + b) * F::EL, b < nblk, i % 8, col, to_fixed, rec, dsum + b * 4);
+                    continue;
+                }
                 block_record<FMT>(xv + (size_t)(b_lo + i / 8) * F::EL, i / 8 < nblk, i % 8, v, to_fixed, dtab + (i / 8) * F::DIG, dsum + (i / 8) * 4 + v * 2);
+            }
         }
         __syncthreads();
     } else {
@@ -259,8 +313,9 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const float f = (t & 1u) ? acc[n][h] : acc[n][h] * 65536.0f;
-                const float y = f + __shfl_xor_sync(0xffffffffu, f, 1);
-                if (!(t & 1u)) dst[(g + 8 * h) * (2 * NT) + 2 * n + (t >> 1)] = y;
+                float y = f + __shfl_xor_sync(0xffffffffu, f, 1);
+                if (ONE) y += __shfl_xor_sync(0xffffffffu, y, 2);
+                if (ONE ? t == 0 : !(t & 1u)) dst[(g + 8 * h) * (2 * NT) + 2 * n + (t >> 1)] = y;
                 acc[n][h] = 0.0f;
             }
         mid = false;
@@ -331,7 +386,10 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
                 }
             }
         };
-        if (nbi == BLK_ITEM) {
+        if constexpr (ONE) {
+#pragma unroll 2
+            for (uint32_t b = 0; b < nbi; b += 2) q1_pair<AL>(rowA + b * F::BB, rowB + b * F::BB, rec + b * F::DIG, trec + b * 16 - t * 4, b + 1 < nbi, lane, acc[0]);
+        } else if (nbi == BLK_ITEM) {
 #pragma unroll(FMT == 0 ? 4 : 2)
             for (uint32_t b = 0; b < BLK_ITEM; b++) block(b);
         } else {
@@ -397,12 +455,12 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
     }
 }
 
-template <int FMT, int NT, bool SW, bool AL>
-int plan_and_launch(BlkArgs a, const LaunchCfg& cfg, bool dry) {
+template <int FMT, int NT, bool SW, bool AL, bool ONE>
+int plan_and_launch_one(BlkArgs a, const LaunchCfg& cfg, bool dry) {
     using F = BlkFmt<FMT>;
     static bool attr_done[64] = {};
     static int clusters[64][4] = {};
-    auto kern = block_rows_kernel<FMT, NT, SW, AL>;
+    auto kern = block_rows_kernel<FMT, NT, SW, AL, ONE>;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ALICE_E_CUDA;
     if (!attr_done[dev]) {
@@ -449,6 +507,13 @@ int plan_and_launch(BlkArgs a, const LaunchCfg& cfg, bool dry) {
         return cudaLaunchKernelEx(&lc, kern, a, S) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
     }
     return ALICE_E_SHAPE;
+}
+
+template <int FMT, int NT, bool SW, bool AL>
+int plan_and_launch(const BlkArgs& a, const LaunchCfg& cfg, bool dry) {
+    if constexpr (FMT == 1 && NT == 1)
+        if (a.batch == 1) return plan_and_launch_one<FMT, NT, SW, AL, true>(a, cfg, dry);
+    return plan_and_launch_one<FMT, NT, SW, AL, false>(a, cfg, dry);
 }
 
 template <int FMT, int NT>

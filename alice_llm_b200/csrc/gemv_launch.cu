@@ -480,8 +480,8 @@ static int launch_split(int (*launch)(const GemvOp&, const LaunchCfg&, bool), co
 static bool one_vector_warp_ring(const GemvOp& op) {
     const WeightDesc& w = *op.w[0];
     switch (w.fmt) {
-        // Q2_0: 51200 x 5120 27.4 against 36.8 us, 4096 x 4096 8.2 against 9.1. Q1_0: 151936 x 1024 16.5 against 31.5, 5120 x 25600 19.8 against
-        // 21.0, 25600 x 5120 15.0 against 14.9, 7168 x 5120 10.7 against 9.8; a 27B model 13.03 against 13.48 ms for two tokens.
+        // Q2_0: 51200 x 5120 27.4 against 36.8 us, 4096 x 4096 8.2 against 9.1. Q1_0: 151936 x 1024 14.3 against 31.5, 5120 x 25600 17.5 against
+        // 21.0, 25600 x 5120 13.0 against 14.9, 7168 x 5120 9.4 against 9.8, 4096 x 4096 7.1 against 8.9.
         case WF_Q1_0: case WF_Q2_0: return true;
         // Widths at which the ring kernel's lanes stand idle (it deals 16-column units to 32 P lanes, 1, 2 or 4 each): 151936 x 5120 148 against
         // 262 us; 32768 x 4096 37.5 against 33.8, 4096 x 14336 27.7 against 22.3.
