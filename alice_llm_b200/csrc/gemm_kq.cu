@@ -6,8 +6,8 @@
 // A CTA (WM x WN warps) owns 32 WM rows x 8 NTW WN tokens and walks the 256-column blocks: raw weight blocks and Q8_K blocks come
 // in with cp.async one to two blocks ahead, a warp unpacks 32 rows of a sub-block into A fragments and uses them for its NTW x 8
 // tokens (32: sums in int32 and f32 then leave room for two CTAs of eight warps an SM). The min / bias term is a pair of products of the scales with base-64 digits of the activation sums, once per block.
-// What bounds it: from 64 tokens on the int8 products (8 clk each and SM quarter) together with the four multiply-adds that
-// scale each of them; below, HBM. Where tiles are fewer than two per SM, a cluster shares the columns of a tile and adds its
+// What bounds it: the instructions around the products (eight to sixteen each), for few tokens HBM. 9 to 64 tokens; more run on tcgen05
+// (csrc/gemm_kq_tc.cu). Where tiles are fewer than two per SM, a cluster shares the columns of a tile and adds its
 // parts through distributed shared memory in a fixed order.
 #include <algorithm>
 

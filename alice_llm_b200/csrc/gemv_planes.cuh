@@ -8,6 +8,9 @@
 // vectors fill the eight B columns, so a second vector costs nothing and every further pair costs its products only: 8 clk
 // per m16n8k32 and SM quarter, measured.
 //
+// 28672 x 8192: one vector 20.0 us (27.8 by the ring kernel), eight 40.2 us (eight times 27.8). What bounds it: one or two vectors the
+// stream and the instructions on it alike (2.9 TB/s), eight the products.
+//
 // Split: a cluster of S CTAs owns a range of 16-row tiles, each of its CTAs 1 / S of the columns, whose digit table stays in
 // shared memory for the whole launch (S is the smallest that makes it fit, or larger where a matrix has fewer tiles than the
 // chip has SMs). Inside a CTA the (tile, segment) pairs are dealt evenly to 16 warps; sums are integers, added in shared memory
