@@ -103,11 +103,21 @@ __device__ __forceinline__ void epi_swiglu_32(const GemmOp& op, uint32_t t, uint
     const size_t o = (size_t)t * op.ldo + c;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        float r[8];
+        float r[8], gb[8], ub[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) gb[j] = ub[j] = 0.0f;
+        if (op.bias) {
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                const float4 x = __ldg(reinterpret_cast<const float4*>(op.bias + c + 8 * i + j)), y = __ldg(reinterpret_cast<const float4*>(op.bias2 + c + 8 * i + j));
+                gb[j] = x.x; gb[j + 1] = x.y; gb[j + 2] = x.z; gb[j + 3] = x.w;
+                ub[j] = y.x; ub[j + 1] = y.y; ub[j + 2] = y.z; ub[j + 3] = y.w;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int k = 8 * i + j;
-            r[j] = op.bias ? silu_ref(g[k] + __ldg(op.bias + c + k)) * (u[k] + __ldg(op.bias2 + c + k)) : silu_ref(g[k]) * u[k];
+            r[j] = silu_ref(g[k] + gb[j]) * (u[k] + ub[j]);
         }
         uint32_t w[4];
 #pragma unroll
