@@ -1,8 +1,8 @@
 // bf16 tiled product on the fifth-generation tensor cores: C[t][n] = sum_k A[t][k] W[n][k].
 //
-// Persistent, one CTA per SM, six warps: warp 0 copies 128 x 64 and BN x 64 tiles by TMA (128-byte swizzle) into a ring of
-// stages, warp 1 issues tcgen05.mma from one thread into one of two TMEM accumulators, warps 2-5 drain the other one and
-// apply the epilogue. Every wait is bounded: when one runs out the kernel records it in the status word, lets its copies and
+// Persistent, one CTA per SM, ten warps: warp 0 copies 128 x 64 and BN x 64 tiles by TMA (128-byte swizzle) into a ring of
+// stages, warp 1 issues tcgen05.mma from one thread into one of two TMEM accumulators, warps 2-9 drain the other one, half of its columns
+// each four, and apply the epilogue. Every wait is bounded: when one runs out the kernel records it in the status word, lets its copies and
 // products finish, gives its TMEM back and returns.
 #pragma once
 #include "dense_epi.cuh"
@@ -10,7 +10,7 @@
 
 namespace alice {
 
-constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 192;
+constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 320;
 template <int BN>
 struct TcGeom {
     static constexpr int STAGES = BN == 256 ? 4 : 6;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int i = 0; i < G::STAGES; i++) { mbar_init(bar(full_, i), 1); mbar_init(bar(empty_, i), 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(bar(tfull_, i), 1); mbar_init(bar(tempty_, i), 128); }
+        for (int i = 0; i < 2; i++) { mbar_init(bar(tfull_, i), 1); mbar_init(bar(tempty_, i), 256); }
         mbar_init(smem_u32(&drain_), 1);
         mbar_fence_init();
         fence_proxy_async();
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             if (!mbar_wait(smem_u32(&drain_), 0)) atomicCAS(a.status, 0, KERR_TC_WAIT);
         }
     } else {
-        const uint32_t quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t quad = warp & 3, row = quad * 32 + lane, half = (warp - 2) >> 2;
         uint32_t i = 0;
         for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, i++) {
             const int b = (int)(i & 1);
@@ -214,19 +214,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             const uint32_t base = tmem + (uint32_t)b * BN + ((quad * 32) << 16);
             if constexpr (EPI == EPI_SWIGLU) {
 #pragma unroll 1
-                for (uint32_t c = 0; c < BN; c += 128) {
+                for (uint32_t p = half * (BN / 128); p < (half + 1) * (BN / 128); p++) {      // 32 outputs each
+                    const uint32_t c = p / 2 * 128, j = p % 2 * 32;
                     if (n0 + c >= op.w.n) break;
-#pragma unroll 1
-                    for (uint32_t j = 0; j < 64; j += 32) {
-                        float g[32], u[32];
-                        tmem_ld32(g, base + c + j);
-                        tmem_ld32(u, base + c + 64 + j);
-                        if (t < op.tokens) epi_swiglu_32(op, t, (n0 + c) / 2 + j, g, u);
-                    }
+                    float g[32], u[32];
+                    tmem_ld32(g, base + c + j);
+                    tmem_ld32(u, base + c + 64 + j);
+                    if (t < op.tokens) epi_swiglu_32(op, t, (n0 + c) / 2 + j, g, u);
                 }
             } else {
 #pragma unroll 1
-                for (uint32_t c = 0; c < BN; c += 32) {
+                for (uint32_t c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
                     if (n0 + c >= op.w.n) break;
                     float v[32];
                     tmem_ld32(v, base + c);
