@@ -170,7 +170,9 @@ int32_t alice_dequantize(alice_engine* e, const alice_weights* w, alice_buf* out
  * pre-quantized Q8_K input when preq != 0): out[0..9] = CTAs, warps per row (or per 16-row tile), row sets per CTA,
  * rows per set per stage, stage-sized row groups in total, ring stages, activation units per lane, 1 if the bit-plane
  * tensor-core kernel is used, column chunks, CTAs per SM. A CTA handles about groups / CTAs stages, so a test can
- * assert that a shape really re-uses the ring. No reference counterpart (diagnostic). */
+ * assert that a shape really re-uses the ring. It describes the ring kernels, which serve single vectors of most shapes and
+ * every tensor-parallel rank; ternary, Q1_0 and Q2_0 matrices and batches run in kernels without that geometry. No reference
+ * counterpart (diagnostic). */
 int32_t alice_plan_query(alice_engine* e, const alice_weights* w, int32_t swiglu, int32_t preq, uint32_t* out, uint32_t n_out);
 
 /* How alice_matvec / alice_swiglu run `batch` input vectors over `w`: the number of kernel launches and how many times
@@ -197,7 +199,7 @@ int32_t alice_engine_tp_info(const alice_engine* e, uint32_t* rank, uint32_t* wo
  * rms_norm -> q/k/v matvec -> RoPE -> KV append -> GQA attention -> o matvec + residual ->
  * rms_norm -> fused SwiGLU gate/up -> down matvec + residual; then output norm and head.
  * One decode step is five large kernels per layer (q/k/v, attention, o, gate/up, down) with a small kernel in front of
- * each matvec that prepares its input once (rms_norm, Q8_K blocks or the f32 vector and its digit table), replayed from a
+ * most matvecs that prepares their input once (rms_norm, Q8_K blocks or the f32 vector), replayed from a
  * CUDA graph; position and token live on the device. K-quant projections use the CPU model's semantics (Q8_K-quantized
  * activations).
  * On an engine that is rank r of a tensor-parallel group of n, the config stays the whole model's and the
