@@ -106,9 +106,10 @@ Q8KView q8_view(uint8_t* base, uint32_t n, uint32_t cap) {
     return v;
 }
 
-// The int8 kernels of Q8_0, Q1_0, Q2_0 and the ternary formats take their input as a finished f32 vector in global memory, left
+// The kernels of Q8_0, Q1_0, Q2_0 and the ternary formats take their input as a finished f32 vector in global memory, left
 // there by the kernel that produced the vector; the K-quant kernels take Q8_K blocks that a small kernel prepares between producer
-// and consumer. A Q8_0 matrix beside one that wants the vector on the Q8_K grid prepares the raw vector in its own prologue.
+// and consumer. A matrix of another prepared format beside a Q1_0 / Q2_0 one, which wants the vector on the Q8_K grid, takes the raw
+// vector and prepares it in its own prologue.
 bool wants_prepared(const WeightDesc& w) {
     return (w.fmt == WF_Q8_0 || w.fmt == WF_Q1_0 || w.fmt == WF_Q2_0 || w.fmt == WF_TERNARY || w.fmt == WF_SPARSE_TERNARY) && w.cols % 4 == 0;
 }
@@ -193,11 +194,11 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     // one-CTA kernel prepares (norm + Q8_K) ahead of the matvec - the matvec is its programmatic dependent, so its CTAs
     // are resident and streaming weights meanwhile (measured on the 8B decode step: 2.23 ms per token this way, 2.28
     // with every CTA of the matvec normalising and quantizing the vector itself); else the raw vector plus the norm
-    // weights, prepared per CTA. `fresh` = the hidden state has changed since the last such preparation.
+    // weights, prepared per CTA. `fresh` = no product since the hidden state changed has had its Q8_K blocks prepared.
     Q8KView hid_view = q8_view(m->hid_q8, H, m->cap);
     auto hidden_input = [&](GemvOp& op, const WeightDesc& w, const float* norm_w, bool via_preq, bool fresh, bool beside_grid = false) -> int {
         op.batch = batch;
-        if (wants_prepared(w) && !(w.fmt == WF_Q8_0 && beside_grid)) { op.x = m->hid_xn; return ALICE_OK; }
+        if (wants_prepared(w) && (!beside_grid || preq_roundtrip(w))) { op.x = m->hid_xn; return ALICE_OK; }
         if (format_uses_q8k(w.fmt)) {
             if (fresh) {
                 Publish p{};
@@ -246,11 +247,13 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
         } else {   // mixed formats (e.g. V kept at higher precision): one launch each
             const WeightDesc* ws[3] = {&L.q, &L.k, &L.v};
             const uint32_t offs[3] = {0, lq, lq + lkv};
+            const bool beside_grid = preq_roundtrip(L.q) || preq_roundtrip(L.k) || preq_roundtrip(L.v);
+            bool blocks = false;       // hid_q8 holds this layer's vector: the first K-quant of the three prepares it, whichever it is
             for (int i = 0; i < 3; i++) {
-                GemvOp op; Q8KView view;
+                GemvOp op;
                 op.w[0] = ws[i];
-                const bool beside_grid = preq_roundtrip(L.q) || preq_roundtrip(L.k) || preq_roundtrip(L.v);
-                if ((rc = hidden_input(op, *ws[i], L.attn_norm, true, i == 0, beside_grid))) return rc;
+                if ((rc = hidden_input(op, *ws[i], L.attn_norm, true, !blocks, beside_grid))) return rc;
+                blocks = blocks || op.q8 != nullptr;
                 op.y = m->qkv + offs[i]; op.y_stride = qkv_stride;
                 if ((rc = gemv(m, op, "q/k/v"))) return rc;
             }
