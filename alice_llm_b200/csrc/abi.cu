@@ -247,7 +247,7 @@ static int run_gemv(alice_engine* e, const alice_weights* w0, const alice_weight
                     float* y, uint32_t batch, const char* who, bool may_alloc = true) {
     GemvOp op;
     const WeightFormat f = w0->d.fmt;
-    if (!format_uses_q8k(f) && f != WF_BF16) {
+    if (!format_uses_q8k(f) && f != WF_Q8_0 && f != WF_BF16) {
         // room for the activation digit table, prepared once ahead of the matvec (csrc/gemv_mma.cuh)
         if (may_alloc) { const int rc = ensure_prep(e, std::max({mma_prep_bytes(w0->d.cols), plane_prep_bytes(w0->d.cols, batch), blocks_prep_bytes(w0->d.cols, batch)})); if (rc) return rc; }
         op.prep = e->prep; op.prep_bytes = e->prep_bytes;

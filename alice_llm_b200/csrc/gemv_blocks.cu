@@ -1,18 +1,25 @@
 // Kernels and launch of csrc/gemv_blocks.cuh.
 //
-// A block is an f16 scale and 32 int8 (Q8_0), 128 signs (Q1_0) or 128 two-bit slots (Q2_0); blocks are 2-byte aligned. The f32
-// activations become 31-bit fixed point (unit 2^-30 of a power of two above the largest) in four signed base-256 digits; the
-// digits of two vectors fill the eight B columns. A operand: the int8 weights themselves, or bytes & (1 << j), or the two bits of a slot at once (0 .. 3 times 4^q). A block's sum is an exact integer (two digits joined in
-// 32 bits: at most 16 bytes x 255 x 128 x 257), the offset of the one- and two-bit codes is taken off in integers too (2 S - T, S - T with T summed over the same
-// digits), and one f32 multiply-add per block scales it.
+// A block is an f16 scale and 32 int8 (Q8_0), 128 signs (Q1_0) or 128 two-bit slots (Q2_0); blocks are 2-byte aligned.
+//
+// Q1_0 and Q2_0 run on the int8 tensor path: the f32 activations become 31-bit fixed point (unit 2^-30 of a power of two above the
+// largest) in four signed base-256 digits; the digits of two vectors fill the eight B columns. A operand: bytes & (1 << j), or the
+// two bits of a slot at once (0 .. 3 times 4^q). A block's sum is an exact integer (two digits joined in 32 bits: at most 16 bytes x
+// 255 x 128 x 257), the offset of the codes is taken off in integers too (2 S - T, S - T with T summed over the same digits), and one
+// f32 multiply-add per block scales it.
+//
+// Q8_0 runs in f32 throughout: fixed point with one exponent for a vector would take the bits of its small elements, and with them the
+// results of rows whose weights at the large ones are near zero. A weight d * q has 19 bits, so it is exact; a lane keeps four rows x
+// four columns of a block in registers and uses them for every vector, whose elements come from shared memory.
 //
 // Every warp has a ring of its own in shared memory (16 rows x 8 blocks a stage, cp.async, no barrier between warps); the digit
-// table of a CTA's columns stays in shared memory for the whole launch. A cluster of S CTAs shares the columns where the table
-// fits no single CTA or a matrix has few rows; the (tile, stage) pairs of a CTA are dealt evenly to its warps and the parts of a
-// tile are added in a fixed order.
+// table (Q8_0: the vectors) of a CTA's columns stays in shared memory for the whole launch. A cluster of S CTAs shares the columns
+// where the table fits no single CTA or a matrix has few rows; the (tile, stage) pairs of a CTA are dealt evenly to its warps and the
+// parts of a tile are added in a fixed order.
 //
-// What bounds it: Q8_0 HBM at any batch (one product per 544 bytes: 32768 x 4096 36.5 us for one vector, 56 for eight); Q1_0 and Q2_0
-// the instructions for one or two vectors (Q1_0 about 75 per 576 bytes for one, an SM issues 100 while those stream: 102400 x 5120 in
+// What bounds it: Q8_0 the instructions (16 weights a lane and block to unpack, scale and multiply with each vector; 151936 x 5120 196 us
+// for one vector, 228 by the ring kernel; 32768 x 4096 44 us for two, 57 for four, 99 for eight, 34 for each by the ring kernel); Q1_0 and
+// Q2_0 the instructions for one or two vectors (Q1_0 about 75 per 576 bytes for one, an SM issues 100 while those stream: 102400 x 5120 in
 // 32.5 us, 2.3 TB/s), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
 #include <algorithm>
 
@@ -28,9 +35,9 @@ constexpr int BLK_WARPS = 16;
 constexpr uint32_t BLK_ITEM = 8;                 // blocks of a row a stage holds
 constexpr uint32_t BLK_SMEM = 224 * 1024, BLK_HDR = 128;
 
-template <int FMT> struct BlkFmt;                // bytes and elements of a block, digit bytes per block and pair of vectors, row pitch of a stage
-// pitch: 32-bit reads of 8 rows x 16 bytes fill the banks once (48 modulo 128)
-template <> struct BlkFmt<0> { static constexpr uint32_t BB = 34, EL = 32, DIG = 256, PITCH = 304; static constexpr bool T = false; };
+template <int FMT> struct BlkFmt;                // bytes and elements of a block, digit (or f32) bytes per block and pair of vectors, row pitch of a stage
+// pitch: 32-bit reads of 8 rows x 16 bytes, or of 4 rows x 32 bytes for Q8_0, fill the banks once (48 or 32 modulo 128)
+template <> struct BlkFmt<0> { static constexpr uint32_t BB = 34, EL = 32, DIG = 256, PITCH = 288; static constexpr bool T = false; };
 template <> struct BlkFmt<1> { static constexpr uint32_t BB = 18, EL = 128, DIG = 1024, PITCH = 176; static constexpr bool T = true; };
 template <> struct BlkFmt<2> { static constexpr uint32_t BB = 34, EL = 128, DIG = 1024, PITCH = 304; static constexpr bool T = true; };
 
@@ -39,7 +46,7 @@ struct BlkArgs {
     uint32_t rows[3], y_off[3], tile0[4], nw;
     const uint8_t* up;
     uint32_t row_bytes, nb;                      // blocks of a row
-    const float* x;                              // one or two vectors: the kernel makes the digits itself; more: the table
+    const float* x;                              // one or two vectors: the kernel makes the digits itself; more: the table. Q8_0: always
     const uint8_t* digits;                       // [nb][NT][DIG]
     const int* tsum;                             // [nb][NT][4]
     const float* kappa;
@@ -69,7 +76,7 @@ __device__ __forceinline__ void block_digits(int f, int (&d)[4]) {
 }
 
 // Digits of one block by eight consecutive lanes (t = u & 3, h = u >> 2) into the block's record, columns 4 col .. + 3, and its two joined
-// digit sums into tsum[0 .. 1]; `live` lanes store. FMT 0: byte 16 h + 4 t + b of the block; 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte
+// digit sums into tsum[0 .. 1]; `live` lanes store. FMT 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte
 // 16 h + 4 t + b, its four slots.
 template <int FMT>
 __device__ __forceinline__ void block_record(const float* x, bool live, uint32_t u, uint32_t col, float to_fixed, uint8_t* rec, int* tsum) {
@@ -78,42 +85,30 @@ __device__ __forceinline__ void block_record(const float* x, bool live, uint32_t
     const uint32_t t = u & 3u, h = u >> 2;
 #pragma unroll
     for (uint32_t b = 0; b < 4; b++) {
-        const uint32_t e = FMT == 0 ? 16 * h + 4 * t + b : FMT == 1 ? 8 * (4 * t + b) + 4 * h : 4 * (16 * h + 4 * t + b);
-        float xe[4] = {0.f, 0.f, 0.f, 0.f};
-        if (live) {
-            if (FMT == 0) {
-                xe[0] = __ldcg(x + e);
-            } else {
-                const float4 q = __ldcg(reinterpret_cast<const float4*>(x + e));
-                xe[0] = q.x; xe[1] = q.y; xe[2] = q.z; xe[3] = q.w;
-            }
-        }
+        const uint32_t e = FMT == 1 ? 8 * (4 * t + b) + 4 * h : 4 * (16 * h + 4 * t + b);
+        const float4 q = live ? __ldcg(reinterpret_cast<const float4*>(x + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float xe[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (uint32_t jj = 0; jj < (FMT == 0 ? 1u : 4u); jj++) {
-            const int sh = FMT == 0 ? 0 : FMT == 1 ? (int)(4 * h + jj) : (int)(2 * jj);
+        for (uint32_t jj = 0; jj < 4; jj++) {
+            const int sh = FMT == 1 ? (int)(4 * h + jj) : (int)(2 * jj);
             const int f = (__float2int_rn(xe[jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
             int dg[4];
             block_digits(f, dg);
 #pragma unroll
             for (int d = 0; d < 4; d++) {
                 out[d][jj] |= (uint32_t)(dg[d] & 255) << (8 * b);
-                if (FMT != 0) ts[d] += dg[d] * (1 << sh);
+                ts[d] += dg[d] * (1 << sh);
             }
         }
     }
-    if (FMT != 0) {
 #pragma unroll
-        for (int d = 0; d < 4; d++)
+    for (int d = 0; d < 4; d++)
 #pragma unroll
-            for (uint32_t o = 1; o < 8; o *= 2) ts[d] += __shfl_xor_sync(0xffffffffu, ts[d], o);
-        if (live && u < 2) tsum[u] = u ? ts[2] * 256 + ts[3] : ts[0] * 256 + ts[1];
-    }
+        for (uint32_t o = 1; o < 8; o *= 2) ts[d] += __shfl_xor_sync(0xffffffffu, ts[d], o);
+    if (live && u < 2) tsum[u] = u ? ts[2] * 256 + ts[3] : ts[0] * 256 + ts[1];
     if (!live) return;
 #pragma unroll
-    for (uint32_t d = 0; d < 4; d++) {
-        if (FMT == 0) reinterpret_cast<uint32_t*>(rec)[((col * 4 + d) * 4 + t) * 2 + h] = out[d][0];
-        else reinterpret_cast<uint4*>(rec)[h * 32 + (col * 4 + d) * 4 + t] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
-    }
+    for (uint32_t d = 0; d < 4; d++) reinterpret_cast<uint4*>(rec)[h * 32 + (col * 4 + d) * 4 + t] = make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
 }
 
 // Digit table of vector blockIdx.y; columns of vectors past the batch stay as they are (a column only reaches its own results).
@@ -151,12 +146,6 @@ __device__ __forceinline__ void mma_u8s8_k32p(int (&c)[4], uint32_t a0, uint32_t
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_s8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-}
-
 __device__ __forceinline__ void mma0_u8s8_k32p(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
@@ -200,13 +189,62 @@ __device__ __forceinline__ void q1_pair(const uint8_t* pA, const uint8_t* pB, co
     acc[1] = fmaf(dB, (float)vB, acc[1]);
 }
 
+// Two f32 numbers in one 64-bit register: an instruction for both.
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 unpack2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+// Sums of a stage of four Q8_0 rows over V vectors: of even and odd columns in the two halves of a register, or, where eight vectors leave
+// no room for twice as many registers, plain.
+template <int V> struct Q8Part {
+    static constexpr bool PAIRS = V <= 4;
+    uint64_t two[PAIRS ? V : 1][4];
+    float one[PAIRS ? 1 : V][4];
+};
+// One Q8_0 block of four rows (columns 4 c .. 4 c + 3 of it; p: where the rows' block begins) times V vectors `pitch` bytes apart. PHASE: p
+// modulo 4, 1 if it is not known ahead.
+template <int V, int PHASE>
+__device__ __forceinline__ void q8_block(const uint8_t* const (&p)[4], const uint8_t* x, uint32_t pitch, uint32_t c, Q8Part<V>& part) {
+    uint64_t w[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float d = f16_bits_to_f32(ld<uint16_t>(p[i]));
+        uint32_t q;
+        if (PHASE == 0) q = __byte_perm(ld<uint32_t>(p[i] + 4 * c), ld<uint32_t>(p[i] + 4 * c + 4), 0x5432);
+        else if (PHASE == 2) q = ld<uint32_t>(p[i] + 2 + 4 * c);
+        else q = ld_u2(p[i] + 2 + 4 * c);
+        q ^= 0x80808080u;      // bias to unsigned
+        // 0x4B000000 | byte is the float 8388608 + byte; less 8388736 it is the int8 value
+        const uint64_t off = pack2(-8388736.0f, -8388736.0f), dd = pack2(d, d);
+        w[i][0] = mul2(add2(pack2(__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7650)), __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7651))), off), dd);
+        w[i][1] = mul2(add2(pack2(__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7652)), __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7653))), off), dd);
+    }
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        if constexpr (Q8Part<V>::PAIRS) {
+            const ulonglong2 e = ld<ulonglong2>(x + v * pitch + c * 16);
+#pragma unroll
+            for (int i = 0; i < 4; i++) part.two[v][i] = fma2(w[i][1], e.y, fma2(w[i][0], e.x, part.two[v][i]));
+        } else {
+            const float4 e = ld<float4>(x + v * pitch + c * 16);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 a = unpack2(w[i][0]), b = unpack2(w[i][1]);
+                part.one[v][i] = fmaf(b.y, e.w, fmaf(b.x, e.z, fmaf(a.y, e.y, fmaf(a.x, e.x, part.one[v][i]))));
+            }
+        }
+    }
+}
+
 // AL: rows are multiples of 16 bytes, so a stage starts on a 16-byte boundary. ONE: one vector, Q1_0 blocks in pairs.
 template <int FMT, int NT, bool SW, bool AL, bool ONE>
 __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __grid_constant__ BlkArgs a, const uint32_t S) {
     extern __shared__ __align__(128) uint8_t smem[];
     using F = BlkFmt<FMT>;
     __shared__ float s_red[BLK_WARPS], s_kappa[2];
-    constexpr int MATS = SW ? 2 : 1;
+    constexpr int MATS = SW ? 2 : 1, V = ONE ? 1 : 2 * NT;
     constexpr uint32_t CH = F::BB * BLK_ITEM / 16 + (AL ? 0 : 1), STAGE = 16 * F::PITCH;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3u;
     const uint32_t rank = S > 1 ? blockIdx.x % S : 0u, cl = blockIdx.x / S, ncl = gridDim.x / S;
@@ -258,7 +296,7 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
 
     pdl_wait();
     bool ok = true;
-    if constexpr (NT == 1) {
+    if constexpr (FMT != 0 && NT == 1) {
         // one or two vectors: every CTA makes the digits of its columns itself, which saves the launch of the table kernel in between
         uint8_t* const dtab = smem + BLK_HDR + BLK_WARPS * a.stages * STAGE;
         int* const dsum = reinterpret_cast<int*>(smem + a.tsum_off);
@@ -285,29 +323,53 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
         __syncthreads();
     } else {
         if (tid == 0) {
-            const uint32_t db = nblk * NT * F::DIG, tb = F::T ? nblk * NT * 16u : 0u;
-            mbar_arrive_expect_tx(bar, db + tb);
-            bulk_g2s(smem_u32(tab), a.digits + (size_t)b_lo * NT * F::DIG, db, bar);
-            if (F::T) bulk_g2s(smem_u32(tsm), a.tsum + (size_t)b_lo * NT * 4, tb, bar);
+            if (FMT == 0) {      // the vectors themselves; those past the batch stay as they are
+                mbar_arrive_expect_tx(bar, a.batch * nblk * 128u);
+                for (uint32_t v = 0; v < a.batch; v++) bulk_g2s(smem_u32(tab) + v * nblk * 128u, a.x + ((size_t)v * a.nb + b_lo) * 32, nblk * 128u, bar);
+            } else {
+                const uint32_t db = nblk * NT * F::DIG, tb = nblk * NT * 16u;
+                mbar_arrive_expect_tx(bar, db + tb);
+                bulk_g2s(smem_u32(tab), a.digits + (size_t)b_lo * NT * F::DIG, db, bar);
+                bulk_g2s(smem_u32(tsm), a.tsum + (size_t)b_lo * NT * 4, tb, bar);
+            }
         }
         ok = mbar_wait_limit(bar, 0, a.wait_limit > 0 ? a.wait_limit : WAIT_CYCLE_LIMIT);
         if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_WAIT_FULL);
     }
 
-    float acc[NT][2] = {};
-    uint32_t tile = i_lo / ns, seg = i_lo - tile * ns, slot = 0, padA = 0, padB = 0;
+    float acc[NT][2] = {}, accf[FMT == 0 ? V : 1][4] = {};     // Q8_0: rows lane / 8 + 4 i, all vectors
+    uint32_t tile = i_lo / ns, seg = i_lo - tile * ns, slot = 0, padA = 0, padB = 0, pad[4] = {0u, 0u, 0u, 0u};
     bool mid = seg != 0;                     // this warp took the tile up in its middle
     auto pads = [&]() {
         if (AL) return;
         uint32_t s, r0;
         const uint8_t* w;
         matrix_of(tile, s, w, r0);
+        if (FMT == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) pad[i] = (min(r0 + (lane >> 3) + 4 * i, a.rows[s] - 1) * a.row_bytes) & 15u;
+            return;
+        }
         padA = (min(r0 + g, a.rows[s] - 1) * a.row_bytes) & 15u;
         padB = (min(r0 + g + 8, a.rows[s] - 1) * a.row_bytes) & 15u;
     };
     if (i_lo < i_hi) pads();
     auto flush = [&]() {
         float* dst = mid ? head + warp * (16 * 2 * NT) : mainp + (size_t)((tile >= nt_loc ? a.tiles_max + (tile - nt_loc) : tile) * 16) * (2 * NT);
+        if constexpr (FMT == 0) {
+#pragma unroll
+            for (int v = 0; v < V; v++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    float y = accf[v][i];
+#pragma unroll
+                    for (int o = 1; o < 8; o *= 2) y += __shfl_xor_sync(0xffffffffu, y, o);
+                    if ((lane & 7u) == (uint32_t)v) dst[((lane >> 3) + 4 * i) * (2 * NT) + v] = y;
+                    accf[v][i] = 0.0f;
+                }
+            mid = false;
+            return;
+        }
 #pragma unroll
         for (int n = 0; n < NT; n++)
 #pragma unroll
@@ -326,25 +388,48 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
         else asm volatile("cp.async.wait_group 2;" ::: "memory");
         __syncwarp();                        // the stage is in for every lane, and every lane is done with the one before
         fetch();
-        const uint8_t* const rowA = smem + BLK_HDR + (warp * a.stages + slot) * STAGE + g * F::PITCH + padA;
-        const uint8_t* const rowB = smem + BLK_HDR + (warp * a.stages + slot) * STAGE + (g + 8) * F::PITCH + padB;
+        const uint8_t* const stage = smem + BLK_HDR + (warp * a.stages + slot) * STAGE;
+        const uint8_t *const rowA = stage + g * F::PITCH + padA, *const rowB = stage + (g + 8) * F::PITCH + padB;
         if (++slot == a.stages) slot = 0;
         const uint32_t b0 = seg * BLK_ITEM, nbi = min(BLK_ITEM, nblk - b0);
-        const uint8_t *const rec = tab + b0 * (NT * F::DIG), *const trec = tsm + b0 * (NT * 16u) + t * 4;
-        auto block = [&](uint32_t b) {
-            const uint8_t *const pA = rowA + b * F::BB, *const pB = rowB + b * F::BB;
-            const float dA = f16_bits_to_f32(ld<uint16_t>(pA)), dB = f16_bits_to_f32(ld<uint16_t>(pB));
-            if constexpr (FMT == 0) {
-                const uint32_t a0 = ld_u2(pA + 2 + 4 * t), a1 = ld_u2(pB + 2 + 4 * t), a2 = ld_u2(pA + 18 + 4 * t), a3 = ld_u2(pB + 18 + 4 * t);
+        if constexpr (FMT == 0) {
+            const uint8_t* p[4];
 #pragma unroll
-                for (int n = 0; n < NT; n++) {
-                    const uint2 x = ld<uint2>(rec + (b * NT + n) * F::DIG + lane * 8);
-                    int c[4];
-                    mma_s8s8_k32(c, a0, a1, a2, a3, x.x, x.y);
-                    acc[n][0] = fmaf(dA, (float)(c[0] * 256 + c[1]), acc[n][0]);
-                    acc[n][1] = fmaf(dB, (float)(c[2] * 256 + c[3]), acc[n][1]);
+            for (int i = 0; i < 4; i++) p[i] = stage + ((lane >> 3) + 4 * i) * F::PITCH + pad[i];
+            const uint8_t* x = tab + b0 * 128u;
+            Q8Part<V> part = {};               // a stage's sum: shorter chains of f32 additions than a row of them
+            auto next = [&](uint32_t n) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) p[i] += n * F::BB;
+                x += n * 128;
+            };
+            if (AL) {                          // whole stages of blocks that begin at 0, 2, 0, 2 .. modulo 4
+#pragma unroll 1
+                for (uint32_t b = 0; b < BLK_ITEM; b += 2) {
+                    q8_block<V, 0>(p, x, nblk * 128u, lane & 7u, part);
+                    next(1);
+                    q8_block<V, 2>(p, x, nblk * 128u, lane & 7u, part);
+                    next(1);
                 }
             } else {
+#pragma unroll 1
+                for (uint32_t b = 0; b < nbi; b++) { q8_block<V, 1>(p, x, nblk * 128u, lane & 7u, part); next(1); }
+            }
+#pragma unroll
+            for (int v = 0; v < V; v++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if constexpr (Q8Part<V>::PAIRS) { const float2 y = unpack2(part.two[v][i]); accf[v][i] += y.x + y.y; }
+                    else accf[v][i] += part.one[v][i];
+                }
+            if (++seg == ns) { flush(); seg = 0; tile++; if (it + 1 < i_hi) pads(); }
+            continue;
+        }
+        const uint8_t *const rec = tab + b0 * (NT * F::DIG), *const trec = tsm + b0 * (NT * 16u) + t * 4;
+        auto block = [&](uint32_t b) {
+            if constexpr (FMT != 0) {
+                const uint8_t *const pA = rowA + b * F::BB, *const pB = rowB + b * F::BB;
+                const float dA = f16_bits_to_f32(ld<uint16_t>(pA)), dB = f16_bits_to_f32(ld<uint16_t>(pB));
                 int c[NT][2][4] = {};        // even and odd bits: two chains
                 if constexpr (FMT == 1) {
                     const uint32_t a0 = ld_u2(pA + 2 + 4 * t), a1 = ld_u2(pB + 2 + 4 * t);
@@ -386,11 +471,11 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
                 }
             }
         };
-        if constexpr (ONE) {
+        if constexpr (ONE && FMT == 1) {
 #pragma unroll 2
             for (uint32_t b = 0; b < nbi; b += 2) q1_pair<AL>(rowA + b * F::BB, rowB + b * F::BB, rec + b * F::DIG, trec + b * 16 - t * 4, b + 1 < nbi, lane, acc[0]);
         } else if (nbi == BLK_ITEM) {
-#pragma unroll(FMT == 0 ? 4 : 2)
+#pragma unroll 2
             for (uint32_t b = 0; b < BLK_ITEM; b++) block(b);
         } else {
 #pragma unroll 1
@@ -437,7 +522,7 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
                     y = r ? y + p : p;
                 }
             }
-            f[q] = (NT == 1 ? s_kappa[v] : __ldg(a.kappa + v)) * y;
+            f[q] = FMT == 0 ? y : (NT == 1 ? s_kappa[v] : __ldg(a.kappa + v)) * y;
         }
         float r = SW ? silu_ref(f[0]) * f[MATS - 1] : f[0];
         const uint32_t yi = a.y_off[s] + row;
@@ -511,7 +596,7 @@ int plan_and_launch_one(BlkArgs a, const LaunchCfg& cfg, bool dry) {
 
 template <int FMT, int NT, bool SW, bool AL>
 int plan_and_launch(const BlkArgs& a, const LaunchCfg& cfg, bool dry) {
-    if constexpr (FMT == 1 && NT == 1)
+    if constexpr (FMT != 2 && NT == 1)
         if (a.batch == 1) return plan_and_launch_one<FMT, NT, SW, AL, true>(a, cfg, dry);
     return plan_and_launch_one<FMT, NT, SW, AL, false>(a, cfg, dry);
 }
@@ -531,7 +616,8 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     a.nb = cols / F::EL;
     const size_t dig = (size_t)a.nb * nt * F::DIG, ts = F::T ? (size_t)a.nb * nt * 16 : 0;
     a.x = op.x;
-    if (!dry && nt > 1) {
+    const bool table = F::T && nt > 1;
+    if (!dry && table) {
         if (!op.prep || ((uintptr_t)op.prep & 15) || dig + ts + 64 > op.prep_bytes) return ALICE_E_SHAPE;
         uint8_t* base = static_cast<uint8_t*>(op.prep);
         a.digits = base; a.tsum = reinterpret_cast<const int*>(base + dig); a.kappa = reinterpret_cast<const float*>(base + dig + ts);
@@ -539,7 +625,7 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     auto rows = [&](bool plan) { return nt == 1 ? launch_nt<FMT, 1>(a, cfg, plan) : nt == 2 ? launch_nt<FMT, 2>(a, cfg, plan) : launch_nt<FMT, 4>(a, cfg, plan); };
     const int rc = rows(true);
     if (rc || dry) return rc;
-    if (nt == 1) return rows(false);
+    if (!table) return rows(false);
     cudaLaunchConfig_t lc = {};
     const uint32_t per_vec = a.nb * 8u;
     lc.gridDim = dim3((per_vec + 255) / 256, op.batch); lc.blockDim = dim3(256); lc.stream = cfg.stream;
@@ -547,7 +633,7 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = cfg.pdl ? 1 : 0;
-    if (cudaLaunchKernelEx(&lc, block_table_kernel<FMT>, op.x, cols, a.nb, nt, const_cast<uint8_t*>(a.digits), const_cast<int*>(a.tsum), const_cast<float*>(a.kappa)) != cudaSuccess)
+    if (cudaLaunchKernelEx(&lc, block_table_kernel<F::T ? FMT : 1>, op.x, cols, a.nb, nt, const_cast<uint8_t*>(a.digits), const_cast<int*>(a.tsum), const_cast<float*>(a.kappa)) != cudaSuccess)
         return ALICE_E_CUDA;
     return rows(false);
 }
@@ -555,7 +641,7 @@ int launch_blk(BlkArgs a, const GemvOp& op, const LaunchCfg& cfg, bool dry) {
 }  // namespace
 
 size_t blocks_prep_bytes(uint32_t cols, uint32_t batch) {
-    return (size_t)((cols + 127) / 128) * pairs_of(batch) * (1024 + 16) + 256;      // Q8_0: 256 per 32 columns, no sums
+    return (size_t)((cols + 127) / 128) * pairs_of(batch) * (1024 + 16) + 256;
 }
 
 int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
