@@ -483,14 +483,17 @@ static bool one_vector_warp_ring(const GemvOp& op) {
         // Q2_0: 51200 x 5120 27.4 against 36.8 us, 4096 x 4096 8.2 against 9.1. Q1_0: 151936 x 1024 14.3 against 31.5, 5120 x 25600 17.5 against
         // 21.0, 25600 x 5120 13.0 against 14.9, 7168 x 5120 9.4 against 9.8, 4096 x 4096 7.1 against 8.9.
         case WF_Q1_0: case WF_Q2_0: return true;
-        // Widths at which the ring kernel's lanes stand idle (it deals 16-column units to 32 P lanes, 1, 2 or 4 each): 151936 x 5120 148 against
-        // 262 us; 32768 x 4096 37.5 against 33.8, 4096 x 14336 27.7 against 22.3.
+        // Widths at which the ring kernel's lanes stand idle (it deals 16-column units to 32 P lanes, 1, 2 or 4 each), and matrices large
+        // enough to hide the way of the vector into shared memory: of 128 MB, 1280 columns 37 against 43 us, 5120 37 against 39, 9216 40
+        // against 48; of 96 MB 28 / 33, 29 / 29, 34 / 36; of 32 MB 13.5 / 12.9, 14.7 / 11.6, 17.3 / 14.2. Other widths: 4096, 139 MB 39 / 34.
         case WF_Q8_0: {
             const uint32_t units = w.cols / 16;
             uint32_t lanes = 32;
             while (lanes < 256 && lanes < units) lanes *= 2;
             const uint32_t each = (units + lanes - 1) / lanes;
-            return 10 * units < 7 * lanes * (each == 3 ? 4 : each);
+            uint64_t bytes = 0;
+            for (uint32_t i = 0; i < op.nw && i < 3; i++) if (op.w[i]) bytes += (uint64_t)op.w[i]->rows * w.row_bytes * (op.up ? 2 : 1);
+            return 10 * units < 7 * lanes * (each == 3 ? 4 : each) && bytes >= 96000000;
         }
         default: return false;
     }
