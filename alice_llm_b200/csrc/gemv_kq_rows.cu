@@ -39,6 +39,7 @@ struct KrArgs {
     const float* resid;
     uint32_t y_stride, batch;
     unsigned long long* argmax_key;
+    uint32_t tile_lo, tiles;                                       // tiles of this launch
     uint32_t tiles_max, stages, acts_off, main_off, head_off;      // shared memory: rings | activations | main | head
 };
 
@@ -54,8 +55,8 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
     constexpr uint32_t CH = F::CH, STAGE = 16 * F::PITCH;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3u;
     const uint32_t rank = S > 1 ? blockIdx.x % S : 0u, cl = blockIdx.x / S, ncl = gridDim.x / S;
-    const uint32_t tiles = a.tile0[a.nw];
-    const uint32_t t_lo = (uint32_t)((uint64_t)tiles * cl / ncl), nt_loc = (uint32_t)((uint64_t)tiles * (cl + 1) / ncl) - t_lo;
+    const uint32_t t_own = (uint32_t)((uint64_t)a.tiles * cl / ncl), nt_loc = (uint32_t)((uint64_t)a.tiles * (cl + 1) / ncl) - t_own;
+    const uint32_t t_lo = a.tile_lo + t_own;
     const uint32_t all = (a.nb + F::NB - 1) / F::NB, s_lo = all * rank / S, ns = all * (rank + 1) / S - s_lo;
     const uint32_t b_lo = s_lo * F::NB, b_hi = min(a.nb, (s_lo + ns) * F::NB), nblk = b_hi - b_lo;
     const uint32_t base = smem_u32(smem), ring = base + warp * a.stages * STAGE;
@@ -227,7 +228,13 @@ int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
-    for (uint32_t S = 1, l2 = 0; S <= 8 && S <= all; S *= 2, l2++) {
+    // The smallest cluster whose CTAs hold the activations of their columns and the sums of all their tiles. Where none does (large matrices:
+    // Q5_K from some 25000 x 8192 on), the one that takes the fewest launches, each over a part of the rows: 28672 x 8192 in Q5_K 57 us
+    // for eight vectors, 261 one vector at a time.
+    constexpr size_t TILE = (size_t)(SW ? 2 : 1) * 16 * 8 * 4, HEAD = (size_t)KR_WARPS * 16 * 8 * 4, STAGE = (size_t)KR_WARPS * 16 * F::PITCH;
+    auto acts_of = [&](uint32_t S) { return (kr_acts_bytes<FMT>((all + S - 1) / S * F::NB) + 15u) & ~(size_t)15; };
+    uint32_t best = 0, best_ncl = 0, launches = 0;
+    for (uint32_t S = 1, l2 = 0; S <= 8 && S <= all && launches != 1; S *= 2, l2++) {
         uint32_t ncl = sms;
         if (S > 1) {      // a cluster's CTAs sit in one GPC: what the chip holds at once is asked for, once per kernel and device
             int& known = clusters[dev][l2];
@@ -241,23 +248,32 @@ int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry) {
             ncl = std::min<uint32_t>((uint32_t)known, sms / S);
         }
         ncl = std::min(ncl, tiles);
-        const uint32_t per = (tiles + ncl - 1) / ncl, slice = (all + S - 1) / S * F::NB;
-        const size_t acts = (kr_acts_bytes<FMT>(slice) + 15u) & ~15u, mn = (size_t)(SW ? 2 : 1) * per * 16 * 8 * 4, hd = (size_t)KR_WARPS * 16 * 8 * 4,
-                     stage = (size_t)KR_WARPS * 16 * F::PITCH, fixed = acts + mn + hd;
-        if (fixed + 2 * stage > KR_SMEM) continue;
+        const size_t fixed = acts_of(S) + HEAD + 2 * STAGE;
+        if (fixed + TILE > KR_SMEM) continue;
         // fewer tiles than half the SMs: let more CTAs share a tile's columns
         if (S < 8 && tiles * S * 2 <= sms && all >= 2 * S) continue;
-        if (dry) return ALICE_OK;
-        a.stages = (uint32_t)std::min<size_t>(4, (KR_SMEM - fixed) / stage);
-        a.tiles_max = per;
-        a.acts_off = (uint32_t)(a.stages * stage); a.main_off = (uint32_t)(a.acts_off + acts); a.head_off = (uint32_t)(a.main_off + mn);
-        at[0].val.clusterDim.x = S;
-        lc.gridDim = dim3(ncl * S); lc.dynamicSmemBytes = fixed + a.stages * stage;
-        lc.attrs = S > 1 ? at : at + 1;
-        lc.numAttrs = (S > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
-        return cudaLaunchKernelEx(&lc, kern, a, S) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
+        const uint64_t room = (uint64_t)ncl * ((KR_SMEM - fixed) / TILE);      // tiles of a launch
+        const uint32_t need = (uint32_t)((tiles + room - 1) / room);
+        if (!best || need < launches) { best = S; best_ncl = ncl; launches = need; }
     }
-    return ALICE_E_SHAPE;
+    if (!best) return ALICE_E_SHAPE;
+    if (dry) return ALICE_OK;
+    const size_t acts = acts_of(best);
+    at[0].val.clusterDim.x = best;
+    lc.attrs = best > 1 ? at : at + 1;
+    lc.numAttrs = (best > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
+    for (uint32_t l = 0; l < launches; l++) {
+        a.tile_lo = (uint32_t)((uint64_t)tiles * l / launches);
+        a.tiles = (uint32_t)((uint64_t)tiles * (l + 1) / launches) - a.tile_lo;
+        const uint32_t ncl = std::min(best_ncl, a.tiles);
+        a.tiles_max = (a.tiles + ncl - 1) / ncl;
+        const size_t mn = a.tiles_max * TILE, fixed = acts + mn + HEAD;
+        a.stages = (uint32_t)std::min<size_t>(4, (KR_SMEM - fixed) / STAGE);
+        a.acts_off = (uint32_t)(a.stages * STAGE); a.main_off = (uint32_t)(a.acts_off + acts); a.head_off = (uint32_t)(a.main_off + mn);
+        lc.gridDim = dim3(ncl * best); lc.dynamicSmemBytes = fixed + a.stages * STAGE;
+        if (cudaLaunchKernelEx(&lc, kern, a, best) != cudaSuccess) return ALICE_E_CUDA;
+    }
+    return ALICE_OK;
 }
 
 }  // namespace

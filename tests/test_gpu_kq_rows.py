@@ -1,5 +1,6 @@
 """K-quants over 2..8 vectors (csrc/gemv_kq_rows.cu) against the kernel of a single vector, which other files hold against the oracle:
-edges of the 16-row tiles, of the one- or two-block stages, of the column split over a cluster, rows that begin anywhere.
+edges of the 16-row tiles, of the one- or two-block stages, of the column split over a cluster, rows that begin anywhere, more tiles than
+the CTAs of a launch have room for (180003 rows of Q5_K).
 
 Both keep the integer block dots; a row adds the scale and the min term of every block in f32, in another order. Either term is up to
 a few times what is left of both (4), and a chain of them rounds a few times (8): 32 times 2^-23 of the sum of magnitudes."""
@@ -26,7 +27,7 @@ def quant(qtype):
 
 
 @pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
-@pytest.mark.parametrize("rows,blocks", [(1, 1), (15, 2), (16, 3), (17, 7), (300, 16), (2500, 1), (40, 56), (4099, 5)])
+@pytest.mark.parametrize("rows,blocks", [(1, 1), (15, 2), (16, 3), (17, 7), (300, 16), (2500, 1), (40, 56), (4099, 5), (180003, 1)])
 def test_every_batch(eng, qtype, rows, blocks):
     cols = 256 * blocks
     rng = np.random.default_rng(rows + cols)
@@ -47,3 +48,12 @@ def test_every_batch(eng, qtype, rows, blocks):
         eng.sync()
         err = np.abs(got - np.array(one[:batch], np.float64)) / bound[:batch]
         assert err.max() <= 1.0, (batch, err.max())
+
+
+@pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("rows,cols,swiglu", [(28672, 8192, False), (28672, 8192, True), (8192, 28672, False), (128256, 4096, False)])
+def test_one_pass_at_the_largest_sizes(eng, qtype, rows, cols, swiglu):
+    w = eng.upload_weights_typed(np.zeros(rows * synth.row_bytes(qtype, cols), np.uint8), rows, cols, quant(qtype))
+    for batch in (2, 3, 8):
+        assert eng.batch_plan(w, batch, swiglu=swiglu)[1] == 1, batch
+    w.free()
