@@ -8,6 +8,7 @@
 // with cp.async while the step before computes, scores and weighted sums from 4 x 2 and 4 x 8 register blocks: 38 us for the same
 // layer (tiles 24.5, join 10, append 3.6). What bounds it: the f32 pipe, and shared-memory reads within 20 % of it.
 #include <algorithm>
+#include <type_traits>
 
 #include "attn_body.cuh"
 #include "common.cuh"
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256, 2) attn_tile_kernel(const __grid_constant
     const float inv_sqrt_d = __fdiv_rn(1.0f, sqrtf(128.0f));
     float m[4], l[4], o[4][8];
     uint32_t last[4];                               // first position the row does not see
+    const uint32_t all_see = min(t1, pos0 + row0 / GROUP + 1);      // positions below it are seen by every row of the tile
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         m[i] = -INFINITY; l[i] = 0.0f;
@@ -141,22 +143,26 @@ __global__ void __launch_bounds__(256, 2) attn_tile_kernel(const __grid_constant
         }
         __syncwarp();      // the 16 threads of a row are half a warp
         const uint32_t pa = smem_u32(sp + ty * 4 * (AT_KEYS + 4)), va = smem_u32(sv + b + tx * 4);
+        auto weigh = [&](auto masked) {
 #pragma unroll 2
-        for (uint32_t t = 0; t < AT_KEYS; t += 4) {
-            float4 p[4];
+            for (uint32_t t = 0; t < AT_KEYS; t += 4) {
+                float4 p[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) p[i] = lds4f(pa + i * (AT_KEYS + 4) * 4 + t * 4);
+                for (int i = 0; i < 4; i++) p[i] = lds4f(pa + i * (AT_KEYS + 4) * 4 + t * 4);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float4 v0 = lds4f(va + (t + j) * AT_PITCH * 4), v1 = lds4f(va + (t + j) * AT_PITCH * 4 + 256);
+                for (int j = 0; j < 4; j++) {
+                    const float4 v0 = lds4f(va + (t + j) * AT_PITCH * 4), v1 = lds4f(va + (t + j) * AT_PITCH * 4 + 256);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float w = j == 0 ? p[i].x : j == 1 ? p[i].y : j == 2 ? p[i].z : p[i].w;
-                    o[i][0] = fmaf(w, v0.x, o[i][0]); o[i][1] = fmaf(w, v0.y, o[i][1]); o[i][2] = fmaf(w, v0.z, o[i][2]); o[i][3] = fmaf(w, v0.w, o[i][3]);
-                    o[i][4] = fmaf(w, v1.x, o[i][4]); o[i][5] = fmaf(w, v1.y, o[i][5]); o[i][6] = fmaf(w, v1.z, o[i][6]); o[i][7] = fmaf(w, v1.w, o[i][7]);
+                    for (int i = 0; i < 4; i++) {
+                        if (masked.value && tb + t + j >= last[i]) continue;      // a value the row does not see may be infinite: 0 times it is not 0
+                        const float w = j == 0 ? p[i].x : j == 1 ? p[i].y : j == 2 ? p[i].z : p[i].w;
+                        o[i][0] = fmaf(w, v0.x, o[i][0]); o[i][1] = fmaf(w, v0.y, o[i][1]); o[i][2] = fmaf(w, v0.z, o[i][2]); o[i][3] = fmaf(w, v0.w, o[i][3]);
+                        o[i][4] = fmaf(w, v1.x, o[i][4]); o[i][5] = fmaf(w, v1.y, o[i][5]); o[i][6] = fmaf(w, v1.z, o[i][6]); o[i][7] = fmaf(w, v1.w, o[i][7]);
+                    }
                 }
             }
-        }
+        };
+        if (tb + AT_KEYS <= all_see) weigh(std::false_type{}); else weigh(std::true_type{});
         __syncthreads();   // this half of the K and V tiles is free
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -204,8 +210,8 @@ __global__ void __launch_bounds__(256) attn_join_kernel(const __grid_constant__ 
         }
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            if (sp0 + j < a.nsplit && ml[j].x > -INFINITY) {
-                const float c = expf(ml[j].x - M);
+            if (sp0 + j < a.nsplit) {      // a share without a maximum: nothing seen (all zeros), or nothing but NaN, which stays
+                const float c = ml[j].x == -INFINITY ? 0.0f : expf(ml[j].x - M);
                 L += ml[j].y * c;
                 A.x += v[j].x * c; A.y += v[j].y * c; A.z += v[j].z * c; A.w += v[j].w * c;
             }
