@@ -1,8 +1,22 @@
-// Largest magnitude of an f32 vector by a whole CTA, for the fixed-point digits of csrc/gemv_planes.cu and csrc/gemv_blocks.cu.
+// Fixed point of f32 vectors, for the digits of csrc/gemv_mma.cuh, csrc/gemv_planes.cu and csrc/gemv_blocks.cu: its unit, and the largest
+// magnitude of a vector by a whole CTA.
 #pragma once
 #include "common.cuh"
 
 namespace alice {
+
+// A factor 2^n, n up to 149, that takes f32 numbers to units: two factors, since 2^128 is no f32.
+struct FixedScale { float a, b; };
+__device__ __forceinline__ int to_units(float x, const FixedScale& s) { return __float2int_rn(x * s.a * s.b); }
+// A unit is BITS bits below a power of two above amax, but not below 2^-149, of which every f32 number is a whole multiple. kappa: its
+// value. A vector that is not finite has units of NaN, and so have all its results.
+template <int BITS>
+__device__ __forceinline__ void fixed_scale(float amax, bool finite, FixedScale& to_fixed, float& kappa) {
+    const uint32_t ebits = (__float_as_uint(amax) >> 23) & 0xffu;
+    const int n = ebits == 0xffu ? BITS : min(BITS + 126 - (int)ebits, 149);
+    to_fixed = {finite ? ldexpf(1.0f, min(n, 100)) : 0.0f, ldexpf(1.0f, max(n - 100, 0))};
+    kappa = finite ? ldexpf(1.0f, -n) : __int_as_float(0x7fffffff);
+}
 
 // THREADS threads take part; red = THREADS / 32 floats of shared memory. 16 loads of 16 bytes a thread are in flight at once.
 template <int THREADS>

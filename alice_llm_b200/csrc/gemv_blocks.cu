@@ -60,13 +60,6 @@ struct BlkArgs {
 };
 
 constexpr int BLK_FIX_BITS = 30;
-// A vector that is not finite has a unit of NaN: so have all its results.
-__device__ __forceinline__ void block_fixed_scale(float amax, bool finite, float& to_fixed, float& kappa) {
-    const uint32_t ebits = (__float_as_uint(amax) >> 23) & 0xffu;
-    const int e = !finite || ebits == 0u ? 0 : max((int)ebits - 126, -96);      // 2^(30 - e) stays an f32
-    to_fixed = finite ? ldexpf(1.0f, BLK_FIX_BITS - e) : 0.0f;
-    kappa = finite ? ldexpf(1.0f, e - BLK_FIX_BITS) : __int_as_float(0x7fffffff);
-}
 // four signed base-256 digits of f, |f| <= 2^30, most significant first
 __device__ __forceinline__ void block_digits(int f, int (&d)[4]) {
     d[3] = (int)(int8_t)(f & 255); f = (f - d[3]) >> 8;
@@ -79,7 +72,7 @@ __device__ __forceinline__ void block_digits(int f, int (&d)[4]) {
 // digit sums into tsum[0 .. 1]; `live` lanes store. FMT 1: byte 4 t + b, bits 4 h .. 4 h + 3; 2: byte
 // 16 h + 4 t + b, its four slots.
 template <int FMT>
-__device__ __forceinline__ void block_record(const float* x, bool live, uint32_t u, uint32_t col, float to_fixed, uint8_t* rec, int* tsum) {
+__device__ __forceinline__ void block_record(const float* x, bool live, uint32_t u, uint32_t col, const FixedScale to_fixed, uint8_t* rec, int* tsum) {
     uint32_t out[4][4] = {};
     int ts[4] = {0, 0, 0, 0};
     const uint32_t t = u & 3u, h = u >> 2;
@@ -91,7 +84,7 @@ __device__ __forceinline__ void block_record(const float* x, bool live, uint32_t
 #pragma unroll
         for (uint32_t jj = 0; jj < 4; jj++) {
             const int sh = FMT == 1 ? (int)(4 * h + jj) : (int)(2 * jj);
-            const int f = (__float2int_rn(xe[jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
+            const int f = (to_units(xe[jj], to_fixed) + ((1 << sh) >> 1)) >> sh;
             int dg[4];
             block_digits(f, dg);
 #pragma unroll
@@ -121,9 +114,10 @@ __global__ void __launch_bounds__(256) block_table_kernel(const float* x, uint32
     const uint32_t v = blockIdx.y, tid = threadIdx.x;
     const float* xv = x + (size_t)v * cols;
     bool finite;
-    float to_fixed, kappa;
+    FixedScale to_fixed;
+    float kappa;
     const float amax = vec_amax<256>(xv, cols, true, red, finite);
-    block_fixed_scale(amax, finite, to_fixed, kappa);
+    fixed_scale<BLK_FIX_BITS>(amax, finite, to_fixed, kappa);
     if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
     const uint32_t i = blockIdx.x * 256 + tid, blk = i / 8;
     const size_t at = (size_t)blk * nt + (v >> 1);
@@ -303,9 +297,10 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
         for (uint32_t v = 0; v < a.batch; v++) {
             const float* xv = a.x + (size_t)v * a.nb * F::EL;
             bool finite;
-            float to_fixed, kappa;
+            FixedScale to_fixed;
+            float kappa;
             const float amax = vec_amax<BLK_WARPS * 32>(xv, a.nb * F::EL, true, s_red, finite);
-            block_fixed_scale(amax, finite, to_fixed, kappa);
+            fixed_scale<BLK_FIX_BITS>(amax, finite, to_fixed, kappa);
             if (tid == 0) s_kappa[v] = kappa;
             for (uint32_t i = tid; i < ((nblk * 8 + 31) & ~31u); i += BLK_WARPS * 32) {
                 if (ONE) {       // odd blocks in columns 4 .. 7, zeros in the others

@@ -18,6 +18,7 @@
 // A warp owns a tile of 16 rows (mma M) and a contiguous range of 16-byte groups of the row; the P warps
 // of a row set split the groups, their f32 partials meet in shared memory exactly as in the scalar path.
 #pragma once
+#include "digits_dev.cuh"
 #include "gemv_stream.cuh"
 
 namespace alice {
@@ -111,7 +112,7 @@ static __device__ __forceinline__ float mma_vec_amax(float* red, const float* x,
 // that builds a slice passes a pointer moved back by the slice's first group) and their block sums into tsum[block].
 template <int CODE>
 static __device__ __forceinline__ void mma_build_digits(const float* x, uint32_t v_lo, uint32_t v_hi, uint8_t* table, uint32_t half_bytes,
-                                                        float* tsum, uint32_t tsum_blocks, float to_fixed) {
+                                                        float* tsum, uint32_t tsum_blocks, const FixedScale to_fixed) {
     const uint32_t tid = threadIdx.x, lane = tid & 31;
 #pragma unroll 1
     for (uint32_t base = v_lo; base < v_hi; base += NCW * 32 * TB_V) {
@@ -139,7 +140,7 @@ static __device__ __forceinline__ void mma_build_digits(const float* x, uint32_t
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         const int j = (int)(i & 1u) * 4 + q;
-                        mma_store_digits(w + q * 4, (__float2int_rn(xq[q] * to_fixed) + ((1 << j) >> 1)) >> j);   // fixed / 2^j, to nearest
+                        mma_store_digits(w + q * 4, (to_units(xq[q], to_fixed) + ((1 << j) >> 1)) >> j);   // fixed / 2^j, to nearest
                     }
                 } else {
                     // this float4 is the four elements of weight byte i: element q owns bits 2q (worth +1) and 2q+1
@@ -149,7 +150,7 @@ static __device__ __forceinline__ void mma_build_digits(const float* x, uint32_t
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         const int sh = 2 * q;
-                        const int f = (__float2int_rn(xq[q] * to_fixed) + ((1 << sh) >> 1)) >> sh;
+                        const int f = (to_units(xq[q], to_fixed) + ((1 << sh) >> 1)) >> sh;
                         uint8_t* w = rec + (size_t)(q >> 1) * half_bytes + ((2 * q) & 3) * 4;
                         mma_store_digits(w, f);
                         mma_store_digits(w + 4, CODE == 1 ? f : -f);
@@ -180,15 +181,6 @@ static __device__ __forceinline__ void mma_zero_tail(uint32_t cols, uint32_t gro
     }
 }
 
-// scale = 2^(exponent(amax) + 1) > amax; inf / nan inputs fall back to scale 1 (their products are garbage in the
-// reference too). to_fixed turns x into 26-bit fixed point, kappa is the value of one unit.
-__device__ __forceinline__ void mma_fixed_scale(float amax, float& to_fixed, float& kappa) {
-    const uint32_t ebits = (__float_as_uint(amax) >> 23) & 0xffu;
-    const int e = (ebits == 0u || ebits == 0xffu) ? 0 : (int)ebits - 126;
-    to_fixed = ldexpf(1.0f, MMA_FIX_BITS - e);
-    kappa = ldexpf(1.0f, e - MMA_FIX_BITS);
-}
-
 // The whole table, built by the NCW consumer warps of a matvec CTA in its own shared memory (the path for callers
 // that give the matvec no room for a prepared copy).
 template <int CODE>
@@ -198,8 +190,9 @@ static __device__ __noinline__ float mma_build_table(StreamSmem* sm, const float
     constexpr uint32_t GE = mma_group_elems<CODE>();
     const uint32_t groups = (cols + GE - 1) / GE;
     const uint32_t half_bytes = groups * 256;
-    float to_fixed, kappa;
-    mma_fixed_scale(mma_vec_amax(reinterpret_cast<float*>(sm->norm_part), x, nvec), to_fixed, kappa);
+    FixedScale to_fixed;
+    float kappa;
+    fixed_scale<MMA_FIX_BITS>(mma_vec_amax(reinterpret_cast<float*>(sm->norm_part), x, nvec), true, to_fixed, kappa);
     mma_build_digits<CODE>(x, 0, nvec, table, half_bytes, tsum, tsum_blocks, to_fixed);
     mma_zero_tail<CODE>(cols, groups, table, half_bytes);
     if (threadIdx.x < 4) reinterpret_cast<uint32_t*>(table + 2 * (size_t)half_bytes)[threadIdx.x] = 0u;   // the zero record
@@ -223,8 +216,9 @@ __global__ void __launch_bounds__(NCW * 32) mma_table_kernel(const float* x, uin
     pdl_wait();   // x comes from the previous kernel; the blob may still be read by the matvec before it
     constexpr uint32_t GE = mma_group_elems<CODE>();
     const uint32_t nvec = cols / 4, groups = (cols + GE - 1) / GE, half_bytes = groups * 256;
-    float to_fixed, kappa;
-    mma_fixed_scale(mma_vec_amax(red, x, nvec), to_fixed, kappa);
+    FixedScale to_fixed;
+    float kappa;
+    fixed_scale<MMA_FIX_BITS>(mma_vec_amax(red, x, nvec), true, to_fixed, kappa);
     const uint32_t e_lo = blockIdx.x * MMA_PREP_ELEMS, e_hi = min(cols, e_lo + MMA_PREP_ELEMS);
     const uint32_t G_lo = e_lo / GE, G_hi = (e_hi + GE - 1) / GE, ng = G_hi - G_lo;   // this CTA's groups
     const uint32_t local_half = ng * 256;

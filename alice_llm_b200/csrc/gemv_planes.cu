@@ -15,7 +15,7 @@ constexpr uint32_t PLANE_HDR = 128;
 // One thread's part of a digit table: word w of quad lane t in a 64-byte segment. Planes: bits 4 h .. 4 h + 3 of its four bytes; codes:
 // the four code places of its four bytes (h = 0). out[digit] = the B words of the four.
 template <bool CODES>
-__device__ __forceinline__ void plane_digits(const float* x, uint32_t cols, bool vec4, float to_fixed, uint32_t seg, uint32_t t, uint32_t w, uint32_t h, uint32_t (&out)[4][4]) {
+__device__ __forceinline__ void plane_digits(const float* x, uint32_t cols, bool vec4, const FixedScale to_fixed, uint32_t seg, uint32_t t, uint32_t w, uint32_t h, uint32_t (&out)[4][4]) {
 #pragma unroll
     for (int d = 0; d < 4; d++) out[d][0] = out[d][1] = out[d][2] = out[d][3] = 0u;
 #pragma unroll
@@ -35,7 +35,7 @@ __device__ __forceinline__ void plane_digits(const float* x, uint32_t cols, bool
         for (uint32_t jj = 0; jj < 4; jj++) {
             // what the consumer's A bytes are worth: 2^j for bits 0 .. 6, 2^6 for bit 7; 2^(2 q) for code place q
             const int sh = CODES ? (int)(2 * jj) : min((int)(4 * h + jj), 6);
-            const int f = (__float2int_rn(xe[jj] * to_fixed) + ((1 << sh) >> 1)) >> sh;
+            const int f = (to_units(xe[jj], to_fixed) + ((1 << sh) >> 1)) >> sh;
             uint8_t dg[193];          // digits land 64 apart
             mma_store_digits(dg, f);
 #pragma unroll
@@ -56,9 +56,11 @@ __global__ void __launch_bounds__(256) plane_table_kernel(const float* x, uint32
     const float* xv = x + (size_t)min(v, batch - 1) * cols;
     const bool vec4 = can_vec4(xv, cols);
     bool finite;
-    float to_fixed, kappa;
-    mma_fixed_scale(vec_amax<256>(xv, cols, vec4, red, finite), to_fixed, kappa);
-    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = finite ? kappa : __int_as_float(0x7fffffff);      // all results of a vector that is not finite are NaN
+    FixedScale to_fixed;
+    float kappa;
+    const float amax = vec_amax<256>(xv, cols, vec4, red, finite);
+    fixed_scale<MMA_FIX_BITS>(amax, finite, to_fixed, kappa);
+    if (blockIdx.x == 0 && tid == 0) kappa_out[v] = kappa;
     constexpr uint32_t RECS = CODES ? 4 : 8;
     const uint32_t i = blockIdx.x * 256 + tid, seg = i / (RECS * 4), t = i & 3u, wh = (i >> 2) % RECS;
     if (seg >= segs) return;
@@ -185,9 +187,11 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
             const float* xv = a.x + (size_t)v * a.cols;
             const bool vec4 = can_vec4(xv, a.cols);
             bool finite;
-            float to_fixed, kappa;
-            mma_fixed_scale(vec_amax<PLANE_WARPS * 32>(xv, a.cols, vec4, s_red, finite), to_fixed, kappa);
-            if (tid == 0) s_kappa[v] = finite ? kappa : __int_as_float(0x7fffffff);
+            FixedScale to_fixed;
+            float kappa;
+            const float amax = vec_amax<PLANE_WARPS * 32>(xv, a.cols, vec4, s_red, finite);
+            fixed_scale<MMA_FIX_BITS>(amax, finite, to_fixed, kappa);
+            if (tid == 0) s_kappa[v] = kappa;
             for (uint32_t i = tid; i < ns * RECS * 4; i += PLANE_WARPS * 32) {
                 const uint32_t sl = i / (RECS * 4), wh = (i >> 2) % RECS;
                 uint32_t out[4][4];

@@ -83,3 +83,21 @@ def test_vectors_that_are_not_finite(eng, qtype):
     assert np.isnan(got[1]).all() and np.isnan(got[2]).all()
     s, bound = exact(qtype, eng.dequantize(w).reshape(rows, cols).astype(np.float64), x[[0, 3]])
     assert (np.abs(got[[0, 3]] - s) <= bound).all()
+
+
+@pytest.mark.parametrize("qtype", [Q1_0, Q2_0])
+@pytest.mark.parametrize("size", [1e-28, 1e-33, 1e-40])
+def test_small_activations(eng, qtype, size):
+    """Units are never below 2^-149, and an element is a multiple of up to 2^7 of them (the place of its bit in a byte)."""
+    rng = np.random.default_rng(4)
+    rows, cols = 40, 1024
+    w = eng.upload_weights_typed(synth.make_weights(qtype, rng, rows, cols), rows, cols, quant(qtype))
+    dense = eng.dequantize(w).reshape(rows, cols).astype(np.float64)
+    x = (synth.make_x(rng, cols, 3).reshape(3, cols).astype(np.float64) * size).astype(np.float32)
+    for batch in (1, 3):
+        y = eng.alloc_f32(batch * rows)
+        eng.matvec_dev(w, eng.upload_f32(x.reshape(-1)), y, batch)
+        got = eng.read_f32(y).reshape(batch, rows)
+        eng.sync()
+        s, bound = exact(qtype, dense, x[:batch])
+        assert (np.abs(got - s) <= bound - 1e-30 + 2.0 ** -143 * np.abs(dense).sum(1) + 2.0 ** -148).all(), batch

@@ -88,3 +88,25 @@ def test_planes_swiglu(eng, oracle, rows, cols, batch):
     silu = a / (1.0 + np.exp(-a))
     bound = 1.1 * off[0] * np.abs(b) + np.abs(silu) * off[1] + 2.0 ** -20 * np.abs(silu * b) + 1e-30
     assert (np.abs(got - silu * b) <= bound).all()
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("size", [1e-30, 1e-35, 1e-38, 1e-42])
+def test_small_activations(eng, oracle, sparse, size):
+    """Down to the smallest f32 numbers. A unit is never below 2^-149, and an element is a multiple of up to 2^6 of them (the place of its
+    bit in a byte): half of that on top of the bound above."""
+    rng = np.random.default_rng(9)
+    rows, cols = 40, 1024
+    m = synth.make_ternary(rng, rows, cols)
+    w = upload(eng, oracle, m, rows, cols, sparse)
+    x = (synth.make_x(rng, cols, 3).reshape(3, cols).astype(np.float64) * size).astype(np.float32)
+    for batch in (1, 3):
+        y = eng.alloc_f32(batch * rows)
+        eng.matvec_dev(w, eng.upload_f32(x.reshape(-1)), y, batch)
+        got = eng.read_f32(y).reshape(batch, rows)
+        eng.sync()
+        t, scale = dense(m, cols), m[2].astype(np.float64)
+        s = x[:batch].astype(np.float64) @ t.T
+        unit = np.maximum(np.abs(x[:batch]).max(1, keepdims=True) * 2.0 ** -20, 2.0 ** -144)
+        bound = scale * (np.abs(t).sum(1) * unit + np.abs(s) * 2.0 ** -22) + 2.0 ** -148
+        assert (np.abs(got - s * scale) <= bound).all(), batch
