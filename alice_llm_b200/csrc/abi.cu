@@ -248,8 +248,10 @@ static int run_gemv(alice_engine* e, const alice_weights* w0, const alice_weight
     GemvOp op;
     const WeightFormat f = w0->d.fmt;
     if (!format_uses_q8k(f) && f != WF_Q8_0 && f != WF_BF16) {
-        // room for the activation digit table, prepared once ahead of the matvec (csrc/gemv_mma.cuh)
-        if (may_alloc) { const int rc = ensure_prep(e, std::max({mma_prep_bytes(w0->d.cols), plane_prep_bytes(w0->d.cols, batch), blocks_prep_bytes(w0->d.cols, batch)})); if (rc) return rc; }
+        // room for the activation digit table, prepared ahead of the matvec (csrc/gemv_mma.cuh): for the most vectors there can be, so that
+        // after one call of a width no other number of them allocates (a caller may be capturing its stream by then)
+        const uint32_t cols = w0->d.cols;
+        if (may_alloc) { const int rc = ensure_prep(e, std::max({mma_prep_bytes(cols), plane_prep_bytes(cols, MAX_BATCH), blocks_prep_bytes(cols, MAX_BATCH)})); if (rc) return rc; }
         op.prep = e->prep; op.prep_bytes = e->prep_bytes;
     }
     op.w[0] = &w0->d; op.up = w1 ? &w1->d : nullptr;
