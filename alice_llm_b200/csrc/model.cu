@@ -508,7 +508,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
         if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
         if (err != cudaSuccess) rc = alice_cuda_fail(err, "alice_model_create: clearing state");
     }
-    if (!rc) rc = m->make_stage();
+    if (!rc) m->make_stage();
     if (rc) { alice_model_destroy(m); return rc; }
     *out = m;
     return ALICE_OK;

@@ -33,9 +33,8 @@ int set_tokens(alice_model* m, const uint32_t* tokens, uint32_t n) {
 
 }  // namespace
 
-int alice_model::make_stage() {
-    MCU(cudaMallocHost(&stage, (size_t)STAGE_ROWS * vocab * 4));
-    return ALICE_OK;
+void alice_model::make_stage() {
+    if (cudaMallocHost(&stage, (size_t)STAGE_ROWS * vocab * 4) != cudaSuccess) { stage = nullptr; cudaGetLastError(); }
 }
 
 extern "C" {
@@ -86,7 +85,7 @@ int32_t alice_model_forward_rows(alice_model* m, const uint32_t* tokens, uint32_
     MCU(cudaSetDevice(m->e->device));
     int rc = check_room(m, n, who);
     uint32_t done = 0;
-    float* const to = nrows <= alice_model::STAGE_ROWS ? m->stage : logits;
+    float* const to = m->stage && nrows <= alice_model::STAGE_ROWS ? m->stage : logits;
     std::vector<uint32_t> local;
     for (uint32_t lo = 0; lo < n && !rc;) {
         const uint32_t k = std::min(m->piece_tokens(), n - lo);
@@ -115,9 +114,10 @@ int32_t alice_model_forward_batch_read(alice_model* m, const uint32_t* tokens, u
 
 int32_t alice_model_read_logits(alice_model* m, float* logits) {
     if (!m || !logits) return alice_fail(ALICE_E_INVALID, "alice_model_read_logits: null argument");
-    MCU(cudaMemcpyAsync(m->stage, m->logits, (size_t)m->vocab * 4, cudaMemcpyDeviceToHost, m->e->stream));
+    float* const to = m->stage ? m->stage : logits;
+    MCU(cudaMemcpyAsync(to, m->logits, (size_t)m->vocab * 4, cudaMemcpyDeviceToHost, m->e->stream));
     const int rc = alice_sync(m->e);
-    memcpy(logits, m->stage, (size_t)m->vocab * 4);
+    if (to != logits) memcpy(logits, to, (size_t)m->vocab * 4);
     return rc;
 }
 

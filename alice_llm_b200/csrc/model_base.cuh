@@ -18,7 +18,8 @@ struct alice_model {
     bool graph_tried = false;
     std::vector<void*> owned;                    // device allocations freed with the model
     // Pinned: logits of up to STAGE_ROWS rows on their way to the caller's pageable memory. The copy runs at link speed and one
-    // wait covers it and the status word (a copy into fresh pageable memory waits by itself, in pieces).
+    // wait covers it and the status word (a copy into fresh pageable memory waits by itself, in pieces). nullptr where no such memory
+    // could be had: the copies then go straight to the caller.
     static constexpr uint32_t STAGE_ROWS = 8;
     float* stage = nullptr;
 
@@ -33,7 +34,7 @@ struct alice_model {
     virtual int enqueue_rows(uint32_t n, const uint32_t* rows, uint32_t nrows, float* host_logits) = 0;
     // Queues clearing of everything a sequence leaves behind.
     virtual int clear_state() = 0;
-    int make_stage();                            // at the end of creation
+    void make_stage();                           // at the end of creation
     // Whether the state after the first p tokens can be had from the present one without running them again.
     virtual bool can_return_to(uint32_t p) const { (void)p; return true; }
 };

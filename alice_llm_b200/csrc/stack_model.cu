@@ -696,7 +696,7 @@ int32_t alice_stack_create(alice_engine* e, const alice_stack_config* cfg, const
     }
     if (!b.rc) build_scratch(b);
     if (!b.rc && cudaDeviceSynchronize() != cudaSuccess) b.rc = alice_cuda_fail(cudaGetLastError(), who);
-    if (!b.rc) b.rc = m->make_stage();
+    if (!b.rc) m->make_stage();
     if (b.rc) { alice_model_destroy(m); return b.rc; }
     *out = m;
     return ALICE_OK;
