@@ -13,6 +13,7 @@
 
 #include "abi_internal.cuh"
 #include "gemv_plan.cuh"
+#include "gemm_kq.cuh"
 #include "gemv_blocks.cuh"
 #include "gemv_planes.cuh"
 #include "tp.cuh"
@@ -332,6 +333,25 @@ int32_t alice_swiglu_preq(alice_engine* e, const alice_weights* gate, const alic
                           alice_buf* y) {
     if (!up) return fail(ALICE_E_INVALID, "alice_swiglu_preq: null argument");
     return preq_common(e, gate, up, q, y, "alice_swiglu_preq");
+}
+
+int32_t alice_debug_prompt_product(alice_engine* e, const alice_weights* w, const alice_weights* up, const alice_q8k* q, const alice_buf* resid, alice_buf* y) {
+    const char* who = "alice_debug_prompt_product";
+    if (!e || !w || !q || !y) return fail(ALICE_E_INVALID, "%s: null argument", who);
+    if (up) { const int rc = check_pair(w, up, who); if (rc) return rc; }
+    const size_t n = (size_t)q->batch * w->d.rows;
+    if (!format_uses_q8k(w->d.fmt) || q->cols != w->d.cols || q->batch <= (uint32_t)MAX_BATCH || y->len < n || (resid && resid->len < n))
+        return fail(ALICE_E_SHAPE, "%s: K-quant weights, more than %d vectors of their width, vectors that hold the result", who, MAX_BATCH);
+    CU(cudaSetDevice(e->device));
+    const int rc = ensure_prep(e, kq_tc_prep_bytes(w->d.cols, q->batch));
+    if (rc) return rc;
+    const Q8KView v = view_of(q, 0);
+    GemvOp op;
+    op.w[0] = &w->d; op.up = up ? &up->d : nullptr;
+    op.q8 = &v; op.resid = resid ? resid->p : nullptr; op.y = y->p; op.batch = q->batch;
+    op.prep = e->prep; op.prep_bytes = e->prep_bytes;
+    op.wait_limit = e->wait_limit;
+    return launch_rc(launch_stream_gemv_op(op, cfg_of(e)), who);
 }
 
 int32_t alice_plan_query(alice_engine* e, const alice_weights* w, int32_t swiglu, int32_t preq, uint32_t* out, uint32_t n_out) {

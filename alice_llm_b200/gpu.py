@@ -148,6 +148,10 @@ class GpuEngine:
         """Queues a hand-over whose flag nobody raises: its bounded wait runs out (self-test of that path)."""
         check(self._lib.alice_debug_expire_wait(self._h))
 
+    def debug_prompt_product(self, w: GpuWeightBuffer, q: Q8KBuffer, y: GpuBuffer, up: GpuWeightBuffer | None = None, resid: GpuBuffer | None = None):
+        """A K-quant product with more than eight vectors, as a prompt runs it (self-test of those kernels)."""
+        check(self._lib.alice_debug_prompt_product(self._h, w._h, up and up._h, q._h, resid and resid._h, y._h))
+
     # -- tensor parallel: one engine (one process) per GPU, rows of every projection sharded over the group --
     TP_ID_BYTES = 128
 

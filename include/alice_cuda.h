@@ -180,6 +180,10 @@ int32_t alice_plan_query(alice_engine* e, const alice_weights* w, int32_t swiglu
  * *_batch4 shaders do, src/gpu.rs:4759; `batch` = one pass per vector). No reference counterpart (diagnostic). */
 int32_t alice_batch_plan(alice_engine* e, const alice_weights* w, int32_t swiglu, uint32_t batch, uint32_t* launches, uint32_t* weight_passes);
 
+/* Self-test of the products a prompt of a K-quant model is made of, which no other call takes by itself, nothing else: w times each of the
+ * (more than 8) vectors of q, with `up` the SwiGLU of both, plus resid where that is not null. y[k * rows + r]. No reference counterpart. */
+int32_t alice_debug_prompt_product(alice_engine* e, const alice_weights* w, const alice_weights* up, const alice_q8k* q, const alice_buf* resid, alice_buf* y);
+
 /* ---- tensor parallel ------------------------------------------------------------------------ */
 /* One engine (one process) per GPU; output rows of every projection are sharded over the group and the
  * full vector is rebuilt on every rank by an NCCL all-gather queued on the engine's stream (the row
