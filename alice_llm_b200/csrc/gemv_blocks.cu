@@ -639,7 +639,8 @@ size_t blocks_prep_bytes(uint32_t cols, uint32_t batch) {
     return (size_t)((cols + 127) / 128) * pairs_of(batch) * (1024 + 16) + 256;
 }
 
-int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+int launch_blocks(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
+    if (launches) *launches = 1;
     const WeightDesc& w0 = *op.w[0];
     if ((w0.fmt != WF_Q8_0 && w0.fmt != WF_Q1_0 && w0.fmt != WF_Q2_0) || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || (op.argmax_key && op.batch > 1)) return ALICE_E_SHAPE;
     if (op.nw < 1 || op.nw > 3 || (op.up && op.nw != 1) || !op.y || !op.x || ((uintptr_t)op.x & 15)) return ALICE_E_SHAPE;

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
 }
 
 template <int FMT, bool SW>
-int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry) {
+int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches_out) {
     using F = KrFmt<FMT>;
     static bool attr_done[64] = {};
     static int clusters[64][4] = {};
@@ -257,6 +257,7 @@ int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry) {
         if (!best || need < launches) { best = S; best_ncl = ncl; launches = need; }
     }
     if (!best) return ALICE_E_SHAPE;
+    if (launches_out) *launches_out = launches;
     if (dry) return ALICE_OK;
     const size_t acts = acts_of(best);
     at[0].val.clusterDim.x = best;
@@ -278,7 +279,7 @@ int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry) {
 
 }  // namespace
 
-int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
     const WeightDesc& w0 = *op.w[0];
     const bool q4 = w0.fmt == WF_Q4_K, q5 = w0.fmt == WF_Q5_K;
     if ((!q4 && !q5 && w0.fmt != WF_Q6_K) || !op.q8 || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || (op.argmax_key && op.batch > 1)) return ALICE_E_SHAPE;
@@ -301,8 +302,8 @@ int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
     a.nw = op.nw; a.row_bytes = w0.row_bytes; a.nb = w0.cols / 256;
     a.qs = op.q8->qs; a.d = op.q8->d; a.bsums = op.q8->bsums;
     a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch; a.argmax_key = op.argmax_key;
-    if (op.up) return q4 ? plan_and_launch<4, true>(a, cfg, dry) : q5 ? plan_and_launch<5, true>(a, cfg, dry) : plan_and_launch<6, true>(a, cfg, dry);
-    return q4 ? plan_and_launch<4, false>(a, cfg, dry) : q5 ? plan_and_launch<5, false>(a, cfg, dry) : plan_and_launch<6, false>(a, cfg, dry);
+    if (op.up) return q4 ? plan_and_launch<4, true>(a, cfg, dry, launches) : q5 ? plan_and_launch<5, true>(a, cfg, dry, launches) : plan_and_launch<6, true>(a, cfg, dry, launches);
+    return q4 ? plan_and_launch<4, false>(a, cfg, dry, launches) : q5 ? plan_and_launch<5, false>(a, cfg, dry, launches) : plan_and_launch<6, false>(a, cfg, dry, launches);
 }
 
 }  // namespace alice

@@ -4,7 +4,7 @@
 
 namespace alice {
 
-// ALICE_E_SHAPE: not a case for this kernel. dry: plan only.
-int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry);
+// ALICE_E_SHAPE: not a case for this kernel. dry: plan only. launches: how many this takes.
+int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
 
 }  // namespace alice

@@ -464,13 +464,14 @@ static GemvOp sub_batch(const GemvOp& op, uint32_t k, uint32_t n, Q8KView& v) {
     return o;
 }
 
+using OnePass = int (*)(const GemvOp&, const LaunchCfg&, bool, uint32_t*);
 // A kernel that takes the whole batch in one pass, or halves of it where the digits of all vectors fit no cluster.
-static int launch_split(int (*launch)(const GemvOp&, const LaunchCfg&, bool), const GemvOp& op, const LaunchCfg& cfg) {
+static int launch_split(OnePass launch, const GemvOp& op, const LaunchCfg& cfg) {
     for (uint32_t n = op.batch; n; n /= 2) {
         Q8KView v;
-        int rc = launch(sub_batch(op, 0, n, v), cfg, false);
+        int rc = launch(sub_batch(op, 0, n, v), cfg, false, nullptr);
         if (rc == ALICE_E_SHAPE) continue;
-        for (uint32_t k = n; k < op.batch && !rc; k += n) rc = launch(sub_batch(op, k, std::min(n, op.batch - k), v), cfg, false);
+        for (uint32_t k = n; k < op.batch && !rc; k += n) rc = launch(sub_batch(op, k, std::min(n, op.batch - k), v), cfg, false, nullptr);
         return rc;
     }
     return ALICE_E_SHAPE;
@@ -499,6 +500,14 @@ static bool one_vector_warp_ring(const GemvOp& op) {
     }
 }
 
+// The one-pass kernel for up to MAX_BATCH vectors, or nullptr: the ring kernels, one vector at a time.
+static OnePass one_pass(const GemvOp& op) {
+    const WeightFormat f = op.w[0]->fmt;
+    if (f == WF_TERNARY || f == WF_SPARSE_TERNARY) return launch_planes;
+    if (op.batch == 1 && !one_vector_warp_ring(op)) return nullptr;
+    return format_uses_q8k(f) ? launch_kq_rows : launch_blocks;
+}
+
 int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
     if (op.batch == 0) return ALICE_E_SHAPE;
     if (op.w[0] && op.w[0]->fmt == WF_BF16) return launch_dense_rows(op, cfg);
@@ -516,10 +525,8 @@ int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
         return ALICE_OK;
     }
     if (op.batch > 1 && op.argmax_key) return ALICE_E_INVALID;
-    const WeightFormat f = op.w[0]->fmt;
-    const bool planes = f == WF_TERNARY || f == WF_SPARSE_TERNARY;
-    if (planes || op.batch > 1 || one_vector_warp_ring(op)) {
-        const int rc = launch_split(planes ? launch_planes : format_uses_q8k(f) ? launch_kq_rows : launch_blocks, op, cfg);
+    if (const OnePass kernel = one_pass(op)) {
+        const int rc = launch_split(kernel, op, cfg);
         if (rc != ALICE_E_SHAPE) return rc;
     }
     if (op.batch == 1) return launch_single(op, cfg);
@@ -539,13 +546,14 @@ size_t mma_prep_bytes(uint32_t cols) {
 }
 
 int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint32_t* weight_passes) {
-    for (uint32_t n = op.batch > 1 ? op.batch : 0; n; n /= 2) {
+    const OnePass kernel = one_pass(op);
+    for (uint32_t n = kernel ? op.batch : 0; n; n /= 2) {
         Q8KView v;
-        const GemvOp part = sub_batch(op, 0, n, v);
-        if (launch_planes(part, cfg, true) == ALICE_OK || launch_blocks(part, cfg, true) == ALICE_OK || launch_kq_rows(part, cfg, true) == ALICE_OK) {
-            *launches = *weight_passes = (op.batch + n - 1) / n;
-            return ALICE_OK;
-        }
+        uint32_t l = 1;
+        if (kernel(sub_batch(op, 0, n, v), cfg, true, &l) != ALICE_OK) continue;
+        *weight_passes = (op.batch + n - 1) / n;
+        *launches = *weight_passes * l;
+        return ALICE_OK;
     }
     GemvOp one = op; one.batch = 1;
     StreamPlan pl;

@@ -377,7 +377,8 @@ size_t plane_prep_bytes(uint32_t cols, uint32_t batch) {
     return (size_t)((cols + 511) / 512) * plane_pairs(batch) * 4096 + 256 + 4096;   // codes: half the bytes for half the columns
 }
 
-int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
+    if (launches) *launches = 1;
     const WeightDesc& w0 = *op.w[0];
     const bool codes = w0.fmt == WF_SPARSE_TERNARY;
     if ((w0.fmt != WF_TERNARY && !codes) || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || (op.argmax_key && op.batch > 1)) return ALICE_E_SHAPE;

@@ -49,7 +49,7 @@ struct PlaneArgs {
 inline uint32_t plane_seg_elems(WeightFormat f) { return f == WF_TERNARY ? 512u : 256u; }
 // Scratch for the digit table of `batch` vectors, for either format.
 size_t plane_prep_bytes(uint32_t cols, uint32_t batch);
-// ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only.
-int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry);
+// ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only. launches: of the product, which is one.
+int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
 
 }  // namespace alice

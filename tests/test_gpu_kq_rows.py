@@ -57,3 +57,19 @@ def test_one_pass_at_the_largest_sizes(eng, qtype, rows, cols, swiglu):
     for batch in (2, 3, 8):
         assert eng.batch_plan(w, batch, swiglu=swiglu)[1] == 1, batch
     w.free()
+
+
+def test_plan_follows_the_kernels(eng):
+    """alice_batch_plan: (launches, passes over the weights) of what really runs, for one vector too."""
+    from alice_llm_b200.gpu import GpuQuantType as Q
+    def plan(t, q, rows, cols, batch, swiglu=False):
+        w = eng.upload_weights_typed(np.zeros(rows * synth.row_bytes(t, cols), np.uint8), rows, cols, q)
+        return eng.batch_plan(w, batch, swiglu=swiglu)
+    assert plan(synth.Q1_0, Q.Q1_0, 256, 28672, 1) == (1, 1)          # the ring kernel would take two column chunks
+    assert plan(synth.Q2_0, Q.Q2_0, 256, 28672, 1) == (1, 1)
+    assert plan(Q5_K, Q.Q5K, 180000, 256, 8) == (2, 1)                # one pass, the rows over two launches
+    assert plan(Q5_K, Q.Q5K, 180000, 256, 1) == (1, 1)
+    assert plan(synth.Q8_0, Q.Q8_0, 256, 4096, 8) == (1, 1)
+    planes = [np.zeros((256, 28672 // 8), np.uint8)] * 2 + [np.ones(256, np.float32)]
+    w = eng.upload_ternary(*planes, 256, 28672)
+    assert eng.batch_plan(w, 1) == (1, 1) and eng.batch_plan(w, 8) == (1, 1)
