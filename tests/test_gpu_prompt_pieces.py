@@ -1,6 +1,7 @@
 """Prompts taken in pieces of up to 256 tokens (csrc/gemm_kq.cu, csrc/attn_tokens.cu) against the same model stepped token by token,
 which the other files hold against the oracle. Token counts at the edges of the 8 / 16 / 32 / 64 / 128-token tiles and of a piece,
-widths that leave part of a row tile, contexts at the edges of the 32-key steps, every query group.
+contexts at the edges of the 32-key steps, every query group, wanted rows in runs of every length. (The widths of a K-quant model are whole row
+tiles; parts of tiles are covered product by product in test_gpu_prompt_products.py.)
 
 All-ternary models are smooth: the two paths differ by the order of f32 sums only (terms up to 1000, two layers: 1e-5, held to
 1e-4). K-quant models round activations to the Q8_K grid, where a last bit moves single values by a step of 1 / 128: 2e-2, as
@@ -29,7 +30,7 @@ def rel_l2(got, ref):
     return float(np.linalg.norm(got - ref) / np.linalg.norm(ref))
 
 
-def compare(eng, mix, heads, hidden, ff, ctx, n, tol):
+def compare(eng, mix, heads, hidden, ff, ctx, n, tol, rows=None):
     from alice_llm_b200.gpu import GpuModel
     cfg = dict(num_layers=2, hidden_dim=hidden, intermediate_dim=ff, num_heads=heads[0], num_kv_heads=heads[1], head_dim=128,
                vocab_size=1000, max_seq_len=ctx + n + 8, rope_theta=500000.0, eps=1e-5)
@@ -37,7 +38,7 @@ def compare(eng, mix, heads, hidden, ff, ctx, n, tol):
     gm = GpuModel.load(eng, soft_model(rng, cfg, mix))
     kv = [(rng.standard_normal((max(ctx, 1), heads[1] * 128), dtype=np.float32), rng.standard_normal((max(ctx, 1), heads[1] * 128), dtype=np.float32)) for _ in range(2)]
     toks = rng.integers(0, 1000, n).tolist()
-    rows = sorted({0, n // 2, max(0, n - 2), n - 1})
+    rows = sorted({0, n // 2, max(0, n - 2), n - 1}) if rows is None else rows
 
     def start():
         gm.reset()
@@ -51,7 +52,7 @@ def compare(eng, mix, heads, hidden, ff, ctx, n, tol):
     ref_kv = [gm.kv_read(l, 0, ctx + n) for l in range(2)]
     start()
     got = gm.forward_rows(toks, rows)
-    assert gm.position() == ctx + n if callable(getattr(gm, "position", None)) else True
+    assert gm.position() == ctx + n
     for i, r in enumerate(rows):
         assert rel_l2(got[i], ref[r]) <= tol, (r, rel_l2(got[i], ref[r]))
     for l in range(2):
@@ -69,3 +70,10 @@ def test_attention_of_many_tokens(eng, heads, ctx, n):
 @pytest.mark.parametrize("mix", [None, Q5KM], ids=["q4km", "q5km"])
 def test_k_quant_prompts(eng, mix, n):
     compare(eng, mix, (4, 2), 512, 256 * 9, 16 if n % 2 else 0, n, 2e-2)
+
+
+@pytest.mark.parametrize("mix", [SMOOTH_MIX, {n: synth.Q8_0 for n in ("q", "k", "v", "o", "gate", "up", "down", "output")}], ids=["ternary", "q8_0"])
+@pytest.mark.parametrize("n,rows", [(20, list(range(20))), (40, [0, 1, 2, 5, 6, *range(9, 27), 30, 39]), (290, [*range(3, 12), *range(250, 262), 280, 289]), (30, [])])
+def test_wanted_rows(eng, mix, n, rows):
+    """Runs of up to eight rows share a launch of the head; more than eight rows leave without the pinned buffer."""
+    compare(eng, mix, (4, 2), 512, 1024, 5, n, 1e-4, rows)
