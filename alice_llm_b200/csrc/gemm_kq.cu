@@ -369,15 +369,14 @@ template <int FMT, bool SW>
 int launch_n(const KqGemmArgs& a, const LaunchCfg& cfg) {
     if (a.batch <= 16) return launch_one<FMT, 4, 1, 2, SW>(a, cfg);
     if (a.batch <= 32) return launch_one<FMT, 4, 1, 4, SW>(a, cfg);
-    if (a.batch <= 64) return launch_one<FMT, 2, 2, 4, SW>(a, cfg);
-    return launch_one<FMT, 2, 4, 4, SW>(a, cfg);
+    return launch_one<FMT, 2, 2, 4, SW>(a, cfg);      // in tiles of 64 also what the tcgen05 kernel could not take (no tensor map, no scratch)
 }
 template <int FMT>
 int launch_fmt(const KqGemmArgs& a, const LaunchCfg& cfg) { return a.up ? launch_n<FMT, true>(a, cfg) : launch_n<FMT, false>(a, cfg); }
 
 }  // namespace
 
-int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
+int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg) {
     const WeightDesc& w0 = *op.w[0];
     const bool q4 = w0.fmt == WF_Q4_K, q5 = w0.fmt == WF_Q5_K;
     if ((!q4 && !q5 && w0.fmt != WF_Q6_K) || !op.q8 || op.argmax_key || op.npeers || op.norm_w) return ALICE_E_SHAPE;
@@ -396,7 +395,6 @@ int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg, bool dry) {
         if (u.fmt != w0.fmt || u.rows != w0.rows || u.cols != w0.cols || u.row_bytes != w0.row_bytes || !u.data || ((uintptr_t)u.data & 15)) return ALICE_E_SHAPE;
         a.up = u.data;
     }
-    if (dry) return ALICE_OK;
     if (op.batch > 64) {
         const int rc = launch_kq_gemm_tc(op, cfg);
         if (rc != ALICE_E_SHAPE) return rc;

@@ -4,8 +4,8 @@
 
 namespace alice {
 
-// Any number of vectors in op.batch with op.q8 prepared. ALICE_E_SHAPE: not a case for this kernel. dry: plan only.
-int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg, bool dry);
+// Any number of vectors in op.batch with op.q8 prepared. ALICE_E_SHAPE: not a case for this kernel.
+int launch_kq_gemm(const GemvOp& op, const LaunchCfg& cfg);
 
 // The same for more than 64 vectors of operands launch_kq_gemm has checked (csrc/gemm_kq_tc.cu), with kq_tc_prep_bytes of scratch in
 // op.prep; ALICE_E_SHAPE without it.

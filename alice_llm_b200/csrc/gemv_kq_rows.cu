@@ -38,7 +38,6 @@ struct KrArgs {
     float* y;
     const float* resid;
     uint32_t y_stride, batch;
-    unsigned long long* argmax_key;
     uint32_t tile_lo, tiles;                                       // tiles of this launch
     uint32_t tiles_max, stages, acts_off, main_off, head_off;      // shared memory: rings | activations | main | head
 };
@@ -169,7 +168,6 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
     }
     const uint32_t R = nt_loc * 16, outs = R * a.batch;
     const uint32_t main_s = base + a.main_off;
-    unsigned long long key = 0ull;
     for (uint32_t i = rank * (KR_WARPS * 32) + tid; i < outs; i += S * (KR_WARPS * 32)) {
         const uint32_t v = i / R, lr = i - v * R, tl = t_lo + lr / 16;
         uint32_t s = 0;
@@ -193,15 +191,10 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
             f[q] = y;
         }
         float r = SW ? silu_ref(f[0]) * f[MATS - 1] : f[0];
-        const uint32_t yi = a.y_off[s] + row;
-        const size_t at = (size_t)v * a.y_stride + yi;
+        const size_t at = (size_t)v * a.y_stride + a.y_off[s] + row;
         if (a.resid != nullptr) r = __fadd_rn(__ldcg(a.resid + at), r);
         a.y[at] = r;
-        const uint32_t b = __float_as_uint(r), ordered = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-        const unsigned long long k = r == r ? ((unsigned long long)ordered << 32) | (0xFFFFFFFFu - yi) : 0ull;
-        key = k > key ? k : key;
     }
-    if (a.argmax_key != nullptr) stream_argmax(a.argmax_key, key, lane);
     if (S > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -282,7 +275,7 @@ int plan_and_launch(KrArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches
 int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
     const WeightDesc& w0 = *op.w[0];
     const bool q4 = w0.fmt == WF_Q4_K, q5 = w0.fmt == WF_Q5_K;
-    if ((!q4 && !q5 && w0.fmt != WF_Q6_K) || !op.q8 || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || (op.argmax_key && op.batch > 1)) return ALICE_E_SHAPE;
+    if ((!q4 && !q5 && w0.fmt != WF_Q6_K) || !op.q8 || op.npeers || op.norm_w || op.batch == 0 || op.batch > 8 || op.argmax_key) return ALICE_E_SHAPE;
     if (op.nw < 1 || op.nw > 3 || (op.up && op.nw != 1) || !op.y || w0.cols % 256 || !w0.cols || op.q8->nb * 256 != w0.cols) return ALICE_E_SHAPE;
     if (!op.q8->qs || ((uintptr_t)op.q8->qs & 15) || ((uintptr_t)op.q8->bsums & 15)) return ALICE_E_SHAPE;
     KrArgs a = {};
@@ -301,7 +294,7 @@ int launch_kq_rows(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* l
     }
     a.nw = op.nw; a.row_bytes = w0.row_bytes; a.nb = w0.cols / 256;
     a.qs = op.q8->qs; a.d = op.q8->d; a.bsums = op.q8->bsums;
-    a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch; a.argmax_key = op.argmax_key;
+    a.y = op.y; a.resid = op.resid; a.y_stride = op.y_stride ? op.y_stride : total; a.batch = op.batch;
     if (op.up) return q4 ? plan_and_launch<4, true>(a, cfg, dry, launches) : q5 ? plan_and_launch<5, true>(a, cfg, dry, launches) : plan_and_launch<6, true>(a, cfg, dry, launches);
     return q4 ? plan_and_launch<4, false>(a, cfg, dry, launches) : q5 ? plan_and_launch<5, false>(a, cfg, dry, launches) : plan_and_launch<6, false>(a, cfg, dry, launches);
 }

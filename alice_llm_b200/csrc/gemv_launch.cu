@@ -515,7 +515,7 @@ int launch_stream_gemv_op(const GemvOp& op, const LaunchCfg& cfg) {
     if (op.batch > (uint32_t)MAX_BATCH) {
         // the tokens of a prompt: K-quants in tiles of tokens (up to eight: 46 us by the kernel below against 90 for the feed-forward
         // block of an 8B model and four tokens), everything else eight at a time
-        const int grc = launch_kq_gemm(op, cfg, false);
+        const int grc = launch_kq_gemm(op, cfg);
         if (grc != ALICE_E_SHAPE) return grc;
         for (uint32_t k = 0; k < op.batch; k += MAX_BATCH) {
             Q8KView v;

@@ -304,8 +304,6 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
 
 uint32_t log2u(uint32_t v) { uint32_t r = 0; while ((1u << (r + 1)) <= v) r++; return r; }
 
-struct PlanePlan { uint32_t S, ncl; size_t smem; };
-
 template <int NT, int PL, bool SW, bool VEC16>
 int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
     static int8_t attr_done[64] = {};

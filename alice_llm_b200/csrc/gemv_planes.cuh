@@ -45,8 +45,6 @@ struct PlaneArgs {
     long long wait_limit;
 };
 
-// Elements a 64-byte segment stands for.
-inline uint32_t plane_seg_elems(WeightFormat f) { return f == WF_TERNARY ? 512u : 256u; }
 // Scratch for the digit table of `batch` vectors, for either format.
 size_t plane_prep_bytes(uint32_t cols, uint32_t batch);
 // ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only. launches: of the product, which is one.
