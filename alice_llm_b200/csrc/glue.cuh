@@ -51,7 +51,7 @@ struct EmbedArgs {
 };
 
 // hidden[k] <- dequantized row tokens[k] of the Q8_0 table; rope_tab[k] <- (sin, cos) of (pos + k) * freq[j]; then the
-// prepared form of hidden for the first projection. One CTA.
+// prepared form of hidden for the first projection. One CTA per token.
 cudaError_t launch_embed_q8_0(const EmbedArgs& a, cudaStream_t st, bool pdl);
 cudaError_t launch_attention(const AttnArgs& a, cudaStream_t st, bool pdl);      // one token
 // `batch` consecutive tokens from position pos0 (the host's copy of *a.pos, which only sizes the split): rotates the queries

@@ -149,7 +149,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     int rc;
 
     // A whole-vector hand-over: what `consumers` need of vector `src` (length len), after rms_norm with norm_w (or none).
-    // A one-CTA kernel behind the producing kernel runs it: on one GPU it prepares the vector; in NCCL mode it follows
+    // A small kernel behind the producing kernel, a CTA per vector, runs it: on one GPU it prepares the vector; in NCCL mode it follows
     // the all-gather; in peer mode it first hands the pushed rows over (flags), then prepares the vector.
     auto vector_pub = [&](Publish& p, const float* src, uint32_t len, const float* norm_w, const Need& nd, uint8_t* q8_base, float* xn,
                           uint32_t flag_idx) {
@@ -165,7 +165,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     // after the kernel: NCCL gather + stand-alone preparation
     auto gather_then_publish = [&](float* vec, uint32_t floats_per_rank, Publish& p) -> int {
         if (n == 1) {
-            // single GPU: a one-CTA kernel between producer and consumer (the consumer is its programmatic dependent
+            // single GPU: a small kernel between producer and consumer (the consumer is its programmatic dependent
             // and streams weights meanwhile) instead of the last CTA of the producer doing the same as a serial tail
             if (p.dst.qs || p.dst.xn) { p.mode = PUB_VECTOR; MCU(launch_publish_vector(p, m->e->status, st, pdl)); }
             return ALICE_OK;
@@ -191,7 +191,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     };
     // input of a matvec over `w` that reads the (normalised) hidden state: the prepared f32 vector for the bit-plane
     // tensor-core kernels; for the K-quants ONE shared copy of the Q8_K blocks (of all vectors of a batch), which a
-    // one-CTA kernel prepares (norm + Q8_K) ahead of the matvec - the matvec is its programmatic dependent, so its CTAs
+    // small kernel prepares (norm + Q8_K) ahead of the matvec - the matvec is its programmatic dependent, so its CTAs
     // are resident and streaming weights meanwhile (measured on the 8B decode step: 2.23 ms per token this way, 2.28
     // with every CTA of the matvec normalising and quantizing the vector itself); else the raw vector plus the norm
     // weights, prepared per CTA. `fresh` = no product since the hidden state changed has had its Q8_K blocks prepared.

@@ -2,8 +2,8 @@
 //
 // Every CTA of a matvec needs its whole input in the form its inner loop reads: Q8_K blocks for the K-quant
 // formats, the RMS-normalised f32 vector for the others. That form is the same in every CTA, so it is computed
-// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel, one CTA; the
-// embedding kernel, itself one CTA, does it for its own output) - and left in global memory; the consumer's CTAs fetch
+// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel, a CTA per vector; the
+// embedding kernel, a CTA per token, does it for its own output) - and left in global memory; the consumer's CTAs fetch
 // it straight into registers. With a tensor-parallel group the same kernel first runs the hand-over of the rows the
 // peers have pushed (publish_peer_gate). Arithmetic: rms_norm (src/llama3.rs:5244-5256:
 // f64 sum of squares, f32 mean / sqrt / divide, (x * scale) * w) and quantize_row_q8_k (src/gguf.rs:1323-1374).

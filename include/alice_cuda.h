@@ -235,6 +235,7 @@ int32_t alice_model_forward_read(alice_model* m, uint32_t token, float* logits);
  * takes exactly 4) in one pass over the weights, token k at position + k attending position + k + 1 rows (causal,
  * src/shaders/attention.wgsl:45); the position advances by n. logits[k * vocab + v]. Together with
  * alice_model_rollback_to this is the verify step of speculative decoding (examples/speculative_dual_gpu.rs:230-322).
+ * Several tokens add their sums in another order than one: the logits agree with stepping to rounding, not to the bit.
  * Single GPU only. */
 int32_t alice_model_forward_batch(alice_model* m, const uint32_t* tokens, uint32_t n);
 int32_t alice_model_forward_batch_read(alice_model* m, const uint32_t* tokens, uint32_t n, float* logits);
@@ -242,6 +243,8 @@ int32_t alice_model_forward_batch_read(alice_model* m, const uint32_t* tokens, u
  * feeds first_token, then n-1 times the argmax of the previous logits; out_tokens[i] = argmax after
  * step i. No host round trip between steps. */
 int32_t alice_model_decode_greedy(alice_model* m, uint32_t first_token, uint32_t n, uint32_t* out_tokens);
+/* The logits of the last token stepped (of alice_model_forward_batch: of its first token). After alice_model_forward_rows they are
+ * unspecified; that call hands out the rows that are wanted. */
 int32_t alice_model_read_logits(alice_model* m, float* logits);
 /* Any number of consecutive tokens (cut into pieces the model takes at once), with the logits of rows[0 .. nrows)
  * (ascending places among these tokens, possibly none) written to logits[i * vocab + v]. Blocks. The prompt phase of
