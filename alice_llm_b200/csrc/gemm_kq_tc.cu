@@ -1,21 +1,24 @@
 // K-quant products with more than 64 vectors on the fifth-generation tensor cores (tcgen05.mma kind::f16).
 //
 // A weight enters as the integer scale x quant, an activation as its Q8_K integer, both exact in f16: up to 63 * 31 for Q4_K / Q5_K;
-// for Q6_K (up to 128 * 32) as a multiple of 32 and a remainder, two products. The f32 accumulators hold the integer dots of q4k_q8k_dot /
-// q6k_q8k_dot (src/gguf.rs:3201-3251, :3282-3319) exactly, whatever the values: the drain takes them at least every 2^24 / (largest
-// product) columns (Q4_K 63 * 15 * 128: 138, so 128; Q5_K 63 * 31 * 128: 67, so 64), and the two products of Q6_K have an accumulator
-// each (multiples of 32 up to 2^22 of them; remainders up to 16 * 128 * 256). One more takes the min term (sums of 16 activations, at
-// most 2048, times the 6-bit mins: at most 63 * 2048 * 16). Scaled by the block's f16 and f32 factors they are added up in f32 registers.
+// for Q6_K (up to 128 * 32) as a multiple of 32 and a remainder, two products. The f32 accumulator of one 256-column block then holds
+// the integer dot of q4k_q8k_dot / q6k_q8k_dot (src/gguf.rs:3201-3251, :3282-3319), a second one the min term (sums of 16 activations,
+// at most 2048, times the 6-bit mins), and both are scaled by the block's f16 and f32 factors and added up in f32 registers once per block.
+//
+// The dot is exact up to 2^24; weights of an ordinary matrix and activations of both signs give some 3e5. Activations of one sign, all near
+// the largest of their block, can pass it (Q5_K reaches 3.8 times 2^24, Q6_K 8 times); every step of 16 columns beyond it then rounds by
+// less than 2^-23 of the sum. Measured on such blocks: 4 to 11 * 2^-24 of a result, 0.6 to 1.2 by integer sums. Draining before 2^24 (every 128
+// or 64 columns) is exact there, but adds a block up in pieces, which costs bits on ordinary blocks (error of a row of 56 blocks 2.0e-7 for
+// two pieces, 2.8e-7 for four, 1.5e-7 for one, 1.6e-7 by integer sums) and a tenth of the time of a prompt.
 //
 // One CTA per SM, 128 rows x 128 vectors, 18 warps: 8 unpack raw blocks (cp.async, a block ahead) into the swizzled A tiles, half a row a
 // thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one thread
-// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the part before (two sets in TMEM). Where
+// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM). Where
 // tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
 // What bounds it: the unpacking and draining warps (issue slots half used, 22 % of the tensor pipe), and the last wave: 448 tiles of the
-// gate and up product of an 8B model over 148 SMs. A 256-token prompt of that model takes 16.5 ms (14.8 with one drain a block, whose sums round above 2^24), 23.0 by the integer path of mma.sync
+// gate and up product of an 8B model over 148 SMs. A 256-token prompt of that model takes 14.9 ms, 23.0 by the integer path of mma.sync
 // (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
 #include <algorithm>
-#include <type_traits>
 
 #include "../../include/alice_cuda.h"
 #include "common.cuh"
@@ -29,11 +32,10 @@ namespace {
 constexpr uint32_t KT_M = 128, KT_N = 128, KT_PROD = 256, KT_EPI = 256, KT_THREADS = KT_PROD + KT_EPI + 64;
 constexpr int KERR_KT_WAIT = 7;      // as the bf16 product: operands or accumulators of a tensor-core product
 
-// bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles, drains of a block and ring depth
-template <int FMT> struct KtFmt;
-template <> struct KtFmt<4> { static constexpr uint32_t BB = 144, CH = 9, PITCH = 144, TILES = 5, ASUB = 1, UNITS = 2, STAGES = 5; };
-template <> struct KtFmt<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 176, TILES = 5, ASUB = 1, UNITS = 4, STAGES = 4; };
-template <> struct KtFmt<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, TILES = 4, ASUB = 2, UNITS = 1, STAGES = 3; };
+template <int FMT> struct KtFmt;     // bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles and ring depth
+template <> struct KtFmt<4> { static constexpr uint32_t BB = 144, CH = 9, PITCH = 144, TILES = 5, ASUB = 1, STAGES = 5; };
+template <> struct KtFmt<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 176, TILES = 5, ASUB = 1, STAGES = 4; };
+template <> struct KtFmt<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, TILES = 4, ASUB = 2, STAGES = 3; };
 
 template <int FMT>
 struct KtGeom {
@@ -195,8 +197,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
     extern __shared__ uint8_t raw_smem[];
     __shared__ __align__(8) uint64_t full_[F::STAGES], empty_[F::STAGES], tfull_[2], tempty_[2], drain_;
     __shared__ uint32_t tmem_base;
-    // Q8_K scales of the vectors, four blocks deep: when the copies of block k are asked for, products of block k - 1 have been issued, for
-    // which a part of block k - 2 had to be drained, so block k - 3 has been
+    // Q8_K scales of the vectors, four blocks deep: when the copies of block k are asked for, block k - 3 has been drained
     __shared__ __align__(16) float dts[4][KT_N];
     uint8_t* const ring = raw_smem + (1024u - (smem_u32(raw_smem) & 1023u));
     uint8_t* const raw = ring + G::RING;
@@ -282,43 +283,35 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
             return FMT == 6 ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(blk + 208)) : __ldg(reinterpret_cast<const uint32_t*>(blk));
         };
         uint32_t hd = head(0);
-        float2 f;
-        // accumulators of unit n of block k: the first one, and with `both` the second (the mins; Q6_K: the remainders)
-        auto take = [&](auto both, uint32_t k, uint32_t n) {
-            const uint32_t b = n & 1u;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(tfull_, b), (n >> 1) & 1));
-            if (!ok) return;
+        for (uint32_t k = 0; k < nblk; k++) {
+            const uint32_t b = k & 1u;
+            const float2 f = __half22float2(u2h(hd));
+            hd = head(k + 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(tfull_, b), (k >> 1) & 1));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t base = tmem + b * KT_N + ch * 64 + ((quad * 32) << 16);
             const float* e = dts[k & 3u] + ch * 64;
 #pragma unroll
-            for (int c = 0; c < 8; c += both.value ? 1 : 2) {
+            for (int c = 0; c < 8; c++) {
                 uint32_t p[8], m[8];
                 tmem_get8(p, base + c * 8);
-                tmem_get8(m, base + (both.value ? 256 + c * 8 : c * 8 + 8));      // without the second accumulator two pieces at a time
+                tmem_get8(m, base + (FMT != 6 ? 256 + c * 8 : (c ^ 1) * 8));      // Q6_K has no second accumulator: two pieces at a time
                 tmem_got8(p, m);
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const float x = e[c * 8 + j], v = __uint_as_float(p[j]), w = __uint_as_float(m[j]);
-                    if (FMT == 6) {
-                        acc[c * 8 + j] = fmaf(f.x * x, v + w, acc[c * 8 + j]);
-                    } else if (both.value) {
-                        acc[c * 8 + j] = fmaf(x, fmaf(-f.y, w, f.x * v), acc[c * 8 + j]);
+                    const float x = e[c * 8 + j];
+                    if (FMT != 6) {
+                        acc[c * 8 + j] = fmaf(x, fmaf(-f.y, __uint_as_float(m[j]), f.x * __uint_as_float(p[j])), acc[c * 8 + j]);
                     } else {
-                        acc[c * 8 + j] = fmaf(f.x * x, v, acc[c * 8 + j]);
-                        acc[c * 8 + 8 + j] = fmaf(f.x * e[c * 8 + 8 + j], w, acc[c * 8 + 8 + j]);
+                        acc[c * 8 + j] = fmaf(f.x * x, __uint_as_float(p[j]), acc[c * 8 + j]);
+                        acc[c * 8 + 8 + j] = fmaf(f.x * e[c * 8 + 8 + j], __uint_as_float(m[j]), acc[c * 8 + 8 + j]);
                     }
                 }
+                if (FMT == 6) c++;
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(bar(tempty_, b));
-        };
-        for (uint32_t k = 0; k < nblk && ok; k++) {
-            f = __half22float2(u2h(hd));
-            hd = head(k + 1);
-#pragma unroll 1
-            for (uint32_t u = 0; u + 1 < F::UNITS && ok; u++) take(std::false_type{}, k, k * F::UNITS + u);
-            if (ok) take(std::true_type{}, k, k * F::UNITS + F::UNITS - 1);
         }
     } else if (warp == 16) {              // ---- B tiles
         if (lane == 0) {
@@ -342,12 +335,12 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
         if (lane == 0) {
             constexpr uint32_t idesc = (1u << 4) | ((KT_N / 8) << 17) | ((KT_M / 16) << 24);      // f16 x f16 -> f32
             uint32_t it = 0;
-            for (uint32_t n = 0; n < nblk * F::UNITS && ok; n++) {
-                const uint32_t b = n & 1u, d = tmem + b * KT_N, c0 = n % F::UNITS * (4 / F::UNITS), c1 = n % F::UNITS == F::UNITS - 1 ? F::TILES : c0 + 4 / F::UNITS;
-                ok = mbar_wait(bar(tempty_, b), ((n >> 1) & 1) ^ 1);
+            for (uint32_t k = 0; k < nblk && ok; k++) {
+                const uint32_t b = k & 1u, d = tmem + b * KT_N;
+                ok = mbar_wait(bar(tempty_, b), ((k >> 1) & 1) ^ 1);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (uint32_t c = c0; c < c1; c++, it++) {
+                for (uint32_t c = 0; c < F::TILES; c++, it++) {
                     const uint32_t st = it % F::STAGES;
                     ok = mbar_wait(bar(full_, st), (it / F::STAGES) & 1);
                     if (!ok) break;
@@ -361,7 +354,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
                         for (uint32_t z = 0; z < F::ASUB; z++) {
                             const uint64_t da = smem_desc(at + z * 16384);
 #pragma unroll
-                            for (int kk = 0; kk < 4; kk++) mma_f16(d + z * 256, da + 2 * kk, db + 2 * kk, idesc, c > c0 || kk > 0);
+                            for (int kk = 0; kk < 4; kk++) mma_f16(d, da + 2 * kk, db + 2 * kk, idesc, c > 0 || z > 0 || kk > 0);
                         }
                     }
                     mma_commit(bar(empty_, st));

@@ -2,10 +2,10 @@
 Q8_K blocks: rows and vectors that leave part of every tile (32 to 128 rows, 16 to 128 vectors), one block to 64, the columns of a
 tile shared by up to eight CTAs, SwiGLU, a residual, several tiles of each.
 
-The block sums are integers. Up to 64 vectors they are summed in 32 bits and rounded to f32 once. Beyond, every f32 accumulator is emptied
-before it can pass 2^24 (half a Q4_K block, a quarter of a Q5_K one, the two parts of Q6_K weights apart), so it is exact too. A result then
-is a sum of f32 terms: scale times integers (three roundings) and one addition each, nb blocks in any order: 2^-24 of the sum of their
-magnitudes, 4 + 2 sqrt(terms) times."""
+The block sums are integers. Up to 64 vectors they are summed in 32 bits and rounded to f32 once; beyond, in f32, exactly up to 2^24. A result
+then is a sum of f32 terms: scale times integers (three roundings) and one addition each, nb blocks in any order: 2^-24 of the sum of
+their magnitudes, 4 + 2 sqrt(terms) times. A sum that passes 2^24 rounds once more in each of the 16 steps of 16 columns (Q6_K 32), by less
+than 2^-23 of what it is by then: test_largest_sums."""
 import numpy as np
 import pytest
 
@@ -130,7 +130,8 @@ def test_residual(eng, qtype, batch):
 @pytest.mark.parametrize("nb", [1, 9])
 @pytest.mark.parametrize("sign", [1, -1])
 def test_largest_sums(eng, qtype, nb, sign):
-    """Weights and activations of one sign near their largest values: block sums of up to 2^27, odd ones among them."""
+    """Weights and activations of one sign near their largest values: block sums of up to 2^27, odd ones among them. All terms have the sign of
+    the sum, so what every step may lose is a share of the result."""
     rows, batch, rng = 150, 100, np.random.default_rng(nb)
     blk = synth.make_weights(qtype, rng, rows, 256 * nb).reshape(-1, BYTES[qtype])
     high = lambda n, lo, hi: rng.integers(lo, hi, (len(blk), n)).astype(np.uint8)
@@ -156,6 +157,8 @@ def test_largest_sums(eng, qtype, nb, sign):
     small = np.concatenate([run(eng, qtype, data, rows, 256 * nb, [a[k:k + 50] for a in q8]) for k in (0, 50)])
     worst = [float((np.abs(v - s) / np.abs(s)).max() * 2 ** 24) for v in (got, small)]
     print("largest sums", qtype, nb, "of 2^-24:", worst)
-    assert (np.abs(got - s) <= bound).all() and (np.abs(small - s) <= bound).all()
-    if nb == 1:            # one block: its sums are exact, so what is left are the roundings of the terms
-        assert max(worst) <= 3.0, worst
+    assert (np.abs(small - s) <= bound).all()
+    steps = 32 if qtype == Q6_K else 16
+    assert (np.abs(got - s) <= bound + steps * 2.0 ** -23 * np.abs(s)).all()
+    if nb == 1:            # one block: integer sums are exact, so what is left are the roundings of the terms
+        assert worst[1] <= 3.0, worst
