@@ -1,6 +1,7 @@
 """K-quant products with more than eight vectors (csrc/gemm_kq.cu, csrc/gemm_kq_tc.cu) one by one against 64-bit numpy, from the same
 Q8_K blocks: rows and vectors that leave part of every tile (32 to 128 rows, 16 to 128 vectors), one block to 64, the columns of a
-tile shared by up to eight CTAs, SwiGLU, a residual, several tiles of each.
+tile shared by up to eight CTAs, SwiGLU, a residual, several tiles of each. One to eight vectors (csrc/gemv_stream.cuh, csrc/gemv_kq_rows.cu)
+against the same.
 
 The block sums are integers. Up to 64 vectors they are summed in 32 bits and rounded to f32 once; beyond, in f32, exactly up to 2^24. A result
 then is a sum of f32 terms: scale times integers (three roundings) and one addition each, nb blocks in any order: 2^-24 of the sum of
@@ -97,6 +98,23 @@ def test_products(eng, qtype, rows, nb):
     s, bound = exact(eng, qtype, data, rows, cols, q8)
     for batch in BATCHES if rows * nb < 4000 else [33, 129]:
         err = np.abs(run(eng, qtype, data, rows, cols, [a[:batch] for a in q8]) - s[:batch]) / bound[:batch]
+        assert err.max() <= 1.0, (batch, err.max())
+
+
+@pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("rows,nb", [(1, 1), (15, 2), (17, 7), (300, 16), (2500, 1), (40, 56), (4099, 5)])
+def test_few_vectors(eng, qtype, rows, nb):
+    cols, rng = 256 * nb, np.random.default_rng(rows + nb)
+    data = synth.make_weights(qtype, rng, rows, cols)
+    q8 = vectors(rng, 8, nb)
+    s, bound = exact(eng, qtype, data, rows, cols, q8)
+    w, y = upload(eng, qtype, data, rows, cols), eng.alloc_f32(8 * rows)
+    for batch in (1, 2, 3, 5, 8):
+        e, qs, bs = (a[:batch] for a in q8)
+        eng.matvec_preq_dev(w, eng.upload_q8k(e, qs, bs, cols, batch), y)
+        got = eng.read_f32(y)[:batch * rows].reshape(batch, rows).astype(np.float64)
+        eng.sync()
+        err = np.abs(got - s[:batch]) / bound[:batch]
         assert err.max() <= 1.0, (batch, err.max())
 
 
