@@ -19,8 +19,8 @@
 //
 // What bounds it: Q8_0 the instructions (16 weights a lane and block to unpack, scale and multiply with each vector; 151936 x 5120 196 us
 // for one vector, 228 by the ring kernel; 32768 x 4096 44 us for two, 57 for four, 99 for eight, 34 for each by the ring kernel); Q1_0 and
-// Q2_0 the instructions for one or two vectors (Q1_0 about 75 per 576 bytes for one, an SM issues 100 while those stream: 102400 x 5120 in
-// 32.5 us, 2.3 TB/s), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
+// Q2_0 the ALU for one or two vectors (Q1_0, one vector: 32 masks among some 60 bit operations per 576 bytes, one every other clk and SM quarter;
+// more warps an SM, 20 to 32, gain nothing: 102400 x 5120 in 29.2 us, 2.5 TB/s, 32.4 with the addresses of every copied piece made anew), the products (8 per 16 rows and block of Q1_0, 4 of Q2_0, for each pair of vectors) for more.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -265,23 +265,48 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
         w = up ? a.up : a.w[s];
         r0 = (tl - a.tile0[s]) * 16;
     };
+    // Where this lane's 16-byte pieces of a stage lie relative to the tile and the slot: a stage is a whole number of them and so are 16
+    // rows, so this is the same for all tiles but a matrix's last one, and a piece costs a few additions and the copy.
+    static_assert(F::BB * BLK_ITEM % 16 == 0, "stages keep the alignment of the rows");
+    constexpr uint32_t PIECES = (16 * CH + 31) / 32;
+    uint32_t rel[PIECES];
+#pragma unroll
+    for (uint32_t j = 0; j < PIECES; j++) {
+        const uint32_t i = j * 32 + lane, r = i / CH, c = i - r * CH;
+        rel[j] = ((r * a.row_bytes) & ~15u) + c * 16;
+    }
+    const uint32_t inside = 16 + (CH * 16 + a.row_bytes - 1) / a.row_bytes;      // rows from a tile's first one on that its whole stages may touch
     uint32_t l_item = i_lo, l_tile = i_lo / ns, l_seg = i_lo - l_tile * ns, l_slot = 0;
-    const uint8_t* lw = nullptr;
+    const uint8_t *lw = nullptr, *lp = nullptr;      // matrix; this stage's columns of the tile's first row
     uint32_t ls = 0, lr0 = 0;
-    if (i_lo < i_hi) matrix_of(l_tile, ls, lw, lr0);
+    auto to_tile = [&]() {
+        matrix_of(l_tile, ls, lw, lr0);
+        lp = lw + (uint64_t)lr0 * a.row_bytes + (uint64_t)(s_lo + l_seg) * (BLK_ITEM * F::BB);
+    };
+    if (i_lo < i_hi) to_tile();
     auto fetch = [&]() {
         if (l_item < i_hi) {
-            const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
-            const uint32_t at = (s_lo + l_seg) * (BLK_ITEM * F::BB), dst = ring + l_slot * STAGE;
+            const uint32_t dst = ring + l_slot * STAGE;
+            if (lr0 + inside <= a.rows[ls]) {
 #pragma unroll
-            for (uint32_t i = lane; i < 16 * CH; i += 32) {
-                const uint32_t r = i / CH, c = i - r * CH;
-                const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
-                const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * F::PITCH + c * 16), "l"(n ? lw + off : lw), "r"(n) : "memory");
+                for (uint32_t j = 0; j < PIECES; j++) {
+                    if (16 * CH % 32 && j * 32 + lane >= 16 * CH) continue;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (j * 32 + lane) * 16 + (j * 32 + lane) / CH * (F::PITCH - CH * 16)), "l"(lp + rel[j]) : "memory");
+                }
+            } else {        // rows past the last repeat it, nothing past the matrix is read
+                const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
+                const uint32_t at = (s_lo + l_seg) * (BLK_ITEM * F::BB);
+#pragma unroll 1
+                for (uint32_t i = lane; i < 16 * CH; i += 32) {
+                    const uint32_t r = i / CH, c = i - r * CH;
+                    const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
+                    const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * F::PITCH + c * 16), "l"(n ? lw + off : lw), "r"(n) : "memory");
+                }
             }
             l_item++;
-            if (++l_seg == ns) { l_seg = 0; l_tile++; if (l_item < i_hi) matrix_of(l_tile, ls, lw, lr0); }
+            lp += BLK_ITEM * F::BB;
+            if (++l_seg == ns) { l_seg = 0; l_tile++; if (l_item < i_hi) to_tile(); }
             if (++l_slot == a.stages) l_slot = 0;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -467,7 +492,11 @@ __global__ void __launch_bounds__(BLK_WARPS * 32, 1) block_rows_kernel(const __g
             }
         };
         if constexpr (ONE && FMT == 1) {
-#pragma unroll 2
+            if (nbi == BLK_ITEM) {
+#pragma unroll
+                for (uint32_t b = 0; b < BLK_ITEM; b += 2) q1_pair<AL>(rowA + b * F::BB, rowB + b * F::BB, rec + b * F::DIG, trec + b * 16 - t * 4, true, lane, acc[0]);
+            } else
+#pragma unroll 1
             for (uint32_t b = 0; b < nbi; b += 2) q1_pair<AL>(rowA + b * F::BB, rowB + b * F::BB, rec + b * F::DIG, trec + b * 16 - t * 4, b + 1 < nbi, lane, acc[0]);
         } else if (nbi == BLK_ITEM) {
 #pragma unroll 2

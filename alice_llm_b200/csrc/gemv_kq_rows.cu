@@ -6,8 +6,10 @@
 // no single CTA, or a matrix has few rows. The (tile, stage) pairs of a CTA are dealt evenly to its warps, the parts of a tile are
 // added in a fixed order.
 //
-// What bounds it: HBM and, close behind, the instructions that unpack (about 230 per 16 rows x 256 columns of Q4_K, where an SM
-// issues 400 while those stream), whatever the batch.
+// What bounds it: HBM at the largest sizes (28672 x 8192 gate and up in Q4_K, four vectors: 52 us, 5.1 TB/s), else start and drain of the launch and,
+// close behind, the ALU, which takes a bit operation every other clk (about 200 instructions per 16 rows x 256 columns of Q4_K, whatever the batch).
+// Addresses of the copies made once a warp instead of for every piece: Q5_K 5003 x 2816, three vectors 8.5 -> 7.9 us, 28672 x 8192, eight
+// vectors 55.0 -> 48.5; Q6_K 128256 x 4096, eight 118.7 -> 110.5.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -73,23 +75,54 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
         w = up ? a.up : a.w[s];
         r0 = (tl - a.tile0[s]) * 16;
     };
+    // Where this lane's 16-byte pieces of a stage lie relative to the tile and the slot: the same for all tiles but a matrix's last one, so a
+    // piece costs an addition and the copy (with the addresses made anew each time, 14 instructions, a quarter of the kernel's).
+    constexpr uint32_t PIECES = (16 * CH + 31) / 32;
+    uint32_t rel[PIECES];
+#pragma unroll
+    for (uint32_t j = 0; j < PIECES; j++) {
+        const uint32_t i = j * 32 + lane, r = i / CH;
+        rel[j] = r * a.row_bytes + (FMT == 6 ? 0u : (i - r * CH) * 16);
+    }
+    const uint32_t inside = 16 + (CH * 16 + a.row_bytes - 1) / a.row_bytes;      // rows from a tile's first one on that its whole stages may touch
     uint32_t l_item = i_lo, l_tile = i_lo / ns, l_seg = i_lo - l_tile * ns, l_slot = 0;
-    const uint8_t* lw = nullptr;
+    const uint8_t *lw = nullptr, *lp = nullptr;      // matrix; this stage's columns of the tile's first row
     uint32_t ls = 0, lr0 = 0;
-    if (i_lo < i_hi) matrix_of(l_tile, ls, lw, lr0);
+    auto to_tile = [&]() {
+        matrix_of(l_tile, ls, lw, lr0);
+        lp = lw + (uint64_t)lr0 * a.row_bytes + (uint64_t)(s_lo + l_seg) * (F::NB * F::BB);
+    };
+    if (i_lo < i_hi) to_tile();
     auto fetch = [&]() {
         if (l_item < i_hi) {
-            const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
-            const uint32_t at = (s_lo + l_seg) * (F::NB * F::BB), dst = ring + l_slot * STAGE;
+            const uint32_t dst = ring + l_slot * STAGE;
+            if (lr0 + inside <= a.rows[ls]) {
 #pragma unroll
-            for (uint32_t i = lane; i < 16 * CH; i += 32) {
-                const uint32_t r = i / CH, c = i - r * CH;
-                const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
-                const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * F::PITCH + c * 16), "l"(n ? lw + off : lw), "r"(n) : "memory");
+                for (uint32_t j = 0; j < PIECES; j++) {
+                    const uint32_t i = j * 32 + lane;
+                    if (16 * CH % 32 && i >= 16 * CH) continue;
+                    if constexpr (FMT != 6) {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(lp + rel[j]) : "memory");
+                    } else {
+                        const uint32_t r = i / CH, c = i - r * CH;
+                        const uint8_t* q = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(lp + rel[j]) & ~(uintptr_t)15);
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * F::PITCH + c * 16), "l"(q + c * 16) : "memory");
+                    }
+                }
+            } else {        // rows past the last repeat it, nothing past the matrix is read
+                const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
+                const uint32_t at = (s_lo + l_seg) * (F::NB * F::BB);
+#pragma unroll 1
+                for (uint32_t i = lane; i < 16 * CH; i += 32) {
+                    const uint32_t r = i / CH, c = i - r * CH;
+                    const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
+                    const uint32_t n = off < total ? (uint32_t)min((uint64_t)16, total - off) : 0u;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * F::PITCH + c * 16), "l"(n ? lw + off : lw), "r"(n) : "memory");
+                }
             }
             l_item++;
-            if (++l_seg == ns) { l_seg = 0; l_tile++; if (l_item < i_hi) matrix_of(l_tile, ls, lw, lr0); }
+            lp += F::NB * F::BB;
+            if (++l_seg == ns) { l_seg = 0; l_tile++; if (l_item < i_hi) to_tile(); }
             if (++l_slot == a.stages) l_slot = 0;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
