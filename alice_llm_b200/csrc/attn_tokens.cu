@@ -21,9 +21,6 @@ constexpr int AT_ROWS = 64, AT_KEYS = 32, AT_PITCH = 132;   // pitch in floats: 
 constexpr uint32_t AT_TILE = AT_KEYS * AT_PITCH;
 constexpr uint32_t AT_SMEM = (AT_ROWS * AT_PITCH + 4 * AT_TILE + AT_ROWS * (AT_KEYS + 4)) * 4;
 
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ float4 lds4f(uint32_t a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));

@@ -313,6 +313,8 @@ int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ALICE_E_CUDA;
     if (!attr_done[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLANE_SMEM) != cudaSuccess) return ALICE_E_CUDA;
+        // the weights come through L1: behind a kernel that had made nearly all of it shared memory (attention) a 70B layer took 8 us more
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 50) != cudaSuccess) return ALICE_E_CUDA;
         attr_done[dev] = 1;
     }
     const uint32_t sms = (uint32_t)std::max(cfg.num_sms, 1), tiles = a.tile0[a.nw];

@@ -47,11 +47,11 @@ __global__ void __launch_bounds__(256) embed_q8_0_kernel(const __grid_constant__
 // for NeoX, freq = 1 / theta^(i_even / d), angle = pos * freq; a lane owns dims 4*lane .. 4*lane+3 of a
 // head vector (head_dim = 128, so a NeoX partner sits in lane ^ 16).
 template <int GROUP>
-__global__ void __launch_bounds__(256, GROUP <= 5 ? 2 : 1) attn_fused_kernel(const __grid_constant__ AttnArgs a) {
-    __shared__ AttnSmem<GROUP> sh;
+__global__ void __launch_bounds__(AD_WARPS * 32, 16 / AD_WARPS) attn_decode_kernel(const __grid_constant__ AttnArgs a) {
+    extern __shared__ __align__(16) uint8_t smem[];
     pdl_launch_dependents();   // the next kernel may become resident (and prefetch its weights) while this one waits
     pdl_wait();
-    attn_fused_body<GROUP>(a, (uint32_t)*a.pos, blockIdx.x, blockIdx.y, &sh);
+    attn_decode_body<GROUP>(a, blockIdx.x, blockIdx.y, reinterpret_cast<AttnSmem<GROUP>*>(smem));
 }
 
 static void launch_cfg(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, dim3 grid, dim3 block, cudaStream_t st, bool pdl) {
@@ -68,18 +68,33 @@ cudaError_t launch_embed_q8_0(const EmbedArgs& a, cudaStream_t st, bool pdl) {
     return cudaLaunchKernelEx(&lc, embed_q8_0_kernel, a);
 }
 
+template <int GROUP>
+static cudaError_t launch_decode(const AttnArgs& a, cudaStream_t st, bool pdl) {
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev >= 64 || !done[dev]) {
+        err = cudaFuncSetAttribute(attn_decode_kernel<GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AttnSmem<GROUP>));
+        if (err != cudaSuccess) return err;
+        if (dev < 64) done[dev] = true;
+    }
+    cudaLaunchConfig_t lc; cudaLaunchAttribute at[1];
+    launch_cfg(lc, at, dim3(a.shape.num_kv_heads, a.nsplit), dim3(AD_WARPS * 32), st, pdl);
+    lc.dynamicSmemBytes = sizeof(AttnSmem<GROUP>);
+    return cudaLaunchKernelEx(&lc, attn_decode_kernel<GROUP>, a);
+}
+
 cudaError_t launch_attention(const AttnArgs& a, cudaStream_t st, bool pdl) {
     const AttnShape& s = a.shape;
     if (s.head_dim != 128 || s.num_heads % s.num_kv_heads) return cudaErrorInvalidValue;
     const uint32_t group = s.num_heads / s.num_kv_heads;
-    cudaLaunchConfig_t lc; cudaLaunchAttribute at[1];
-    launch_cfg(lc, at, dim3(s.num_kv_heads, a.nsplit), dim3(256), st, pdl);
     switch (group) {
-        case 1: return cudaLaunchKernelEx(&lc, attn_fused_kernel<1>, a);
-        case 2: return cudaLaunchKernelEx(&lc, attn_fused_kernel<2>, a);
-        case 4: return cudaLaunchKernelEx(&lc, attn_fused_kernel<4>, a);
-        case 5: return cudaLaunchKernelEx(&lc, attn_fused_kernel<5>, a);
-        case 8: return cudaLaunchKernelEx(&lc, attn_fused_kernel<8>, a);
+        case 1: return launch_decode<1>(a, st, pdl);
+        case 2: return launch_decode<2>(a, st, pdl);
+        case 4: return launch_decode<4>(a, st, pdl);
+        case 5: return launch_decode<5>(a, st, pdl);
+        case 8: return launch_decode<8>(a, st, pdl);
         default: return cudaErrorInvalidValue;
     }
 }

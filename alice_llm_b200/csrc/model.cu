@@ -281,6 +281,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
             for (uint32_t q = 0; q < m->npeers; q++) aa.peer_out[q] = reinterpret_cast<float*>(on_peer(q, m->attn_out)) + (size_t)r * lq;
         }
         if (batch == 1) {
+            aa.nsplit = std::max<uint32_t>(1, std::min(m->nsplit, (uint32_t)m->e->num_sms / shape.num_kv_heads));      // a CTA an SM
             MCU(launch_attention(aa, st, pdl));
         } else {
             MCU(launch_attention_tokens(aa, m->qkv, batch, m->pos, m->part_vectors, m->e->num_sms, st, pdl));
