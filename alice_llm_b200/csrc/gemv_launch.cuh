@@ -75,7 +75,7 @@ int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint3
 // out[r*cols + c] = dequantized weight, bit-exact with the reference dequantizers.
 int launch_dequantize(const WeightDesc& w, float* out, cudaStream_t stream);
 
-// The stand-alone form of csrc/publish.cuh: one CTA per vector of `p.batch` (optional rms_norm, then Q8_K and / or
+// The stand-alone form of csrc/publish.cuh: a warp per block of 256 elements of `p.batch` vectors (optional rms_norm, then Q8_K and / or
 // f32) - used where no producing kernel can do it (the embedding, NCCL-gathered vectors).
 cudaError_t launch_publish_vector(const Publish& p, int* status, cudaStream_t stream, bool pdl);
 

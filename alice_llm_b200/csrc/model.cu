@@ -149,7 +149,7 @@ int LlamaModel::step(uint32_t batch, bool greedy_feed, const uint32_t* rows, uin
     int rc;
 
     // A whole-vector hand-over: what `consumers` need of vector `src` (length len), after rms_norm with norm_w (or none).
-    // A small kernel behind the producing kernel, a CTA per vector, runs it: on one GPU it prepares the vector; in NCCL mode it follows
+    // A small kernel behind the producing kernel, a warp per block, runs it: on one GPU it prepares the vector; in NCCL mode it follows
     // the all-gather; in peer mode it first hands the pushed rows over (flags), then prepares the vector.
     auto vector_pub = [&](Publish& p, const float* src, uint32_t len, const float* norm_w, const Need& nd, uint8_t* q8_base, float* xn,
                           uint32_t flag_idx) {

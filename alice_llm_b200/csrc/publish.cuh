@@ -2,7 +2,7 @@
 //
 // Every CTA of a matvec needs its whole input in the form its inner loop reads: Q8_K blocks for the K-quant
 // formats, the RMS-normalised f32 vector for the others. That form is the same in every CTA, so it is computed
-// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel, a CTA per vector; the
+// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel, a warp per block of 256; the
 // embedding kernel, a CTA per token, does it for its own output) - and left in global memory; the consumer's CTAs fetch
 // it straight into registers. With a tensor-parallel group the same kernel first runs the hand-over of the rows the
 // peers have pushed (publish_peer_gate). Arithmetic: rms_norm (src/llama3.rs:5244-5256:
@@ -112,44 +112,34 @@ __device__ __forceinline__ void pub_emit_block(const PublishDst& dst, const Q8KL
     }
 }
 
-// Whole-vector form, run by NW warps (threads 0 .. NW*32-1 of the CTA) that meet on named barrier `BAR`.
-// Warp w owns the 256-element blocks w, w + NW, ...; a lane owns 8 consecutive elements of each. Up to PUB_REG_BLOCKS
-// blocks per warp stay in registers between the sum of squares and the second pass (one trip to L2 for vectors of up to
-// NW * PUB_REG_BLOCKS * 256 elements), longer vectors are read twice. `red` = NW doubles of shared memory.
-//
-// One CTA prepares vector k: a batch is a grid of as many CTAs. (One CTA walking through all of them took 24.4 us for eight
-// vectors of 4096, one CTA each 6 us.)
-constexpr int PUB_REG_BLOCKS = 2;
+// Vector k, blocks part * NW + warp, + parts * NW ...: run by NW warps (threads 0 .. NW*32-1 of the CTA) that meet on named barrier `BAR`. A
+// block of 256 elements is a warp's, 8 consecutive ones a lane's. With a norm every CTA of the vector takes the sum over all of it (f64, its
+// loads in flight together), so the CTAs need nothing of each other. `red` = NW doubles of shared memory.
 template <int NW, int BAR>
-static __device__ __noinline__ void publish_vector(const Publish& p, double* red, uint32_t k) {
+static __device__ __noinline__ void publish_vector(const Publish& p, double* red, uint32_t k, uint32_t part = 0, uint32_t parts = 1) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n = p.n, nblk = (n + QK_K - 1) / QK_K;
-    const bool in_regs = nblk <= (uint32_t)(NW * PUB_REG_BLOCKS);
+    const uint32_t n = p.n, nblk = (n + QK_K - 1) / QK_K, b0 = part * NW + warp;
     const float* x = p.src + (size_t)k * n;
-    Q8KLaneInput xv[PUB_REG_BLOCKS], wv[PUB_REG_BLOCKS];
+    Q8KLaneInput xv{}, wv{};
     float scale = 1.0f;
-    if (in_regs) {
-#pragma unroll
-        for (int i = 0; i < PUB_REG_BLOCKS; i++) {
-            const uint32_t b = warp + (uint32_t)i * NW;
-            if (b < nblk) {
-                xv[i] = pub_load8(x, b * QK_K + lane * 8, n);
-                if (p.norm_w != nullptr) wv[i] = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
-            }
-        }
+    if (b0 < nblk) {
+        xv = pub_load8(x, b0 * QK_K + lane * 8, n);
+        if (p.norm_w != nullptr) wv = pub_load8_w(p.norm_w, b0 * QK_K + lane * 8, n);
     }
     if (p.norm_w != nullptr) {
-        double ss = 0.0;
-        if (in_regs) {
+        constexpr int LB = 4;
+        double ss[2] = {0.0, 0.0};
+        for (uint32_t b = warp; b < nblk; b += LB * NW) {
+            Q8KLaneInput v[LB];
 #pragma unroll
-            for (int i = 0; i < PUB_REG_BLOCKS; i++)
-                if (warp + (uint32_t)i * NW < nblk) ss += pub_sumsq(xv[i]);
-        } else {
-            for (uint32_t b = warp; b < nblk; b += NW) ss += pub_sumsq(pub_load8(x, b * QK_K + lane * 8, n));
+            for (int i = 0; i < LB; i++) v[i] = pub_load8(x, (b + i * NW) * QK_K + lane * 8, n);      // zeros past the end
+#pragma unroll
+            for (int i = 0; i < LB; i++) ss[i & 1] += pub_sumsq(v[i]);
         }
+        double s1 = ss[0] + ss[1];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) red[warp] = ss;
+        for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        if (lane == 0) red[warp] = s1;
         asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");
         double tot = 0.0;
 #pragma unroll
@@ -157,18 +147,12 @@ static __device__ __noinline__ void publish_vector(const Publish& p, double* red
         const float mean = (float)(tot / (double)n);
         scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
     }
-    if (in_regs) {
-#pragma unroll
-        for (int i = 0; i < PUB_REG_BLOCKS; i++) {
-            const uint32_t b = warp + (uint32_t)i * NW;
-            if (b < nblk) pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv[i], scale, wv[i]) : xv[i], lane, k, b, n);
+    for (uint32_t b = b0; b < nblk; b += parts * NW) {
+        if (b != b0) {
+            xv = pub_load8(x, b * QK_K + lane * 8, n);
+            if (p.norm_w != nullptr) wv = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
         }
-    } else {
-        for (uint32_t b = warp; b < nblk; b += NW) {
-            const Q8KLaneInput v = pub_load8(x, b * QK_K + lane * 8, n);
-            if (p.norm_w != nullptr) pub_emit_block(p.dst, pub_scale(v, scale, pub_load8_w(p.norm_w, b * QK_K + lane * 8, n)), lane, k, b, n);
-            else pub_emit_block(p.dst, v, lane, k, b, n);
-        }
+        pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv, scale, wv) : xv, lane, k, b, n);
     }
 }
 

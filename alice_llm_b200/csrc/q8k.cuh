@@ -53,22 +53,16 @@ __device__ __forceinline__ void q8k_quantize_block_warp(const Q8KLaneInput in, u
                                                         int16_t* bsums, float* rt = nullptr) {
     const float4 a = in.a, b = in.b;
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    // local first-maximum, then a warp max over (|x| bits, reversed index) keys
+    // first maximum of the lane, the largest of the warp, its first lane: lanes own consecutive elements
     float lmax = 0.0f, lval = 0.0f;
-    uint32_t lidx = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const float av = fabsf(v[i]);
-        if (av > lmax) { lmax = av; lval = v[i]; lidx = i; }
+        if (av > lmax) { lmax = av; lval = v[i]; }
     }
-    unsigned long long best = ((unsigned long long)__float_as_uint(lmax) << 32) | (0xFFFFFFFFu - (lane * 8 + lidx));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other > best ? other : best;
-    }
-    const float amax = __uint_as_float((uint32_t)(best >> 32));
-    const uint32_t win_lane = (0xFFFFFFFFu - (uint32_t)best) >> 3;
+    const uint32_t best = __reduce_max_sync(0xffffffffu, __float_as_uint(lmax));
+    const float amax = __uint_as_float(best);
+    const uint32_t win_lane = __ffs(__ballot_sync(0xffffffffu, __float_as_uint(lmax) == best)) - 1;
     const float max_val = __shfl_sync(0xffffffffu, lval, win_lane);
     uint32_t w0 = 0, w1 = 0;
     int lsum = 0;
