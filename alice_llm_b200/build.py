@@ -17,7 +17,7 @@ LIB = os.path.join(HERE, "libalice_cuda.so")
 LIB_STACK = os.path.join(HERE, "libalice_stack.so")
 STACK_SOURCES = ["engine.cu", "tp.cu", "step.cu", "model_api.cu", "stack_model.cu", "stack_ops.cu", "dense_rows.cu", "dense_gemm.cu", "delta.cu",
                  "latent.cu", "latent_decode.cu", "latent_prefill.cu", "grouped.cu", "grouped_decode.cu", "grouped_prefill.cu"]
-SOURCES = STACK_SOURCES + ["abi.cu", "gemv_launch.cu", "gemv_planes.cu", "gemv_blocks.cu", "gemv_kq_rows.cu", "gemm_kq.cu", "gemm_kq_tc.cu", "q8k.cu", "dequant.cu", "ternarize.cu", "glue.cu", "attn_tokens.cu", "model.cu"]
+SOURCES = STACK_SOURCES + ["abi.cu", "gemv_launch.cu", "gemv_planes.cu", "gemv_planes_tc.cu", "gemv_blocks.cu", "gemv_kq_rows.cu", "gemm_kq.cu", "gemm_kq_tc.cu", "q8k.cu", "dequant.cu", "ternarize.cu", "glue.cu", "attn_tokens.cu", "model.cu"]
 # never --use_fast_math: dequantization and the Q8_K quantizer must round like the reference
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-strict-aliasing"]

@@ -464,6 +464,20 @@ static GemvOp sub_batch(const GemvOp& op, uint32_t k, uint32_t n, Q8KView& v) {
     return o;
 }
 
+// Ternary planes and codes: three vectors and more of matrices large enough for tcgen05, with rows that begin on 16-byte boundaries. Its start costs 2 us
+// more: 4096 x 4096 (4 MB) four vectors 10.1 us against 8.5, eight 10.5 / 12.0; 5120 x 5120 three 12.8 / 10.0, eight 12.7 / 13.0; 30000 x 2048 (15 MB) four
+// 14.4 / 13.1; 8192 x 8192 (17 MB) three 13.2 / 15.5; 1024 x 8192 (2 MB) eight 10.5 / 9.4.
+static int launch_ternary(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
+    const WeightDesc& w = *op.w[0];
+    uint64_t bytes = 0;
+    for (uint32_t i = 0; i < op.nw && i < 3; i++) if (op.w[i]) bytes += (uint64_t)op.w[i]->rows * w.row_bytes * (op.up ? 2 : 1);
+    if (op.batch > 2 && plane_rows_aligned(w) && bytes >= (op.batch > 4 ? 4000000u : 16000000u)) {
+        const int rc = launch_planes_tc(op, cfg, dry, launches);
+        if (rc != ALICE_E_SHAPE) return rc;
+    }
+    return launch_planes(op, cfg, dry, launches);
+}
+
 using OnePass = int (*)(const GemvOp&, const LaunchCfg&, bool, uint32_t*);
 // A kernel that takes the whole batch in one pass, or halves of it where the digits of all vectors fit no cluster.
 static int launch_split(OnePass launch, const GemvOp& op, const LaunchCfg& cfg) {
@@ -503,7 +517,7 @@ static bool one_vector_warp_ring(const GemvOp& op) {
 // The one-pass kernel for up to MAX_BATCH vectors, or nullptr: the ring kernels, one vector at a time.
 static OnePass one_pass(const GemvOp& op) {
     const WeightFormat f = op.w[0]->fmt;
-    if (f == WF_TERNARY || f == WF_SPARSE_TERNARY) return launch_planes;
+    if (f == WF_TERNARY || f == WF_SPARSE_TERNARY) return launch_ternary;
     if (op.batch == 1 && !one_vector_warp_ring(op)) return nullptr;
     return format_uses_q8k(f) ? launch_kq_rows : launch_blocks;
 }

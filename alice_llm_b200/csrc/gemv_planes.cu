@@ -5,6 +5,7 @@
 #include "digits_dev.cuh"
 #include "gemv_mma.cuh"
 #include "gemv_planes.cuh"
+#include "planes_dev.cuh"
 
 namespace alice {
 namespace {
@@ -43,7 +44,6 @@ __device__ __forceinline__ void plane_digits(const float* x, uint32_t cols, bool
         }
     }
 }
-__device__ __forceinline__ bool can_vec4(const float* x, uint32_t cols) { return cols % 4 == 0 && ((uintptr_t)x & 15) == 0; }
 
 // Digit table of one vector per blockIdx.y (columns 4 (v & 1) .. + 3 of pair v >> 1); vectors past `batch` are zero columns. With
 // RECS records of 512 bytes to a segment and pair: table[((seg * NT + pair) * RECS + record) * 32 + 4 * column + t].
@@ -101,13 +101,6 @@ __device__ __forceinline__ PlaneTile plane_tile(const PlaneArgs& a, uint32_t til
     return {w + (size_t)min(r0 + g, last) * a.row_bytes, w + (size_t)min(r0 + g + 8, last) * a.row_bytes};
 }
 
-__device__ __forceinline__ long long ld_cluster_s64(uint32_t addr, uint32_t rank) {
-    uint32_t remote;
-    long long v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(remote) : "memory");
-    return v;
-}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -8,8 +8,8 @@
 // vectors fill the eight B columns, so a second vector costs nothing and every further pair costs its products only: 8 clk
 // per m16n8k32 and SM quarter, measured.
 //
-// 28672 x 8192: one vector 20.0 us (27.8 by the ring kernel), eight 40.2 us (eight times 27.8). What bounds it: one or two vectors the
-// stream and the instructions on it alike (2.9 TB/s), eight the products.
+// 28672 x 8192: one vector 20.0 us (27.8 by the ring kernel). What bounds it: the stream and the instructions on it alike (2.9 TB/s). Three vectors
+// and more of larger matrices go to csrc/gemv_planes_tc.cu (eight: 38.9 us here, 26.1 there).
 //
 // Split: a cluster of S CTAs owns a range of 16-row tiles, each of its CTAs 1 / S of the columns, whose digit table stays in
 // shared memory for the whole launch (S is the smallest that makes it fit, or larger where a matrix has fewer tiles than the
@@ -45,9 +45,13 @@ struct PlaneArgs {
     long long wait_limit;
 };
 
+// Rows (planes of rows) that begin on 16-byte boundaries.
+inline bool plane_rows_aligned(const WeightDesc& w) { return (w.fmt == WF_SPARSE_TERNARY ? w.row_bytes : w.row_bytes / 2) % 16 == 0; }
 // Scratch for the digit table of `batch` vectors, for either format.
 size_t plane_prep_bytes(uint32_t cols, uint32_t batch);
 // ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only. launches: of the product, which is one.
 int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
+// The same for three vectors and more on tcgen05, where plane_rows_aligned.
+int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
 
 }  // namespace alice

@@ -20,6 +20,19 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 __device__ __forceinline__ uint64_t smem_desc_n(uint32_t addr, uint32_t block) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(block >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
+// One lane of a converged warp, in a form that leaves the compiler sure of it: products that a lane picked by its number issues take a loop over
+// the lanes each (44 clk a product instead of 8).
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{ .reg .pred p; .reg .b32 r; elect.sync r|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+    return p != 0;
+}
+// One lane waits for its warp: 32 of them polling take the shared-memory pipe from the other warps.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long limit = WAIT_CYCLE_LIMIT) {
+    bool ok = true;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait_limit(bar, parity, limit);
+    return __all_sync(0xffffffffu, ok);
+}
 // Instruction descriptor: bf16 x bf16 -> f32, M x N.
 __host__ __device__ constexpr uint32_t mma_desc(uint32_t m, uint32_t n, bool b_rows_k = false) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_rows_k << 16) | ((n / 8) << 17) | ((m / 16) << 24);

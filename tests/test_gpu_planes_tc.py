@@ -1,0 +1,84 @@
+"""Ternary planes and packed codes of larger matrices over three vectors and more (csrc/gemv_planes_tc.cu): rows dealt unevenly, ragged last tiles, columns
+that end inside a segment, fewer segments than a cluster has CTAs, more tiles than accumulators fit (two launches), gate and up, three matrices in one launch.
+
+Sums are integers and activations are rounded alike, so every vector's result equals, to the bit, that of the vector alone, which
+tests/test_gpu_planes.py holds against 64-bit numpy."""
+import numpy as np
+import pytest
+
+from alice_llm_b200 import synth
+from softmodel import SMOOTH_MIX, soft_model
+from test_gpu_planes import upload
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from alice_llm_b200.gpu import GpuEngine
+    e = GpuEngine(0)
+    yield e
+    e.close()
+
+
+def run(eng, call, x, rows):
+    """x [batch, cols] through `call` at once and one by one."""
+    y = eng.alloc_f32(len(x) * rows)
+    call(eng.upload_f32(x.reshape(-1)), y, len(x))
+    got = eng.read_f32(y)[:len(x) * rows].reshape(len(x), rows).copy()
+    for k in range(len(x)):
+        call(eng.upload_f32(x[k]), y, 1)
+        one = eng.read_f32(y)[:rows]
+        eng.sync()
+        assert np.array_equal(got[k], one), (k, np.abs(got[k] - one).max())
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("rows,cols,batch", [(4097, 8192, 5), (16500, 1152, 8), (2300, 7808, 6), (9001, 8192, 3), (70000, 512, 7), (300000, 256, 8), (700, 28672, 8), (18000, 4096, 4)])
+def test_as_alone(eng, oracle, rows, cols, batch, sparse):
+    rng = np.random.default_rng(rows + cols + batch)
+    m = synth.make_ternary(rng, rows, cols)
+    w = upload(eng, oracle, m, rows, cols, sparse)
+    x = synth.make_x(rng, cols, batch).reshape(batch, cols) * (10.0 ** rng.integers(-3, 4, (batch, 1))).astype(np.float32)
+    run(eng, lambda xd, y, n: eng.matvec_dev(w, xd, y, n), x, rows)
+    w.free()
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(3000, 4224, 8), (6001, 8192, 3), (20000, 8192, 8)])
+def test_gate_and_up(eng, oracle, rows, cols, batch):
+    rng = np.random.default_rng(rows)
+    g, u = (upload(eng, oracle, synth.make_ternary(rng, rows, cols), rows, cols, False) for _ in range(2))
+    x = synth.make_x(rng, cols, batch).reshape(batch, cols)
+    run(eng, lambda xd, y, n: eng.swiglu_dev(g, u, xd, y, n), x, rows)
+    g.free(), u.free()
+
+
+def test_not_finite_stays_with_its_vector(eng, oracle):
+    rng = np.random.default_rng(3)
+    rows, cols = 2500, 8192
+    w = upload(eng, oracle, synth.make_ternary(rng, rows, cols), rows, cols, False)
+    x = synth.make_x(rng, cols, 6).reshape(6, cols)
+    x[2, 77] = np.inf
+    y = eng.alloc_f32(6 * rows)
+    eng.matvec_dev(w, eng.upload_f32(x.reshape(-1)), y, 6)
+    got = eng.read_f32(y).reshape(6, rows)
+    eng.sync()
+    assert np.isnan(got[2]).all() and np.isfinite(np.delete(got, 2, 0)).all()
+    w.free()
+
+
+def test_model_with_three_matrices_in_a_launch(eng):
+    """Eight drafted tokens against the same tokens stepped: attention adds in another order, everything else is the same to the bit."""
+    from alice_llm_b200.gpu import GpuModel
+    cfg = dict(num_layers=1, hidden_dim=4096, intermediate_dim=4096, num_heads=32, num_kv_heads=8, head_dim=128, vocab_size=500, max_seq_len=32,
+               rope_theta=500000.0, eps=1e-5)
+    model = soft_model(np.random.default_rng(11), cfg, SMOOTH_MIX)
+    a, b = GpuModel.load(eng, model), GpuModel.load(eng, model)
+    toks = [3, 499, 41, 7, 8, 250, 1, 0]
+    got = np.asarray(a.forward_batch_and_read(toks), np.float64).reshape(8, 500)
+    want = np.asarray([b.forward_and_read(t) for t in toks], np.float64)
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+    ka, va = a.kv_read(0, 0, 8)
+    kb, vb = b.kv_read(0, 0, 8)
+    assert np.array_equal(ka, kb) and np.array_equal(va, vb)      # of the one layer: nothing of attention is in them
+    a.free(), b.free()
