@@ -267,6 +267,15 @@ static int check_pair(const alice_weights* g, const alice_weights* u, const char
     return ALICE_OK;
 }
 
+// Whether the CTAs of a matvec make the Q8_K blocks of its one vector themselves. Two launches cost a caller that queues call behind call 8 us; a product
+// that is over before that gains a launch less, though its own start is longer: Q4_K 4096 x 4096 8.0 -> 6.1 us a call (replayed from a graph 5.8 ->
+// 6.3), 1024 x 4096 7.8 -> 5.2, Q6_K 8192 x 4096 (28 MB) 9.8 -> 9.3, Q4_K 32768 x 1024 8.4 -> 7.8, 1024 x 8192 (5 MB) 7.9 -> 6.7, but 14336 x 4096 (33 MB) 8.9 -> 9.0,
+// 4096 x 8192 (19 MB) 7.9 -> 7.9 (graph 7.7 -> 8.6), 2048 x 14336 7.9 -> 9.1: up to 16 blocks of 256 two warps' worth each, up to 32 where little else is to do.
+static bool quantized_in_matvec(const WeightDesc& w, bool two, uint32_t batch) {
+    const uint64_t bytes = (uint64_t)w.rows * w.row_bytes * (two ? 2 : 1);
+    return batch == 1 && ((w.cols <= 4096 && bytes <= 28000000) || (w.cols <= 8192 && bytes <= 8000000));
+}
+
 // f32 input of a matvec. K-quant weights want it as Q8_K blocks (q4k_matvec = quantize_row_q8_k + q4k_matvec_preq,
 // src/gguf.rs:3600-3603): a small quantizer kernel runs ahead of the matvec, which is launched as its programmatic
 // dependent - its CTAs become resident and stream weights while the blocks are being written. (Measured on the FFN
@@ -283,6 +292,7 @@ static int matvec_common(alice_engine* e, const alice_weights* w0, const alice_w
     if (!format_uses_q8k(d.fmt)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
     if ((uintptr_t)x->p & 15) return fail(ALICE_E_INVALID, "%s: input vector must be 16-byte aligned", who);
     const uint32_t nb = d.cols / 256;
+    if (quantized_in_matvec(d, w1 != nullptr, batch)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
     int rc = ensure_scratch(e, Q8KLayout::make(nb, batch).total);
     if (rc) return rc;
     launch_quantize_q8k(x->p, d.cols, batch, e->scratch, e->stream, e->pdl);
@@ -361,15 +371,14 @@ int32_t alice_plan_query(alice_engine* e, const alice_weights* w, int32_t swiglu
     if (swiglu) op.up = &w->d;
     alignas(16) static float dummy[4];
     Q8KView v{};
-    (void)preq;     // the input always reaches the kernel prepared; the plan does not depend on who prepared it
-    if (format_uses_q8k(w->d.fmt)) { v.qs = reinterpret_cast<const int8_t*>(dummy); v.nb = w->d.cols / 256; op.q8 = &v; }
+    if (format_uses_q8k(w->d.fmt) && (preq || !quantized_in_matvec(w->d, swiglu != 0, 1))) { v.qs = reinterpret_cast<const int8_t*>(dummy); v.nb = w->d.cols / 256; op.q8 = &v; }
     else op.x = dummy;
     op.y = dummy;   // planning never dereferences the vectors
     StreamPlan pl;
     const int rc = plan_stream_gemv(op, cfg_of(e), pl);
     if (rc) return launch_rc(rc, "alice_plan_query");
     const StreamArgs& a = pl.args;
-    out[0] = pl.grid; out[1] = a.P; out[2] = a.slots; out[3] = a.rps; out[4] = a.groups; out[5] = a.nstages;
+    out[0] = pl.grid; out[1] = a.P; out[2] = a.slots; out[3] = a.rps; out[4] = pl.mma ? a.groups : walk_stages(pl); out[5] = a.nstages;
     out[6] = pl.kl; out[7] = pl.mma ? 1u : 0u; out[8] = pl.ksplit; out[9] = pl.ctas_per_sm;
     return ALICE_OK;
 }

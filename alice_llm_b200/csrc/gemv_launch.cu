@@ -329,24 +329,29 @@ int plan_stream_gemv(const GemvOp& op, const LaunchCfg& cfg, StreamPlan& pl) {
     }
     for (uint32_t i = op.nw; i < 4; i++) a.seg_t0[i] = total_sets;
     pl.grid = std::min(ctas, total_sets);
-    // the number of stages the walk produces, over all CTAs (what alice_plan_query reports)
-    a.groups = 0;
-    for (uint32_t cta = 0; cta < pl.grid; cta++) {
-        uint32_t t = (uint32_t)((uint64_t)total_sets * cta / pl.grid);
-        const uint32_t t_end = (uint32_t)((uint64_t)total_sets * (cta + 1) / pl.grid);
-        for (uint32_t sg = 0; t < t_end;) {
-            while (sg + 1 < op.nw && t >= a.seg_t0[sg + 1]) sg++;
-            const uint32_t T = std::min(t_end, a.seg_t0[sg + 1]) - t;
-            a.groups += (T + rps - 1) / rps;
-            t += T;
-        }
-    }
     a.tab_off = HDR_BYTES + nst * stage;
     pl.smem = HDR_BYTES + (size_t)nst * stage + act_bytes;
     pl.kl = kl; pl.swiglu = sw; pl.stage = stage;
     pl.mma = false; pl.ksplit = 1; pl.ctas_per_sm = per_sm;
     pl.args = a;
     return ALICE_OK;
+}
+
+uint32_t walk_stages(const StreamPlan& pl) {
+    const StreamArgs& a = pl.args;
+    const uint32_t total = a.seg_t0[a.nseg];
+    uint32_t n = 0;
+    for (uint32_t cta = 0; cta < pl.grid; cta++) {
+        uint32_t t = (uint32_t)((uint64_t)total * cta / pl.grid);
+        const uint32_t t_end = (uint32_t)((uint64_t)total * (cta + 1) / pl.grid);
+        for (uint32_t sg = 0; t < t_end;) {
+            while (sg + 1 < a.nseg && t >= a.seg_t0[sg + 1]) sg++;
+            const uint32_t T = std::min(t_end, a.seg_t0[sg + 1]) - t;
+            n += (T + a.rps - 1) / a.rps;
+            t += T;
+        }
+    }
+    return n;
 }
 
 namespace {

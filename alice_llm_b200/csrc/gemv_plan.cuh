@@ -18,6 +18,8 @@ struct StreamPlan {
     uint32_t ksplit = 1;      // column chunks, one launch each, accumulating into y (mma kernels with rows too wide for shared memory)
 };
 
+// Stages the row walk of the per-lane kernel makes, over all CTAs.
+uint32_t walk_stages(const StreamPlan& pl);
 int plan_stream_gemv(const GemvOp& op, const LaunchCfg& cfg, StreamPlan& pl);
 
 constexpr uint32_t STREAM_HDR_BYTES = (sizeof(StreamSmem) + 127) & ~127u;
