@@ -15,9 +15,8 @@
 // thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one thread
 // copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM). Where
 // tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
-// What bounds it: the unpacking and draining warps (issue slots half used, 22 % of the tensor pipe), and the last wave: 448 tiles of the
-// gate and up product of an 8B model over 148 SMs. A 256-token prompt of that model takes 14.9 ms, 23.0 by the integer path of mma.sync
-// (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
+// What bounds it: the unpacking and draining warps (issue slots half used, 22 % of the tensor pipe). A 256-token prompt of an 8B model takes
+// 14.2 ms, 23.0 by the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -54,7 +53,7 @@ struct KtArgs {
     const float* dt;             // [nb][dstride]: Q8_K scales
     float* y;
     const float* resid;
-    uint32_t y_stride, batch;
+    uint32_t y_stride, batch, tile_lo;      // tile_lo: first tile of the launch
     int* status;
     CUtensorMap tb;
 };
@@ -204,7 +203,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
     const uint32_t ring_s = smem_u32(ring);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     auto bar = [](uint64_t* b, uint32_t i) { return smem_u32(b + i); };
-    const uint32_t rank = KS > 1 ? blockIdx.x % KS : 0u, tile = blockIdx.x / KS, tok0 = blockIdx.y * KT_N;
+    const uint32_t rank = KS > 1 ? blockIdx.x % KS : 0u, tile = a.tile_lo + blockIdx.x / KS, tok0 = blockIdx.y * KT_N;
     uint32_t s = 0;
     if (!SW) while (s + 1 < a.nw && tile >= a.tile0[s + 1]) s++;
     constexpr uint32_t OUT = SW ? KT_M / 2 : KT_M;
@@ -446,13 +445,24 @@ int launch_tc(KtArgs a, const GemvOp& op, const LaunchCfg& cfg) {
     lc.attrs = at + 1; lc.numAttrs = cfg.pdl ? 1 : 0;
     if (cudaLaunchKernelEx(&lc, kt_prepare_kernel<FMT>, op.q8->qs, op.q8->d, op.q8->bsums, a.batch, a.nb, a.dstride, x, dt) != cudaSuccess) return ALICE_E_CUDA;
     const uint32_t tiles = a.tile0[a.nw], sms = (uint32_t)std::max(cfg.num_sms, 1);
-    uint32_t KS = 1;
-    while (KS < 8 && tiles * toks * KS * 2 <= sms && a.nb >= 8 * KS) KS *= 2;
-    at[0].val.clusterDim.x = KS;
-    lc.gridDim = dim3(tiles * KS, toks); lc.blockDim = dim3(KT_THREADS); lc.dynamicSmemBytes = G::SMEM;
-    lc.attrs = KS > 1 ? at : at + 1;
-    lc.numAttrs = (KS > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
-    return cudaLaunchKernelEx(&lc, kern, a, KS) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
+    // CTAs that share the columns of each of n tiles, where these leave SMs idle
+    auto shares = [&](uint32_t n, uint32_t least) { uint32_t k = 1; while (k < 8 && n * toks * k * 2 <= sms && a.nb >= least * k) k *= 2; return k; };
+    // Tiles over whole waves of the SMs, up to half a wave of them, are a launch of its own ahead of the others, their columns shared by clusters: a CTA
+    // takes its blocks and, in blocks, 1.5 for its start, 2.5 with a cluster's sum, the launch 2.5, so from a.nb = 7 on it is shorter than a wave. Measured
+    // with 256 vectors, without and with: gate and up of an 8B model (448 CTAs on 148 SMs) 162 and 140 us (Q5_K 195 and 161), 9728 x 4096 81
+    // and 53, 13312 x 4096 (60 CTAs over) 82 and 70, 10240 x 2048 48 and 35, 13312 x 2048 49 and 49. Shares of the main launch, eight blocks at least.
+    uint32_t rest = tiles * toks > sms ? (tiles * toks % sms + toks - 1) / toks : 0u;
+    if (rest && (rest * toks * 2 > sms || a.nb / shares(rest, 2) + 6 > a.nb)) rest = 0;
+    auto launch = [&](uint32_t lo, uint32_t n, uint32_t ks) {
+        a.tile_lo = lo;
+        at[0].val.clusterDim.x = ks;
+        lc.gridDim = dim3(n * ks, toks); lc.blockDim = dim3(KT_THREADS); lc.dynamicSmemBytes = G::SMEM;
+        lc.attrs = ks > 1 ? at : at + 1;
+        lc.numAttrs = (ks > 1 ? 1 : 0) + (cfg.pdl ? 1 : 0);
+        return cudaLaunchKernelEx(&lc, kern, a, ks) == cudaSuccess ? ALICE_OK : ALICE_E_CUDA;
+    };
+    const int rc = rest ? launch(tiles - rest, rest, shares(rest, 2)) : ALICE_OK;
+    return rc ? rc : launch(0, tiles - rest, shares(tiles - rest, 8));
 }
 
 }  // namespace

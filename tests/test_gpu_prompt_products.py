@@ -133,6 +133,25 @@ def test_swiglu(eng, qtype, rows, nb, batch):
     assert (np.abs(got - g * sig * u) <= bound).all(), (np.abs(got - g * sig * u) / bound).max()
 
 
+@pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("rows,nb,batch,swiglu", [(9600, 9, 256, False), (9601, 8, 200, False), (14000, 10, 256, False), (19000, 17, 128, False), (6300, 16, 300, False), (4800, 9, 200, True)])
+def test_tiles_over_whole_waves(eng, qtype, rows, nb, batch, swiglu):
+    """Up to half a wave of tiles over whole waves of 148: their columns shared by clusters of two to eight, the other tiles whole"""
+    cols, rng = 256 * nb, np.random.default_rng(rows + nb)
+    gate, up = (synth.make_weights(qtype, rng, rows, cols) for _ in range(2))
+    q8 = vectors(rng, batch, nb)
+    q8[0][:] /= np.float32(np.sqrt(cols))
+    g, dg = exact(eng, qtype, gate, rows, cols, q8)
+    got = run(eng, qtype, gate, rows, cols, q8, up if swiglu else None)
+    if not swiglu:
+        assert (np.abs(got - g) <= dg).all(), (np.abs(got - g) / dg).max()
+        return
+    u, du = exact(eng, qtype, up, rows, cols, q8)
+    sig = 1.0 / (1.0 + np.exp(-np.clip(g, -700, 700)))
+    bound = 1.1 * dg * (np.abs(u) + du) + np.abs(g * sig) * du + 2.0 ** -20 * np.abs(g * sig * u) + 1e-30
+    assert (np.abs(got - g * sig * u) <= bound).all(), (np.abs(got - g * sig * u) / bound).max()
+
+
 @pytest.mark.parametrize("qtype", [Q4_K, Q6_K])
 @pytest.mark.parametrize("batch", [20, 100])
 def test_residual(eng, qtype, batch):
