@@ -66,6 +66,13 @@ def test_attention_of_many_tokens(eng, heads, ctx, n):
     compare(eng, SMOOTH_MIX, heads, 512, 1024, ctx, n, 1e-4)
 
 
+@pytest.mark.parametrize("heads", [(2, 2), (10, 2), (16, 2), (32, 8)])
+@pytest.mark.parametrize("ctx,n", [(0, 3), (120, 5), (250, 6), (257, 6), (2048, 8), (5000, 2), (1000, 48)])
+def test_shares_of_attention(eng, heads, ctx, n):
+    """Tiles of 16, 32, 48 and 64 rows; one share, two to eight in a cluster, more through the scratch, clusters where that is too small"""
+    compare(eng, SMOOTH_MIX, heads, 512, 512, ctx, n, 1e-4)
+
+
 @pytest.mark.parametrize("n", [2, 9, 16, 17, 33, 64, 65, 129, 256, 300])
 @pytest.mark.parametrize("mix", [None, Q5KM], ids=["q4km", "q5km"])
 def test_k_quant_prompts(eng, mix, n):
