@@ -1,7 +1,7 @@
 // K-quant products with more than 64 vectors on the fifth-generation tensor cores (tcgen05.mma kind::f16).
 //
 // A weight enters as the integer scale x quant, an activation as its Q8_K integer, both exact in f16: up to 63 * 31 for Q4_K / Q5_K;
-// for Q6_K (up to 128 * 32) as a multiple of 32 and a remainder, two products. The f32 accumulator of one 256-column block then holds
+// for Q6_K (up to 128 * 32) the scale as a multiple of 16 and -8 .. 7, two products. The f32 accumulator of one 256-column block then holds
 // the integer dot of q4k_q8k_dot / q6k_q8k_dot (src/gguf.rs:3201-3251, :3282-3319), a second one the min term (sums of 16 activations,
 // at most 2048, times the 6-bit mins), and both are scaled by the block's f16 and f32 factors and added up in f32 registers once per block.
 //
@@ -11,12 +11,15 @@
 // or 64 columns) is exact there, but adds a block up in pieces, which costs bits on ordinary blocks (error of a row of 56 blocks 2.0e-7 for
 // two pieces, 2.8e-7 for four, 1.5e-7 for one, 1.6e-7 by integer sums) and a tenth of the time of a prompt.
 //
-// One CTA per SM, 128 rows x 128 vectors, 18 warps: 8 unpack raw blocks (cp.async, a block ahead) into the swizzled A tiles, half a row a
-// thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one thread
-// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM). Where
+// One CTA per SM, 128 rows x 128 vectors, 20 warps: 8 unpack raw blocks (cp.async, a block ahead) into the swizzled A tiles, half a row a
+// thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one warp
+// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM), 16 vectors ahead, which
+// takes registers the other warps give up (72 and 48 against 144; with 96 for all and 8 vectors at a time 137 us for that product, 128 so). Where
 // tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
-// What bounds it: the unpacking and draining warps (issue slots half used, 22 % of the tensor pipe). A 256-token prompt of an 8B model takes
-// 14.2 ms, 23.0 by the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
+// What bounds it: the unpacking warps, a chain of wait, read, compute, store and hand over for each k-tile: 128 us of which 104 are left without unpacking
+// and draining. Q6_K reads its words for two k-tiles at a time and multiplies by the two parts of the scale: 4096 x 14336 with 256 vectors 126 -> 102
+// us. Waits by one lane of a warp, or a row a thread and every other k-tile, are no faster (150, 132 us). A 256-token prompt of an 8B model takes
+// 12.5 ms, 23.0 by the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -28,7 +31,9 @@
 namespace alice {
 namespace {
 
-constexpr uint32_t KT_M = 128, KT_N = 128, KT_PROD = 256, KT_EPI = 256, KT_THREADS = KT_PROD + KT_EPI + 64;
+constexpr uint32_t KT_M = 128, KT_N = 128, KT_PROD = 256, KT_EPI = 256, KT_THREADS = KT_PROD + KT_EPI + 128;
+constexpr uint32_t KT_R = 96, KT_RU = 72, KT_RD = 144, KT_RM = 48;      // registers a thread at launch, then of the unpacking, draining and other warps
+static_assert(KT_PROD * KT_RU + KT_EPI * KT_RD + 128 * KT_RM <= KT_THREADS * KT_R, "a warpgroup would wait for registers for good");
 constexpr int KERR_KT_WAIT = 7;      // as the bf16 product: operands or accumulators of a tensor-core product
 
 template <int FMT> struct KtFmt;     // bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles and ring depth
@@ -136,33 +141,44 @@ __device__ __forceinline__ void kt_unpack(const uint8_t* raw, uint32_t scales, u
                 *reinterpret_cast<uint4*>(at + r * 128 + ((piece ^ (r & 7u)) * 16)) = make_uint4(out[4 * k], out[4 * k + 1], out[4 * k + 2], out[4 * k + 3]);
             }
         }
-    } else {
-        const uint32_t n = c >> 1, z = 2 * (c & 1) + half;       // quadrant z of half n of the block
-        const uint8_t* ql = raw + 64 * n + 32 * (z & 1);
-        const uint8_t* qh = raw + 128 + 32 * n;
-        const __half2 m2 = __float2half2_rn(49152.0f);           // sums with it are multiples of 32
+    }
+}
+// Q6_K: the words with the quants of k-tiles c and c + 1 (c even), word w = (k + r / 8) % 4 of either 16 columns: rows eight apart meet the same banks.
+__device__ __forceinline__ void k6_load(const uint8_t* raw, uint32_t c, uint32_t half, uint32_t rot, uint32_t (&l)[8], uint32_t (&h)[8]) {
+    const uint8_t* ql = raw + 32 * c + 32 * half;
+    const uint8_t* qh = raw + 128 + 16 * c;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int sc = (int)(int8_t)raw[192 + 8 * n + 2 * z + i];
-            const __half2 s2 = __half2half2(__int2half_rn(sc));
+    for (uint32_t j = 0; j < 8; j++) {
+        const uint32_t at = 16 * (j >> 2) + 4 * ((j + rot) & 3u);
+        l[j] = kld_u2(ql + at);
+        h[j] = kld_u2(qh + at);
+    }
+}
+// 32 weights (k-half `half` of k-tile c) into row r of the two A tiles at `at`: quant times a multiple of 16 next to the scale, and times the rest.
+__device__ __forceinline__ void k6_unpack(const uint8_t* raw, const uint32_t (&l)[8], const uint32_t (&h)[8], uint32_t c, uint32_t half, uint32_t rot, uint8_t* at, uint32_t r) {
+    const uint32_t z = 2 * (c & 1) + half;                    // quadrant of half c / 2 of the block
+    uint8_t* const row = at + r * 128;
+    const uint32_t base = (4 * half ^ (r & 7u)) << 4;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++) {
-                const uint32_t w = (k + (r >> 3)) & 3u;          // rows eight apart meet the same banks: let them take another word
-                const uint32_t l = kld_u2(ql + 16 * i + 4 * w) >> (z >> 1 ? 4 : 0), h = kld_u2(qh + 16 * i + 4 * w) >> (2 * z);
-                const uint32_t q = (l & 0x0f0f0f0fu) | ((h & 0x03030303u) << 4);
-                uint32_t hi[2], lo[2];
+    for (uint32_t i = 0; i < 2; i++) {
+        const int sc = (int)(int8_t)raw[192 + 8 * (c >> 1) + 2 * z + i], up = (sc + 8) & ~15;
+        const __half2 s_hi = __half2half2(__int2half_rn(up)), s_lo = __half2half2(__int2half_rn(sc - up));
 #pragma unroll
-                for (int p = 0; p < 2; p++) {                    // bytes 2 p and 2 p + 1, in order
-                    const uint32_t b = __byte_perm(q, 0x64u, p ? 0x4342u : 0x4140u);
-                    const __half2 u = __hsub2(u2h(b), __float2half2_rn(1056.0f));          // quant - 32
-                    const __half2 a = __hsub2(__hfma2(u, s2, m2), m2);                     // the multiple of 32 next to scale * quant
-                    hi[p] = h2u(a);
-                    lo[p] = h2u(__hfma2(u, s2, __hneg2(a)));
-                }
-                const uint32_t to = r * 128 + (((4 * half + 2 * i + (w >> 1)) ^ (r & 7u)) * 16) + (w & 1u) * 8;
-                *reinterpret_cast<uint2*>(at + to) = make_uint2(hi[0], hi[1]);
-                *reinterpret_cast<uint2*>(at + 16384 + to) = make_uint2(lo[0], lo[1]);
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t w = (k + rot) & 3u, j = 4 * i + k;
+            const uint32_t lw = c & 1 ? l[j] >> 4 : l[j];
+            const uint32_t hx = c & 1 ? h[j] >> (2 * half) : (half ? h[j] << 2 : h[j] << 4);
+            const uint32_t q = ((lw & 0x0f0f0f0fu) | (hx & 0xf0f0f0f0u)) & 0x3f3f3f3fu;
+            uint32_t hi[2], lo[2];
+#pragma unroll
+            for (int p = 0; p < 2; p++) {                     // bytes 2 p and 2 p + 1, in order
+                const __half2 u = __hsub2(u2h(__byte_perm(q, 0x64u, p ? 0x4342u : 0x4140u)), __float2half2_rn(1056.0f));      // quant - 32
+                hi[p] = h2u(__hmul2(u, s_hi));
+                lo[p] = h2u(__hmul2(u, s_lo));
             }
+            const uint32_t to = base ^ (i << 5) ^ (w << 3);
+            *reinterpret_cast<uint2*>(row + to) = make_uint2(hi[0], hi[1]);
+            *reinterpret_cast<uint2*>(row + 16384 + to) = make_uint2(lo[0], lo[1]);
         }
     }
 }
@@ -174,20 +190,28 @@ __device__ __forceinline__ void kt_mins(uint32_t m, uint32_t half, uint8_t* at, 
     *reinterpret_cast<uint4*>(at + r * 128 + ((half ^ (r & 7u)) * 16)) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-__device__ __forceinline__ void tmem_get8(uint32_t (&r)[8], uint32_t addr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+__device__ __forceinline__ void tmem_get16(uint32_t (&r)[16], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(addr)
         : "memory");
 }
-// what tmem_get8 asked for is there
-__device__ __forceinline__ void tmem_got8(uint32_t (&r)[8], uint32_t (&q)[8]) {
+// what was asked for is there
+__device__ __forceinline__ void tmem_got16(uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-          "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7])
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
         :
         : "memory");
 }
+__device__ __forceinline__ void tmem_got16(uint32_t (&r)[16], uint32_t (&q)[16]) {
+    tmem_got16(r);
+#pragma unroll
+    for (int i = 0; i < 16; i++) asm volatile("" : "+r"(q[i]));      // not before the wait
+}
+template <uint32_t N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <uint32_t N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 template <int FMT, bool SW>
 __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_constant__ KtArgs a, const uint32_t KS) {
@@ -228,10 +252,12 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
     // row of the matrix behind row i of the tile: with SwiGLU 64 gate rows, then the same 64 of up
     auto matrix = [&](uint32_t i) { return SW && i >= KT_M / 2 ? a.up : a.w[s]; };
     auto matrix_row = [&](uint32_t i) { return min(r0 + (SW ? i & (KT_M / 2 - 1) : i), seg_rows - 1); };
-    float acc[64];
+    float* const part = reinterpret_cast<float*>(ring);            // [vector][128 rows]
+    constexpr uint32_t PP = KT_M + 1;
     bool ok = true;
 
     if (warp < 8) {                       // ---- unpack
+        regs_down<KT_RU>();
         const uint32_t r = tid >> 1, half = tid & 1u;
         const uint64_t total = (uint64_t)seg_rows * a.row_bytes;
         auto fetch = [&](uint32_t k) {
@@ -256,7 +282,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
             fetch(k + 1);
             const uint8_t* src = raw + (k & 1u) * G::RAW + r * F::PITCH;
             if (FMT == 6) src += (matrix_row(r) * a.row_bytes + (b_lo + k) * F::BB) & 15u;
-            uint32_t sl = 0, sh = 0, ml = 0, mh = 0;
+            uint32_t sl = 0, sh = 0, ml = 0, mh = 0, ql[8], qh[8];
+            const uint32_t rot = r >> 3;
             if (FMT != 6) k4_unpack(kld<uint4>(src), sl, sh, ml, mh);
 #pragma unroll
             for (uint32_t c = 0; c < F::TILES; c++, it++) {
@@ -264,13 +291,26 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
                 ok = __all_sync(0xffffffffu, ok && mbar_wait(bar(empty_, st), ((it / F::STAGES) & 1) ^ 1));
                 if (!ok) break;
                 uint8_t* const at = ring + st * G::STAGE;
-                if (FMT != 6 && c == 4) kt_mins(half ? mh : ml, half, at, r); else kt_unpack<FMT>(src, half ? (c < 2 ? sl >> 8 : sh >> 8) : (c < 2 ? sl : sh), c, half, at, r);
+                if constexpr (FMT == 6) {
+                    if (!(c & 1)) k6_load(src, c, half, rot, ql, qh);
+                    k6_unpack(src, ql, qh, c, half, rot, at, r);
+                } else if (c == 4) {
+                    kt_mins(half ? mh : ml, half, at, r);
+                } else {
+                    kt_unpack<FMT>(src, half ? (c < 2 ? sl >> 8 : sh >> 8) : (c < 2 ? sl : sh), c, half, at, r);
+                }
                 fence_proxy_async();
                 mbar_arrive(bar(full_, st));
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();                  // the ring is free: all products and copies are done
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        regs_up<KT_R>();
     } else if (warp < 16) {               // ---- drain
+        regs_up<KT_RD>();
+        float acc[64];
         const uint32_t quad = warp & 3u, ch = (warp - 8) >> 2, i = quad * 32 + lane;
         const uint8_t* wrow = matrix(i) + (uint64_t)matrix_row(i) * a.row_bytes;
 #pragma unroll
@@ -291,28 +331,40 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t base = tmem + b * KT_N + ch * 64 + ((quad * 32) << 16);
             const float* e = dts[k & 3u] + ch * 64;
+            uint32_t p[2][16], m[2][16];      // a piece of 16 vectors ahead
+            tmem_get16(p[0], base);
+            if (FMT != 6) tmem_get16(m[0], base + 256);
 #pragma unroll
-            for (int c = 0; c < 8; c++) {
-                uint32_t p[8], m[8];
-                tmem_get8(p, base + c * 8);
-                tmem_get8(m, base + (FMT != 6 ? 256 + c * 8 : (c ^ 1) * 8));      // Q6_K has no second accumulator: two pieces at a time
-                tmem_got8(p, m);
+            for (int c = 0; c < 4; c++) {
+                if (FMT != 6) tmem_got16(p[c & 1], m[c & 1]); else tmem_got16(p[c & 1]);
+                if (c < 3) {
+                    tmem_get16(p[(c + 1) & 1], base + 16 * c + 16);
+                    if (FMT != 6) tmem_get16(m[(c + 1) & 1], base + 256 + 16 * c + 16);
+                }
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float x = e[c * 8 + j];
-                    if (FMT != 6) {
-                        acc[c * 8 + j] = fmaf(x, fmaf(-f.y, __uint_as_float(m[j]), f.x * __uint_as_float(p[j])), acc[c * 8 + j]);
-                    } else {
-                        acc[c * 8 + j] = fmaf(f.x * x, __uint_as_float(p[j]), acc[c * 8 + j]);
-                        acc[c * 8 + 8 + j] = fmaf(f.x * e[c * 8 + 8 + j], __uint_as_float(m[j]), acc[c * 8 + 8 + j]);
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 x4 = *reinterpret_cast<const float4*>(e + 16 * c + j);
+                    const float x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        float& y = acc[16 * c + j + q];
+                        if (FMT != 6) y = fmaf(x[q], fmaf(-f.y, __uint_as_float(m[c & 1][j + q]), f.x * __uint_as_float(p[c & 1][j + q])), y);
+                        else y = fmaf(f.x * x[q], __uint_as_float(p[c & 1][j + q]), y);
                     }
                 }
-                if (FMT == 6) c++;
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(bar(tempty_, b));
         }
-    } else if (warp == 16) {              // ---- B tiles
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();                  // the ring is free: all products and copies are done
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 64; j++) part[(ch * 64 + j) * PP + i] = acc[j];
+        regs_down<KT_R>();
+    } else {
+    regs_down<KT_RM>();
+    if (warp == 16) {              // ---- B tiles
         if (lane == 0) {
             pdl_wait();
             uint32_t it = 0;
@@ -330,52 +382,50 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
             for (uint32_t j = it - last; j < it; j++) mbar_wait(bar(full_, j % F::STAGES), (j / F::STAGES) & 1);
         }
         __syncwarp();
-    } else {                              // ---- products
-        if (lane == 0) {
+    } else if (warp == 17) {                              // ---- products
+        {
             constexpr uint32_t idesc = (1u << 4) | ((KT_N / 8) << 17) | ((KT_M / 16) << 24);      // f16 x f16 -> f32
             uint32_t it = 0;
             for (uint32_t k = 0; k < nblk && ok; k++) {
                 const uint32_t b = k & 1u, d = tmem + b * KT_N;
-                ok = mbar_wait(bar(tempty_, b), ((k >> 1) & 1) ^ 1);
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(tempty_, b), ((k >> 1) & 1) ^ 1));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (uint32_t c = 0; c < F::TILES; c++, it++) {
                     const uint32_t st = it % F::STAGES;
-                    ok = mbar_wait(bar(full_, st), (it / F::STAGES) & 1);
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(full_, st), (it / F::STAGES) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t at = ring_s + st * G::STAGE;
                     const uint64_t db = smem_desc(at + G::A);
-                    if (FMT != 6 && c == 4) {
-                        mma_f16(d + 256, smem_desc(at), db, idesc, false);
-                    } else {
+                    if (elect_lane()) {
+                        if (FMT != 6 && c == 4) {
+                            mma_f16(d + 256, smem_desc(at), db, idesc, false);
+                        } else {
 #pragma unroll
-                        for (uint32_t z = 0; z < F::ASUB; z++) {
-                            const uint64_t da = smem_desc(at + z * 16384);
+                            for (uint32_t z = 0; z < F::ASUB; z++) {
+                                const uint64_t da = smem_desc(at + z * 16384);
 #pragma unroll
-                            for (int kk = 0; kk < 4; kk++) mma_f16(d, da + 2 * kk, db + 2 * kk, idesc, c > 0 || z > 0 || kk > 0);
+                                for (int kk = 0; kk < 4; kk++) mma_f16(d, da + 2 * kk, db + 2 * kk, idesc, c > 0 || z > 0 || kk > 0);
+                            }
                         }
+                        mma_commit(bar(empty_, st));
+                        if (c + 1 == F::TILES) mma_commit(bar(tfull_, b));
                     }
-                    mma_commit(bar(empty_, st));
+                    __syncwarp();
                 }
-                if (ok) mma_commit(bar(tfull_, b));
             }
-            mma_commit(smem_u32(&drain_));
-            ok = mbar_wait(smem_u32(&drain_), 0) && ok;
+            if (elect_lane()) mma_commit(smem_u32(&drain_));
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&drain_), 0)) && ok;
         }
         __syncwarp();
     }
-    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_KT_WAIT);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();                      // the ring is free: all products and copies are done
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float* const part = reinterpret_cast<float*>(ring);            // [vector][128 rows]
-    constexpr uint32_t PP = KT_M + 1;
-    if (warp >= 8 && warp < 16) {
-        const uint32_t i = (warp & 3u) * 32 + lane, ch = (warp - 8) >> 2;
-#pragma unroll
-        for (int j = 0; j < 64; j++) part[(ch * 64 + j) * PP + i] = acc[j];
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();                  // the ring is free: all products and copies are done
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        regs_up<KT_R>();
     }
+    if (!ok && lane == 0) atomicCAS(a.status, 0, KERR_KT_WAIT);
     auto meet = [&]() {
         if (KS > 1) {
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
