@@ -27,11 +27,10 @@ __device__ __forceinline__ bool elect_lane() {
     asm volatile("{ .reg .pred p; .reg .b32 r; elect.sync r|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
     return p != 0;
 }
-// One lane waits for its warp: 32 of them polling take the shared-memory pipe from the other warps.
+// A warp waits, all lanes at once: with one lane of it asking, the others stand behind a branch, which the next step of a chain feels (ternary, eight vectors:
+// 8192 x 8192 13.4 against 12.4 us, gate and up of 28672 x 8192 53.3 against 52.2; K-quant prompt products 150 against 136).
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long limit = WAIT_CYCLE_LIMIT) {
-    bool ok = true;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait_limit(bar, parity, limit);
-    return __all_sync(0xffffffffu, ok);
+    return __all_sync(0xffffffffu, mbar_wait_limit(bar, parity, limit));
 }
 // Instruction descriptor: bf16 x bf16 -> f32, M x N.
 __host__ __device__ constexpr uint32_t mma_desc(uint32_t m, uint32_t n, bool b_rows_k = false) {
