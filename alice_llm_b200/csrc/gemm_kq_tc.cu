@@ -16,10 +16,11 @@
 // copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM), 16 vectors ahead, which
 // takes registers the other warps give up (72 and 48 against 144; with 96 for all and 8 vectors at a time 137 us for that product, 128 so). Where
 // tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
-// What bounds it: the unpacking warps, a chain of wait, read, compute, store and hand over for each k-tile: 128 us of which 104 are left without unpacking
-// and draining. Q6_K reads its words for two k-tiles at a time and multiplies by the two parts of the scale: 4096 x 14336 with 256 vectors 126 -> 102
-// us. Waits by one lane of a warp, or a row a thread and every other k-tile, are no faster (150, 132 us). A 256-token prompt of an 8B model takes
-// 12.5 ms, 23.0 by the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
+// What bounds it: the unpacking warps, a chain of wait, read, compute, store and hand over: of 128 us 104 are left without unpacking and
+// draining. Two k-tiles to a hand-over make it 122 for Q4_K; the shallower rings of the others lose by it (Q5_K 152 and 164). Q6_K reads its
+// words for two k-tiles at a time and multiplies by the two parts of the scale: 4096 x 14336 with 256 vectors 126 -> 102 us. Waits by one lane
+// of a warp, or a row a thread and every other k-tile, are no faster (150, 132 us). A 256-token prompt of an 8B model takes 12.4 ms, 23.0 by
+// the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -36,10 +37,10 @@ constexpr uint32_t KT_R = 96, KT_RU = 72, KT_RD = 144, KT_RM = 48;      // regis
 static_assert(KT_PROD * KT_RU + KT_EPI * KT_RD + 128 * KT_RM <= KT_THREADS * KT_R, "a warpgroup would wait for registers for good");
 constexpr int KERR_KT_WAIT = 7;      // as the bf16 product: operands or accumulators of a tensor-core product
 
-template <int FMT> struct KtFmt;     // bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles and ring depth
-template <> struct KtFmt<4> { static constexpr uint32_t BB = 144, CH = 9, PITCH = 144, TILES = 5, ASUB = 1, STAGES = 5; };
-template <> struct KtFmt<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 176, TILES = 5, ASUB = 1, STAGES = 4; };
-template <> struct KtFmt<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, TILES = 4, ASUB = 2, STAGES = 3; };
+template <int FMT> struct KtFmt;     // bytes of a raw block, 16-byte pieces and pitch of a raw row, k-tiles of a block, A tiles, ring depth, k-tiles unpacked at once
+template <> struct KtFmt<4> { static constexpr uint32_t BB = 144, CH = 9, PITCH = 144, TILES = 5, ASUB = 1, STAGES = 5, PER = 2; };
+template <> struct KtFmt<5> { static constexpr uint32_t BB = 176, CH = 11, PITCH = 176, TILES = 5, ASUB = 1, STAGES = 4, PER = 1; };
+template <> struct KtFmt<6> { static constexpr uint32_t BB = 210, CH = 14, PITCH = 240, TILES = 4, ASUB = 2, STAGES = 3, PER = 1; };
 
 template <int FMT>
 struct KtGeom {
@@ -286,21 +287,29 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kq_gemm_tc_kernel(const __grid_
             const uint32_t rot = r >> 3;
             if (FMT != 6) k4_unpack(kld<uint4>(src), sl, sh, ml, mh);
 #pragma unroll
-            for (uint32_t c = 0; c < F::TILES; c++, it++) {
-                const uint32_t st = it % F::STAGES;
-                ok = __all_sync(0xffffffffu, ok && mbar_wait(bar(empty_, st), ((it / F::STAGES) & 1) ^ 1));
+            for (uint32_t c0 = 0; c0 + F::PER <= F::TILES; c0 += F::PER) {
+                const uint32_t n = c0 + 2 * F::PER > F::TILES ? F::TILES - c0 : F::PER;      // the last takes the rest along
+#pragma unroll
+                for (uint32_t j = 0; j < n; j++) ok = ok && mbar_wait(bar(empty_, (it + j) % F::STAGES), (((it + j) / F::STAGES) & 1) ^ 1);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                uint8_t* const at = ring + st * G::STAGE;
-                if constexpr (FMT == 6) {
-                    if (!(c & 1)) k6_load(src, c, half, rot, ql, qh);
-                    k6_unpack(src, ql, qh, c, half, rot, at, r);
-                } else if (c == 4) {
-                    kt_mins(half ? mh : ml, half, at, r);
-                } else {
-                    kt_unpack<FMT>(src, half ? (c < 2 ? sl >> 8 : sh >> 8) : (c < 2 ? sl : sh), c, half, at, r);
+#pragma unroll
+                for (uint32_t j = 0; j < n; j++) {
+                    const uint32_t c = c0 + j;
+                    uint8_t* const at = ring + (it + j) % F::STAGES * G::STAGE;
+                    if constexpr (FMT == 6) {
+                        if (!(c & 1)) k6_load(src, c, half, rot, ql, qh);
+                        k6_unpack(src, ql, qh, c, half, rot, at, r);
+                    } else if (c == 4) {
+                        kt_mins(half ? mh : ml, half, at, r);
+                    } else {
+                        kt_unpack<FMT>(src, half ? (c < 2 ? sl >> 8 : sh >> 8) : (c < 2 ? sl : sh), c, half, at, r);
+                    }
                 }
                 fence_proxy_async();
-                mbar_arrive(bar(full_, st));
+#pragma unroll
+                for (uint32_t j = 0; j < n; j++) mbar_arrive(bar(full_, (it + j) % F::STAGES));
+                it += n;
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
