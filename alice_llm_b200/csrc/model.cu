@@ -449,7 +449,7 @@ int32_t alice_model_create(alice_engine* e, const alice_model_config* cfg, const
         m->layers.push_back(L);
     }
     m->nsplit = std::max<uint32_t>(1, std::min<uint32_t>(64, (2 * (uint32_t)e->num_sms) / (c.num_kv_heads / n)));
-    // (measured on the 8B and 27B decode steps: one wave of 2 CTAs per SM is the optimum; 18 or 64 splits cost 4-10 %)
+    // (room for two CTAs an SM, which several tokens take; one token takes a CTA an SM)
     const size_t kv_elems = (size_t)c.num_layers * c.max_seq_len * lkv;
     if (!rc) rc = upload_norm(m, &m->out_norm, output_norm, c.hidden_dim);
     constexpr uint32_t PIECE = 256;

@@ -51,6 +51,28 @@ def test_every_batch(eng, qtype, rows, blocks):
 
 
 @pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("cols,limit", [(256, 28000000), (4096, 28000000), (4352, 8000000), (8192, 8000000), (8448, 0)])
+def test_vector_quantized_in_the_product(eng, qtype, swiglu, cols, limit):
+    """A small product makes the Q8_K blocks of its vector itself: the same bits as from blocks made ahead, on both sides of the limits"""
+    rng = np.random.default_rng(cols)
+    most = limit // (synth.row_bytes(qtype, cols) * (2 if swiglu else 1))
+    x = eng.upload_f32(synth.make_x(rng, cols))
+    q = eng.alloc_q8k(cols, 1)
+    eng.quantize_q8k(x, q)
+    for rows in (5, most, most + 1) if cols > 256 and limit else (5, 3000):
+        w, u = (eng.upload_weights_typed(synth.make_weights(qtype, rng, rows, cols), rows, cols, quant(qtype)) for _ in range(2))
+        y = eng.alloc_f32(rows)
+        out = []
+        for product in (lambda: eng.swiglu_dev(w, u, x, y, 1), lambda: eng.swiglu_preq_dev(w, u, q, y)) if swiglu else (lambda: eng.matvec_dev(w, x, y, 1), lambda: eng.matvec_preq_dev(w, q, y)):
+            product()
+            out.append(eng.read_f32(y).view(np.uint32).copy())
+            eng.sync()
+        assert np.array_equal(out[0], out[1]), rows
+        w.free(), u.free()
+
+
+@pytest.mark.parametrize("qtype", [Q4_K, Q5_K, Q6_K])
 @pytest.mark.parametrize("rows,cols,swiglu", [(28672, 8192, False), (28672, 8192, True), (8192, 28672, False), (128256, 4096, False)])
 def test_one_pass_at_the_largest_sizes(eng, qtype, rows, cols, swiglu):
     w = eng.upload_weights_typed(np.zeros(rows * synth.row_bytes(qtype, cols), np.uint8), rows, cols, quant(qtype))
