@@ -275,6 +275,10 @@ static bool quantized_in_matvec(const WeightDesc& w, bool two, uint32_t batch) {
     const uint64_t bytes = (uint64_t)w.rows * w.row_bytes * (two ? 2 : 1);
     return batch == 1 && ((w.cols <= 4096 && bytes <= 28000000) || (w.cols <= 8192 && bytes <= 8000000));
 }
+static bool overlap(const float* a, size_t na, const float* b, size_t nb) {
+    const uintptr_t pa = (uintptr_t)a, pb = (uintptr_t)b;
+    return pa < pb + nb * sizeof(float) && pb < pa + na * sizeof(float);
+}
 
 // f32 input of a matvec. K-quant weights want it as Q8_K blocks (q4k_matvec = quantize_row_q8_k + q4k_matvec_preq,
 // src/gguf.rs:3600-3603): a small quantizer kernel runs ahead of the matvec, which is launched as its programmatic
@@ -292,7 +296,8 @@ static int matvec_common(alice_engine* e, const alice_weights* w0, const alice_w
     if (!format_uses_q8k(d.fmt)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
     if ((uintptr_t)x->p & 15) return fail(ALICE_E_INVALID, "%s: input vector must be 16-byte aligned", who);
     const uint32_t nb = d.cols / 256;
-    if (quantized_in_matvec(d, w1 != nullptr, batch)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
+    // a CTA that quantizes reads all of x, maybe behind the first rows that another has stored: not where x and y meet
+    if (quantized_in_matvec(d, w1 != nullptr, batch) && !overlap(x->p, d.cols, y->p, d.rows)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
     int rc = ensure_scratch(e, Q8KLayout::make(nb, batch).total);
     if (rc) return rc;
     launch_quantize_q8k(x->p, d.cols, batch, e->scratch, e->stream, e->pdl);

@@ -152,7 +152,8 @@ int32_t alice_weights_download(alice_engine* e, const alice_weights* w, uint8_t*
 /* quantized_matvec / q4k_matvec / q5k_matvec / q6k_matvec / q8_0_matvec / ternary_matvec /
  * sparse_ternary_matvec (src/gguf.rs:4214, 3600, 3502, 4077, 3811, 5303, 5808) and
  * GpuPass::matvec_* / matvec_auto (src/gpu.rs:1022-1392, 1795-1960): y = W x for `batch`
- * input vectors (1..8). K-quant weights quantize x to Q8_K first, as the CPU path does. */
+ * input vectors (1..8). K-quant weights quantize x to Q8_K first, as the CPU path does. x and y may share memory with
+ * K-quant weights only: there all of x is read before a row of y is stored. The same holds for alice_swiglu. */
 int32_t alice_matvec(alice_engine* e, const alice_weights* w, const alice_buf* x, alice_buf* y, uint32_t batch);
 /* quantized_matvec_preq / q4k_matvec_preq / ... (src/gguf.rs:4574, 3607, 3509, 4084). For Q1_0 /
  * Q2_0 weights the Q8_K blocks are turned back into f32 first (src/gguf.rs:4593-4605). */
