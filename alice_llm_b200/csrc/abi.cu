@@ -53,10 +53,11 @@ Q8KView view_of(const alice_q8k* q, uint32_t k) {
 int ensure_scratch(alice_engine* e, size_t bytes) {
     if (bytes <= e->scratch_bytes) return ALICE_OK;
     CU(cudaStreamSynchronize(e->stream));
-    if (e->scratch) CU(cudaFree(e->scratch));
-    e->scratch = nullptr; e->scratch_bytes = 0;
-    CU(cudaMalloc(&e->scratch, bytes));
-    e->scratch_bytes = bytes;
+    bytes = std::max(bytes, 2 * e->scratch_bytes);
+    void* p = nullptr;
+    CU(cudaMalloc(&p, bytes));
+    if (e->scratch) e->outgrown[e->n_outgrown++] = e->scratch;
+    e->scratch = p; e->scratch_bytes = bytes;
     return ALICE_OK;
 }
 
@@ -275,6 +276,18 @@ static bool quantized_in_matvec(const WeightDesc& w, bool two, uint32_t batch) {
     const uint64_t bytes = (uint64_t)w.rows * w.row_bytes * (two ? 2 : 1);
     return batch == 1 && ((w.cols <= 4096 && bytes <= 28000000) || (w.cols <= 8192 && bytes <= 8000000));
 }
+// The same for a caller that captures its stream: a launch less gains it nothing when the graph is replayed, so what counts is the time on the device.
+// In the product and with blocks ahead: Q4_K 2048 wide 3.7 / 3.7 us (2 MB) and 5.4 / 5.9 (16 MB), 3072 4.0 / 3.7 (2 MB), 5.6 / 5.6 (10 MB), 7.5 / 7.9
+// (24 MB), 4096 4.3 / 3.8 (2 MB), 5.7 / 5.3 (10 MB), 8.0 / 7.9 (28 MB), 8192 5.3 / 3.9 (2 MB); Q6_K 4096 4.4 / 4.5 (2 MB), 7.0 / 7.4 (16 MB), 8192 5.5 / 4.6 (2 MB).
+static bool quantized_in_replay(const WeightDesc& w, bool two) {
+    const uint64_t bytes = (uint64_t)w.rows * w.row_bytes * (two ? 2 : 1);
+    return w.cols <= 2048 || (w.cols <= 3072 && bytes >= 10000000) || (w.cols <= 4096 && w.fmt == WF_Q6_K);
+}
+static bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) { cudaGetLastError(); return false; }
+    return s != cudaStreamCaptureStatusNone;
+}
 static bool overlap(const float* a, size_t na, const float* b, size_t nb) {
     const uintptr_t pa = (uintptr_t)a, pb = (uintptr_t)b;
     return pa < pb + nb * sizeof(float) && pb < pa + na * sizeof(float);
@@ -296,10 +309,15 @@ static int matvec_common(alice_engine* e, const alice_weights* w0, const alice_w
     if (!format_uses_q8k(d.fmt)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
     if ((uintptr_t)x->p & 15) return fail(ALICE_E_INVALID, "%s: input vector must be 16-byte aligned", who);
     const uint32_t nb = d.cols / 256;
+    const size_t blocks = Q8KLayout::make(nb, batch).total;
+    int rc;
     // a CTA that quantizes reads all of x, maybe behind the first rows that another has stored: not where x and y meet
-    if (quantized_in_matvec(d, w1 != nullptr, batch) && !overlap(x->p, d.cols, y->p, d.rows)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
-    int rc = ensure_scratch(e, Q8KLayout::make(nb, batch).total);
-    if (rc) return rc;
+    if (quantized_in_matvec(d, w1 != nullptr, batch) && !overlap(x->p, d.cols, y->p, d.rows)) {
+        const bool graph = capturing(e->stream);
+        if (!graph && (rc = ensure_scratch(e, blocks))) return rc;      // a later capture cannot allocate
+        if (!graph || blocks > e->scratch_bytes || quantized_in_replay(d, w1 != nullptr)) return run_gemv(e, w0, w1, nullptr, x->p, y->p, batch, who);
+    }
+    if ((rc = ensure_scratch(e, blocks))) return rc;
     launch_quantize_q8k(x->p, d.cols, batch, e->scratch, e->stream, e->pdl);
     CU(cudaGetLastError());
     const Q8KView v = view_at(e->scratch, nb, batch);

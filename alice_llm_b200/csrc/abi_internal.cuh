@@ -18,6 +18,8 @@ struct alice_engine {
     int* status_host = nullptr;   // pinned host word alice_sync copies it into
     void* scratch = nullptr;      // engine-owned scratch: Q8_K of the current input, or its f32 form
     size_t scratch_bytes = 0;
+    void* outgrown[64] = {};      // scratch of before, whose address graphs of the caller's may hold; each at most half of the next, all together
+    uint32_t n_outgrown = 0;      // less than scratch_bytes
     void* prep = nullptr;         // engine-owned scratch of the bit-plane kernels: the activation digit table of the current input
     size_t prep_bytes = 0;
     long long wait_limit = 0;          // SM cycles a kernel wait may take (0 = about one second)

@@ -135,6 +135,7 @@ int32_t alice_engine_destroy(alice_engine* e) {
     cudaStreamSynchronize(e->stream);
     alice::tp_release(e);
     if (e->scratch) cudaFree(e->scratch);
+    for (; e->n_outgrown; e->n_outgrown--) cudaFree(e->outgrown[e->n_outgrown - 1]);
     if (e->prep) cudaFree(e->prep);
     if (e->status) cudaFree(e->status);
     if (e->status_host) cudaFreeHost(e->status_host);
