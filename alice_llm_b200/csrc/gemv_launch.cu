@@ -584,10 +584,11 @@ int batch_plan(const GemvOp& op, const LaunchCfg& cfg, uint32_t* launches, uint3
 
 // ---- stand-alone hand-over kernel ----------------------------------------------------------------------------
 namespace {
-constexpr int PUB_WARPS = 4;
-
-__global__ void __launch_bounds__(PUB_WARPS * 32) publish_vector_kernel(const __grid_constant__ Publish p, int* status) {
-    __shared__ double red[PUB_WARPS];
+// WHOLE: a CTA of NW warps has a vector, else a part of one. Bounds on registers: CTAs of four warps are there to become resident beside those of a matvec
+// (110 instead of 72 registers: a decoded token of 8B shapes 4 % longer, eight tokens of a ternary model 7 %).
+template <int NW, bool WHOLE>
+__global__ void __launch_bounds__(NW * 32, NW == 4 ? 7 : 2) publish_vector_kernel(const __grid_constant__ Publish p, int* status) {
+    __shared__ double red[NW];
     __shared__ int ok;
     pdl_launch_dependents();
     pdl_wait();
@@ -596,24 +597,29 @@ __global__ void __launch_bounds__(PUB_WARPS * 32) publish_vector_kernel(const __
         __syncthreads();
         if (!ok) return;
     }
-    if (p.dst.qs != nullptr || p.dst.xn != nullptr) publish_vector<PUB_WARPS, 1>(p, red, blockIdx.y, blockIdx.x, gridDim.x);
+    if (p.dst.qs == nullptr && p.dst.xn == nullptr) return;
+    if (WHOLE) publish_vector<NW, 1>(p, red, blockIdx.y);
+    else publish_part<NW, 1>(p, red, blockIdx.y, blockIdx.x, gridDim.x);
 }
 }  // namespace
 
-// A block a warp, four warps a CTA: small enough to become resident beside the CTAs of the matvec it waits for, and no warp has a second
-// block (one CTA of 16 warps a vector: a decoded token of 8B shapes 70.8 us a layer with two such launches, 69.2 this way; 27B 91.8 -> 89.2).
+// The vectors of a step: a block a warp, four warps a CTA, small enough to become resident beside the CTAs of the matvec it waits for (one CTA of 16 warps
+// a vector: a decoded token of 8B shapes 70.8 us a layer with two such launches, 69.2 this way; 27B 91.8 -> 89.2). A CTA of 16 warps a vector where
+// that is not what counts: the vectors of a prompt, of which every CTA of four warps would take the sum over all again (256 of 4096 elements 5.1 against
+// 3.6 us, of 8192 11.2 against 4.9), and behind peers, where one CTA has all of it (4096 and 8192 elements: 4 warps 4.3 and 6.9 us, 16 warps 2.5 and 3.3).
 cudaError_t launch_publish_vector(const Publish& p, int* status, cudaStream_t stream, bool pdl) {
-    const uint32_t blocks = (p.n + QK_K - 1) / QK_K, parts = p.npeers ? 1 : (blocks + PUB_WARPS - 1) / PUB_WARPS;
+    const uint32_t blocks = (p.n + QK_K - 1) / QK_K;
+    const bool many = p.npeers || p.batch > (uint32_t)MAX_BATCH;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(parts, p.npeers ? 1 : p.batch);
-    lc.blockDim = dim3(PUB_WARPS * 32);
+    lc.gridDim = dim3(many ? 1 : (blocks + 3) / 4, p.npeers ? 1 : p.batch);
+    lc.blockDim = dim3(many ? 512 : 128);
     lc.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at;
     lc.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&lc, publish_vector_kernel, p, status);
+    return cudaLaunchKernelEx(&lc, many ? publish_vector_kernel<16, true> : blocks <= 4 ? publish_vector_kernel<4, true> : publish_vector_kernel<4, false>, p, status);
 }
 
 }  // namespace alice

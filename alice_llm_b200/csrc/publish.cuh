@@ -2,9 +2,9 @@
 //
 // Every CTA of a matvec needs its whole input in the form its inner loop reads: Q8_K blocks for the K-quant
 // formats, the RMS-normalised f32 vector for the others. That form is the same in every CTA, so it is computed
-// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel, a warp per block of 256; the
+// once - by a small stand-alone kernel launched between producer and consumer (publish_vector_kernel; the
 // embedding kernel, a CTA per token, does it for its own output) - and left in global memory; the consumer's CTAs fetch
-// it straight into registers. With a tensor-parallel group the same kernel first runs the hand-over of the rows the
+// it straight into registers. With a tensor-parallel group one CTA of the same kernel first runs the hand-over of the rows the
 // peers have pushed (publish_peer_gate). Arithmetic: rms_norm (src/llama3.rs:5244-5256:
 // f64 sum of squares, f32 mean / sqrt / divide, (x * scale) * w) and quantize_row_q8_k (src/gguf.rs:1323-1374).
 #pragma once
@@ -112,11 +112,25 @@ __device__ __forceinline__ void pub_emit_block(const PublishDst& dst, const Q8KL
     }
 }
 
-// Vector k, blocks part * NW + warp, + parts * NW ...: run by NW warps (threads 0 .. NW*32-1 of the CTA) that meet on named barrier `BAR`. A
-// block of 256 elements is a warp's, 8 consecutive ones a lane's. With a norm every CTA of the vector takes the sum over all of it (f64, its
-// loads in flight together), so the CTAs need nothing of each other. `red` = NW doubles of shared memory.
+// rms_norm's factor from what each lane has added up (f64): NW warps that meet on named barrier `BAR`, `red` = NW doubles of shared memory.
 template <int NW, int BAR>
-static __device__ __noinline__ void publish_vector(const Publish& p, double* red, uint32_t k, uint32_t part = 0, uint32_t parts = 1) {
+__device__ __forceinline__ float pub_norm_scale(double ss, double* red, uint32_t n, float eps) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");
+    double tot = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; w++) tot += red[w];
+    const float mean = (float)(tot / (double)n);
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+}
+
+// Vector k, blocks part * NW + warp, + parts * NW ...: run by the NW warps of a CTA (threads 0 .. NW*32-1). A block of 256 elements is a
+// warp's, 8 consecutive ones a lane's. With a norm every CTA of the vector takes the sum over all of it (its loads in flight together), so the
+// CTAs need nothing of each other.
+template <int NW, int BAR>
+__device__ __forceinline__ void publish_part(const Publish& p, double* red, uint32_t k, uint32_t part, uint32_t parts) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = p.n, nblk = (n + QK_K - 1) / QK_K, b0 = part * NW + warp;
     const float* x = p.src + (size_t)k * n;
@@ -136,16 +150,7 @@ static __device__ __noinline__ void publish_vector(const Publish& p, double* red
 #pragma unroll
             for (int i = 0; i < LB; i++) ss[i & 1] += pub_sumsq(v[i]);
         }
-        double s1 = ss[0] + ss[1];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        if (lane == 0) red[warp] = s1;
-        asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NW * 32) : "memory");
-        double tot = 0.0;
-#pragma unroll
-        for (int w = 0; w < NW; w++) tot += red[w];
-        const float mean = (float)(tot / (double)n);
-        scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
+        scale = pub_norm_scale<NW, BAR>(ss[0] + ss[1], red, n, p.eps);
     }
     for (uint32_t b = b0; b < nblk; b += parts * NW) {
         if (b != b0) {
@@ -153,6 +158,41 @@ static __device__ __noinline__ void publish_vector(const Publish& p, double* red
             if (p.norm_w != nullptr) wv = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
         }
         pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv, scale, wv) : xv, lane, k, b, n);
+    }
+}
+
+// Vector k by one CTA: up to two blocks a warp stay in registers between the sum and the second pass (one trip to L2), longer vectors are read twice.
+template <int NW, int BAR>
+__device__ __forceinline__ void publish_vector(const Publish& p, double* red, uint32_t k) {
+    constexpr int HELD = 2;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t n = p.n, nblk = (n + QK_K - 1) / QK_K;
+    if (nblk > (uint32_t)(NW * HELD)) {
+        publish_part<NW, BAR>(p, red, k, 0, 1);
+        return;
+    }
+    const float* x = p.src + (size_t)k * n;
+    Q8KLaneInput xv[HELD], wv[HELD];
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+        const uint32_t b = warp + (uint32_t)i * NW;
+        if (b < nblk) {
+            xv[i] = pub_load8(x, b * QK_K + lane * 8, n);
+            if (p.norm_w != nullptr) wv[i] = pub_load8_w(p.norm_w, b * QK_K + lane * 8, n);
+        }
+    }
+    float scale = 1.0f;
+    if (p.norm_w != nullptr) {
+        double ss = 0.0;
+#pragma unroll
+        for (int i = 0; i < HELD; i++)
+            if (warp + (uint32_t)i * NW < nblk) ss += pub_sumsq(xv[i]);
+        scale = pub_norm_scale<NW, BAR>(ss, red, n, p.eps);
+    }
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+        const uint32_t b = warp + (uint32_t)i * NW;
+        if (b < nblk) pub_emit_block(p.dst, p.norm_w != nullptr ? pub_scale(xv[i], scale, wv[i]) : xv[i], lane, k, b, n);
     }
 }
 

@@ -73,6 +73,13 @@ def test_shares_of_attention(eng, heads, ctx, n):
     compare(eng, SMOOTH_MIX, heads, 512, 512, ctx, n, 1e-4)
 
 
+@pytest.mark.parametrize("hidden", [256, 1184, 2048, 2304, 8192, 8448])
+@pytest.mark.parametrize("n", [8, 9])
+def test_prepared_vectors(eng, hidden, n):
+    """Up to eight vectors are prepared by CTAs of four warps, more by one of sixteen each: vectors that fit the registers of either and that do not"""
+    compare(eng, SMOOTH_MIX, (4, 2), hidden, 512, 20, n, 1e-4)
+
+
 @pytest.mark.parametrize("n", [2, 9, 16, 17, 33, 64, 65, 129, 256, 300])
 @pytest.mark.parametrize("mix", [None, Q5KM], ids=["q4km", "q5km"])
 def test_k_quant_prompts(eng, mix, n):
