@@ -7,6 +7,8 @@
 //   o_t = S^T (G_t q_t) + sum_s B_ts u_s,   S <- G_W S + sum_s (P_sW k_s) u_s^T.
 // A, B and the inverse depend on the projections only and are made for all blocks at once; what remains on the path from
 // block to block are three small products per block, in f32. Decays enter as products, never as quotients.
+#include <algorithm>
+
 #include "dense_dev.cuh"
 #include "mixers.cuh"
 
@@ -238,11 +240,11 @@ __device__ __forceinline__ float4 reduce64(float (&v)[64], uint32_t lane) {
 template <int DP, int NW>
 struct ScanStage {
     float k[W][DP], q[W][DP], g[W][DP], v[W][8 * NW], inv[W][W], b[W][W];
-    float end[DP];                 // decay over the whole block
 };
-template <int DP, int NW>
+template <int DP, int NW, bool AHEAD>
 struct ScanSmem {
-    ScanStage<DP, NW> st[3];
+    ScanStage<DP, NW> st[AHEAD ? 3 : 2];
+    float end[AHEAD ? 3 : 1][DP];  // decay over the whole block (two CTAs of keys 256 wide just fit an SM without AHEAD)
     float w[W][8 * NW];            // v - S^T (G k)
     float y[W][8 * NW];            // S^T (G q)
     float2 u[W][8 * NW];           // writes, twice each
@@ -269,15 +271,39 @@ __device__ __forceinline__ void scan_fetch(ScanStage<DP, NW>& st, const DeltaArg
     }
 }
 
-// grid (vp / (8 NW), heads), 2 NW warps. A warp of the first NW owns eight columns of the state, four per half-warp, a lane DP / 16 of their
-// rows (register pairs). The others bring the tokens in, two blocks ahead, and work out their decays, one block ahead: in the same warps these were a
-// chain of sixteen steps between the blocks of a chain (2048 tokens of eight layers, four of them scans of 32 heads: 13.35 -> 12.42 ms). What bounds it:
-// latency, a warp a scheduler has the state, 128 blocks one after the other.
+// In place: k -> G k, q -> G q, g -> (decays after s) k_s; absent tokens have k = q = 0 and decay 1.
 template <int DP, int NW>
-__global__ void __launch_bounds__(2 * NW * 32) delta_scan_kernel(const __grid_constant__ DeltaArgs a, uint32_t tokens) {
+__device__ __forceinline__ void scan_decays(ScanStage<DP, NW>& st, float* end, uint32_t n, uint32_t tid) {
+    for (uint32_t d = tid; d < DP; d += NW * 32) {
+        float k[W], g[W], p = 1.0f;
+#pragma unroll
+        for (int t = 0; t < W; t++) {
+            k[t] = st.k[t][d];
+            g[t] = (uint32_t)t < n ? st.g[t][d] : 1.0f;
+            p *= g[t];
+            st.k[t][d] = p * k[t];
+            st.q[t][d] *= p;
+        }
+        end[d] = p;
+        p = 1.0f;
+#pragma unroll
+        for (int t = W - 1; t >= 0; t--) {
+            st.g[t][d] = p * k[t];
+            p *= g[t];
+        }
+    }
+}
+
+// grid (vp / (8 NW), heads). A warp of the first NW owns eight columns of the state, four per half-warp, a lane DP / 16 of their
+// rows (register pairs). AHEAD: as many warps again bring the tokens in, two blocks ahead, and work out their decays, one block ahead: in the same
+// warps these are a chain of sixteen steps between the blocks of a chain (2048 tokens of eight layers, four of them scans of 32 heads: 13.35 -> 12.42
+// ms). What bounds it: latency, a warp a scheduler has the state, 128 blocks one after the other. Such a CTA takes more of an SM: see scan_width.
+template <int DP, int NW, bool AHEAD>
+__global__ void __launch_bounds__((AHEAD ? 2 : 1) * NW * 32) delta_scan_kernel(const __grid_constant__ DeltaArgs a, uint32_t tokens) {
     constexpr int EL = DP / 16, NP = EL / 2, NC = EL / 4, COLS = 8 * NW;   // rows per lane, in NC runs of four
+    constexpr uint32_t STAGES = AHEAD ? 3 : 2;
     extern __shared__ __align__(16) uint8_t raw[];
-    auto& sm = *reinterpret_cast<ScanSmem<DP, NW>*>(raw);
+    auto& sm = *reinterpret_cast<ScanSmem<DP, NW, AHEAD>*>(raw);
     const DeltaShape& s = a.s;
     const uint32_t tid = threadIdx.x, lane = tid & 31, dg = lane & 15, warp = tid >> 5, h = blockIdx.y, kh = h / (s.heads / s.kv_heads), c0 = blockIdx.x * COLS;
     const uint32_t cw = warp * 8, cl = cw + (lane >> 4) * 4;   // first column of the warp, of the lane
@@ -292,43 +318,21 @@ __global__ void __launch_bounds__(2 * NW * 32) delta_scan_kernel(const __grid_co
         }
     };
     const uint32_t nblk = (tokens + W - 1) / W;
-    if (warp >= NW) {
+    auto fetch = [&](uint32_t blk, uint32_t thread) {
+        if (blk < nblk) scan_fetch<DP, NW>(sm.st[blk % STAGES], a, blk * W, min(tokens - blk * W, (uint32_t)W), h, kh, c0, thread);
+        cp_commit();
+    };
+    auto decays = [&](uint32_t blk, uint32_t thread) { scan_decays<DP, NW>(sm.st[blk % STAGES], sm.end[AHEAD ? blk % STAGES : 0], min(tokens - blk * W, (uint32_t)W), thread); };
+    if (AHEAD && warp >= NW) {
         const uint32_t pt = tid - NW * 32;
-        auto fetch = [&](uint32_t blk) {
-            if (blk < nblk) scan_fetch<DP, NW>(sm.st[blk % 3], a, blk * W, min(tokens - blk * W, (uint32_t)W), h, kh, c0, pt);
-            cp_commit();
-        };
-        // in place: k -> G k, q -> G q, g -> (decays after s) k_s; absent tokens have k = q = 0 and decay 1
-        auto decays = [&](uint32_t blk) {
-            ScanStage<DP, NW>& st = sm.st[blk % 3];
-            const uint32_t n = min(tokens - blk * W, (uint32_t)W);
-            for (uint32_t d = pt; d < DP; d += NW * 32) {
-                float k[W], g[W], p = 1.0f;
-#pragma unroll
-                for (int t = 0; t < W; t++) {
-                    k[t] = st.k[t][d];
-                    g[t] = (uint32_t)t < n ? st.g[t][d] : 1.0f;
-                    p *= g[t];
-                    st.k[t][d] = p * k[t];
-                    st.q[t][d] *= p;
-                }
-                st.end[d] = p;
-                p = 1.0f;
-#pragma unroll
-                for (int t = W - 1; t >= 0; t--) {
-                    st.g[t][d] = p * k[t];
-                    p *= g[t];
-                }
-            }
-        };
-        fetch(0);
-        fetch(1);
+        fetch(0, pt);
+        fetch(1, pt);
         for (uint32_t blk = 0; blk <= nblk; blk++) {      // works on block blk; the state's warps on the one before
             cp_wait<1>();
             asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");      // the copies of all of these warps
-            if (blk < nblk) decays(blk);
+            if (blk < nblk) decays(blk, pt);
             __syncthreads();
-            fetch(blk + 2);                               // in the place of block blk - 1
+            fetch(blk + 2, pt);                           // in the place of block blk - 1
         }
         cp_wait<0>();
         return;
@@ -336,10 +340,18 @@ __global__ void __launch_bounds__(2 * NW * 32) delta_scan_kernel(const __grid_co
     float2 S[4][NP];
 #pragma unroll
     for (int c = 0; c < 4; c++) rows(sp + c * DP, S[c]);
-    __syncthreads();                                      // block 0 is ready
+    if (AHEAD) __syncthreads();                           // block 0 is ready
+    else fetch(0, tid);
     for (uint32_t blk = 0; blk < nblk; blk++) {
         const uint32_t t0 = blk * W, n = min(tokens - t0, (uint32_t)W);
-        const ScanStage<DP, NW>& st = sm.st[blk % 3];
+        const ScanStage<DP, NW>& st = sm.st[blk % STAGES];
+        if (!AHEAD) {
+            fetch(blk + 1, tid);
+            cp_wait<1>();
+            __syncthreads();
+            decays(blk, tid);
+            __syncthreads();
+        }
 #pragma unroll 1
         for (int pass = 0; pass < 2; pass++) {   // S^T (G k), then S^T (G q)
             float v[64];
@@ -398,7 +410,7 @@ __global__ void __launch_bounds__(2 * NW * 32) delta_scan_kernel(const __grid_co
                     if (tl + 4 * i < n) a.o[((size_t)(t0 + tl + 4 * i) * s.heads + h) * s.vdim + c0 + c] = o[i];
         }
         float2 e[NP];
-        rows(st.end + dg * 4, e);
+        rows(sm.end[AHEAD ? blk % STAGES : 0] + dg * 4, e);
 #pragma unroll
         for (int c = 0; c < 4; c++)
 #pragma unroll
@@ -586,13 +598,44 @@ cudaError_t step_e(const DeltaStepArgs& a, cudaStream_t st, bool pdl) {
     return cudaLaunchKernelEx(&lc, delta_step_kernel<E>, a);
 }
 
-template <int DP, int NW>
+template <int DP, int NW, bool AHEAD>
 cudaError_t scan_inst(const DeltaArgs& a, uint32_t tokens, cudaStream_t st, bool pdl) {
+    return launch_pdl(delta_scan_kernel<DP, NW, AHEAD>, dim3(a.s.vp / (8 * NW), a.s.heads), dim3((AHEAD ? 2 : 1) * NW * 32), sizeof(ScanSmem<DP, NW, AHEAD>), st, pdl, a, tokens);
+}
+// CTAs that the chip holds at once, asked for once per device.
+template <int DP, int NW, bool AHEAD>
+cudaError_t scan_room(uint32_t& ctas) {
     static bool done[64] = {};
-    constexpr size_t smem = sizeof(ScanSmem<DP, NW>);
-    const cudaError_t err = allow_smem(delta_scan_kernel<DP, NW>, smem, done);
+    static uint32_t known[64] = {};
+    constexpr size_t smem = sizeof(ScanSmem<DP, NW, AHEAD>);
+    int dev = 0, per = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) err = allow_smem(delta_scan_kernel<DP, NW, AHEAD>, smem, done);
     if (err != cudaSuccess) return err;
-    return launch_pdl(delta_scan_kernel<DP, NW>, dim3(a.s.vp / (8 * NW), a.s.heads), dim3(2 * NW * 32), smem, st, pdl, a, tokens);
+    if (dev < 64 && known[dev]) { ctas = known[dev]; return cudaSuccess; }
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, delta_scan_kernel<DP, NW, AHEAD>, (AHEAD ? 2 : 1) * NW * 32, smem);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess) return err;
+    ctas = (uint32_t)std::max(per * sms, 1);
+    if (dev < 64) known[dev] = ctas;
+    return cudaSuccess;
+}
+// Warps that work ahead make a CTA larger: an SM holds two instead of three of keys 128 wide, one instead of two of 256. They pay unless that means
+// another wave of CTAs (four layers of 1024 tokens, without and with: 16 heads 256 x 256 3.00 and 2.11 ms, 20 heads 3.36 and 3.51, 48 heads 5.40 and 5.55; 64
+// heads 128 x 128 3.48 and 2.85, 80 heads 3.79 and 3.86). Of keys 64 wide an SM holds enough for its schedulers either way (250 heads 5.04 and 4.79).
+template <int DP, int NW>
+cudaError_t scan_width(const DeltaArgs& a, uint32_t tokens, cudaStream_t st, bool pdl) {
+    uint32_t ahead = 0;
+    cudaError_t err = scan_room<DP, NW, true>(ahead);
+    if (err != cudaSuccess) return err;
+    if constexpr (DP > 64) {
+        uint32_t plain = 0;
+        err = scan_room<DP, NW, false>(plain);
+        if (err != cudaSuccess) return err;
+        const uint32_t ctas = a.s.heads * (a.s.vp / (8 * NW));
+        if ((ctas + ahead - 1) / ahead > (ctas + plain - 1) / plain) return scan_inst<DP, NW, false>(a, tokens, st, pdl);
+    }
+    return scan_inst<DP, NW, true>(a, tokens, st, pdl);
 }
 template <int DP>
 cudaError_t scan_dim(const DeltaArgs& a, uint32_t tokens, cudaStream_t st, bool pdl) {
@@ -603,7 +646,7 @@ cudaError_t scan_dim(const DeltaArgs& a, uint32_t tokens, cudaStream_t st, bool 
     err = launch_pdl(delta_pairs_kernel<DP>, dim3((tokens + W - 1) / W, a.s.heads), dim3(256), smem, st, pdl, a, tokens);
     if (err != cudaSuccess) return err;
     // few columns: narrower CTAs, so that more SMs have one
-    return a.s.heads * (a.s.vp / 32) < 100 ? scan_inst<DP, 2>(a, tokens, st, pdl) : scan_inst<DP, 4>(a, tokens, st, pdl);
+    return a.s.heads * (a.s.vp / 32) < 100 ? scan_width<DP, 2>(a, tokens, st, pdl) : scan_width<DP, 4>(a, tokens, st, pdl);
 }
 
 }  // namespace

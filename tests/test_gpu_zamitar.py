@@ -104,6 +104,18 @@ def test_each_mechanism_alone(eng, name, dtype):
     m.free()
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim", [(74, 37, 128), (75, 25, 128), (18, 18, 256), (19, 19, 256), (10, 5, 256)])
+def test_scans_of_many_heads(eng, heads, kv_heads, dim):
+    """On both sides of the counts of heads from which the scan's CTAs would take another wave with warps that work ahead; blocks of 16, a last one of 5"""
+    cfg = zm.config([zm.delta(heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, ff=0)])
+    w = zm.weights(cfg, 5)
+    toks = np.random.default_rng(6).integers(0, cfg["vocab"], 72)
+    logits = ref.forward(cfg, zm.floats(w), toks)
+    m = GpuModel.load_stack(eng, (cfg, w), dtype="float32", max_seq_len=80)
+    close(run_portions(m, toks, [69, 1]), logits, "float32")
+    m.free()
+
+
 # ---- whole models ----------------------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", DTYPES)
