@@ -9,7 +9,7 @@
 // What bounds it: HBM at the largest sizes (28672 x 8192 gate and up in Q4_K, four vectors: 52 us, 5.1 TB/s), else start and drain of the launch and,
 // close behind, the ALU, which takes a bit operation every other clk (about 200 instructions per 16 rows x 256 columns of Q4_K, whatever the batch).
 // Addresses of the copies made once a warp instead of for every piece: Q5_K 5003 x 2816, three vectors 8.5 -> 7.9 us, 28672 x 8192, eight
-// vectors 55.0 -> 48.5; Q6_K 128256 x 4096, eight 118.7 -> 110.5.
+// vectors 55.0 -> 48.5; Q6_K 28672 x 8192, four 61.1 -> 55.4, 128256 x 4096, eight 121 -> 109.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"
@@ -112,7 +112,9 @@ __global__ void __launch_bounds__(KR_WARPS * 32, 1) kq_rows_kernel(const __grid_
             } else {        // rows past the last repeat it, nothing past the matrix is read
                 const uint64_t total = (uint64_t)a.rows[ls] * a.row_bytes;
                 const uint32_t at = (s_lo + l_seg) * (F::NB * F::BB);
-#pragma unroll 1
+                // Unrolled for Q6_K, though hardly ever run: the compiler then schedules the other path better (28672 x 8192, four vectors 63.9 us as a loop, 55.4
+                // unrolled; 61.1 with no other path). Of Q4_K and Q5_K it is the loop (4096 x 4096, eight vectors 7.0 and 8.3 us).
+#pragma unroll (FMT == 6 ? PIECES : 1)
                 for (uint32_t i = lane; i < 16 * CH; i += 32) {
                     const uint32_t r = i / CH, c = i - r * CH;
                     const uint64_t off = (((uint64_t)min(lr0 + r, a.rows[ls] - 1) * a.row_bytes + at) & ~(uint64_t)15) + c * 16;
