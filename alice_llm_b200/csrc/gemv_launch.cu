@@ -469,16 +469,23 @@ static GemvOp sub_batch(const GemvOp& op, uint32_t k, uint32_t n, Q8KView& v) {
     return o;
 }
 
-// Ternary planes and codes: three vectors and more of matrices large enough for tcgen05, with rows that begin on 16-byte boundaries. Its start costs 2 us
-// more: 4096 x 4096 (4 MB) four vectors 10.1 us against 8.5, eight 10.5 / 12.0; 5120 x 5120 three 12.8 / 10.0, eight 12.7 / 13.0; 30000 x 2048 (15 MB) four
-// 14.4 / 13.1; 8192 x 8192 (17 MB) three 13.2 / 15.5; 1024 x 8192 (2 MB) eight 10.5 / 9.4.
+// Ternary planes and codes: the tcgen05 kernel for three vectors and more, with rows that begin on 16-byte boundaries, where it is the faster one by what each
+// kernel's plan has to do (both fitted to 500 sizes: 3 to 60 MB, 512 to 28672 columns, 3 to 8 vectors; about 6 % off). Its steps take 128 rows whether
+// a CTA has them or not, and each of its launches costs 7 us and more: 4096 x 4096 (4 MB), eight vectors 9.5 against 10.9 us; 8192 x 8192, three 11.3 / 13.1; 2048 wide,
+// eight, 10 MB 11.8 / 14.7, 40 MB (three launches) 37.6 / 29.2; codes 8192 wide, 60 MB, three 27.1 / 23.5, eight 29.8 / 40.6; codes 1536 wide, 17 MB (two launches),
+// five 23.6 / 16.6. Below 4 MB (16 for three and four vectors) neither has enough to do.
 static int launch_ternary(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
     const WeightDesc& w = *op.w[0];
     uint64_t bytes = 0;
     for (uint32_t i = 0; i < op.nw && i < 3; i++) if (op.w[i]) bytes += (uint64_t)op.w[i]->rows * w.row_bytes * (op.up ? 2 : 1);
     if (op.batch > 2 && plane_rows_aligned(w) && bytes >= (op.batch > 4 ? 4000000u : 16000000u)) {
-        const int rc = launch_planes_tc(op, cfg, dry, launches);
-        if (rc != ALICE_E_SHAPE) return rc;
+        float tc = 0.0f, rows = 0.0f;
+        int rc = launch_planes(op, cfg, true, nullptr, &rows);
+        if (rc && rc != ALICE_E_SHAPE) return rc;
+        if (rc || (launch_planes_tc(op, cfg, true, nullptr, &tc) == ALICE_OK && tc < rows)) {
+            rc = launch_planes_tc(op, cfg, dry, launches);
+            if (rc != ALICE_E_SHAPE) return rc;
+        }
     }
     return launch_planes(op, cfg, dry, launches);
 }

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(PLANE_WARPS * 32, 1) plane_rows_kernel(const _
 uint32_t log2u(uint32_t v) { uint32_t r = 0; while ((1u << (r + 1)) <= v) r++; return r; }
 
 template <int NT, int PL, bool SW, bool VEC16>
-int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
+int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry, float* us) {
     static int8_t attr_done[64] = {};
     static int clusters[64][4] = {};
     auto kern = plane_rows_kernel<NT, PL, SW, VEC16>;
@@ -340,6 +340,11 @@ int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
         if (smem > PLANE_SMEM) continue;
         // fewer tiles than half the SMs: let more CTAs share a tile's columns
         if (S < 8 && tiles * S * 2 <= sms && a.segs >= 2 * S) continue;
+        if (us) {      // start; steps of 16 rows and a segment that a warp makes; bytes of digits and of sums in shared memory
+            constexpr float start = PL == 2 ? (NT < 4 ? 6.5f : 6.1f) : NT < 4 ? 5.3f : 6.1f, step = PL == 2 ? (NT < 4 ? 1.2f : 1.9f) : NT < 4 ? 0.57f : 1.0f;
+            constexpr float digit = PL == 2 ? (NT < 4 ? 1.8e-5f : 2.6e-5f) : NT < 4 ? 2.2e-5f : 2.5e-5f, sum = NT < 4 ? (PL == 2 ? 1.30e-4f : 1.49e-4f) : PL == 2 ? 1.52e-4f : 1.43e-4f;
+            *us = start + step * (SW ? 2 : 1) * per * slice / PLANE_WARPS + digit * table + sum * acc;
+        }
         if (dry) return ALICE_OK;
         a.tiles_max = per;
         a.acc_off = (uint32_t)(PLANE_HDR + table);
@@ -353,13 +358,13 @@ int plan_and_launch(PlaneArgs a, const LaunchCfg& cfg, bool dry) {
 }
 
 template <int NT, int PL>
-int launch_pl(const PlaneArgs& a, bool vec16, const LaunchCfg& cfg, bool dry) {
-    if (a.up) return vec16 ? plan_and_launch<NT, PL, true, true>(a, cfg, dry) : plan_and_launch<NT, PL, true, false>(a, cfg, dry);
-    return vec16 ? plan_and_launch<NT, PL, false, true>(a, cfg, dry) : plan_and_launch<NT, PL, false, false>(a, cfg, dry);
+int launch_pl(const PlaneArgs& a, bool vec16, const LaunchCfg& cfg, bool dry, float* us) {
+    if (a.up) return vec16 ? plan_and_launch<NT, PL, true, true>(a, cfg, dry, us) : plan_and_launch<NT, PL, true, false>(a, cfg, dry, us);
+    return vec16 ? plan_and_launch<NT, PL, false, true>(a, cfg, dry, us) : plan_and_launch<NT, PL, false, false>(a, cfg, dry, us);
 }
 template <int NT>
-int launch_nt(const PlaneArgs& a, bool codes, bool vec16, const LaunchCfg& cfg, bool dry) {
-    return codes ? launch_pl<NT, 1>(a, vec16, cfg, dry) : launch_pl<NT, 2>(a, vec16, cfg, dry);
+int launch_nt(const PlaneArgs& a, bool codes, bool vec16, const LaunchCfg& cfg, bool dry, float* us) {
+    return codes ? launch_pl<NT, 1>(a, vec16, cfg, dry, us) : launch_pl<NT, 2>(a, vec16, cfg, dry, us);
 }
 // pairs of vectors the kernels are built for
 uint32_t plane_pairs(uint32_t batch) { return batch <= 2 ? 1u : batch <= 4 ? 2u : 4u; }
@@ -370,7 +375,7 @@ size_t plane_prep_bytes(uint32_t cols, uint32_t batch) {
     return (size_t)((cols + 511) / 512) * plane_pairs(batch) * 4096 + 256 + 4096;   // codes: half the bytes for half the columns
 }
 
-int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
+int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches, float* us) {
     if (launches) *launches = 1;
     const WeightDesc& w0 = *op.w[0];
     const bool codes = w0.fmt == WF_SPARSE_TERNARY;
@@ -408,7 +413,7 @@ int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* la
         a.table = static_cast<const uint4*>(op.prep);
         a.kappa = reinterpret_cast<const float*>(static_cast<const uint8_t*>(op.prep) + table);
     }
-    auto rows = [&](bool plan) { return nt == 1 ? launch_nt<1>(a, codes, vec16, cfg, plan) : nt == 2 ? launch_nt<2>(a, codes, vec16, cfg, plan) : launch_nt<4>(a, codes, vec16, cfg, plan); };
+    auto rows = [&](bool plan) { return nt == 1 ? launch_nt<1>(a, codes, vec16, cfg, plan, us) : nt == 2 ? launch_nt<2>(a, codes, vec16, cfg, plan, us) : launch_nt<4>(a, codes, vec16, cfg, plan, us); };
     int rc = rows(true);
     if (rc || dry) return rc;
     if (nt == 1) return rows(false);

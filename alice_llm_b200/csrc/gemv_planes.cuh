@@ -49,9 +49,10 @@ struct PlaneArgs {
 inline bool plane_rows_aligned(const WeightDesc& w) { return (w.fmt == WF_SPARSE_TERNARY ? w.row_bytes : w.row_bytes / 2) % 16 == 0; }
 // Scratch for the digit table of `batch` vectors, for either format.
 size_t plane_prep_bytes(uint32_t cols, uint32_t batch);
-// ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only. launches: of the product, which is one.
-int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
+// ALICE_E_SHAPE: not a case for this kernel (the caller goes on to the ring kernels). dry: plan only. launches: of the product, which is one. us: about what
+// three vectors and more take, tables included.
+int launch_planes(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr, float* us = nullptr);
 // The same for three vectors and more on tcgen05, where plane_rows_aligned.
-int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr);
+int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches = nullptr, float* us = nullptr);
 
 }  // namespace alice

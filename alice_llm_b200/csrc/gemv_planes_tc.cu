@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) plane_tc_kernel(const __grid_co
 }
 
 template <int N, int PL, bool SW>
-int plan_and_launch(PtArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches_out) {
+int plan_and_launch(PtArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches_out, float* us) {
     using G = PtGeom<PL>;
     constexpr uint32_t MATS = SW ? 2 : 1, MOST = std::min<uint32_t>(PT_TILES, (512 - PT_D) / N);
     static bool attr_done[64] = {};
@@ -417,6 +417,22 @@ int plan_and_launch(PtArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches
     const uint64_t most = (uint64_t)(MOST / MATS - (a.nw - 1)) * 128 * best_ncl;
     const uint32_t launches = (uint32_t)((total + most - 1) / most);
     if (launches_out) *launches_out = launches;
+    if (us) {      // start of a launch; steps of 128 rows, full or not, and a segment; sums of a cluster's rows at its end
+        constexpr float start = PL == 2 ? (N == 16 ? 7.1f : 8.2f) : N == 16 ? 6.8f : 7.2f, step = PL == 2 ? (N == 16 ? 0.54f : 0.63f) : N == 16 ? 0.38f : 0.43f;
+        constexpr float sum = N == 16 ? 4.3e-4f : PL == 2 ? 2.4e-4f : 2.1e-4f;
+        const uint32_t n = total / launches, per = (n + best_ncl - 1) / best_ncl;
+        uint32_t tiles = 0;      // of the cluster that has most: rows of several matrices make more of them
+        for (uint32_t c = 0; c < best_ncl; c++) {
+            const uint32_t lo = (uint32_t)((uint64_t)n * c / best_ncl), hi = (uint32_t)((uint64_t)n * (c + 1) / best_ncl);
+            uint32_t t = 0;
+            for (uint32_t i = 0; i < a.nw; i++) {
+                const uint32_t from = std::max(lo, a.row0[i]), to = std::min(hi, a.row0[i + 1]);
+                if (from < to) t += (to - from + 127) / 128;
+            }
+            tiles = std::max(tiles, t);
+        }
+        *us = launches * (start + step * MATS * tiles * ((a.segs + best - 1) / best) + sum * MATS * per * a.batch) * (SW ? 0.9f : 1.0f);
+    }
     if (dry) return ALICE_OK;
     a.stages = (uint32_t)std::min<size_t>(PT_STAGES, (PT_SMEM - table_of(best)) / G::STAGE);
     a.tab_off = a.stages * G::STAGE;
@@ -435,14 +451,14 @@ int plan_and_launch(PtArgs a, const LaunchCfg& cfg, bool dry, uint32_t* launches
 }
 
 template <int PL>
-int launch_n(const PtArgs& a, const LaunchCfg& cfg, bool dry, uint32_t* l) {
-    if (a.up) return a.batch <= 4 ? plan_and_launch<16, PL, true>(a, cfg, dry, l) : plan_and_launch<32, PL, true>(a, cfg, dry, l);
-    return a.batch <= 4 ? plan_and_launch<16, PL, false>(a, cfg, dry, l) : plan_and_launch<32, PL, false>(a, cfg, dry, l);
+int launch_n(const PtArgs& a, const LaunchCfg& cfg, bool dry, uint32_t* l, float* us) {
+    if (a.up) return a.batch <= 4 ? plan_and_launch<16, PL, true>(a, cfg, dry, l, us) : plan_and_launch<32, PL, true>(a, cfg, dry, l, us);
+    return a.batch <= 4 ? plan_and_launch<16, PL, false>(a, cfg, dry, l, us) : plan_and_launch<32, PL, false>(a, cfg, dry, l, us);
 }
 
 }  // namespace
 
-int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches) {
+int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t* launches, float* us) {
     const WeightDesc& w0 = *op.w[0];
     const bool codes = w0.fmt == WF_SPARSE_TERNARY;
     if ((w0.fmt != WF_TERNARY && !codes) || op.npeers || op.norm_w || op.batch < 3 || op.batch > 8 || op.argmax_key) return ALICE_E_SHAPE;
@@ -475,7 +491,7 @@ int launch_planes_tc(const GemvOp& op, const LaunchCfg& cfg, bool dry, uint32_t*
         a.table = static_cast<const uint4*>(op.prep);
         a.kappa = reinterpret_cast<const float*>(static_cast<const uint8_t*>(op.prep) + table);
     }
-    auto rows = [&](bool plan) { return codes ? launch_n<1>(a, cfg, plan, launches) : launch_n<2>(a, cfg, plan, launches); };
+    auto rows = [&](bool plan) { return codes ? launch_n<1>(a, cfg, plan, launches, us) : launch_n<2>(a, cfg, plan, launches, us); };
     int rc = rows(true);
     if (rc || dry) return rc;
     cudaLaunchConfig_t lc = {};

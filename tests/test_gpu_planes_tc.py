@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from alice_llm_b200 import synth
+from graph_kernels import block_sizes
 from softmodel import SMOOTH_MIX, soft_model
 from test_gpu_planes import upload
 
@@ -82,3 +83,37 @@ def test_model_with_three_matrices_in_a_launch(eng):
     kb, vb = b.kv_read(0, 0, 8)
     assert np.array_equal(ka, kb) and np.array_equal(va, vb)      # of the one layer: nothing of attention is in them
     a.free(), b.free()
+
+
+TC_THREADS = 672      # of a block of csrc/gemv_planes_tc.cu, and of no other kernel
+
+
+@pytest.mark.parametrize("rows,cols,batch,sparse,launches", [
+    (4097, 8192, 5, False, 1), (2300, 7808, 6, False, 1), (8300, 8192, 3, False, 1), (8300, 8192, 4, False, 1), (70000, 512, 7, False, 1), (300000, 256, 8, False, 2), (60000, 6144, 5, False, 2),
+    (4097, 8192, 8, True, 1), (70000, 512, 7, True, 1), (300000, 256, 8, True, 2), (700, 28672, 8, False, 0), (700, 28672, 8, True, 0), (8300, 8192, 2, False, 0), (16500, 1152, 8, False, 0),
+    (4097, 8200, 8, False, 0), (7000, 8192, 4, False, 0), (1900, 8192, 5, False, 0)])
+def test_kernel_by_size(eng, oracle, rows, cols, batch, sparse, launches):
+    """Launches of the tcgen05 kernel: by what the plans cost, none for two vectors, planes that begin off 16-byte boundaries and less than 4 or 16 MB"""
+    rng = np.random.default_rng(rows)
+    m = synth.make_ternary(rng, rows, cols)
+    w = upload(eng, oracle, m, rows, cols, sparse)
+    x = synth.make_x(rng, cols, batch).reshape(batch, cols)
+    call = lambda xd, y, n: eng.matvec_dev(w, xd, y, n)
+    run(eng, call, x, rows)
+    xd, y = eng.upload_f32(x.reshape(-1)), eng.alloc_f32(batch * rows)
+    assert block_sizes(eng, lambda: call(xd, y, batch)).count(TC_THREADS) == launches
+    assert eng.batch_plan(w, batch) == (max(launches, 1), 1)
+    w.free()
+
+
+@pytest.mark.parametrize("rows,cols,batch,sparse,launches", [
+    (3000, 4224, 8, False, 1), (6001, 8192, 3, False, 1), (20000, 8192, 8, False, 2), (10000, 4096, 4, False, 1), (3000, 4224, 8, True, 1), (10000, 4096, 6, True, 1), (3500, 13312, 4, True, 1)])
+def test_gate_and_up_of_either_format(eng, oracle, rows, cols, batch, sparse, launches):
+    rng = np.random.default_rng(rows + batch)
+    g, u = (upload(eng, oracle, synth.make_ternary(rng, rows, cols), rows, cols, sparse) for _ in range(2))
+    x = synth.make_x(rng, cols, batch).reshape(batch, cols)
+    call = lambda xd, y, n: eng.swiglu_dev(g, u, xd, y, n)
+    run(eng, call, x, rows)
+    xd, y = eng.upload_f32(x.reshape(-1)), eng.alloc_f32(batch * rows)
+    assert block_sizes(eng, lambda: call(xd, y, batch)).count(TC_THREADS) == launches
+    g.free(), u.free()
