@@ -85,8 +85,8 @@ __device__ __forceinline__ void add_share(float& M, float& L, float4& A, float m
     M = mx;
 }
 
-// blockIdx: key / value head, tile of 16 I (token, head) rows, share of the tile's positions; a cluster of `cs` shares adds up in its CTAs, in rank
-// order. nsplit == cs: the finished output; else (max, sum, sums) of the cluster's shares into a.part[row][split / cs].
+// blockIdx: key / value head, tile of 16 I (token, head) rows, share of the tile's positions. cs > 1: the nsplit = cs shares are a cluster, which adds
+// them up in rank order; cs = 1: each of more than one share leaves (max, sum, sums) in a.part[row][share].
 template <int I>
 __global__ void __launch_bounds__(AT_THREADS, 2) attn_tile_kernel(const __grid_constant__ AttnArgs a, uint32_t batch, uint32_t cs) {
     extern __shared__ __align__(16) float sm[];
@@ -211,21 +211,19 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_tile_kernel(const __grid_c
         if (tb + AT_KEYS <= all_see) weigh(std::false_type{}); else weigh(std::true_type{});
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const uint32_t parts = a.nsplit / cs;
-    auto target = [&](uint32_t row) {
-        const uint32_t k = row / group, head = kvh * group + row % group;
-        return parts == 1 ? a.attn_out + (size_t)k * a.out_stride + (size_t)head * 128 : a.part + (((size_t)k * s.num_heads + head) * parts + split / cs) * 132;
-    };
+    auto output = [&](uint32_t row) { return a.attn_out + (size_t)(row / group) * a.out_stride + (size_t)(kvh * group + row % group) * 128; };
     if (cs == 1) {
 #pragma unroll
         for (int i = 0; i < I; i++) {
             const uint32_t row = row0 + ty + 16 * i;
             if (row >= nrows) continue;
-            float* out = target(row);
-            const float f = parts > 1 ? 1.0f : l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
-            if (parts > 1) {
+            float* out = output(row);
+            float f = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+            if (a.nsplit > 1) {
+                out = a.part + (((size_t)(row / group) * s.num_heads + kvh * group + row % group) * a.nsplit + split) * 132;
                 if (tx == 0) { out[0] = m[i]; out[1] = l[i]; }
                 out += 4;
+                f = 1.0f;
             }
 #pragma unroll
             for (int d = 0; d < 4; d++) {
@@ -249,7 +247,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_tile_kernel(const __grid_c
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const uint32_t lane = tid & 31;
-    for (uint32_t r = split % cs + cs * (tid >> 5); r < ROWS && row0 + r < nrows; r += cs * (AT_THREADS / 32)) {      // a warp a row, four dimensions a lane
+    for (uint32_t r = split + cs * (tid >> 5); r < ROWS && row0 + r < nrows; r += cs * (AT_THREADS / 32)) {      // a warp a row, four dimensions a lane
         float2 ml[8];
         float4 v[8];
         float M = -INFINITY;
@@ -266,13 +264,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_tile_kernel(const __grid_c
 #pragma unroll
         for (uint32_t q = 0; q < 8; q++)
             if (q < cs) add_share(L, A, ml[q], v[q], M);
-        float* out = target(row0 + r);
-        const float f = parts > 1 ? 1.0f : L > 0.0f ? 1.0f / L : 0.0f;
-        if (parts > 1) {
-            if (lane == 0) { out[0] = M; out[1] = L; }
-            out += 4;
-        }
-        reinterpret_cast<float4*>(out)[lane] = make_float4(A.x * f, A.y * f, A.z * f, A.w * f);
+        const float f = L > 0.0f ? 1.0f / L : 0.0f;
+        reinterpret_cast<float4*>(output(row0 + r))[lane] = make_float4(A.x * f, A.y * f, A.z * f, A.w * f);
     }
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // no CTA leaves while others read its sums
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
@@ -368,8 +361,7 @@ cudaError_t launch_attention_tokens(const AttnArgs& args, float* qkv, uint32_t b
         case 3: err = launch_tile<3>(lc, a, batch, cs); break;
         default: err = launch_tile<4>(lc, a, batch, cs);
     }
-    a.nsplit /= cs;
-    if (err != cudaSuccess || a.nsplit == 1) return err;
+    if (err != cudaSuccess || cs > 1 || a.nsplit == 1) return err;
     lc.attrs = at + 1; lc.numAttrs = pdl ? 1 : 0;
     lc.gridDim = dim3(batch * s.num_heads); lc.blockDim = dim3(128); lc.dynamicSmemBytes = 0;
     return cudaLaunchKernelEx(&lc, attn_join_kernel, a);
