@@ -337,11 +337,12 @@ cudaError_t launch_attention_tokens(const AttnArgs& args, float* qkv, uint32_t b
     if (group != 1 && group != 2 && group != 4 && group != 5 && group != 8) return cudaErrorInvalidValue;
     // Shares of the positions: two CTAs an SM. Up to eight are a cluster, which adds up by itself (11.8 against 14.5 us for 2 tokens behind 500); more go
     // through the scratch and a join, since clusters leave slots empty when the chip is full (64 heads behind 2048, 33 shares: clusters of
-    // 2 and 4 34 and 48 us, none 27.8). What the scratch does not hold (prompts) is a cluster again: 45 us for 256 tokens, 63 with one share.
-    const uint32_t slots = std::max(1u, 2 * (uint32_t)num_sms / (s.num_kv_heads * tiles)), total = (pos0 + batch + AT_KEYS - 1) / AT_KEYS;
-    const uint32_t steps = (total + slots - 1) / slots, n = (total + steps - 1) / steps;
+    // 2 and 4 34 and 48 us, none 27.8), as many of them as the scratch holds (two key / value heads of 8, eight tokens behind 8000: 315 us for four
+    // layers, 882 in clusters). Where it holds no more than a cluster has (prompts), clusters again: 45 us for 256 tokens, 63 with one share.
+    const uint32_t slots = std::max(1u, 2 * (uint32_t)num_sms / (s.num_kv_heads * tiles)), room = part_vectors / (batch * s.num_heads);
+    const uint32_t total = (pos0 + batch + AT_KEYS - 1) / AT_KEYS, most = room > 8 ? std::min(slots, room) : slots, steps = (total + most - 1) / most, n = (total + steps - 1) / steps;
     uint32_t cs = 1;
-    if (n <= 8 || n > part_vectors / (batch * s.num_heads)) while (cs < 8 && 2 * cs <= std::min(slots, total)) cs *= 2;
+    if (n <= 8 || room <= 8) while (cs < 8 && 2 * cs <= std::min(slots, total)) cs *= 2;
     a.nsplit = cs > 1 ? cs : n;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute at[2];
