@@ -333,16 +333,23 @@ cudaError_t launch_attention_tokens(const AttnArgs& args, float* qkv, uint32_t b
     AttnArgs a = args;
     const AttnShape& s = a.shape;
     if (s.head_dim != 128 || s.num_heads % s.num_kv_heads || a.npeers) return cudaErrorInvalidValue;
-    const uint32_t group = s.num_heads / s.num_kv_heads, per16 = std::min(4u, (batch * group + 15) / 16), tiles = (batch * group + 16 * per16 - 1) / (16 * per16);
+    const uint32_t group = s.num_heads / s.num_kv_heads, rows = batch * group, total = (pos0 + batch + AT_KEYS - 1) / AT_KEYS;
+    // Tiles of 64 rows, smaller ones where a few steps would leave SMs without any (four layers of 8 x 4 heads, prompts of 17 and 64 tokens: 475 -> 429 us and
+    // 583 -> 550; behind 500, 16 steps, of 8 x 8 heads 364 -> 372).
+    auto tiles_of = [&](uint32_t per16) { return (rows + 16 * per16 - 1) / (16 * per16); };
+    uint32_t per16 = std::min(4u, (rows + 15) / 16);
+    while (per16 > 1 && total <= 8 && s.num_kv_heads * tiles_of(per16) * total < (uint32_t)num_sms) per16 = (per16 + 1) / 2;
+    const uint32_t tiles = tiles_of(per16);
     if (group != 1 && group != 2 && group != 4 && group != 5 && group != 8) return cudaErrorInvalidValue;
-    // Shares of the positions: two CTAs an SM. Up to eight are a cluster, which adds up by itself (11.8 against 14.5 us for 2 tokens behind 500); more go
+    // Shares of the positions: two CTAs an SM. Up to eight are a cluster, which adds up by itself (11.8 against 14.5 us for 2 tokens behind 500), of a power
+    // of two: rather an empty share than two steps in one (four layers of 8 x 4 heads, eight tokens behind 200, seven steps: 278 us with eight, 312 with four); more go
     // through the scratch and a join, since clusters leave slots empty when the chip is full (64 heads behind 2048, 33 shares: clusters of
     // 2 and 4 34 and 48 us, none 27.8), as many of them as the scratch holds (two key / value heads of 8, eight tokens behind 8000: 315 us for four
     // layers, 882 in clusters). Where it holds no more than a cluster has (prompts), clusters again: 45 us for 256 tokens, 63 with one share.
     const uint32_t slots = std::max(1u, 2 * (uint32_t)num_sms / (s.num_kv_heads * tiles)), room = part_vectors / (batch * s.num_heads);
-    const uint32_t total = (pos0 + batch + AT_KEYS - 1) / AT_KEYS, most = room > 8 ? std::min(slots, room) : slots, steps = (total + most - 1) / most, n = (total + steps - 1) / steps;
+    const uint32_t most = room > 8 ? std::min(slots, room) : slots, steps = (total + most - 1) / most, n = (total + steps - 1) / steps;
     uint32_t cs = 1;
-    if (n <= 8 || room <= 8) while (cs < 8 && 2 * cs <= std::min(slots, total)) cs *= 2;
+    if (n <= 8 || room <= 8) while (cs < 8 && cs < total && 2 * cs <= slots) cs *= 2;
     a.nsplit = cs > 1 ? cs : n;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute at[2];

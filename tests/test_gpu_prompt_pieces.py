@@ -74,9 +74,10 @@ def test_shares_of_attention(eng, heads, ctx, n):
 
 
 @pytest.mark.parametrize("heads", [(4, 2), (16, 2), (32, 4)])
-@pytest.mark.parametrize("ctx,n", [(2040, 8), (2041, 8), (4100, 8), (240, 8), (249, 8), (0, 17), (0, 48)])
+@pytest.mark.parametrize("ctx,n", [(2040, 8), (2041, 8), (4100, 8), (240, 8), (249, 8), (60, 8), (140, 3), (0, 17), (0, 48)])
 def test_shares_and_tiles_at_their_limits(eng, heads, ctx, n):
-    """64 steps of 32 positions and 65, where the scratch holds 64 shares for eight tokens; eight steps and nine, where tiles are smaller up to eight"""
+    """64 steps of 32 positions and 65, where the scratch holds 64 shares for eight tokens; eight steps and nine, where tiles are smaller up to eight;
+    three and five, whose clusters have empty shares"""
     compare(eng, SMOOTH_MIX, heads, 512, 512, ctx, n, 1e-4)
 
 
