@@ -16,6 +16,7 @@
 #include "attn_body.cuh"
 #include "common.cuh"
 #include "glue.cuh"
+#include "packed_f32.cuh"
 
 namespace alice {
 namespace {
@@ -24,32 +25,12 @@ constexpr uint32_t AT_THREADS = 128, AT_KEYS = 32, AT_PITCH = 132, AT_PPITCH = 2
 constexpr uint32_t AT_TILE = AT_KEYS * AT_PITCH, AT_RING = 3;
 constexpr uint32_t at_smem(uint32_t rows) { return (rows * AT_PITCH + AT_RING * AT_TILE + rows * AT_PPITCH) * 4; }
 
-// Two f32 side by side (fma.rn.f32x2: each half rounds as fmaf does).
+// Four f32 as two pairs.
 struct F2x2 { uint64_t a, b; };
 __device__ __forceinline__ F2x2 lds_2x2(uint32_t at) {
     F2x2 v;
     asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(v.a), "=l"(v.b) : "r"(at));
     return v;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
-    return r;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t x, uint64_t y) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
-    return r;
 }
 
 // Rotates the queries in place and appends the rotated keys and the values to the cache: a warp per head vector.

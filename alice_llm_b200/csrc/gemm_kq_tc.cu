@@ -191,26 +191,6 @@ __device__ __forceinline__ void kt_mins(uint32_t m, uint32_t half, uint8_t* at, 
     *reinterpret_cast<uint4*>(at + r * 128 + ((half ^ (r & 7u)) * 16)) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-__device__ __forceinline__ void tmem_get16(uint32_t (&r)[16], uint32_t addr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(addr)
-        : "memory");
-}
-// what was asked for is there
-__device__ __forceinline__ void tmem_got16(uint32_t (&r)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-        :
-        : "memory");
-}
-__device__ __forceinline__ void tmem_got16(uint32_t (&r)[16], uint32_t (&q)[16]) {
-    tmem_got16(r);
-#pragma unroll
-    for (int i = 0; i < 16; i++) asm volatile("" : "+r"(q[i]));      // not before the wait
-}
 template <uint32_t N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 

@@ -27,6 +27,7 @@
 #include "digits_dev.cuh"
 #include "gemv_blocks.cuh"
 #include "gemv_mma.cuh"
+#include "packed_f32.cuh"
 
 namespace alice {
 namespace {
@@ -182,13 +183,6 @@ __device__ __forceinline__ void q1_pair(const uint8_t* pA, const uint8_t* pB, co
     acc[0] = fmaf(dA, (float)vA, acc[0]);
     acc[1] = fmaf(dB, (float)vB, acc[1]);
 }
-
-// Two f32 numbers in one 64-bit register: an instruction for both.
-__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float2 unpack2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 // Sums of a stage of four Q8_0 rows over V vectors: of even and odd columns in the two halves of a register, or, where eight vectors leave
 // no room for twice as many registers, plain.
