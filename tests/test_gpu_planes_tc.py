@@ -85,6 +85,20 @@ def test_model_with_three_matrices_in_a_launch(eng):
     a.free(), b.free()
 
 
+def test_model_of_few_vectors(eng):
+    """Three drafted tokens: 16 digit columns, with the residual of a wide output projection"""
+    from alice_llm_b200.gpu import GpuModel
+    cfg = dict(num_layers=1, hidden_dim=4096, intermediate_dim=512, num_heads=128, num_kv_heads=16, head_dim=128, vocab_size=500, max_seq_len=16,
+               rope_theta=500000.0, eps=1e-5)
+    model = soft_model(np.random.default_rng(12), cfg, SMOOTH_MIX)
+    a = GpuModel.load(eng, model)
+    toks = [3, 499, 41]
+    got = np.asarray(a.forward_batch_and_read(toks), np.float64).reshape(3, 500)
+    a.reset()
+    want = np.asarray([a.forward_and_read(t) for t in toks], np.float64)
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+    a.free()
+
 TC_THREADS = 672      # of a block of csrc/gemv_planes_tc.cu, and of no other kernel
 
 
