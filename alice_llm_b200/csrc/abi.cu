@@ -269,9 +269,9 @@ static int check_pair(const alice_weights* g, const alice_weights* u, const char
 }
 
 // Whether the CTAs of a matvec make the Q8_K blocks of its one vector themselves. Two launches cost a caller that queues call behind call 8 us; a product
-// that is over before that gains a launch less, though its own start is longer: Q4_K 4096 x 4096 8.0 -> 6.1 us a call (replayed from a graph 5.8 ->
-// 6.3), 1024 x 4096 7.8 -> 5.2, Q6_K 8192 x 4096 (28 MB) 9.8 -> 9.3, Q4_K 32768 x 1024 8.4 -> 7.8, 1024 x 8192 (5 MB) 7.9 -> 6.7, but 14336 x 4096 (33 MB) 8.9 -> 9.0,
-// 4096 x 8192 (19 MB) 7.9 -> 7.9 (graph 7.7 -> 8.6), 2048 x 14336 7.9 -> 9.1: up to 16 blocks of 256 two warps' worth each, up to 32 where little else is to do.
+// that is over before that gains a launch less, though its own start is longer: Q4_K 4096 x 4096 7.4 -> 6.1 us a call, 1024 x 4096 7.8 -> 4.7,
+// Q6_K 8192 x 4096 (28 MB) 9.8 -> 9.3, Q4_K 32768 x 1024 8.4 -> 7.8, 1024 x 8192 (5 MB) 7.9 -> 6.7, but 14336 x 4096 (33 MB) 8.9 -> 9.0, 4096 x 8192 (19 MB) 7.9 ->
+// 7.9, 2048 x 14336 7.9 -> 9.1: up to 16 blocks of 256 two warps' worth each, up to 32 where little else is to do.
 static bool quantized_in_matvec(const WeightDesc& w, bool two, uint32_t batch) {
     const uint64_t bytes = (uint64_t)w.rows * w.row_bytes * (two ? 2 : 1);
     return batch == 1 && ((w.cols <= 4096 && bytes <= 28000000) || (w.cols <= 8192 && bytes <= 8000000));

@@ -12,15 +12,16 @@
 // two pieces, 2.8e-7 for four, 1.5e-7 for one, 1.6e-7 by integer sums) and a tenth of the time of a prompt.
 //
 // One CTA per SM, 128 rows x 128 vectors, 20 warps: 8 unpack raw blocks (cp.async, a block ahead) into the swizzled A tiles, half a row a
-// thread (with four, the products waited for them: 216 us for the gate and up product of an 8B model and 256 tokens), one warp
-// copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM), 16 vectors ahead, which
-// takes registers the other warps give up (72 and 48 against 144; with 96 for all and 8 vectors at a time 137 us for that product, 128 so). Where
-// tiles are fewer than the SMs a cluster shares the columns and adds its parts through distributed shared memory in rank order.
-// What bounds it: the unpacking warps, a chain of wait, read, compute, store and hand over: of 128 us 104 are left without unpacking and
-// draining. Two k-tiles to a hand-over make it 122 for Q4_K; the shallower rings of the others lose by it (Q5_K 152 and 164). Q6_K reads its
-// words for two k-tiles at a time and multiplies by the two parts of the scale: 4096 x 14336 with 256 vectors 126 -> 102 us. Waits by one lane
-// of a warp, or a row a thread and every other k-tile, are no faster (150, 132 us). A 256-token prompt of an 8B model takes 12.4 ms, 23.0 by
-// the integer path of mma.sync (csrc/gemm_kq.cu), which spends some 16 instructions per product on scales and unpacking.
+// thread, one warp copies the B tiles by TMA, one issues the products, 8 drain the accumulators of the block before (two sets in TMEM), 16 vectors
+// ahead, which takes registers the other warps give up (72 and 48 against 144). Where tiles are fewer than the SMs a cluster shares the
+// columns and adds its parts through distributed shared memory in rank order.
+// Gate and up of an 8B model with 256 vectors, step by step: 216 us with four unpacking warps, 162 with eight, 140 with the tiles over whole waves split by
+// columns (launch_tc), 128 with the registers moved and 16 vectors at a time (137 with 96 registers for all and 8), 122 with two k-tiles to a hand-over (Q4_K; the
+// shallower rings of the others lose by it, Q5_K 152 and 164). Q6_K reads its words for two k-tiles at a time and multiplies by the two parts of the
+// scale: 4096 x 14336 with 256 vectors 126 -> 102 us. Waits by one lane of a warp, or a row a thread and every other k-tile, are no faster (150, 132 us).
+// What bounds it: the hand-overs. No unit is near its peak (ALU 34 %, tensor pipe 28, shared memory 45, issue slots 57), and without unpacking and
+// draining 104 of the 128 us were left. A 256-token prompt of an 8B model takes 12.2 ms, 23.0 by the integer path of mma.sync (csrc/gemm_kq.cu), which
+// spends some 16 instructions per product on scales and unpacking.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"

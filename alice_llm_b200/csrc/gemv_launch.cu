@@ -245,7 +245,7 @@ int plan_stream_gemv(const GemvOp& op, const LaunchCfg& cfg, StreamPlan& pl) {
         if (wi->fmt != w0.fmt || wi->cols != w0.cols || wi->row_bytes != w0.row_bytes) return ALICE_E_SHAPE;
         total_rows += wi->rows;
     }
-    // the input arrives prepared: Q8_K blocks for the K-quants, the f32 vector for everything else
+    // the input: for the K-quants Q8_K blocks, or the f32 vector that the CTAs make them of themselves; the f32 vector for everything else
     if (format_uses_q8k(w0.fmt)) {
         if (q8 ? q8->qs == nullptr : x == nullptr) return ALICE_E_INVALID;
         if (q8 && q8->nb * 256u != w0.cols) return ALICE_E_SHAPE;

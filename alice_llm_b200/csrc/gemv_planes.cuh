@@ -9,7 +9,7 @@
 // per m16n8k32 and SM quarter, measured.
 //
 // 28672 x 8192: one vector 20.0 us (27.8 by the ring kernel). What bounds it: the stream and the instructions on it alike (2.9 TB/s). Three vectors
-// and more of larger matrices go to csrc/gemv_planes_tc.cu (eight: 38.9 us here, 26.1 there).
+// and more go to csrc/gemv_planes_tc.cu where that is the faster (eight: 37.5 us here, 24.5 there).
 //
 // Split: a cluster of S CTAs owns a range of 16-row tiles, each of its CTAs 1 / S of the columns, whose digit table stays in
 // shared memory for the whole launch (S is the smallest that makes it fit, or larger where a matrix has fewer tiles than the

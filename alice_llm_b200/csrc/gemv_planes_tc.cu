@@ -9,8 +9,9 @@
 // wait. A cluster shares the columns, so that the digits of a CTA's fit beside its ring; accumulators of all of a CTA's tiles stay in tensor memory until the
 // end, where a sum's digits meet in 64 bits and the CTAs of a cluster add theirs. Rows are dealt evenly, not in whole tiles.
 //
-// Measured: 28672 x 8192, eight vectors 38.9 -> 26.1 us, 8192 x 28672 46.6 -> 32.9, 8192 x 8192 20.1 -> 14.7 (digit tables included). What bounds it: bit
-// operations (an ALU instruction every other clk and SM quarter; 14 for 32 weights) and the hand-overs between the warps.
+// Measured against csrc/gemv_planes.cu, eight vectors, digit tables included: 28672 x 8192 37.5 -> 24.5 us, 8192 x 28672 45.3 -> 29.8, 8192 x 8192 19.1 -> 12.3; gate
+// and up of 28672 x 8192 64.1 -> 52.9. What bounds it: the hand-overs between the warps and the start and end of a launch (7 us). No unit is near its
+// peak: ALU 49 % (14 bit operations for 32 weights, one every other clk and SM quarter), tensor pipe 17, HBM 24, shared memory 14.
 #include <algorithm>
 
 #include "../../include/alice_cuda.h"

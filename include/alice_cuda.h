@@ -172,7 +172,8 @@ int32_t alice_dequantize(alice_engine* e, const alice_weights* w, alice_buf* out
  * rows per set per stage, stage-sized row groups in total, ring stages, activation units per lane, 1 if the bit-plane
  * tensor-core kernel is used, column chunks, CTAs per SM. A CTA handles about groups / CTAs stages, so a test can
  * assert that a shape really re-uses the ring. It describes the ring kernels, which serve single vectors of most shapes and
- * every tensor-parallel rank; ternary, Q1_0 and Q2_0 matrices and batches run in kernels without that geometry. No reference
+ * every tensor-parallel rank; ternary, Q1_0 and Q2_0 matrices and batches run in kernels without that geometry. A K-quant call
+ * without preq is taken to be outside a stream capture, its x and y apart (else it has the plan with preq). No reference
  * counterpart (diagnostic). */
 int32_t alice_plan_query(alice_engine* e, const alice_weights* w, int32_t swiglu, int32_t preq, uint32_t* out, uint32_t n_out);
 
